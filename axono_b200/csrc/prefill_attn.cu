@@ -13,7 +13,8 @@
 // maximum moves by more than a threshold.  One lane each of two more warps launches the MMAs and the
 // TMA loads; the sides meet only on mbarriers (tcgen05.commit for MMA completion).  K/V tiles are
 // multi-buffered and S is computed two tiles ahead, so tensor core and softmax overlap.  Every wait
-// is bounded.  Other dtypes and head sizes run row by row on the decode kernels (correct, not fast).
+// is bounded.  From 256 rows on, and for narrower heads, the 256-row form below; FLOAT32 and head sizes that are
+// not a multiple of 8 up to 128 go to prefill_tiled.cu, and what that does not take to the decode kernels, row by row.
 //
 // Semantics as the reference's CPU op (src/ops/cpu/sequence.cpp:236-301): q (sq,hq,d), k/v
 // (skv,hkv,d) token-major, head h reads KV head h / (hq/hkv), scale 1/sqrt(d); with is_causal row t
@@ -53,7 +54,7 @@ constexpr float kLog2e = 1.4426950408889634f;
 
 struct PrefillParams {
   void *out;
-  int sq, hq, hkv, skv, causal;
+  int sq, hq, hkv, skv, causal, d;
   float scale_log2;
 };
 
@@ -338,6 +339,22 @@ constexpr int kPairOffQ = 0, kPairOffK = 2 * kPairTileBytes, kPairOffV = kPairOf
 constexpr int kPairOffBar = kPairOffV + 2 * kPairTileBytes;
 constexpr int kPairSmemBytes = kPairOffBar + 256;  // 192 KB + barriers
 
+// Two fp16 parts of a pair of weights: hi + lo holds 22 bits of each (2^-24 absolute where a part is subnormal).
+__device__ __forceinline__ uint32_t split_half2(float a, float b, uint32_t &lo) {
+  const __half2 hi = __floats2half2_rn(a, b);
+  const float2 f = __half22float2(hi);
+  lo = pack_half2(a - f.x, b - f.y);
+  return *reinterpret_cast<const uint32_t *>(&hi);
+}
+
+// kNarrow: head sizes below 128 (multiples of 8).  They ran on the FMA pipe before, whose weights were fp32, so P enters
+// P.V as two fp16 parts here: P's two parts take the two halves of S_g, and a tile costs 16 products for P.V instead of 8.
+// Elements past the head size are zeros that TMA fills in; head sizes up to 64 leave the second 64-wide block of every tile
+// out - Q.K^T does not step into it, and the columns of O that P.V forms from whatever stands there are never stored.
+// P.V keeps N = 128 whatever the head size: products of one shape need no wait between P.V and the S that overwrites P.
+// Bound by the products of P.V and the softmax about equally.  2700 x 2700 keys, 16 heads of 64, not causal:
+// 121 us against 1921 us on the FMA pipe, the same error against 64 bits (2.1e-4, the rounding of the result).
+template <bool kNarrow>
 __global__ void __launch_bounds__(kPairThreads, 1)
 prefill_attn_f16_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                              const __grid_constant__ CUtensorMap tmV, const PrefillParams p) {
@@ -388,6 +405,8 @@ prefill_attn_f16_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __gr
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;  // S_g at g * 128, O_g at 256 + g * 128
+  const bool two_blocks = !kNarrow || p.d > 64;
+  const uint32_t tile_bytes = two_blocks ? kPairTileBytes : kPairTileBytes / 2;
 
   if (warp == kPairLoadWarp) {
     // ================= TMA warp (one lane) =================
@@ -395,14 +414,15 @@ prefill_attn_f16_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __gr
       tma_prefetch_descriptor(&tmQ);
       tma_prefetch_descriptor(&tmK);
       tma_prefetch_descriptor(&tmV);
-      mbar_arrive_expect_tx(bar_q, 3 * kPairTileBytes);
+      auto load_tile = [&](uint8_t *dst, const CUtensorMap *map, uint64_t *bar, int head, int row) {
+        tma_load_3d(dst, map, bar, 0, head, row);
+        if (two_blocks) tma_load_3d(dst + kPairTileBytes / 2, map, bar, 64, head, row);
+      };
+      mbar_arrive_expect_tx(bar_q, 3 * tile_bytes);
 #pragma unroll
-      for (int g = 0; g < 2; ++g) {  // rows past sq are zero-filled
-        tma_load_3d(smem + kPairOffQ + g * kPairTileBytes, &tmQ, bar_q, 0, h, q0 + g * kBlockM);
-        tma_load_3d(smem + kPairOffQ + g * kPairTileBytes + kPairTileBytes / 2, &tmQ, bar_q, 64, h, q0 + g * kBlockM);
-      }
-      tma_load_3d(smem + kPairOffK, &tmK, bar_q, 0, hk, 0);
-      tma_load_3d(smem + kPairOffK + kPairTileBytes / 2, &tmK, bar_q, 64, hk, 0);
+      for (int g = 0; g < 2; ++g)  // rows past sq are zero-filled
+        load_tile(smem + kPairOffQ + g * kPairTileBytes, &tmQ, bar_q, h, q0 + g * kBlockM);
+      load_tile(smem + kPairOffK, &tmK, bar_q, hk, 0);
       bool ok = true;
       for (int j = 0; j < nkv && ok; ++j) {  // pair j: V_j into V stage j & 1, K_{j+1} into K stage (j+1) & 1
         const int s = j & 1;
@@ -411,15 +431,10 @@ prefill_attn_f16_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __gr
         if (j >= 1) ok = mbar_wait_bounded(&empty_kv[s], s ? ((j - 1) >> 1) & 1 : ((j >> 1) - 1) & 1, abort_flag);
         if (!ok) break;
         const bool with_k = j + 1 < nkv;
-        mbar_arrive_expect_tx(&full_kv[s], with_k ? 2 * kPairTileBytes : kPairTileBytes);
-        if (with_k) {  // first: S_g(j+1) is what the softmax warps wait for
-          uint8_t *kd = smem + kPairOffK + (s ^ 1) * kPairTileBytes;
-          tma_load_3d(kd, &tmK, &full_kv[s], 0, hk, (j + 1) * kPairN);
-          tma_load_3d(kd + kPairTileBytes / 2, &tmK, &full_kv[s], 64, hk, (j + 1) * kPairN);
-        }
-        uint8_t *vd = smem + kPairOffV + s * kPairTileBytes;
-        tma_load_3d(vd, &tmV, &full_kv[s], 0, hk, j * kPairN);
-        tma_load_3d(vd + kPairTileBytes / 2, &tmV, &full_kv[s], 64, hk, j * kPairN);
+        mbar_arrive_expect_tx(&full_kv[s], with_k ? 2 * tile_bytes : tile_bytes);
+        if (with_k)  // first: S_g(j+1) is what the softmax warps wait for
+          load_tile(smem + kPairOffK + (s ^ 1) * kPairTileBytes, &tmK, &full_kv[s], hk, (j + 1) * kPairN);
+        load_tile(smem + kPairOffV + s * kPairTileBytes, &tmV, &full_kv[s], hk, j * kPairN);
       }
     }
   } else if (warp == kPairMmaWarp) {
@@ -431,11 +446,13 @@ prefill_attn_f16_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __gr
       const uint64_t dq = smem_desc(smem_u32(smem + kPairOffQ), 16, 1024);
       const uint64_t dk = smem_desc(smem_u32(smem + kPairOffK), 16, 1024);
       const uint64_t dv = smem_desc(smem_u32(smem + kPairOffV), kPairTileBytes / 2, 1024);
+      const int d_steps = kNarrow ? (p.d + 15) / 16 : kD / 16;
       auto issue_s = [&](int g, int j) {  // S_g(j) = Q_g . K_j^T; K_j is known to have landed
         const uint64_t dqg = dq + (uint64_t)(g * (kPairTileBytes >> 4));
         const uint64_t dks = dk + (uint64_t)((j & 1) * (kPairTileBytes >> 4));
 #pragma unroll
         for (int ks = 0; ks < 8; ++ks) {  // head_dim 128 = 8 steps of 16; each 64-wide half of d is one box
+          if (kNarrow && ks >= d_steps) break;
           const uint32_t off = ((ks >> 2) * (kPairTileBytes / 2) + (ks & 3) * 32) >> 4;
           umma_f16(tmem_base + g * 128, dqg + off, dks + off, idesc_qk, ks > 0);
         }
@@ -461,9 +478,11 @@ prefill_attn_f16_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __gr
           // O_g += P_g(j) . V_j: P from tensor memory (16 keys = 8 columns); V as the MN-major B
           // operand: the two 64-wide d atoms are one box (16 KB) apart, 8-key groups 1 KB apart
 #pragma unroll
-          for (int ks = 0; ks < kPairN / 16; ++ks)
-            umma_f16_ts(tmem_base + 256 + g * 128, tmem_base + g * 128 + ks * 8, dvs + (uint64_t)(ks * (2048 >> 4)),
-                        idesc_pv, j > 0 || ks > 0);
+          for (int part = 0; part < (kNarrow ? 2 : 1); ++part)
+#pragma unroll
+            for (int ks = 0; ks < kPairN / 16; ++ks)
+              umma_f16_ts(tmem_base + 256 + g * 128, tmem_base + g * 128 + part * 64 + ks * 8, dvs + (uint64_t)(ks * (2048 >> 4)),
+                          idesc_pv, j > 0 || part > 0 || ks > 0);
           if (j == nkv_g[g] - 1) umma_commit(&bar_fin[g]);
           if (j + 1 < nkv_g[g]) issue_s(g, j + 1);
         }
@@ -516,23 +535,28 @@ prefill_attn_f16_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __gr
       float sum4[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
       for (int c = 0; c < 4; ++c) {
-        uint32_t packed[16];
+        uint32_t packed[16], low[16];
 #pragma unroll
         for (int i = 0; i < 32; i += 2) {
           const float xa = fmaf(__uint_as_float(sr[c][i]), p.scale_log2, -m_safe);
           const float xb = fmaf(__uint_as_float(sr[c][i + 1]), p.scale_log2, -m_safe);
           const float a = fast_exp2(xa), b = fast_exp2(xb);
           sum4[(i >> 1) & 3] += a + b;
-          packed[i >> 1] = pack_half2(a, b);
+          if (kNarrow)
+            packed[i >> 1] = split_half2(a, b, low[i >> 1]);
+          else
+            packed[i >> 1] = pack_half2(a, b);
         }
         // P: 32 keys = 16 columns over the front of this thread's own S row (all scores are in registers)
         tmem_st16(tmem_s + c * 16, packed);
+        if (kNarrow) tmem_st16(tmem_s + 64 + c * 16, low);
       }
       l_run = l_run * corr + ((sum4[0] + sum4[1]) + (sum4[2] + sum4[3]));
       // S_g(j) was queued behind P_g(j-1).V_{j-1}, so that product is complete: O_g may be rescaled
       if (j > 0 && moved) {
 #pragma unroll
         for (int c = 0; c < 4; ++c) {
+          if (kNarrow && c * 32 >= p.d) break;
           uint32_t r[32];
           tmem_ld32(tmem_o + c * 32, r);
 #pragma unroll
@@ -550,14 +574,16 @@ prefill_attn_f16_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __gr
     tc_fence_after();
     if (ok && my_nkv > 0) {
       const float inv = l_run > 0.f ? 1.0f / l_run : 0.f;
-      __half *dst = reinterpret_cast<__half *>(p.out) + ((size_t)t_row * p.hq + h) * kD;
+      __half *dst = reinterpret_cast<__half *>(p.out) + ((size_t)t_row * p.hq + h) * (kNarrow ? p.d : kD);
 #pragma unroll
       for (int c = 0; c < 4; ++c) {
+        if (kNarrow && c * 32 >= p.d) break;
         uint32_t r[32];
         tmem_ld32(tmem_o + c * 32, r);
         if (t_row < p.sq) {
 #pragma unroll
           for (int u = 0; u < 4; ++u) {
+            if (kNarrow && c * 32 + u * 8 >= p.d) break;
             uint4 w;
             w.x = pack_half2(__uint_as_float(r[u * 8 + 0]) * inv, __uint_as_float(r[u * 8 + 1]) * inv);
             w.y = pack_half2(__uint_as_float(r[u * 8 + 2]) * inv, __uint_as_float(r[u * 8 + 3]) * inv);
@@ -576,12 +602,12 @@ prefill_attn_f16_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __gr
 }
 
 
-// (rows, heads, 128) fp16 token-major -> tensor map with boxes of [box_rows rows][64 halves], 128-byte swizzle
-bool rows_map(CUtensorMap *map, const void *base, int64_t rows, int heads, int box_rows) {
+// (rows, heads, d) fp16 token-major -> tensor map with boxes of [box_rows rows][64 halves], 128-byte swizzle
+bool rows_map(CUtensorMap *map, const void *base, int64_t rows, int heads, int d, int box_rows) {
   EncodeTiledFn fn = tensor_map_encoder();
   if (!fn) return false;
-  cuuint64_t dims[3] = {(cuuint64_t)kD, (cuuint64_t)heads, (cuuint64_t)rows};
-  cuuint64_t strides[2] = {(cuuint64_t)kD * 2, (cuuint64_t)heads * kD * 2};
+  cuuint64_t dims[3] = {(cuuint64_t)d, (cuuint64_t)heads, (cuuint64_t)rows};
+  cuuint64_t strides[2] = {(cuuint64_t)d * 2, (cuuint64_t)heads * d * 2};
   cuuint32_t box[3] = {64, 1, (cuuint32_t)box_rows}, es[3] = {1, 1, 1};
   return fn(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 3, const_cast<void *>(base), dims, strides, box, es,
             CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
@@ -610,19 +636,22 @@ int axb200_sdpa(const void *q, const void *k, const void *v, void *out, int sq, 
   if (sq <= 0 || hq <= 0 || hkv <= 0 || d <= 0 || skv <= 0 || skv > 0x7fffffff - 4096) return AXB200_INVALID_ARGUMENT;
   if (hq % hkv != 0) return AXB200_SHAPE_MISMATCH;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  const bool tensor_path = dtype == AXB200_FLOAT16 && d == axb::kD && hq <= 65535 && axb::aligned16(q) &&
+  // fp16 heads of 128, and prompts of narrower heads: a TMA row is a multiple of 16 bytes, and below 16 rows (of 128 that a
+  // tile holds) the row-by-row form is the cheaper one
+  const bool narrow = d < axb::kD && d % 8 == 0 && sq >= 16;
+  const bool tensor_path = dtype == AXB200_FLOAT16 && (d == axb::kD || narrow) && hq <= 65535 && axb::aligned16(q) &&
                            axb::aligned16(k) && axb::aligned16(v) && axb::aligned16(out) && axb::tensor_map_encoder();
   if (!tensor_path) {
     if (axb::sdpa_tiled_supported(sq, hq, hkv, d, skv))
       return axb::sdpa_tiled(q, k, v, out, sq, hq, hkv, d, skv, is_causal, dtype, st);
     return axb::sdpa_rows_fallback(q, k, v, out, sq, hq, hkv, d, skv, is_causal, dtype, workspace, workspace_bytes, st);
   }
-  // 256 query rows per CTA once there are that many; the 128-row form below that
-  const bool pair = sq >= 2 * axb::kBlockM;
+  // 256 query rows per CTA once there are that many; the 128-row form (heads of 128 only) below that
+  const bool pair = narrow || sq >= 2 * axb::kBlockM;
   const int kv_box = pair ? axb::kPairN : axb::kBlockN;
   CUtensorMap mq, mk, mv;
-  if (!axb::rows_map(&mq, q, sq, hq, axb::kBlockM) || !axb::rows_map(&mk, k, skv, hkv, kv_box) ||
-      !axb::rows_map(&mv, v, skv, hkv, kv_box))
+  if (!axb::rows_map(&mq, q, sq, hq, d, axb::kBlockM) || !axb::rows_map(&mk, k, skv, hkv, d, kv_box) ||
+      !axb::rows_map(&mv, v, skv, hkv, d, kv_box))
     return AXB200_INTERNAL_ERROR;
   static std::mutex mu;
   static bool opted[64] = {false};
@@ -633,7 +662,9 @@ int axb200_sdpa(const void *q, const void *k, const void *v, void *out, int sq, 
     if (!opted[dev]) {
       if (cudaFuncSetAttribute(axb::prefill_attn_f16_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                axb::kSmemBytes) != cudaSuccess ||
-          cudaFuncSetAttribute(axb::prefill_attn_f16_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+          cudaFuncSetAttribute(axb::prefill_attn_f16_pair_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                               axb::kPairSmemBytes) != cudaSuccess ||
+          cudaFuncSetAttribute(axb::prefill_attn_f16_pair_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                axb::kPairSmemBytes) != cudaSuccess)
         return AXB200_DEVICE_ERROR;
       opted[dev] = true;
@@ -646,10 +677,12 @@ int axb200_sdpa(const void *q, const void *k, const void *v, void *out, int sq, 
   p.hkv = hkv;
   p.skv = (int)skv;
   p.causal = is_causal != 0;
+  p.d = d;
   p.scale_log2 = (1.0f / sqrtf((float)d)) * axb::kLog2e;
   if (pair) {
     const dim3 grid((sq + 2 * axb::kBlockM - 1) / (2 * axb::kBlockM), hq);
-    axb::prefill_attn_f16_pair_kernel<<<grid, axb::kPairThreads, axb::kPairSmemBytes, st>>>(mq, mk, mv, p);
+    auto *kernel = narrow ? axb::prefill_attn_f16_pair_kernel<true> : axb::prefill_attn_f16_pair_kernel<false>;
+    kernel<<<grid, axb::kPairThreads, axb::kPairSmemBytes, st>>>(mq, mk, mv, p);
   } else {
     const dim3 grid((sq + axb::kBlockM - 1) / axb::kBlockM, hq);
     axb::prefill_attn_f16_kernel<<<grid, axb::kThreads, axb::kSmemBytes, st>>>(mq, mk, mv, p);
