@@ -35,7 +35,6 @@ constexpr int kConsumerThreads = kConsumerWarps * 32;
 constexpr int kThreads = kConsumerThreads + 32;  // + one producer warp
 constexpr int kStageBytes = 32768;               // K tile 16 KB + V tile 16 KB
 constexpr int kTileTokensF16 = 64;
-constexpr int kTileTokensF32 = 32;
 constexpr int kMaxGroupMma = 16;
 constexpr int kMaxChunks = 256;  // the reference's kMaxSplits (src/ops/cuda/gqa.cu:27)
 constexpr float kLog2e = 1.4426950408889634f;
@@ -1168,12 +1167,45 @@ gqa_split_f16_kernel(const __grid_constant__ CUtensorMap tmK,
 }
 
 // ---- fp32 split kernel: FMA on unswizzled tiles ----------------------------------------------
-// Tile = 32 tokens x 128 floats; warp w owns tokens [8w, 8w+8), lane owns dims [4*lane, +4).
-template <bool kPaged, int kStages, int kGroup>
+// A stage is a K tile and a V tile of 16 KB each: 32 tokens of kD = 128 floats or 64 tokens of 64.  The head size p.d is
+// any multiple of 4 up to kD; columns past it lie outside the tensor map and arrive as zeros, as in the fp16 kernel.
+// A warp owns a quarter of a tile's tokens and takes eight rows of 512 bytes at a time - a token each (kD = 128), or two
+// tokens, one per half-warp (kD = 64) - with four dims per lane.  The eight partial dots of a head are summed over the lanes
+// by exchanges that halve the number of values a lane still holds (4 + 2 + 1, then one value each): 9 or 8 shuffles
+// instead of 40, and every lane ends with the score of one token, so that a token's exponential is taken by the 4 or 2
+// lanes that hold it instead of all 32.
+// Bound by HBM at long lengths, by the latency of its one wave at short ones.  us per call, 16 / 8 heads: d = 128, 1000
+// tokens 10.4 before the exchanges and 9.1 with them, 32768 tokens 48.5 and 47.2 (5.7 TB/s); d = 64, 16001 tokens 66.5 on
+// the generic kernel and 17.4 here; d = 96, 26000 tokens 136 and 31; d = 8, 4096 tokens (8 / 8 heads) 21.3 and 6.6.
+__host__ __device__ constexpr int f32_tile_width(int d) { return d <= 64 ? 64 : 128; }
+__host__ __device__ constexpr int f32_tile_tokens(int tile_width) { return kStageBytes / 2 / 4 / tile_width; }
+
+// v[0 .. 7], partial sums of eight values in every lane of a group of kLanes -> the full sum of value
+// (bit 2, 1, 0 = the group's lane bits from the highest) in each lane.
+template <int kLanes>
+__device__ __forceinline__ float reduce_eight(const float (&v)[8], int lane) {
+  float a[4], b[2];
+  const bool hi = lane & (kLanes / 2), mid = lane & (kLanes / 4), lo = lane & (kLanes / 8);
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+    a[i] = (hi ? v[i + 4] : v[i]) + __shfl_xor_sync(0xffffffffu, hi ? v[i] : v[i + 4], kLanes / 2);
+#pragma unroll
+  for (int i = 0; i < 2; ++i)
+    b[i] = (mid ? a[i + 2] : a[i]) + __shfl_xor_sync(0xffffffffu, mid ? a[i] : a[i + 2], kLanes / 4);
+  float c = (lo ? b[1] : b[0]) + __shfl_xor_sync(0xffffffffu, lo ? b[0] : b[1], kLanes / 8);
+#pragma unroll
+  for (int off = kLanes / 16; off > 0; off >>= 1) c += __shfl_xor_sync(0xffffffffu, c, off);
+  return c;
+}
+
+template <bool kPaged, int kStages, int kGroup, int kD>
 __global__ void __launch_bounds__(kThreads, 2)
 gqa_split_f32_kernel(const __grid_constant__ CUtensorMap tmK,
                      const __grid_constant__ CUtensorMap tmV, const DecodeParams p,
                      const GatherParams gp) {
+  constexpr int kTile = f32_tile_tokens(kD), kRowLanes = kD / 4, kRows = 32 / kRowLanes;  // rows a warp reads at once
+  constexpr int kWarpTokens = kTile / kConsumerWarps;                                    // = 8 * kRows
+  static_assert(kWarpTokens == 8 * kRows, "a warp's tokens are eight reads");
   extern __shared__ uint8_t smem_raw[];
   __shared__ int s_plan[kPlanWords];
   uint8_t *smem = align_1024(smem_raw);
@@ -1203,7 +1235,7 @@ gqa_split_f32_kernel(const __grid_constant__ CUtensorMap tmK,
   if (warp == kConsumerWarps) {
     if (kPaged && !p.balanced) {
       spec_start = blockIdx.x * p.chunk_tokens;
-      const int slot = (spec_start + lane * kTileTokensF32) / p.page_tokens;
+      const int slot = (spec_start + lane * kTile) / p.page_tokens;
       if (slot < p.max_blocks) spec_page = p.block_table[(size_t)blockIdx.z * p.max_blocks + slot];
     }
   }
@@ -1221,25 +1253,28 @@ gqa_split_f32_kernel(const __grid_constant__ CUtensorMap tmK,
   int start = chunk * w.ct;
   const int end = min(L, start + w.ct);
   if (end <= first) return;  // the whole chunk lies before the window
-  if (start < first) start = first / kTileTokensF32 * kTileTokensF32;  // skip whole tiles before it
-  const int ntiles = (end - start + kTileTokensF32 - 1) / kTileTokensF32;
+  if (start < first) start = first / kTile * kTile;  // skip whole tiles before it
+  const int ntiles = (end - start + kTile - 1) / kTile;
   const bool direct = p.direct_ok && w.n - c_first == 1;
 
   if (warp == kConsumerWarps) {
-    produce_tiles<kPaged, kStages, kTileTokensF32, 1, 128>(&tmK, &tmV, p, smem, full, empty, abort_flag, b, hk,
-                                                           start, ntiles, lane, spec_start, spec_page);
+    produce_tiles<kPaged, kStages, kTile, 1, kD>(&tmK, &tmV, p, smem, full, empty, abort_flag, b, hk,
+                                                 start, ntiles, lane, spec_start, spec_page);
     return;
   }
 
+  // lane: dims [4 * col, +4) of row `sub` of the rows a read covers
+  const int col = lane % kRowLanes, sub = lane / kRowLanes;
+  const bool has_dims = col * 4 < p.d;
   const float *qf = reinterpret_cast<const float *>(p.q);
   float4 qr[kGroup];
 #pragma unroll
   for (int r = 0; r < kGroup; ++r)
-    qr[r] = *reinterpret_cast<const float4 *>(
-        qf + ((size_t)b * p.hq + (size_t)hk * kGroup + r) * kHeadDim + lane * 4);
+    qr[r] = has_dims ? *reinterpret_cast<const float4 *>(qf + ((size_t)b * p.hq + (size_t)hk * kGroup + r) * p.d + col * 4)
+                     : make_float4(0.f, 0.f, 0.f, 0.f);
 
   float4 o[kGroup];
-  float m[kGroup], l[kGroup];  // m: running max of the raw dot products
+  float m[kGroup], l[kGroup];  // m: running max of the raw dot products; l: of this lane's own tokens
 #pragma unroll
   for (int r = 0; r < kGroup; ++r) {
     o[r] = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -1247,6 +1282,9 @@ gqa_split_f32_kernel(const __grid_constant__ CUtensorMap tmK,
     l[r] = 0.f;
   }
   const float sl2 = p.scale * kLog2e;
+  // the token (within the warp's part of a tile) whose score this lane holds, and the lane that holds a token's
+  const int my_read = ((lane & (kRowLanes / 2)) ? 4 : 0) | ((lane & (kRowLanes / 4)) ? 2 : 0) | ((lane & (kRowLanes / 8)) ? 1 : 0);
+  const int my_token = my_read * kRows + sub;
 
   bool ok = true;
   for (int i = 0; i < ntiles && ok; ++i) {
@@ -1254,53 +1292,39 @@ gqa_split_f32_kernel(const __grid_constant__ CUtensorMap tmK,
     const uint32_t phase = (i / kStages) & 1;
     ok = mbar_wait_bounded(&full[s], phase, abort_flag, p.wait_ns);
     if (!ok) break;
-    const float *Ks = reinterpret_cast<const float *>(smem + (size_t)s * kStageBytes);
-    const float *Vs = Ks + kTileTokensF32 * kHeadDim;
-    const int valid = end - (start + i * kTileTokensF32 + warp * 8);  // tokens of this warp that exist
-    const int lo = first - (start + i * kTileTokensF32 + warp * 8);   // tokens below lo precede the window
+    const float *Ks = reinterpret_cast<const float *>(smem + (size_t)s * kStageBytes) + warp * kWarpTokens * kD + lane * 4;
+    const float *Vs = Ks + kTile * kD;
+    const int valid = end - (start + i * kTile + warp * kWarpTokens);  // tokens of this warp that exist
+    const int lo = first - (start + i * kTile + warp * kWarpTokens);   // tokens below lo precede the window
 
-    float sc[kGroup][8];
+    float4 kv[8];
 #pragma unroll
-    for (int t = 0; t < 8; ++t) {
-      const float4 kv = *reinterpret_cast<const float4 *>(Ks + (warp * 8 + t) * kHeadDim + lane * 4);
-#pragma unroll
-      for (int r = 0; r < kGroup; ++r) {
-        float a = qr[r].x * kv.x;
-        a = fmaf(qr[r].y, kv.y, a);
-        a = fmaf(qr[r].z, kv.z, a);
-        a = fmaf(qr[r].w, kv.w, a);
-        sc[r][t] = a;
-      }
-    }
+    for (int t = 0; t < 8; ++t) kv[t] = *reinterpret_cast<const float4 *>(Ks + t * kRows * kD);
+    float pw[kGroup];
 #pragma unroll
     for (int r = 0; r < kGroup; ++r) {
+      float part[8];
 #pragma unroll
       for (int t = 0; t < 8; ++t) {
-        float a = sc[r][t];
-        a += __shfl_xor_sync(0xffffffffu, a, 16);
-        a += __shfl_xor_sync(0xffffffffu, a, 8);
-        a += __shfl_xor_sync(0xffffffffu, a, 4);
-        a += __shfl_xor_sync(0xffffffffu, a, 2);
-        a += __shfl_xor_sync(0xffffffffu, a, 1);
-        sc[r][t] = (t < valid && t >= lo) ? a : -INFINITY;
+        float a = qr[r].x * kv[t].x;
+        a = fmaf(qr[r].y, kv[t].y, a);
+        a = fmaf(qr[r].z, kv[t].z, a);
+        part[t] = fmaf(qr[r].w, kv[t].w, a);
       }
+      const float dot = reduce_eight<kRowLanes>(part, lane);
+      pw[r] = (my_token < valid && my_token >= lo) ? dot : -INFINITY;
     }
 #pragma unroll
     for (int r = 0; r < kGroup; ++r) {
-      float mx = sc[r][0];
+      float mx = pw[r];
 #pragma unroll
-      for (int t = 1; t < 8; ++t) mx = fmaxf(mx, sc[r][t]);
+      for (int off = 16; off >= kRowLanes / 8; off >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, off));
       const float mn = fmaxf(m[r], mx);
       const float ms = (mn == -INFINITY) ? 0.f : mn;
       const float corr = exp2f((m[r] - ms) * sl2);
       m[r] = mn;
-      float sum = 0.f;
-#pragma unroll
-      for (int t = 0; t < 8; ++t) {
-        sc[r][t] = exp2f((sc[r][t] - ms) * sl2);
-        sum += sc[r][t];
-      }
-      l[r] = l[r] * corr + sum;
+      pw[r] = exp2f((pw[r] - ms) * sl2);
+      l[r] = l[r] * corr + pw[r];
       o[r].x *= corr;
       o[r].y *= corr;
       o[r].z *= corr;
@@ -1308,18 +1332,33 @@ gqa_split_f32_kernel(const __grid_constant__ CUtensorMap tmK,
     }
 #pragma unroll
     for (int t = 0; t < 8; ++t) {
-      float4 vv = *reinterpret_cast<const float4 *>(Vs + (warp * 8 + t) * kHeadDim + lane * 4);
-      if (t >= valid || t < lo) vv = make_float4(0.f, 0.f, 0.f, 0.f);  // stale rows outside the range
+      float4 vv = *reinterpret_cast<const float4 *>(Vs + t * kRows * kD);
+      const int token = t * kRows + sub;
+      if (token >= valid || token < lo) vv = make_float4(0.f, 0.f, 0.f, 0.f);  // stale rows outside the range
+      const int holder = sub * kRowLanes + ((t & 4) ? kRowLanes / 2 : 0) + ((t & 2) ? kRowLanes / 4 : 0) + ((t & 1) ? kRowLanes / 8 : 0);
 #pragma unroll
       for (int r = 0; r < kGroup; ++r) {
-        o[r].x = fmaf(sc[r][t], vv.x, o[r].x);
-        o[r].y = fmaf(sc[r][t], vv.y, o[r].y);
-        o[r].z = fmaf(sc[r][t], vv.z, o[r].z);
-        o[r].w = fmaf(sc[r][t], vv.w, o[r].w);
+        const float wt = __shfl_sync(0xffffffffu, pw[r], holder);
+        o[r].x = fmaf(wt, vv.x, o[r].x);
+        o[r].y = fmaf(wt, vv.y, o[r].y);
+        o[r].z = fmaf(wt, vv.z, o[r].z);
+        o[r].w = fmaf(wt, vv.w, o[r].w);
       }
     }
     __syncwarp();
     if (lane == 0) mbar_arrive(&empty[s]);
+  }
+#pragma unroll
+  for (int r = 0; r < kGroup; ++r) {
+#pragma unroll
+    for (int off = 16; off >= kRowLanes / 8; off >>= 1) l[r] += __shfl_xor_sync(0xffffffffu, l[r], off);
+#pragma unroll
+    for (int off = kRowLanes; off < 32; off <<= 1) {  // the rows of a read were summed apart
+      o[r].x += __shfl_xor_sync(0xffffffffu, o[r].x, off);
+      o[r].y += __shfl_xor_sync(0xffffffffu, o[r].y, off);
+      o[r].z += __shfl_xor_sync(0xffffffffu, o[r].z, off);
+      o[r].w += __shfl_xor_sync(0xffffffffu, o[r].w, off);
+    }
   }
 
   named_bar_sync(1, kConsumerThreads);
@@ -1329,20 +1368,20 @@ gqa_split_f32_kernel(const __grid_constant__ CUtensorMap tmK,
   float *mL = mM + kConsumerWarps * kMaxGroupMma;
 #pragma unroll
   for (int r = 0; r < kGroup; ++r) {
-    *reinterpret_cast<float4 *>(mO + (warp * kMaxGroupMma + r) * kHeadDim + lane * 4) = o[r];
+    if (sub == 0) *reinterpret_cast<float4 *>(mO + (warp * kMaxGroupMma + r) * kD + col * 4) = o[r];
     if (lane == 0) {
       mM[warp * kMaxGroupMma + r] = m[r];
       mL[warp * kMaxGroupMma + r] = l[r];
     }
   }
   named_bar_sync(1, kConsumerThreads);
-  finalize_chunk<float, kHeadDim>(p, gp, mO, mM, mL, b, hk, chunk, threadIdx.x, sl2, direct);
+  finalize_chunk<float, kD>(p, gp, mO, mM, mL, b, hk, chunk, threadIdx.x, sl2, direct);
   finish_item<float>(p, gp, w, hk, c_first, direct, sl2, threadIdx.x, kConsumerThreads, s_word, mO,
                      [] { named_bar_sync(1, kConsumerThreads); });
 }
 
 // ---- generic split kernel: any head_dim <= 256, any group, any alignment ---------------------------
-// For the shapes the TMA kernels do not take (head_dim != 128, pointers off 16 bytes, odd groups).
+// For the shapes the TMA kernels do not take (head sizes, pointers off 16 bytes, odd groups).
 // Same split-K scheme and partial format; tiles of keys are staged in shared memory as fp32 with plain
 // coalesced loads (a warp reads a row), every query head of the KV head works on the staged tile:
 //   scores   thread = (key, head subset): one K value from shared memory feeds all its heads
@@ -1728,26 +1767,25 @@ int sm_count() {
 // 4-D tensor map over a cache.  Paged: dims (d, page_tokens, hkv, num_pages), box
 // (box_d, tile, 1, 1).  Token-major: dims (d, hkv, skv, 1), box (box_d, 1, tile, 1).
 bool make_map(CUtensorMap *map, const void *base, int dtype, bool paged, int d, int hkv,
-              int64_t tokens_or_page_tokens, int64_t num_pages, int tile) {
+              int64_t tokens_or_page_tokens, int64_t num_pages, int tile, int box_d) {
   EncodeTiledFn fn = encode_fn();
   if (!fn) return false;
   const size_t es = dtype_size(dtype);
   const bool f16 = dtype == AXB200_FLOAT16;
   cuuint64_t dims[4], strides[3];
   cuuint32_t box[4], estr[4] = {1, 1, 1, 1};
-  const cuuint32_t box_d = f16 ? 64 : 128;
   if (paged) {
     dims[0] = d; dims[1] = tokens_or_page_tokens; dims[2] = hkv; dims[3] = num_pages;
     strides[0] = d * es;
     strides[1] = tokens_or_page_tokens * d * es;
     strides[2] = (cuuint64_t)hkv * tokens_or_page_tokens * d * es;
-    box[0] = box_d; box[1] = tile; box[2] = 1; box[3] = 1;
+    box[0] = (cuuint32_t)box_d; box[1] = tile; box[2] = 1; box[3] = 1;
   } else {
     dims[0] = d; dims[1] = hkv; dims[2] = tokens_or_page_tokens; dims[3] = 1;
     strides[0] = d * es;
     strides[1] = (cuuint64_t)hkv * d * es;
     strides[2] = (cuuint64_t)tokens_or_page_tokens * hkv * d * es;
-    box[0] = box_d; box[1] = 1; box[2] = tile; box[3] = 1;
+    box[0] = (cuuint32_t)box_d; box[1] = 1; box[2] = tile; box[3] = 1;
   }
   CUresult r = fn(map, f16 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4,
                   const_cast<void *>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
@@ -1874,13 +1912,20 @@ int launch_f16(const CUtensorMap &mk, const CUtensorMap &mv, const DecodeParams 
                    : launch_f16_d<kPaged, 128, false>(mk, mv, p, g, grid, st, none);
 }
 
-template <bool kPaged, int kGroup>
-int launch_f32_g(const CUtensorMap &mk, const CUtensorMap &mv, const DecodeParams &p,
+template <bool kPaged, int kGroup, int kD>
+int launch_f32_d(const CUtensorMap &mk, const CUtensorMap &mv, const DecodeParams &p,
                  const GatherParams &g, dim3 grid, cudaStream_t st) {
-  auto kern = gqa_split_f32_kernel<kPaged, kStagesDefault, kGroup>;
+  auto kern = gqa_split_f32_kernel<kPaged, kStagesDefault, kGroup, kD>;
   constexpr int smem = SmemLayout<kStagesDefault>::kDynamicBytes;
   if (!set_smem(reinterpret_cast<const void *>(kern), smem)) return AXB200_DEVICE_ERROR;
   return launch_split(kern, grid, kThreads, smem, st, g_dependent_launch, mk, mv, p, g);
+}
+
+template <bool kPaged, int kGroup>
+int launch_f32_g(const CUtensorMap &mk, const CUtensorMap &mv, const DecodeParams &p,
+                 const GatherParams &g, dim3 grid, cudaStream_t st) {
+  return f32_tile_width(p.d) == 64 ? launch_f32_d<kPaged, kGroup, 64>(mk, mv, p, g, grid, st)
+                                   : launch_f32_d<kPaged, kGroup, 128>(mk, mv, p, g, grid, st);
 }
 
 template <bool kPaged>
@@ -2006,10 +2051,9 @@ int decode_impl(bool paged, const void *q, void *out, const void *k, const void 
   const float dom = p.scale * kLog2e;
 
   const bool f16_in = dtype == AXB200_FLOAT16;
-  // fp16: any head size that is a multiple of 8 up to 128 (rows stay 16-byte multiples for the tensor
-  // map; narrower heads ride in the 64- or 128-wide tile with zero fill); fp32: 128
-  bool tiled = (d == kHeadDim || (f16_in && d % 8 == 0 && d <= kHeadDim)) && aligned16(k) && aligned16(v) &&
-               aligned16(q) && encode_fn();
+  // any head size up to 128 whose rows are multiples of 16 bytes, as the tensor map wants them; narrower heads ride in the
+  // 64- or 128-wide tile with zero fill
+  bool tiled = d <= kHeadDim && d % (f16_in ? 8 : 4) == 0 && aligned16(k) && aligned16(v) && aligned16(q) && encode_fn();
   if (tiled && f16 && p.group > kMaxGroupMma) tiled = false;
   if (tiled && !f16 && !(p.group == 1 || p.group == 2 || p.group == 4 || p.group == 8))
     tiled = false;
@@ -2021,10 +2065,11 @@ int decode_impl(bool paged, const void *q, void *out, const void *k, const void 
 
   CUtensorMap mk, mv;
   if (tiled) {
-    const int tile = f16 ? kTileTokensF16 : kTileTokensF32;
+    const int box_d = f16 ? 64 : f32_tile_width(d);
+    const int tile = f16 ? kTileTokensF16 : f32_tile_tokens(box_d);
     const int64_t tok = paged ? page_tokens : max_len;
-    if (!make_map(&mk, k, dtype, paged, d, hkv, tok, num_pages, tile) ||
-        !make_map(&mv, v, dtype, paged, d, hkv, tok, num_pages, tile))
+    if (!make_map(&mk, k, dtype, paged, d, hkv, tok, num_pages, tile, box_d) ||
+        !make_map(&mv, v, dtype, paged, d, hkv, tok, num_pages, tile, box_d))
       return AXB200_INTERNAL_ERROR;
   }
   int status;
