@@ -64,8 +64,8 @@ latent_prefill_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
     if (threadIdx.x == 0) atomicOr(&g_error_word, AXB200_ERR_WAIT_TIMEOUT);
     return;
   }
-  // heaviest blocks first: the last query block has the most key tiles
-  const int h = blockIdx.y, q0 = (gridDim.x - 1 - blockIdx.x) * 2 * kRows;
+  // heaviest blocks of all heads first: the last query block has the most key tiles
+  const int h = blockIdx.x % p.heads, q0 = (int)((gridDim.x - 1 - blockIdx.x) / p.heads) * 2 * kRows;
   const int warp = uniform_warp(), lane = threadIdx.x & 31;
   const int hk = h / p.group;
   const int tile0 = p.window > 0 ? max(0, p.start + q0 + 1 - p.window) / kKeys : 0;  // the first key tile
@@ -237,12 +237,7 @@ latent_prefill_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
           for (int i = 0; i < 32; ++i)
             if (n0 + c * 32 + i >= kv_end) sr[c][i] = 0xff800000u;  // -inf
       }
-      float mx4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
-#pragma unroll
-      for (int c = 0; c < 4; ++c)
-#pragma unroll
-        for (int i = 0; i < 32; ++i) mx4[i & 3] = fmaxf(mx4[i & 3], __uint_as_float(sr[c][i]));
-      const float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3]));
+      const float mx = row_max(sr);
       // scale may be negative or zero in principle: the running maximum is kept of the scaled scores
       const float m_tile = mx * p.scale_log2;
       float corr = 1.f;
@@ -253,20 +248,22 @@ latent_prefill_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
         m_run = m_new;
       }
       const float m_safe = (m_run == -INFINITY) ? 0.f : m_run;
-      float sum4[4] = {0.f, 0.f, 0.f, 0.f};
+      const uint64_t scale2 = pack_f32x2(p.scale_log2, p.scale_log2), shift2 = pack_f32x2(-m_safe, -m_safe);
+      uint64_t sum2[4] = {0, 0, 0, 0};
 #pragma unroll
       for (int c = 0; c < 4; ++c) {
         uint32_t packed[16];
 #pragma unroll
         for (int i = 0; i < 32; i += 2) {
-          const float a = fast_exp2(fmaf(__uint_as_float(sr[c][i]), p.scale_log2, -m_safe));
-          const float b = fast_exp2(fmaf(__uint_as_float(sr[c][i + 1]), p.scale_log2, -m_safe));
-          sum4[(i >> 1) & 3] += a + b;
+          const float2 x = unpack_f32x2(fma_f32x2(pack_f32x2(__uint_as_float(sr[c][i]), __uint_as_float(sr[c][i + 1])), scale2, shift2));
+          const float a = fast_exp2(x.x), b = fast_exp2(x.y);
+          sum2[(i >> 1) & 3] = add_f32x2(sum2[(i >> 1) & 3], pack_f32x2(a, b));
           packed[i >> 1] = pack_bf16x2(a, b);
         }
         tmem_st16(tp + c * 16, packed);
       }
-      l_run = l_run * corr + ((sum4[0] + sum4[1]) + (sum4[2] + sum4[3]));
+      const float2 sum = unpack_f32x2(add_f32x2(add_f32x2(sum2[0], sum2[1]), add_f32x2(sum2[2], sum2[3])));
+      l_run = l_run * corr + (sum.x + sum.y);
       // bar_s of tile j was committed after P(j-1).V_{j-1}: that product is complete and O_g may be rescaled
       if (j > 0 && moved) {
 #pragma unroll
@@ -345,7 +342,7 @@ int launch(const CUtensorMap (&m)[5], const Params &p, cudaStream_t st) {
       opted[dev] = true;
     }
   }
-  const dim3 grid((p.n + 2 * kRows - 1) / (2 * kRows), p.heads);
+  const dim3 grid((unsigned)p.heads * ((p.n + 2 * kRows - 1) / (2 * kRows)));
   return launch_dependent(kernel, grid, dim3(kThreads), L::kSmem, st, m[0], m[1], m[2], m[3], m[4], p);
 }
 
