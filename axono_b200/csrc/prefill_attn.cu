@@ -13,8 +13,8 @@
 // maximum moves by more than a threshold.  One lane each of two more warps launches the MMAs and the
 // TMA loads; the sides meet only on mbarriers (tcgen05.commit for MMA completion).  K/V tiles are
 // multi-buffered and S is computed two tiles ahead, so tensor core and softmax overlap.  Every wait
-// is bounded.  From 256 rows on, and for narrower heads, the 256-row form below; FLOAT32 and head sizes that are
-// not a multiple of 8 up to 128 go to prefill_tiled.cu, and what that does not take to the decode kernels, row by row.
+// is bounded.  From 256 rows on, and for narrower heads, the 256-row form below; FLOAT32 goes to prefill_f32.cu, head sizes
+// that are not a multiple of 8 up to 128 to prefill_tiled.cu, and what that does not take to the decode kernels, row by row.
 //
 // Semantics as the reference's CPU op (src/ops/cpu/sequence.cpp:236-301): q (sq,hq,d), k/v
 // (skv,hkv,d) token-major, head h reads KV head h / (hq/hkv), scale 1/sqrt(d); with is_causal row t
@@ -32,11 +32,14 @@ int sdpa_rows_fallback(const void *q, const void *k, const void *v, void *out, i
                        int d, int64_t skv, int is_causal, int dtype, void *workspace,
                        size_t workspace_bytes, cudaStream_t st);
 size_t sdpa_rows_workspace_bytes(int sq, int hq, int hkv, int d, int64_t skv);
-// Tiled evaluation on the FMA pipe (prefill_tiled.cu): FLOAT32 and the head sizes the tensor-core kernels
-// do not take.
+// Tiled evaluation on the FMA pipe (prefill_tiled.cu): what the tensor-core kernels do not take.
 bool sdpa_tiled_supported(int sq, int hq, int hkv, int d, int64_t skv);
 int sdpa_tiled(const void *q, const void *k, const void *v, void *out, int sq, int hq, int hkv, int d, int64_t skv,
                int is_causal, int dtype, cudaStream_t st);
+// FLOAT32 on the tensor cores (prefill_f32.cu); the scratch it wants is 0 where it does not apply.
+size_t sdpa_split_workspace_bytes(int sq, int hq, int hkv, int d, int64_t skv);
+int sdpa_split(const void *q, const void *k, const void *v, void *out, int sq, int hq, int hkv, int d, int64_t skv, int is_causal,
+               void *workspace, cudaStream_t st);
 
 namespace {
 
@@ -624,7 +627,8 @@ size_t axb200_sdpa_workspace_bytes(int sq, int hq, int hkv, int d, int64_t skv, 
   // the tensor-core kernels and the tiled FMA kernel keep everything on chip; only the row-by-row
   // evaluation on the decode kernels needs room for partials
   // (whatever the tensor-core path does not take - unaligned pointers, say - the tiled kernel does)
-  if (hkv > 0 && hq % hkv == 0 && axb::sdpa_tiled_supported(sq, hq, hkv, d, skv)) return 0;
+  if (hkv > 0 && hq % hkv == 0 && axb::sdpa_tiled_supported(sq, hq, hkv, d, skv))
+    return dtype == AXB200_FLOAT32 ? axb::sdpa_split_workspace_bytes(sq, hq, hkv, d, skv) : 0;
   return axb::sdpa_rows_workspace_bytes(sq, hq, hkv, d, skv);
 }
 
@@ -641,7 +645,12 @@ int axb200_sdpa(const void *q, const void *k, const void *v, void *out, int sq, 
   const bool tensor_path = dtype == AXB200_FLOAT16 && (d == axb::kD || narrow) && hq <= 65535 && axb::aligned16(q) &&
                            axb::aligned16(k) && axb::aligned16(v) && axb::aligned16(out) && axb::tensor_map_encoder();
   if (!tensor_path) {
-    if (axb::sdpa_tiled_supported(sq, hq, hkv, d, skv))
+    const bool tiled = axb::sdpa_tiled_supported(sq, hq, hkv, d, skv);
+    const size_t split = tiled && dtype == AXB200_FLOAT32 ? axb::sdpa_split_workspace_bytes(sq, hq, hkv, d, skv) : 0;
+    if (split && workspace && workspace_bytes >= split && axb::aligned16(workspace) && axb::aligned16(q) && axb::aligned16(k) &&
+        axb::aligned16(v) && axb::aligned16(out))
+      return axb::sdpa_split(q, k, v, out, sq, hq, hkv, d, skv, is_causal, workspace, st);
+    if (tiled)
       return axb::sdpa_tiled(q, k, v, out, sq, hq, hkv, d, skv, is_causal, dtype, st);
     return axb::sdpa_rows_fallback(q, k, v, out, sq, hq, hkv, d, skv, is_causal, dtype, workspace, workspace_bytes, st);
   }

@@ -1,9 +1,7 @@
 // Prefill attention on the FMA pipe: many queries, optional causal mask, FLOAT32 or FLOAT16 storage
 // with fp32 arithmetic throughout, any head_dim that is a multiple of 4 up to 256.  It serves what the
-// tensor-core kernel does not take - above all FLOAT32, the only type the reference's own
-// ScaledDotProductAttention accepts (src/ops/cuda/sequence.cu:451-472), where a tensor-core product
-// (fp16 or tf32 operands) could not hold the 1e-5 parity bound.  Before this kernel those shapes ran
-// row by row on the decode kernels, which re-read K and V once per query row.
+// tensor-core kernels do not take: FLOAT32 heads above 128 and the smallest FLOAT32 prompts, FLOAT16 head sizes that are not a
+// multiple of 8, unaligned tensors, and the FLOAT32 inputs that have no exact bf16 parts (see prefill_f32.cu).
 //
 // One CTA per (block of query rows, KV head): the `group` query heads of the KV head times the rows
 // of the block make 64 virtual rows that share every staged K / V tile.  Per tile of 64 keys:
@@ -41,7 +39,19 @@ struct TiledParams {
   int sq, hq, hkv, group, skv, causal, d;
   int bq;  // query rows per CTA: virtual rows / group
   float scale;
+  // not null: only the KV heads of which some flag is set are computed.  kv_flags: kv_tiles per head for the keys, then for
+  // the values; q_flags: q_blocks per query head
+  const uint32_t *kv_flags, *q_flags;
+  int kv_tiles, q_blocks;
 };
+
+__device__ __forceinline__ bool tp_flagged(const TiledParams &p, int hk) {
+  int any = 0;
+  for (int i = threadIdx.x; i < p.kv_tiles; i += kTpThreads)
+    any |= p.kv_flags[(size_t)hk * p.kv_tiles + i] | p.kv_flags[((size_t)p.hkv + hk) * p.kv_tiles + i];
+  for (int i = threadIdx.x; i < p.group * p.q_blocks; i += kTpThreads) any |= p.q_flags[(size_t)hk * p.group * p.q_blocks + i];
+  return __syncthreads_or(any);
+}
 
 template <typename T>
 __device__ __forceinline__ float tp_f32(T v);
@@ -71,6 +81,7 @@ sdpa_tiled_kernel(const TiledParams p) {
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   // heaviest blocks first under the causal mask
   const int qb = gridDim.x - 1 - blockIdx.x, hk = blockIdx.y;
+  if (p.kv_flags && !tp_flagged(p, hk)) return;
   const int q0 = qb * p.bq;
   const T *qg = reinterpret_cast<const T *>(p.q), *kg = reinterpret_cast<const T *>(p.k),
           *vg = reinterpret_cast<const T *>(p.v);
@@ -298,9 +309,9 @@ int tp_dispatch_cols(const TiledParams &p, cudaStream_t st) {
 }
 }  // namespace
 
-int sdpa_tiled(const void *q, const void *k, const void *v, void *out, int sq, int hq, int hkv, int d, int64_t skv,
-               int is_causal, int dtype, cudaStream_t st) {
-  TiledParams p{};
+namespace {
+int tp_run(const void *q, const void *k, const void *v, void *out, int sq, int hq, int hkv, int d, int64_t skv, int is_causal,
+           int dtype, TiledParams p, cudaStream_t st) {
   p.q = q;
   p.k = k;
   p.v = v;
@@ -319,6 +330,24 @@ int sdpa_tiled(const void *q, const void *k, const void *v, void *out, int sq, i
   if (dtype == AXB200_FLOAT32)
     return big ? tp_dispatch_cols<float, 128, 4>(p, st) : tp_dispatch_cols<float, 64, 2>(p, st);
   return big ? tp_dispatch_cols<__half, 128, 4>(p, st) : tp_dispatch_cols<__half, 64, 2>(p, st);
+}
+}  // namespace
+
+int sdpa_tiled(const void *q, const void *k, const void *v, void *out, int sq, int hq, int hkv, int d, int64_t skv,
+               int is_causal, int dtype, cudaStream_t st) {
+  return tp_run(q, k, v, out, sq, hq, hkv, d, skv, is_causal, dtype, TiledParams{}, st);
+}
+
+// FLOAT32, only the KV heads that some flag names (see TiledParams).
+int sdpa_tiled_flagged(const void *q, const void *k, const void *v, void *out, int sq, int hq, int hkv, int d, int64_t skv,
+                       int is_causal, const uint32_t *kv_flags, int kv_tiles, const uint32_t *q_flags, int q_blocks,
+                       cudaStream_t st) {
+  TiledParams p{};
+  p.kv_flags = kv_flags;
+  p.kv_tiles = kv_tiles;
+  p.q_flags = q_flags;
+  p.q_blocks = q_blocks;
+  return tp_run(q, k, v, out, sq, hq, hkv, d, skv, is_causal, AXB200_FLOAT32, p, st);
 }
 
 }  // namespace axb

@@ -36,3 +36,48 @@ def test_fp16_narrow_heads_on_tensor_cores(d, sq, skv):
             err = (out - ref).abs()
             assert (err <= ref.abs() * 2.0 ** -11 + ref.abs().max() * 2.0 ** -20).all(), (causal, hq, err.max())
     assert ops.last_error() == 0
+
+
+def by_fma(q, k, v, causal):
+    """The same through the kernel that a call without scratch takes."""
+    from axono_b200 import _capi
+
+    lib, out = _capi.lib(), torch.empty_like(q)
+    st = lib.axb200_sdpa(q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), q.shape[0], q.shape[1], k.shape[1], q.shape[2],
+                         k.shape[0], int(causal), _capi.FLOAT32, None, 0, torch.cuda.current_stream().cuda_stream)
+    assert st == 0
+    return out
+
+
+@pytest.mark.parametrize("d", [4, 20, 64, 68, 80, 128])
+@pytest.mark.parametrize("sq,skv", [(16, 64), (16, 129), (128, 66), (127, 129), (129, 128), (300, 511), (1030, 1100)])
+def test_fp32_on_tensor_cores(d, sq, skv):
+    """A score is off by 2^-21 of the largest one (its sum of products and its exponent), which changes a weight by as much;
+    sums over keys and the result by 2^-20."""
+    from axono_b200 import ops
+
+    for causal in (True, False):
+        for hq, hkv, spread in ((4, 2, 1.0), (3, 3, 6.0)):
+            q, k, v = tensors(sq, skv, hq, hkv, d, torch.float32, spread)
+            out = ops.scaled_dot_product_attention(q, k, v, causal).double()
+            ref = attention(q, k, v, causal)
+            top = (torch.einsum("qhd,khd->hqk", q, k.repeat_interleave(hq // hkv, 1)).abs().max() * d ** -0.5).item()
+            err = (out - ref).abs().max().item()
+            assert err <= v.abs().max().item() * (2 * top * 2.0 ** -21 + 2.0 ** -20), (causal, hq, err)
+    assert ops.last_error() == 0
+
+
+@pytest.mark.parametrize("d", [64, 128])
+def test_fp32_values_without_three_parts(d):
+    """Infinities, NaN, the largest floats and subnormal ones: heads that hold them come out as from the FMA kernel."""
+    from axono_b200 import ops
+
+    for causal in (True, False):
+        q, k, v = tensors(200, 260, 8, 4, d, torch.float32)
+        k[70, 0, 3] = float("-inf")
+        v[199, 1, 2] = 1e-39
+        v[10, 2, 0] = float("nan")
+        q[150, 7, 1] = 3.4e38  # a head of KV head 3
+        out, ref = ops.scaled_dot_product_attention(q, k, v, causal), by_fma(q, k, v, causal)
+        assert torch.equal(torch.nan_to_num(out, 9e9, 8e9, 7e9), torch.nan_to_num(ref, 9e9, 8e9, 7e9))
+    assert ops.last_error() == 0
