@@ -24,6 +24,7 @@ constexpr int kMTile = 128, kKTile = 64, kATile = kMTile * kKTile * 2;
 template <int kN>
 struct Shape {
   static constexpr int kBTile = kN * kKTile * 2;
+  static constexpr int kBox = kN < 64 ? kN : 64;  // rows per load
   static constexpr int kStageBytes = 2 * kATile + kBTile;
   static constexpr int kStages = kN <= 32 ? 3 : kN == 64 ? 5 : kN == 128 ? 4 : 3;
   static constexpr int kCtasPerSm = kN <= 32 ? 2 : 1;
@@ -61,6 +62,10 @@ moe_umma_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__
   int4 tile;  // expert, first row, rows
   if (m0 >= p.out || !moe_tile(p, shared ? blockIdx.y : blockIdx.y - up.shared_tiles, kN, tile)) return;
   const int steps = (p.in + kKTile - 1) / kKTile;
+  // A tile takes the columns and the loads that its rows need: the last tile of an expert is rarely full (187 rows per expert in
+  // tiles of 256: 27 % of the products and a quarter of the operand traffic of whole tiles went to other experts' rows;
+  // 12000 routed rows of 2048 x 1408: gate and up 234 us, down 142; now 207 and 116).
+  const int cols = (tile.z + 15) & ~15, boxes = (cols + S::kBox - 1) / S::kBox;
 
   if (threadIdx.x == 0) {
     for (int i = 0; i < 2 * S::kStages + 1; ++i) mbar_init(&full[i], 1);
@@ -87,10 +92,11 @@ moe_umma_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__
         const int s = k % S::kStages;
         if (k >= S::kStages && !mbar_wait_bounded(&empty[s], (k / S::kStages - 1) & 1, abort_flag, p.wait_ns)) break;
         uint8_t *dst = smem + s * S::kStageBytes;
-        mbar_arrive_expect_tx(&full[s], S::kStageBytes);
+        mbar_arrive_expect_tx(&full[s], 2 * kATile + boxes * (S::kBox * kKTile * 2));
         tma_load_3d(dst, mw, &full[s], k * kKTile, m0, mat0);
         tma_load_3d(dst + kATile, mw, &full[s], k * kKTile, row1, mat1);
-        tma_load_2d(dst + 2 * kATile, mx, &full[s], k * kKTile, tile.y);
+        for (int b = 0; b < boxes; ++b)
+          tma_load_2d(dst + 2 * kATile + b * (S::kBox * kKTile * 2), mx, &full[s], k * kKTile, tile.y + b * S::kBox);
       }
       // after a wait that ran out: no copy may still be on its way when the CTA leaves
       if (*abort_flag)
@@ -101,8 +107,8 @@ moe_umma_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__
   } else if (warp == kMmaWarp) {
     const uint32_t lead = lane == 0;  // the warp walks, one lane issues
     {
-      // fp32 accumulate, bf16 operands, both K-major, M = 128, N = kN
-      constexpr uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(kN >> 3) << 17) | ((kMTile >> 4) << 24);
+      // fp32 accumulate, bf16 operands, both K-major, M = 128, N = the tile's rows to a multiple of 16
+      const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(cols >> 3) << 17) | ((kMTile >> 4) << 24);
       const uint64_t base = smem_desc(smem_u32(smem), 16, 1024);
       bool ok = true;
       for (int k = 0; k < steps && ok; ++k) {
@@ -175,7 +181,7 @@ bool maps_of(const MoeProduct &p, bool gate_up, int n_tile, CUtensorMap *w, CUte
   const cuuint64_t ws[2] = {(cuuint64_t)p.in * 2, (cuuint64_t)p.in * p.out * 2};
   const cuuint32_t wb[3] = {kKTile, kMTile, 1};
   const cuuint64_t xd[2] = {(cuuint64_t)p.in, (cuuint64_t)p.rows}, xs[1] = {(cuuint64_t)p.in * 2};
-  const cuuint32_t xb[2] = {kKTile, (cuuint32_t)n_tile};
+  const cuuint32_t xb[2] = {kKTile, (cuuint32_t)(n_tile < 64 ? n_tile : 64)};
   return encode(w, p.w, 3, wd, ws, wb) && encode(x, p.x, 2, xd, xs, xb);
 }
 
