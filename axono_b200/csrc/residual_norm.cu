@@ -73,7 +73,22 @@ __global__ void __launch_bounds__(kThreads) residual_layer_norm_kernel(const Res
       for (int i = 0; i < kVec; ++i) add[i] += t[i];
     }
     if (p.expert_rows) {
-      for (int k = 0; k < p.top; ++k) {
+      // four rows at a time: one after the other, a row's address and then the row were waited for `top` times
+      // (2000 rows of 2048, 6 experts: 33.7 us, now 32.1, its start under the kernel before included)
+      int k = 0;
+      for (; k + 4 <= p.top; k += 4) {
+        float wt[4], e[4][kVec];
+        int at[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) wt[u] = p.weight[r * p.top + k + u], at[u] = p.slot[r * p.top + k + u];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) load_vec<kVec>(p.expert_rows + (size_t)at[u] * p.width + c, e[u]);
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+#pragma unroll
+          for (int i = 0; i < kVec; ++i) add[i] = fmaf(wt[u], e[u][i], add[i]);
+      }
+      for (; k < p.top; ++k) {
         const float wt = p.weight[r * p.top + k];
         load_vec<kVec>(p.expert_rows + (size_t)p.slot[r * p.top + k] * p.width + c, t);
 #pragma unroll
