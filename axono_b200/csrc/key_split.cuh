@@ -1,0 +1,143 @@
+// Blocks of query rows whose keys are divided among several CTAs, and the kernel that joins their partial results.
+//
+// The blocks of a prompt are few (a block is 256 rows of a head) and, under a causal mask, of very different length, so that
+// the last of them leave most SMs without work: 2700 rows of 16 heads are 176 blocks, one full wave and 28 more that
+// take as long again.  A plan divides the blocks that would run alone; the parts leave un-normalised sums, their maxima and
+// denominators in scratch memory.
+#pragma once
+
+#include <math.h>
+
+#include "common.cuh"
+
+namespace axb {
+
+constexpr int kMostUnits = 448, kSms = 148;
+
+// What CTAs work on, per head: unit u is part `part` of `parts` of row block `block`.  units == 0: blocks as they are.
+struct KeySplit {
+  int units;
+  uint16_t block[kMostUnits];
+  uint8_t part[kMostUnits], parts[kMostUnits];
+};
+
+// The first tile of part i of n.
+__host__ __device__ inline int split_begin(int tiles, int part, int parts) { return (int)((int64_t)tiles * part / parts); }
+
+// Tiles in a row that a division has to save: joining takes 4 to 6 us with its launch, a tile of a block about 2.  2000 rows of
+// 8 heads of 128 under a causal mask, 4 tiles saved: 37 us whole, 35 in parts; 4096 rows of 2 heads, 22 saved: 68 and 25.
+constexpr float kLeastGain = 6.f, kPartCost = 1.5f;  // what a part costs beside its tiles, in tiles
+
+// blocks row blocks of `heads` heads; tiles(b) key tiles in block b, not decreasing in b.
+template <typename Tiles>
+KeySplit plan_key_split(int64_t blocks, int heads, bool causal, Tiles tiles) {
+  KeySplit plan;
+  plan.units = 0;
+  if (blocks > kMostUnits || heads > 2 * kSms) return plan;
+  const int most = tiles((int)blocks - 1);
+  int unsplit = 0, parts = 1, limit = 0;
+  if (causal) {
+    // The time of parts of at most `at_most` tiles: the longest where all run at once, else an even share and a short one.
+    const auto estimate = [&](int at_most) {
+      int64_t count = 0, total = 0;
+      int longest = 0;
+      for (int b = 0; b < blocks; ++b) {
+        const int t = tiles(b), n = (t + at_most - 1) / at_most;
+        count += n;
+        total += t;
+        longest = (t + n - 1) / n > longest ? (t + n - 1) / n : longest;
+      }
+      const float alone = longest + kPartCost;
+      if (count * heads <= kSms) return alone;
+      const float even = (total + kPartCost * count) * heads / kSms + (float)total / count + kPartCost;
+      return even > alone ? even : alone;
+    };
+    float best = estimate(most) - kLeastGain;
+    int64_t total = 0;
+    for (int b = 0; b < blocks; ++b) total += tiles(b);
+    const int first = (int)((total * heads + kSms - 1) / kSms);
+    for (int at_most = first < 2 ? 2 : first; at_most < most && at_most < first + 8; ++at_most) {
+      const float time = estimate(at_most);
+      if (time < best) best = time, limit = at_most;
+    }
+    if (limit == 0) return plan;
+  } else {
+    // blocks of one length: whole waves of them as they are, the rest in parts that fill one, two or three rounds of the SMs
+    const int64_t all = blocks * heads, waves = all / kSms;
+    unsplit = (int)(waves * kSms / heads);
+    const int64_t rest = all - (int64_t)unsplit * heads;
+    float best = ((all + kSms - 1) / kSms - waves) * (most + kPartCost) - kLeastGain;
+    for (int rounds = 1; rounds <= 3; ++rounds) {
+      const int64_t n = rest ? rounds * kSms / rest : 0;
+      const float time = n > 1 ? rounds * ((float)most / n + kPartCost) : INFINITY;
+      if (n <= 16 && n * 2 <= most && time < best) best = time, parts = (int)n;
+    }
+    if (parts == 1) return plan;
+  }
+  int units = 0;
+  for (int i = 0; i < blocks; ++i) {
+    const int b = (int)blocks - 1 - i;  // under a causal mask the longest first
+    const int n = causal ? (tiles(b) + limit - 1) / limit : i < unsplit ? 1 : parts;
+    if (units + n > kMostUnits || n > 255) return plan;
+    for (int part = 0; part < n; ++part, ++units) {
+      plan.block[units] = (uint16_t)b;
+      plan.part[units] = (uint8_t)part;
+      plan.parts[units] = (uint8_t)n;
+    }
+  }
+  plan.units = units;
+  return plan;
+}
+
+// Scratch of a plan: per unit and head `rows` rows of d floats, and (maximum, denominator) of each row.
+inline size_t key_split_bytes(const KeySplit &plan, int heads, int rows, int d) {
+  return (size_t)plan.units * heads * rows * (d + 2) * sizeof(float);
+}
+
+struct Partials {
+  float *sums;  // (unit, head, row, d)
+  float2 *ml;   // (unit, head, row): maximum in powers of two (-inf: no key), denominator
+};
+inline Partials partials_at(void *scratch, const KeySplit &plan, int heads, int rows) {
+  Partials p{nullptr, nullptr};
+  if (plan.units == 0) return p;
+  p.ml = static_cast<float2 *>(scratch);
+  p.sums = reinterpret_cast<float *>(p.ml + (size_t)plan.units * heads * rows);
+  return p;
+}
+
+// A warp per row of a divided block: out = sum_i 2^(m_i - m) sums_i / sum_i 2^(m_i - m) l_i.  blockIdx.y: unit (those that are no
+// first part of several leave at once); blockIdx.x: head and 8 rows.  d: a multiple of 4 up to 128.
+template <typename O, int kRowsPerBlock>
+__global__ void __launch_bounds__(256) join_parts_kernel(const __grid_constant__ KeySplit plan, const Partials p, O *out, int sq, int hq, int d) {
+  const int u = blockIdx.y, n = plan.parts[u];
+  if (n == 1 || plan.part[u] != 0) return;
+  grid_dependency_wait();
+  const int h = blockIdx.x / (kRowsPerBlock / 8), row = blockIdx.x % (kRowsPerBlock / 8) * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  const int64_t t = (int64_t)plan.block[u] * kRowsPerBlock + row;
+  if (t >= sq) return;
+  const size_t step = (size_t)hq * kRowsPerBlock, first = ((size_t)u * hq + h) * kRowsPerBlock + row;
+  float m = -INFINITY;
+  for (int i = 0; i < n; ++i) m = fmaxf(m, p.ml[first + i * step].x);
+  float l = 0.f;
+  float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+  for (int i = 0; i < n; ++i) {
+    const float2 ml = p.ml[first + i * step];
+    if (ml.x == -INFINITY && ml.y == 0.f) continue;  // no key, and perhaps nothing stored
+    const float w = exp2f(ml.x - m);
+    l = fmaf(w, ml.y, l);
+    if (lane * 4 < d) {
+      const float4 v = *reinterpret_cast<const float4 *>(p.sums + (first + i * step) * d + lane * 4);
+      acc.x = fmaf(w, v.x, acc.x), acc.y = fmaf(w, v.y, acc.y), acc.z = fmaf(w, v.z, acc.z), acc.w = fmaf(w, v.w, acc.w);
+    }
+  }
+  if (lane * 4 >= d) return;
+  const float inv = l > 0.f ? 1.0f / l : 0.f;
+  O *dst = out + ((size_t)t * hq + h) * d + lane * 4;
+  stf(dst, acc.x * inv);
+  stf(dst + 1, acc.y * inv);
+  stf(dst + 2, acc.z * inv);
+  stf(dst + 3, acc.w * inv);
+}
+
+}  // namespace axb

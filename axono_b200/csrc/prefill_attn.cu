@@ -23,6 +23,7 @@
 
 #include <mutex>
 
+#include "key_split.cuh"
 #include "tcgen05.cuh"
 
 namespace axb {
@@ -359,11 +360,12 @@ __device__ __forceinline__ uint32_t split_half2(float a, float b, uint32_t &lo) 
 // out - Q.K^T does not step into it, and the columns of O that P.V forms from whatever stands there are never stored.
 // P.V keeps N = 128 whatever the head size: products of one shape need no wait between P.V and the S that overwrites P.
 // Bound by the products of P.V and the softmax about equally.  2700 x 2700 keys, 16 heads of 64, not causal:
-// 111 us against 1921 us on the FMA pipe, the same error against 64 bits (2.1e-4, the rounding of the result).
+// 111 us (91 with the last blocks divided, key_split.cuh) against 1921 us on the FMA pipe, the same error against 64 bits (2.1e-4, the rounding of the result).
 template <bool kNarrow>
 __global__ void __launch_bounds__(kPairThreads, 1)
 prefill_attn_f16_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
-                             const __grid_constant__ CUtensorMap tmV, const PrefillParams p) {
+                             const __grid_constant__ CUtensorMap tmV, const PrefillParams p, const __grid_constant__ KeySplit split,
+                             const Partials partials) {
   extern __shared__ __align__(1024) uint8_t smem[];
   uint64_t *bars = reinterpret_cast<uint64_t *>(smem + kPairOffBar);
   // K/V tiles travel in pairs (V_j, K_{j+1}) - what one key-tile step of the MMA warp consumes - under
@@ -380,7 +382,10 @@ prefill_attn_f16_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __gr
     return;
   }
   // heaviest blocks of all heads first: under a causal mask the last query block has the most key tiles
-  const int h = blockIdx.x % p.hq, qb = (gridDim.x - 1 - blockIdx.x) / p.hq;
+  // (or in the plan's order, where keys are divided)
+  const int h = blockIdx.x % p.hq, unit = blockIdx.x / p.hq;
+  const int qb = split.units ? split.block[unit] : (int)((gridDim.x - 1 - blockIdx.x) / p.hq);
+  const int parts = split.units ? split.parts[unit] : 1;
   const int hk = h / (p.hq / p.hkv);
   const int q0 = qb * 2 * kBlockM;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -394,7 +399,14 @@ prefill_attn_f16_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __gr
     const int kv_end_max = p.causal ? min(t_last + 1, p.skv) : p.skv;
     nkv_g[g] = first < p.sq ? (kv_end_max + kPairN - 1) / kPairN : 0;
   }
-  const int nkv = max(nkv_g[0], nkv_g[1]);
+  int nkv = max(nkv_g[0], nkv_g[1]), tile0 = 0;
+  if (parts > 1) {
+    const int part = split.part[unit], end = split_begin(nkv, part + 1, parts);
+    tile0 = split_begin(nkv, part, parts);
+#pragma unroll
+    for (int g = 0; g < 2; ++g) nkv_g[g] = max(0, min(nkv_g[g], end) - tile0);
+    nkv = end - tile0;
+  }
 
   if (threadIdx.x == 0) {
     for (int i = 0; i < 9; ++i) mbar_init(&bars[i], 1);
@@ -428,7 +440,7 @@ prefill_attn_f16_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __gr
 #pragma unroll
       for (int g = 0; g < 2; ++g)  // rows past sq are zero-filled
         load_tile(smem + kPairOffQ + g * kPairTileBytes, &tmQ, bar_q, h, q0 + g * kBlockM);
-      load_tile(smem + kPairOffK, &tmK, bar_q, hk, 0);
+      load_tile(smem + kPairOffK, &tmK, bar_q, hk, tile0 * kPairN);
       bool ok = true;
       for (int j = 0; j < nkv && ok; ++j) {  // pair j: V_j into V stage j & 1, K_{j+1} into K stage (j+1) & 1
         const int s = j & 1;
@@ -439,8 +451,8 @@ prefill_attn_f16_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __gr
         const bool with_k = j + 1 < nkv;
         mbar_arrive_expect_tx(&full_kv[s], with_k ? 2 * tile_bytes : tile_bytes);
         if (with_k)  // first: S_g(j+1) is what the softmax warps wait for
-          load_tile(smem + kPairOffK + (s ^ 1) * kPairTileBytes, &tmK, &full_kv[s], hk, (j + 1) * kPairN);
-        load_tile(smem + kPairOffV + s * kPairTileBytes, &tmV, &full_kv[s], hk, j * kPairN);
+          load_tile(smem + kPairOffK + (s ^ 1) * kPairTileBytes, &tmK, &full_kv[s], hk, (tile0 + j + 1) * kPairN);
+        load_tile(smem + kPairOffV + s * kPairTileBytes, &tmV, &full_kv[s], hk, (tile0 + j) * kPairN);
       }
     }
   } else if (warp == kPairMmaWarp) {
@@ -515,7 +527,7 @@ prefill_attn_f16_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __gr
 #pragma unroll
       for (int c = 0; c < 4; ++c) tmem_ld32_async(tmem_s + c * 32, sr[c]);
       tmem_wait_ld();
-      const int n0 = j * kPairN;
+      const int n0 = (tile0 + j) * kPairN;
       if (n0 + kPairN > kv_end) {
 #pragma unroll
         for (int c = 0; c < 4; ++c)
@@ -574,7 +586,27 @@ prefill_attn_f16_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __gr
     // ---- epilogue: O / l -> out ----
     if (ok && my_nkv > 0) ok = __all_sync(0xffffffffu, mbar_wait_bounded(&bar_fin[g], 0, abort_flag));
     tc_fence_after();
-    if (ok && my_nkv > 0) {
+    if (parts > 1) {
+      const size_t at = ((size_t)unit * p.hq + h) * (2 * kBlockM) + g * kBlockM + row;
+      const bool any = ok && my_nkv > 0;
+      if (t_row < p.sq) partials.ml[at] = any ? make_float2(m_run, l_run) : make_float2(-INFINITY, 0.f);
+      if (any) {
+        float *dst = partials.sums + at * p.d;
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+          if (kNarrow && c * 32 >= p.d) break;
+          uint32_t r[32];
+          tmem_ld32(tmem_o + c * 32, r);
+          if (t_row < p.sq) {
+#pragma unroll
+            for (int u = 0; u < 8; ++u) {
+              if (kNarrow && c * 32 + u * 4 >= p.d) break;
+              *reinterpret_cast<uint4 *>(dst + c * 32 + u * 4) = make_uint4(r[u * 4], r[u * 4 + 1], r[u * 4 + 2], r[u * 4 + 3]);
+            }
+          }
+        }
+      }
+    } else if (ok && my_nkv > 0) {
       const float inv = l_run > 0.f ? 1.0f / l_run : 0.f;
       __half *dst = reinterpret_cast<__half *>(p.out) + ((size_t)t_row * p.hq + h) * (kNarrow ? p.d : kD);
 #pragma unroll
@@ -616,6 +648,21 @@ bool rows_map(CUtensorMap *map, const void *base, int64_t rows, int heads, int d
             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
+// The 256-row form's plan.
+KeySplit pair_plan(int sq, int hq, int64_t skv, int is_causal) {
+  const auto tiles = [&](int b) {
+    const int64_t last = ((int64_t)b + 1) * 2 * kBlockM, end = last < sq ? last : sq;
+    return (int)(((is_causal && end < skv ? end : skv) + kPairN - 1) / kPairN);
+  };
+  return plan_key_split(((int64_t)sq + 2 * kBlockM - 1) / (2 * kBlockM), hq, is_causal != 0, tiles);
+}
+
+// Heads below 128 in prompts: a TMA row is a multiple of 16 bytes, and below 16 rows (of 128 that a tile holds) the
+// row-by-row form is the cheaper one.
+bool narrow_heads(int sq, int d) { return d < kD && d % 8 == 0 && sq >= 16; }
+// 256 query rows per CTA once there are that many; the 128-row form (heads of 128 only) below that.
+bool pair_form(int sq, int d) { return narrow_heads(sq, d) || (d == kD && sq >= 2 * kBlockM); }
+
 bool aligned16(const void *p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
 
 }  // namespace
@@ -627,9 +674,15 @@ size_t axb200_sdpa_workspace_bytes(int sq, int hq, int hkv, int d, int64_t skv, 
   // the tensor-core kernels and the tiled FMA kernel keep everything on chip; only the row-by-row
   // evaluation on the decode kernels needs room for partials
   // (whatever the tensor-core path does not take - unaligned pointers, say - the tiled kernel does)
-  if (hkv > 0 && hq % hkv == 0 && axb::sdpa_tiled_supported(sq, hq, hkv, d, skv))
-    return dtype == AXB200_FLOAT32 ? axb::sdpa_split_workspace_bytes(sq, hq, hkv, d, skv) : 0;
-  return axb::sdpa_rows_workspace_bytes(sq, hq, hkv, d, skv);
+  const bool tiled = hkv > 0 && hq % hkv == 0 && axb::sdpa_tiled_supported(sq, hq, hkv, d, skv);
+  if (tiled && dtype == AXB200_FLOAT32) return axb::sdpa_split_workspace_bytes(sq, hq, hkv, d, skv);
+  size_t most = tiled ? 0 : axb::sdpa_rows_workspace_bytes(sq, hq, hkv, d, skv);
+  if (dtype == AXB200_FLOAT16 && sq > 0 && hq > 0 && skv > 0 && axb::pair_form(sq, d))
+    for (int causal = 0; causal < 2; ++causal) {  // the caller does not name the mask here
+      const size_t n = axb::key_split_bytes(axb::pair_plan(sq, hq, skv, causal), hq, 2 * axb::kBlockM, d);
+      most = n > most ? n : most;
+    }
+  return most;
 }
 
 int axb200_sdpa(const void *q, const void *k, const void *v, void *out, int sq, int hq, int hkv, int d,
@@ -639,9 +692,7 @@ int axb200_sdpa(const void *q, const void *k, const void *v, void *out, int sq, 
   if (sq <= 0 || hq <= 0 || hkv <= 0 || d <= 0 || skv <= 0 || skv > 0x7fffffff - 4096) return AXB200_INVALID_ARGUMENT;
   if (hq % hkv != 0) return AXB200_SHAPE_MISMATCH;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  // fp16 heads of 128, and prompts of narrower heads: a TMA row is a multiple of 16 bytes, and below 16 rows (of 128 that a
-  // tile holds) the row-by-row form is the cheaper one
-  const bool narrow = d < axb::kD && d % 8 == 0 && sq >= 16;
+  const bool narrow = axb::narrow_heads(sq, d);
   const bool tensor_path = dtype == AXB200_FLOAT16 && (d == axb::kD || narrow) && hq <= 65535 && axb::aligned16(q) &&
                            axb::aligned16(k) && axb::aligned16(v) && axb::aligned16(out) && axb::tensor_map_encoder();
   if (!tensor_path) {
@@ -654,8 +705,7 @@ int axb200_sdpa(const void *q, const void *k, const void *v, void *out, int sq, 
       return axb::sdpa_tiled(q, k, v, out, sq, hq, hkv, d, skv, is_causal, dtype, st);
     return axb::sdpa_rows_fallback(q, k, v, out, sq, hq, hkv, d, skv, is_causal, dtype, workspace, workspace_bytes, st);
   }
-  // 256 query rows per CTA once there are that many; the 128-row form (heads of 128 only) below that
-  const bool pair = narrow || sq >= 2 * axb::kBlockM;
+  const bool pair = axb::pair_form(sq, d);
   const int kv_box = pair ? axb::kPairN : axb::kBlockN;
   CUtensorMap mq, mk, mv;
   if (!axb::rows_map(&mq, q, sq, hq, d, axb::kBlockM) || !axb::rows_map(&mk, k, skv, hkv, d, kv_box) ||
@@ -688,9 +738,17 @@ int axb200_sdpa(const void *q, const void *k, const void *v, void *out, int sq, 
   p.d = d;
   p.scale_log2 = (1.0f / sqrtf((float)d)) * axb::kLog2e;
   if (pair) {
-    const dim3 grid((unsigned)hq * ((sq + 2 * axb::kBlockM - 1) / (2 * axb::kBlockM)));
+    axb::KeySplit split = axb::pair_plan(sq, hq, skv, is_causal);
+    if (split.units && (!workspace || !axb::aligned16(workspace) || workspace_bytes < axb::key_split_bytes(split, hq, 2 * axb::kBlockM, d)))
+      split.units = 0;
+    const axb::Partials partials = axb::partials_at(workspace, split, hq, 2 * axb::kBlockM);
+    const dim3 grid((unsigned)hq * (split.units ? split.units : (sq + 2 * axb::kBlockM - 1) / (2 * axb::kBlockM)));
     auto *kernel = narrow ? axb::prefill_attn_f16_pair_kernel<true> : axb::prefill_attn_f16_pair_kernel<false>;
-    kernel<<<grid, axb::kPairThreads, axb::kPairSmemBytes, st>>>(mq, mk, mv, p);
+    kernel<<<grid, axb::kPairThreads, axb::kPairSmemBytes, st>>>(mq, mk, mv, p, split, partials);
+    if (split.units && cudaPeekAtLastError() == cudaSuccess)
+      return axb::launch_dependent(axb::join_parts_kernel<__half, 2 * axb::kBlockM>,
+                                   dim3((unsigned)hq * (2 * axb::kBlockM / 8), split.units), dim3(256), 0, st, split, partials,
+                                   static_cast<__half *>(out), sq, hq, d);
   } else {
     const dim3 grid((sq + axb::kBlockM - 1) / axb::kBlockM, hq);
     axb::prefill_attn_f16_kernel<<<grid, axb::kThreads, axb::kSmemBytes, st>>>(mq, mk, mv, p);

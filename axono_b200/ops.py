@@ -552,10 +552,10 @@ def scaled_dot_product_attention(q, k, v, is_causal: bool = False):
     q, k, v = _c(q), _c(k), _c(v)
     out = torch.empty_like(q)
     lib = _capi.lib()
-    # of this call alone: calls on several streams may overlap
-    ws = torch.empty(lib.axb200_sdpa_workspace_bytes(sq, hq, hkv, d, skv, dt), dtype=torch.uint8, device=q.device)
+    need = lib.axb200_sdpa_workspace_bytes(sq, hq, hkv, d, skv, dt)
+    ws = torch.empty(need, dtype=torch.uint8, device=q.device) if need else None  # of this call alone: streams may overlap
     _call(lib.axb200_sdpa(q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), sq, hq, hkv, d, skv,
-                          int(bool(is_causal)), dt, ws.data_ptr(), ws.numel(), _stream(q)), op)
+                          int(bool(is_causal)), dt, ws.data_ptr() if need else None, need, _stream(q)), op)
     return out
 
 

@@ -38,13 +38,13 @@ def test_fp16_narrow_heads_on_tensor_cores(d, sq, skv):
     assert ops.last_error() == 0
 
 
-def by_fma(q, k, v, causal):
-    """The same through the kernel that a call without scratch takes."""
+def without_scratch(q, k, v, causal):
+    """The same through the kernels that a call without scratch takes: FMA kernel in fp32, whole blocks in fp16."""
     from axono_b200 import _capi
 
     lib, out = _capi.lib(), torch.empty_like(q)
     st = lib.axb200_sdpa(q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), q.shape[0], q.shape[1], k.shape[1], q.shape[2],
-                         k.shape[0], int(causal), _capi.FLOAT32, None, 0, torch.cuda.current_stream().cuda_stream)
+                         k.shape[0], int(causal), _capi.FLOAT32 if q.dtype == torch.float32 else _capi.FLOAT16, None, 0, torch.cuda.current_stream().cuda_stream)
     assert st == 0
     return out
 
@@ -78,6 +78,28 @@ def test_fp32_values_without_three_parts(d):
         v[199, 1, 2] = 1e-39
         v[10, 2, 0] = float("nan")
         q[150, 7, 1] = 3.4e38  # a head of KV head 3
-        out, ref = ops.scaled_dot_product_attention(q, k, v, causal), by_fma(q, k, v, causal)
+        out, ref = ops.scaled_dot_product_attention(q, k, v, causal), without_scratch(q, k, v, causal)
         assert torch.equal(torch.nan_to_num(out, 9e9, 8e9, 7e9), torch.nan_to_num(ref, 9e9, 8e9, 7e9))
+    assert ops.last_error() == 0
+
+
+@pytest.mark.parametrize("d", [8, 64, 128])
+@pytest.mark.parametrize("sq,skv,hq,hkv", [(256, 4100, 2, 1), (300, 1500, 3, 3), (1300, 1300, 2, 2), (2700, 2700, 16, 8),
+                                           (2305, 900, 16, 16), (3000, 3100, 4, 2)])
+def test_fp16_keys_divided_among_blocks(d, sq, skv, hq, hkv):
+    """Blocks of rows whose keys several CTAs share: the parts of a row are joined in fp32.  The result's rounding is 2^-11 of
+    it; a weight is off by 2^-21 of the largest score (its sum of products and its exponent) and, for heads of 128, by its
+    rounding to fp16, 2^-11; and a small weight, as multiples of 2^-24 of a sum that is at least one, by 2^-25.  The same
+    bound for undivided blocks."""
+    from axono_b200 import ops
+
+    for causal in (True, False):
+        q, k, v = tensors(sq, skv, hq, hkv, d, torch.float16, 3.0)
+        ref, mass = attention(q, k, v, causal), attention(q, k, v.abs(), causal)
+        top = (torch.einsum("qhd,khd->hqk", q.float(), k.float().repeat_interleave(hq // hkv, 1)).abs().max() * d ** -0.5).item()
+        weight = 2 * top * 2.0 ** -21 + 2.0 ** -20 + (2.0 ** -11 if d == 128 else 0.0)
+        for out in (ops.scaled_dot_product_attention(q, k, v, causal), without_scratch(q, k, v, causal)):
+            err = (out.double() - ref).abs()
+            small = 2.0 ** -25 * v.double().abs().sum(0).repeat_interleave(hq // hkv, 0)
+            assert (err <= ref.abs() * 2.0 ** -11 + weight * mass + small + 2.0 ** -24).all(), (causal, err.max())
     assert ops.last_error() == 0
