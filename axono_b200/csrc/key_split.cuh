@@ -1,6 +1,6 @@
 // Blocks of query rows whose keys are divided among several CTAs, and the kernel that joins their partial results.
 //
-// The blocks of a prompt are few (a block is 256 rows of a head) and, under a causal mask, of very different length, so that
+// The blocks of a prompt are few (a block is 128 or 256 rows of a head) and, under a causal mask, of very different length, so that
 // the last of them leave most SMs without work: 2700 rows of 16 heads are 176 blocks, one full wave and 28 more that
 // take as long again.  A plan divides the blocks that would run alone; the parts leave un-normalised sums, their maxima and
 // denominators in scratch memory.
@@ -24,35 +24,33 @@ struct KeySplit {
 // The first tile of part i of n.
 __host__ __device__ inline int split_begin(int tiles, int part, int parts) { return (int)((int64_t)tiles * part / parts); }
 
-// Tiles in a row that a division has to save: joining takes 4 to 6 us with its launch, a tile of a block about 2.  2000 rows of
-// 8 heads of 128 under a causal mask, 4 tiles saved: 37 us whole, 35 in parts; 4096 rows of 2 heads, 22 saved: 68 and 25.
-constexpr float kLeastGain = 6.f, kPartCost = 1.5f;  // what a part costs beside its tiles, in tiles
-
-// blocks row blocks of `heads` heads; tiles(b) key tiles in block b, not decreasing in b.
+// blocks row blocks of `heads` heads; tiles(b) key tiles in block b, not decreasing in b; part_cost: what a block or part costs beside
+// its tiles, in tiles; least_gain: tiles in a row that a division has to save, as many as joining takes (4 to 6 us with its launch).
 template <typename Tiles>
-KeySplit plan_key_split(int64_t blocks, int heads, bool causal, Tiles tiles) {
+KeySplit plan_key_split(int64_t blocks, int heads, bool causal, float part_cost, float least_gain, Tiles tiles) {
   KeySplit plan;
   plan.units = 0;
   if (blocks > kMostUnits || heads > 2 * kSms) return plan;
   const int most = tiles((int)blocks - 1);
   int unsplit = 0, parts = 1, limit = 0;
   if (causal) {
-    // The time of parts of at most `at_most` tiles: the longest where all run at once, else an even share and a short one.
+    // The time of parts of at most `at_most` tiles: the longest where all run at once, else an even share and half of the last.
     const auto estimate = [&](int at_most) {
       int64_t count = 0, total = 0;
-      int longest = 0;
+      int longest = 0, shortest = most;
       for (int b = 0; b < blocks; ++b) {
         const int t = tiles(b), n = (t + at_most - 1) / at_most;
         count += n;
         total += t;
         longest = (t + n - 1) / n > longest ? (t + n - 1) / n : longest;
+        shortest = t / n < shortest ? t / n : shortest;
       }
-      const float alone = longest + kPartCost;
+      const float alone = longest + part_cost;
       if (count * heads <= kSms) return alone;
-      const float even = (total + kPartCost * count) * heads / kSms + (float)total / count + kPartCost;
+      const float even = (total + part_cost * count) * heads / kSms + (shortest + part_cost) / 2;
       return even > alone ? even : alone;
     };
-    float best = estimate(most) - kLeastGain;
+    float best = estimate(most) - least_gain;
     int64_t total = 0;
     for (int b = 0; b < blocks; ++b) total += tiles(b);
     const int first = (int)((total * heads + kSms - 1) / kSms);
@@ -66,11 +64,13 @@ KeySplit plan_key_split(int64_t blocks, int heads, bool causal, Tiles tiles) {
     const int64_t all = blocks * heads, waves = all / kSms;
     unsplit = (int)(waves * kSms / heads);
     const int64_t rest = all - (int64_t)unsplit * heads;
-    float best = ((all + kSms - 1) / kSms - waves) * (most + kPartCost) - kLeastGain;
+    float best = ((all + kSms - 1) / kSms - waves) * (most + part_cost) - least_gain;
     for (int rounds = 1; rounds <= 3; ++rounds) {
-      const int64_t n = rest ? rounds * kSms / rest : 0;
-      const float time = n > 1 ? rounds * ((float)most / n + kPartCost) : INFINITY;
-      if (n <= 16 && n * 2 <= most && time < best) best = time, parts = (int)n;
+      int64_t n = rest ? rounds * kSms / rest : 0;
+      n = n > 16 ? 16 : n;
+      n = n > most / 2 ? most / 2 : n;
+      const float time = n > 1 ? rounds * ((float)most / n + part_cost) : INFINITY;
+      if (time < best) best = time, parts = (int)n;
     }
     if (parts == 1) return plan;
   }

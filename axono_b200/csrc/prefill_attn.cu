@@ -648,13 +648,14 @@ bool rows_map(CUtensorMap *map, const void *base, int64_t rows, int heads, int d
             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-// The 256-row form's plan.
+// The 256-row form's plan; a tile of 128 keys takes about 2 us of a block.  2000 rows of 8 heads of 128 under a causal mask, 4
+// tiles saved: 37 us whole, 35 in parts; 4096 rows of 2 heads, 22 saved: 68 and 25.
 KeySplit pair_plan(int sq, int hq, int64_t skv, int is_causal) {
   const auto tiles = [&](int b) {
     const int64_t last = ((int64_t)b + 1) * 2 * kBlockM, end = last < sq ? last : sq;
     return (int)(((is_causal && end < skv ? end : skv) + kPairN - 1) / kPairN);
   };
-  return plan_key_split(((int64_t)sq + 2 * kBlockM - 1) / (2 * kBlockM), hq, is_causal != 0, tiles);
+  return plan_key_split(((int64_t)sq + 2 * kBlockM - 1) / (2 * kBlockM), hq, is_causal != 0, 1.5f, 6.f, tiles);
 }
 
 // Heads below 128 in prompts: a TMA row is a multiple of 16 bytes, and below 16 rows (of 128 that a tile holds) the

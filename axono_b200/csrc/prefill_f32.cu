@@ -27,6 +27,7 @@
 
 #include <mutex>
 
+#include "key_split.cuh"
 #include "tcgen05.cuh"
 
 namespace axb {
@@ -46,7 +47,7 @@ constexpr size_t kMostScratch = (size_t)2 << 30;  // 170 K tokens of 8 heads of 
 template <int kB>
 struct Layout {
   static constexpr int kPart = kB * kBox, kTile = 3 * kPart;
-  static constexpr int kOffV = 2 * kTile, kOffCorr = 4 * kTile, kOffL = kOffCorr + 2 * kRows * 4, kOffBar = kOffL + kRows * 4;
+  static constexpr int kOffV = 2 * kTile, kOffCorr = 4 * kTile, kOffL = kOffCorr + 2 * kRows * 4, kOffBar = kOffL + 2 * kRows * 4;
   static constexpr int kSmem = kOffBar + 256;
   static constexpr int kQCols = 96 * kB, kSpCols = 96, kColO = kQCols + 2 * kSpCols;
 };
@@ -110,7 +111,7 @@ split_kernel(const Params p) {
 
 template <int kB>
 __global__ void __launch_bounds__(kThreads, 1)
-split_attn_kernel(const Params p) {
+split_attn_kernel(const Params p, const __grid_constant__ KeySplit split, const Partials partials) {
   using L = Layout<kB>;
   extern __shared__ __align__(1024) uint8_t smem[];
   uint64_t *bars = reinterpret_cast<uint64_t *>(smem + L::kOffBar);
@@ -128,11 +129,17 @@ split_attn_kernel(const Params p) {
     if (threadIdx.x == 0) atomicOr(&g_error_word, AXB200_ERR_WAIT_TIMEOUT);
     return;
   }
-  const int h = blockIdx.x % p.hq, qb = (int)((gridDim.x - 1 - blockIdx.x) / p.hq);
+  const int h = blockIdx.x % p.hq, unit = blockIdx.x / p.hq;
+  const int qb = split.units ? split.block[unit] : (int)((gridDim.x - 1 - blockIdx.x) / p.hq);
+  const int parts = split.units ? split.parts[unit] : 1;
   const int hk = h / (p.hq / p.hkv), q0 = qb * kRows;
   const int warp = uniform_warp(), lane = threadIdx.x & 31;
   const int kv_end_max = p.causal ? min(min(q0 + kRows, p.sq), p.skv) : p.skv;
-  const int nkv = (kv_end_max + kKeys - 1) / kKeys;
+  int nkv = (kv_end_max + kKeys - 1) / kKeys, tile0 = 0;
+  if (parts > 1) {
+    tile0 = split_begin(nkv, split.part[unit], parts);
+    nkv = split_begin(nkv, split.part[unit] + 1, parts) - tile0;
+  }
 
   if (threadIdx.x == 0) {
     for (int i = 0; i < 11; ++i) mbar_init(&bars[i], 1);
@@ -184,7 +191,7 @@ split_attn_kernel(const Params p) {
   if (warp == kLoadWarp) {
     if (lane == 0) {
       grid_dependency_wait();  // the tiles
-      const uint8_t *k_tiles = p.tiles + (size_t)hk * p.n_tiles * L::kTile;
+      const uint8_t *k_tiles = p.tiles + ((size_t)hk * p.n_tiles + tile0) * L::kTile;
       const uint8_t *v_tiles = k_tiles + (size_t)p.hkv * p.n_tiles * L::kTile;
       bool ok = true;
       int nk = 0, nv = 0;  // copies begun
@@ -276,7 +283,7 @@ split_attn_kernel(const Params p) {
       tmem_ld32_async(sp, sr[0]);
       tmem_ld32_async(sp + 32, sr[1]);
       tmem_wait_ld();
-      const int n0 = j * kKeys;
+      const int n0 = (tile0 + j) * kKeys;
       if (n0 + kKeys > kv_end) {
 #pragma unroll
         for (int c = 0; c < 2; ++c)
@@ -316,6 +323,7 @@ split_attn_kernel(const Params p) {
       if (lane == 0) mbar_arrive(&bar_p[s]);
     }
     l_s[row] = l_run;
+    l_s[kRows + row] = m_run * p.scale_log2;
     __syncwarp();
     if (lane == 0) mbar_arrive(bar_l);
   } else {
@@ -349,8 +357,15 @@ split_attn_kernel(const Params p) {
     }
     if (ok) ok = mbar_wait_warp(bar_l, 0, abort_flag, p.wait_ns);
     if (ok && t_row < p.sq) {
-      const float l = l_s[row], inv = l > 0.f ? 1.0f / l : 0.f;
+      const float l = l_s[row];
+      float inv = l > 0.f ? 1.0f / l : 0.f;
       float *dst = p.out + ((size_t)t_row * p.hq + h) * p.d;
+      if (parts > 1) {  // un-normalised
+        const size_t at = ((size_t)unit * p.hq + h) * kRows + row;
+        partials.ml[at] = make_float2(l_s[kRows + row], l);
+        dst = partials.sums + at * p.d;
+        inv = 1.f;
+      }
 #pragma unroll
       for (int i = 0; i < 16 * kB; ++i) {
         if (i * 4 >= p.d) break;
@@ -361,17 +376,29 @@ split_attn_kernel(const Params p) {
   }
   tc_fence_before();
   __syncthreads();
-  if (threadIdx.x == 0) p.q_flags[h * p.q_blocks + qb] = *q_bad;
+  if (threadIdx.x == 0) p.q_flags[h * p.q_blocks + qb] = *q_bad;  // the same from every part
   if (warp == kMmaWarp)
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;" ::"r"(tmem) : "memory");
 }
 
 size_t up256(size_t n) { return (n + 255) & ~(size_t)255; }
 int blocks_of(int d) { return d > 64 ? 2 : 1; }
+size_t tile_bytes(int hkv, int64_t n_tiles, int d) { return (size_t)2 * hkv * n_tiles * 3 * blocks_of(d) * kBox; }
 size_t kv_flag_bytes(int hkv, int64_t n_tiles) { return up256((size_t)2 * hkv * n_tiles * 4); }
 
+// A tile of 64 keys takes 2 to 3 us of a block, a block three tiles more (Q's parts, the first copies, the result).  1536 rows of 16
+// heads of 128, not causal: 176 us whole, 140 in parts; 4096 rows of 2 heads, causal: 208 and 91.  Where the SMs are nearly full
+// a division gains nothing (1536 rows of 16 heads, causal: 92 us both, before the joining), hence the five tiles.
+KeySplit split_plan(int sq, int hq, int64_t skv, int is_causal) {
+  const auto tiles = [&](int b) {
+    const int64_t last = ((int64_t)b + 1) * kRows, end = last < sq ? last : sq;
+    return (int)(((is_causal && end < skv ? end : skv) + kKeys - 1) / kKeys);
+  };
+  return plan_key_split(((int64_t)sq + kRows - 1) / kRows, hq, is_causal != 0, 3.f, 5.f, tiles);
+}
+
 template <int kB>
-int launch(const Params &p, cudaStream_t st) {
+int launch(const Params &p, void *parts_at, cudaStream_t st) {
   static std::mutex mu;
   static bool opted[64] = {false};
   int dev = 0;
@@ -386,7 +413,13 @@ int launch(const Params &p, cudaStream_t st) {
   }
   split_kernel<kB><<<dim3(p.n_tiles, p.hkv, 2), kSplitThreads, 0, st>>>(p);
   if (cudaGetLastError() != cudaSuccess) return AXB200_DEVICE_ERROR;
-  return launch_dependent(split_attn_kernel<kB>, dim3((unsigned)p.hq * p.q_blocks), dim3(kThreads), Layout<kB>::kSmem, st, p);
+  const KeySplit split = split_plan(p.sq, p.hq, p.skv, p.causal);
+  const Partials partials = partials_at(parts_at, split, p.hq, kRows);
+  const int rc = launch_dependent(split_attn_kernel<kB>, dim3((unsigned)p.hq * (split.units ? split.units : p.q_blocks)), dim3(kThreads),
+                                  Layout<kB>::kSmem, st, p, split, partials);
+  if (rc != AXB200_OK || split.units == 0) return rc;
+  return launch_dependent(join_parts_kernel<float, kRows>, dim3((unsigned)p.hq * (kRows / 8), split.units), dim3(256), 0, st, split,
+                          partials, p.out, p.sq, p.hq, p.d);
 }
 
 }  // namespace
@@ -399,8 +432,13 @@ size_t sdpa_split_workspace_bytes(int sq, int hq, int hkv, int d, int64_t skv) {
   const int64_t rows = (int64_t)sq * (hq / hkv);
   if (d % 4 || d > 128 || sq < 16 || hkv > 65535 || in_a_row < (rows >= kRows ? 2 : 3)) return 0;
   const int64_t n_tiles = (skv + kKeys - 1) / kKeys, q_blocks = ((int64_t)sq + kRows - 1) / kRows;
+  size_t parts = 0;
+  for (int causal = 0; causal < 2; ++causal) {  // the caller does not name the mask here
+    const size_t n = key_split_bytes(split_plan(sq, hq, skv, causal), hq, kRows, d);
+    parts = n > parts ? n : parts;
+  }
   const size_t total = up256((size_t)hq * q_blocks * 4) + kv_flag_bytes(hkv, n_tiles) +
-                       (size_t)2 * hkv * n_tiles * 3 * blocks_of(d) * kBox;
+                       tile_bytes(hkv, n_tiles, d) + parts;
   return total <= kMostScratch ? total : 0;
 }
 
@@ -427,7 +465,8 @@ int sdpa_split(const void *q, const void *k, const void *v, void *out, int sq, i
   at += up256((size_t)hq * p.q_blocks * 4);
   p.kv_flags = reinterpret_cast<uint32_t *>(at);
   p.tiles = at + kv_flag_bytes(hkv, p.n_tiles);
-  const int status = blocks_of(d) == 2 ? launch<2>(p, st) : launch<1>(p, st);
+  void *parts_at = p.tiles + tile_bytes(hkv, p.n_tiles, d);
+  const int status = blocks_of(d) == 2 ? launch<2>(p, parts_at, st) : launch<1>(p, parts_at, st);
   if (status != AXB200_OK) return status;
   return sdpa_tiled_flagged(q, k, v, out, sq, hq, hkv, d, skv, is_causal, p.kv_flags, p.n_tiles, p.q_flags, p.q_blocks, st);
 }
