@@ -360,7 +360,8 @@ __device__ __forceinline__ uint32_t split_half2(float a, float b, uint32_t &lo) 
 // out - Q.K^T does not step into it, and the columns of O that P.V forms from whatever stands there are never stored.
 // P.V keeps N = 128 whatever the head size: products of one shape need no wait between P.V and the S that overwrites P.
 // Bound by the products of P.V and the softmax about equally.  2700 x 2700 keys, 16 heads of 64, not causal:
-// 111 us (91 with the last blocks divided, key_split.cuh) against 1921 us on the FMA pipe, the same error against 64 bits (2.1e-4, the rounding of the result).
+// 111 us, 91 with the last blocks divided (key_split.cuh), against 1921 us on the FMA pipe; the same error against 64 bits
+// (2.1e-4, the rounding of the result).
 template <bool kNarrow>
 __global__ void __launch_bounds__(kPairThreads, 1)
 prefill_attn_f16_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
@@ -672,9 +673,8 @@ bool aligned16(const void *p) { return (reinterpret_cast<uintptr_t>(p) & 15u) ==
 extern "C" {
 
 size_t axb200_sdpa_workspace_bytes(int sq, int hq, int hkv, int d, int64_t skv, int dtype) {
-  // the tensor-core kernels and the tiled FMA kernel keep everything on chip; only the row-by-row
-  // evaluation on the decode kernels needs room for partials
-  // (whatever the tensor-core path does not take - unaligned pointers, say - the tiled kernel does)
+  // the row-by-row evaluation on the decode kernels needs room for partials, the fp32 form for the tiles of parts, the
+  // 256-row form for what divided blocks leave (without it FMA kernel and whole blocks)
   const bool tiled = hkv > 0 && hq % hkv == 0 && axb::sdpa_tiled_supported(sq, hq, hkv, d, skv);
   if (tiled && dtype == AXB200_FLOAT32) return axb::sdpa_split_workspace_bytes(sq, hq, hkv, d, skv);
   size_t most = tiled ? 0 : axb::sdpa_rows_workspace_bytes(sq, hq, hkv, d, skv);

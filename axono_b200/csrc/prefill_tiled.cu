@@ -20,6 +20,7 @@
 
 #include <mutex>
 #include <set>
+#include <type_traits>
 
 #include "axono_b200.h"
 #include "common.cuh"
@@ -39,7 +40,7 @@ struct TiledParams {
   int sq, hq, hkv, group, skv, causal, d;
   int bq;  // query rows per CTA: virtual rows / group
   float scale;
-  // not null: only the KV heads of which some flag is set are computed.  kv_flags: kv_tiles per head for the keys, then for
+  // of the flagged form: only the KV heads of which some flag is set are computed.  kv_flags: kv_tiles per head for the keys, then for
   // the values; q_flags: q_blocks per query head
   const uint32_t *kv_flags, *q_flags;
   int kv_tiles, q_blocks;
@@ -69,8 +70,8 @@ inline size_t tp_smem_bytes(int d, int rows) {
 }
 
 // kCols: 16-byte column chunks per thread = head_dim / 64, rounded up; kTpRows virtual rows per CTA,
-// kTpRpt of them per thread.
-template <typename T, int kCols, int kTpRows, int kTpRpt>
+// kTpRpt of them per thread; kFlagged: only the KV heads that some flag names.
+template <typename T, int kCols, int kTpRows, int kTpRpt, bool kFlagged>
 __global__ void __launch_bounds__(kTpThreads)
 sdpa_tiled_kernel(const TiledParams p) {
   static_assert((kTpRows / kTpRpt) * 16 == kTpThreads, "thread tile does not cover the CTA tile");
@@ -81,7 +82,7 @@ sdpa_tiled_kernel(const TiledParams p) {
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   // heaviest blocks first under the causal mask
   const int qb = gridDim.x - 1 - blockIdx.x, hk = blockIdx.y;
-  if (p.kv_flags && !tp_flagged(p, hk)) return;
+  if (kFlagged && !tp_flagged(p, hk)) return;
   const int q0 = qb * p.bq;
   const T *qg = reinterpret_cast<const T *>(p.q), *kg = reinterpret_cast<const T *>(p.k),
           *vg = reinterpret_cast<const T *>(p.v);
@@ -279,7 +280,10 @@ bool tp_set_smem(const void *kernel, int bytes) {
 
 template <typename T, int kCols, int kRows, int kRpt>
 int tp_launch(const TiledParams &p, cudaStream_t st) {
-  auto kern = sdpa_tiled_kernel<T, kCols, kRows, kRpt>;
+  auto kern = sdpa_tiled_kernel<T, kCols, kRows, kRpt, false>;
+  if constexpr (std::is_same_v<T, float> && kCols <= 2) {  // what prefill_f32.cu takes
+    if (p.kv_flags) kern = sdpa_tiled_kernel<T, kCols, kRows, kRpt, true>;
+  }
   const int smem = (int)tp_smem_bytes(p.d, kRows);
   if (!tp_set_smem(reinterpret_cast<const void *>(kern), 200 * 1024)) return AXB200_DEVICE_ERROR;
   const dim3 grid((p.sq + p.bq - 1) / p.bq, p.hkv);

@@ -1179,8 +1179,8 @@ def run_prefill(args):
         peak, kind = 1590.0, "fallback"
     kernel = "prefill_attn_f16_pair_kernel" if S >= 256 else "prefill_attn_f16_kernel"
     bound = "tensor"
-    if f32:
-        peak, kind, kernel, bound = 148 * 128 * 2 * 1.965e9 / 1e12, "nominal fp32 FMA", "sdpa_tiled_kernel<float>", "fma"
+    if f32:  # six bf16 products of parts for one of floats
+        peak, kind, kernel = peak / 6, f"{kind} bf16 / 6", "split_attn_kernel"
     err = ops.last_error()
     print(json.dumps({
         "metric": "prefill_attention_tflops", "value": tflops, "unit": "TFLOP/s", "n_gpus": 1, "steps": args.steps,

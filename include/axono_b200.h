@@ -195,11 +195,13 @@ int axb200_gqa_decode_paged_window(const void *q, void *out, const void *k_pages
  * Replaces axono::ops::cuda::ScaledDotProductAttention (include/axono/ops/cuda/sequence.h:37-39,
  * src/ops/cuda/sequence.cu:105-163,451-472): q (sq,hq,d), k/v (skv,hkv,d) token-major, out (sq,hq,d);
  * scale 1/sqrt(d); head h reads KV head h/(hq/hkv); with is_causal row t sees keys [0, t] when
- * skv >= t+1 and every key otherwise (src/ops/cpu/sequence.cpp:269-270).  fp16 with d == 128 runs on
- * the tcgen05 tensor cores; FLOAT32 and other head sizes (d a multiple of 4 up to 192, sq >= 16) on a
- * tiled FMA kernel with fp32 arithmetic; neither needs scratch.  The remaining cases run row by row
- * on the decode kernels and need axb200_sdpa_workspace_bytes of scratch (0 for the first two).
- * There is no shared-memory limit on skv. */
+ * skv >= t+1 and every key otherwise (src/ops/cpu/sequence.cpp:269-270).  fp16 with d == 128, or a multiple
+ * of 8 below it, and FLOAT32 with d a multiple of 4 up to 128 run on the tcgen05 tensor cores (FLOAT32 as
+ * products of three bf16 parts per value, the error of fp32 arithmetic); other head sizes (d a multiple
+ * of 4 up to 192, sq >= 16) on a tiled FMA kernel with fp32 arithmetic; the remaining cases row by row on
+ * the decode kernels.  Scratch: axb200_sdpa_workspace_bytes, a multiple of 16 bytes in address, of this call
+ * alone while it runs.  The row-by-row form cannot do without it; with less or none FLOAT32 takes the FMA
+ * kernel and fp16 does not divide a block's keys among CTAs.  There is no shared-memory limit on skv. */
 size_t axb200_sdpa_workspace_bytes(int sq, int hq, int hkv, int d, int64_t skv, int dtype);
 int axb200_sdpa(const void *q, const void *k, const void *v, void *out,
                 int sq, int hq, int hkv, int d, int64_t skv, int is_causal, int dtype,
