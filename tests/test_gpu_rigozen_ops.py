@@ -19,7 +19,7 @@ def tol(dtype):
 
 # ---- the residual stream ----------------------------------------------------------------------------------
 @pytest.mark.parametrize("dtype", DTYPES)
-@pytest.mark.parametrize("width", [76, 256, 7168])
+@pytest.mark.parametrize("width", [76, 256, 2048, 2056, 4096, 4104, 7168])  # held in registers up to 2048 and 4096, staged above
 def test_residual_post_norm(dtype, width):
     from axono_b200 import ops
 
