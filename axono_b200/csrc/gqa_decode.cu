@@ -1407,9 +1407,12 @@ __host__ __device__ inline int gen_head_batch(int d, int group) {
 }
 inline size_t gen_smem_bytes(int d, int group) {
   const int tt = gen_tile_tokens(d), gb = gen_head_batch(d, group);
-  return sizeof(float) * ((size_t)2 * tt * gen_row_stride(d) + (((size_t)gb * d + 3) & ~size_t(3)) + (size_t)gb * tt +
-                          3 * kGenMaxHeads) +
-         sizeof(long long) * 64 + 8;
+  const size_t tiles = sizeof(float) * ((size_t)2 * tt * gen_row_stride(d) + (((size_t)gb * d + 3) & ~size_t(3)) +
+                                        (size_t)gb * tt + 3 * kGenMaxHeads) +
+                       sizeof(long long) * 64 + 8;
+  // the merge of the chunks takes the place of the tiles, and wants more where d = 4 (two heads: 4224 bytes, tiles 3816)
+  const size_t merge = sizeof(float) * 2 * (kGenThreads / 32) * kMergeRow;
+  return tiles > merge ? tiles : merge;
 }
 
 // Scores of one key against kNh query heads (sub, sub + nsub, ...): the K value is read once per

@@ -48,3 +48,23 @@ def test_fp32_head_sizes(d, hq, hkv):
     for i, n in enumerate(LENGTHS):
         close(out[i], reference(q[i], k[i, max(0, n - 70):n], v[i, max(0, n - 70):n]))
     assert ops.last_error() == 0
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.float32])
+@pytest.mark.parametrize("hq,hkv", [(4, 2), (6, 2), (3, 3)])
+def test_heads_of_four(dtype, hq, hkv):
+    """The kernel for any head size at its smallest: two heads' merge of the chunks takes more shared memory than the tiles do.
+    Tensors one element off 16 bytes, so that fp32 comes here too; fp16 rounds the result by 2^-11."""
+    from axono_b200 import ops
+
+    g = torch.Generator(device="cuda").manual_seed(hq)
+
+    def off(*s):
+        n = s[0] * s[1] * s[2]
+        return torch.randn(n + 1, generator=g, device="cuda").to(dtype)[1:].view(s)
+
+    for n in (1, 64, 300, 1025, 4097):
+        q, k, v = off(1, hq, 4), off(n, hkv, 4), off(n, hkv, 4)
+        out, ref = ops.gqa_decode_attention(q, k, v)[0].double(), reference(q[0], k, v)
+        assert ((out - ref).abs() <= TOL * ref.abs().max() + (ref.abs() * 2.0 ** -11 if dtype == torch.float16 else 0.0)).all()
+    assert ops.last_error() == 0
