@@ -249,7 +249,9 @@ latent_prefill_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
       }
       const float m_safe = (m_run == -INFINITY) ? 0.f : m_run;
       const uint64_t scale2 = pack_f32x2(p.scale_log2, p.scale_log2), shift2 = pack_f32x2(-m_safe, -m_safe);
-      uint64_t sum2[4] = {0, 0, 0, 0};
+      // neighbours first: the order of these additions shows in the last bit of the results (even and odd scores apart, two
+      // additions per instruction: 152 us instead of 157 at 2048 rows over 8192 keys, 16 heads of 128)
+      float sum4[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
       for (int c = 0; c < 4; ++c) {
         uint32_t packed[16];
@@ -257,13 +259,12 @@ latent_prefill_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
         for (int i = 0; i < 32; i += 2) {
           const float2 x = unpack_f32x2(fma_f32x2(pack_f32x2(__uint_as_float(sr[c][i]), __uint_as_float(sr[c][i + 1])), scale2, shift2));
           const float a = fast_exp2(x.x), b = fast_exp2(x.y);
-          sum2[(i >> 1) & 3] = add_f32x2(sum2[(i >> 1) & 3], pack_f32x2(a, b));
+          sum4[(i >> 1) & 3] += a + b;
           packed[i >> 1] = pack_bf16x2(a, b);
         }
         tmem_st16(tp + c * 16, packed);
       }
-      const float2 sum = unpack_f32x2(add_f32x2(add_f32x2(sum2[0], sum2[1]), add_f32x2(sum2[2], sum2[3])));
-      l_run = l_run * corr + (sum.x + sum.y);
+      l_run = l_run * corr + ((sum4[0] + sum4[1]) + (sum4[2] + sum4[3]));
       // bar_s of tile j was committed after P(j-1).V_{j-1}: that product is complete and O_g may be rescaled
       if (j > 0 && moved) {
 #pragma unroll

@@ -213,6 +213,23 @@ def test_expanded_form_with_window_and_sink(heads, kv_heads, dim, rot, vdim):
             close(got, want, 1.5e-2)
 
 
+def test_latent_prefill_denominators_add_neighbours_first():
+    """The order in which a row's weights are added: 1 beside 0.85 x 2^-24 is 1, four times, so the denominator is 4 and the
+    result stands halfway between two values (the even one is the larger).  Odd and even keys summed apart would give
+    4 + 54 x 2^-24, and the smaller one."""
+    from axono_b200 import ops
+
+    step, n, m, d = torch.finfo(torch.bfloat16).eps, 256, 384, 128
+    q, k, v = (torch.zeros(s, d, dtype=torch.bfloat16) for s in (n, m, m))
+    q[:, 0] = 1
+    k[:, 0] = -480.0  # 2^-61: nothing
+    k[1:128:2, 0] = -190.0  # 2^-24.2
+    k[0:8:2, 0] = 0
+    v[0:4:2], v[4:8:2] = 1 + step, 1 + 2 * step
+    out = ops.latent_prefill(q.cuda(), m - n, k.cuda(), v.cuda(), None, 1, d, 0, d, d ** -0.5)
+    assert (out == 1 + 2 * step).all() and ops.last_error() == 0
+
+
 # ---- the gated delta rule ----------------------------------------------------------------------------------
 class Mixer:
     """Random weights of one mixer, its inputs, and the plain evaluation of a whole sequence."""
