@@ -60,6 +60,7 @@ struct PrefillParams {
   void *out;
   int sq, hq, hkv, skv, causal, d;
   float scale_log2;
+  const __half *q, *k, *v;  // for rows that the tensor core cannot finish
 };
 
 constexpr float kLazyLog2 = 8.0f;
@@ -354,6 +355,71 @@ __device__ __forceinline__ uint32_t split_half2(float a, float b, uint32_t &lo) 
   return *reinterpret_cast<const uint32_t *>(&hi);
 }
 
+// One row over the keys [key0, key1) with a weight of one part, as the definition has it.  A weight in two parts meets V twice, and
+// where V is infinite hi * V + lo * V is NaN (lo may be 0 or negative) though the row's value is +-inf; and every row of a block
+// multiplies the V of all its tiles, also those that its mask hides.  So a thread whose row is not finite does it over - only
+// inputs that are not finite lead here.  ml: where un-normalised sums go instead of the result.
+__device__ __noinline__ void redo_narrow_row(const PrefillParams &p, int t_row, int h, int key0, int key1, float *sums, float2 *ml) {
+  constexpr int kMost = kD / 8 - 1;  // 16-byte pieces of a row
+  const int hk = h / (p.hq / p.hkv), pieces = p.d / 8;
+  const size_t step = (size_t)p.hkv * p.d;
+  const __half *k = p.k + (size_t)hk * p.d, *v = p.v + (size_t)hk * p.d;
+  const uint4 *from = reinterpret_cast<const uint4 *>(p.q + ((size_t)t_row * p.hq + h) * p.d);
+  uint4 q[kMost];
+#pragma unroll
+  for (int c = 0; c < kMost; ++c)
+    if (c < pieces) q[c] = from[c];
+  const auto dot2 = [](uint32_t a, uint32_t b, float s) {
+    const float2 x = __half22float2(*reinterpret_cast<const __half2 *>(&a)), y = __half22float2(*reinterpret_cast<const __half2 *>(&b));
+    return fmaf(x.y, y.y, fmaf(x.x, y.x, s));
+  };
+  const auto score = [&](int key) {
+    const uint4 *row = reinterpret_cast<const uint4 *>(k + key * step);
+    float s = 0.f;
+#pragma unroll
+    for (int c = 0; c < kMost; ++c)
+      if (c < pieces) {
+        const uint4 x = row[c];
+        s = dot2(q[c].w, x.w, dot2(q[c].z, x.z, dot2(q[c].y, x.y, dot2(q[c].x, x.x, s))));
+      }
+    return s;
+  };
+  float m = -INFINITY;
+  for (int key = key0; key < key1; ++key) m = fmaxf(m, score(key));
+  for (int c0 = 0; c0 < p.d; c0 += 32) {
+    float acc[32], l = 0.f;
+#pragma unroll
+    for (int i = 0; i < 32; ++i) acc[i] = 0.f;
+    for (int key = key0; key < key1; ++key) {
+      const float s = score(key), w = s == -INFINITY ? 0.f : exp2f((s - m) * p.scale_log2);
+      l += w;
+#pragma unroll
+      for (int u = 0; u < 4; ++u)
+        if (c0 + u * 8 < p.d) {
+          const uint4 x = *reinterpret_cast<const uint4 *>(v + key * step + c0 + u * 8);
+          const uint32_t part[4] = {x.x, x.y, x.z, x.w};
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            const float2 f = __half22float2(*reinterpret_cast<const __half2 *>(&part[i]));
+            acc[u * 8 + 2 * i] = fmaf(w, f.x, acc[u * 8 + 2 * i]);
+            acc[u * 8 + 2 * i + 1] = fmaf(w, f.y, acc[u * 8 + 2 * i + 1]);
+          }
+        }
+    }
+    const float inv = l > 0.f ? 1.0f / l : 0.f;
+    __half *out = reinterpret_cast<__half *>(p.out) + ((size_t)t_row * p.hq + h) * p.d + c0;
+#pragma unroll
+    for (int i = 0; i < 32; ++i)
+      if (c0 + i < p.d) {
+        if (ml)
+          sums[c0 + i] = acc[i];
+        else
+          out[i] = __float2half_rn(acc[i] * inv);
+      }
+    if (ml) *ml = make_float2(m * p.scale_log2, l);
+  }
+}
+
 // kNarrow: head sizes below 128 (multiples of 8).  They ran on the FMA pipe before, whose weights were fp32, so P enters
 // P.V as two fp16 parts here: P's two parts take the two halves of S_g, and a tile costs 16 products for P.V instead of 8.
 // Elements past the head size are zeros that TMA fills in; head sizes up to 64 leave the second 64-wide block of every tile
@@ -365,7 +431,8 @@ __device__ __forceinline__ uint32_t split_half2(float a, float b, uint32_t &lo) 
 template <bool kNarrow>
 __global__ void __launch_bounds__(kPairThreads, 1)
 prefill_attn_f16_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
-                             const __grid_constant__ CUtensorMap tmV, const PrefillParams p, const __grid_constant__ KeySplit split,
+                             const __grid_constant__ CUtensorMap tmV, const __grid_constant__ PrefillParams p,
+                             const __grid_constant__ KeySplit split,
                              const Partials partials) {
   extern __shared__ __align__(1024) uint8_t smem[];
   uint64_t *bars = reinterpret_cast<uint64_t *>(smem + kPairOffBar);
@@ -587,8 +654,9 @@ prefill_attn_f16_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __gr
     // ---- epilogue: O / l -> out ----
     if (ok && my_nkv > 0) ok = __all_sync(0xffffffffu, mbar_wait_bounded(&bar_fin[g], 0, abort_flag));
     tc_fence_after();
+    const size_t at = ((size_t)unit * p.hq + h) * (2 * kBlockM) + g * kBlockM + row;  // of divided blocks
+    float bad = 0.f;  // NaN once a stored sum is not finite
     if (parts > 1) {
-      const size_t at = ((size_t)unit * p.hq + h) * (2 * kBlockM) + g * kBlockM + row;
       const bool any = ok && my_nkv > 0;
       if (t_row < p.sq) partials.ml[at] = any ? make_float2(m_run, l_run) : make_float2(-INFINITY, 0.f);
       if (any) {
@@ -602,6 +670,9 @@ prefill_attn_f16_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __gr
 #pragma unroll
             for (int u = 0; u < 8; ++u) {
               if (kNarrow && c * 32 + u * 4 >= p.d) break;
+              if (kNarrow)
+#pragma unroll
+                for (int i = 0; i < 4; ++i) bad = fmaf(__uint_as_float(r[u * 4 + i]), 0.f, bad);
               *reinterpret_cast<uint4 *>(dst + c * 32 + u * 4) = make_uint4(r[u * 4], r[u * 4 + 1], r[u * 4 + 2], r[u * 4 + 3]);
             }
           }
@@ -619,6 +690,9 @@ prefill_attn_f16_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __gr
 #pragma unroll
           for (int u = 0; u < 4; ++u) {
             if (kNarrow && c * 32 + u * 8 >= p.d) break;
+            if (kNarrow)
+#pragma unroll
+              for (int i = 0; i < 8; ++i) bad = fmaf(__uint_as_float(r[u * 8 + i]), 0.f, bad);
             uint4 w;
             w.x = pack_half2(__uint_as_float(r[u * 8 + 0]) * inv, __uint_as_float(r[u * 8 + 1]) * inv);
             w.y = pack_half2(__uint_as_float(r[u * 8 + 2]) * inv, __uint_as_float(r[u * 8 + 3]) * inv);
@@ -629,6 +703,9 @@ prefill_attn_f16_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __gr
         }
       }
     }
+    if (kNarrow && bad != 0.f)
+      redo_narrow_row(p, t_row, h, tile0 * kPairN, min((tile0 + my_nkv) * kPairN, kv_end), partials.sums + at * p.d,
+                      parts > 1 ? partials.ml + at : nullptr);
   }
   tc_fence_before();
   __syncthreads();
@@ -738,6 +815,9 @@ int axb200_sdpa(const void *q, const void *k, const void *v, void *out, int sq, 
   p.causal = is_causal != 0;
   p.d = d;
   p.scale_log2 = (1.0f / sqrtf((float)d)) * axb::kLog2e;
+  p.q = static_cast<const __half *>(q);
+  p.k = static_cast<const __half *>(k);
+  p.v = static_cast<const __half *>(v);
   if (pair) {
     axb::KeySplit split = axb::pair_plan(sq, hq, skv, is_causal);
     if (split.units && (!workspace || !axb::aligned16(workspace) || workspace_bytes < axb::key_split_bytes(split, hq, 2 * axb::kBlockM, d)))

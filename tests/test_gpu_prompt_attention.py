@@ -103,3 +103,36 @@ def test_fp16_keys_divided_among_blocks(d, sq, skv, hq, hkv):
             small = 2.0 ** -25 * v.double().abs().sum(0).repeat_interleave(hq // hkv, 0)
             assert (err <= ref.abs() * 2.0 ** -11 + weight * mass + small + 2.0 ** -24).all(), (causal, err.max())
     assert ops.last_error() == 0
+
+
+@pytest.mark.parametrize("d", [8, 64, 72])
+@pytest.mark.parametrize("sq,skv,hq,hkv", [(200, 260, 4, 2), (300, 4100, 2, 1), (1300, 1300, 2, 2)])  # the later two divide keys
+def test_fp16_narrow_heads_with_infinities(d, sq, skv, hq, hkv):
+    """Infinite and NaN values, keys and queries: rows that see them come out as the definition's, rows that the mask keeps
+    from them as if they were not there."""
+    from axono_b200 import ops
+
+    inf, nan = float("inf"), float("nan")
+    for causal in (True, False):
+        q, k, v = tensors(sq, skv, hq, hkv, d, torch.float16)
+        clean = ops.scaled_dot_product_attention(q, k, v, causal)
+        at, group = {0: inf, 1: -inf, 2: nan}, hq // hkv
+        for head in range(hkv):
+            vb = v.clone()
+            for c, x in at.items():
+                vb[100, head, c] = x
+            want = clean.clone()
+            seen = torch.arange(sq, device="cuda") >= (100 if causal else 0)
+            for c, x in at.items():
+                for h in range(head * group, (head + 1) * group):
+                    want[seen, h, c] = x
+            out = ops.scaled_dot_product_attention(q, k, vb, causal)
+            torch.testing.assert_close(out, want, rtol=2.0 ** -10, atol=1e-5, equal_nan=True)
+        kb, qb = k.clone(), q.clone()
+        kb[100, 0, 3], qb[150, hq - 1, 4] = nan, inf  # NaN scores; scores of +inf (and -inf: nothing)
+        out = ops.scaled_dot_product_attention(qb, kb, v, causal)
+        want = clean.clone()
+        want[seen, 0:group] = nan
+        want[150, hq - 1] = nan
+        torch.testing.assert_close(out, want, rtol=2.0 ** -10, atol=1e-5, equal_nan=True)
+    assert ops.last_error() == 0
