@@ -256,11 +256,17 @@ latent_prefill_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
       for (int c = 0; c < 4; ++c) {
         uint32_t packed[16];
 #pragma unroll
-        for (int i = 0; i < 32; i += 2) {
-          const float2 x = unpack_f32x2(fma_f32x2(pack_f32x2(__uint_as_float(sr[c][i]), __uint_as_float(sr[c][i + 1])), scale2, shift2));
-          const float a = fast_exp2(x.x), b = fast_exp2(x.y);
-          sum4[(i >> 1) & 3] += a + b;
-          packed[i >> 1] = pack_bf16x2(a, b);
+        for (int i = 0; i < 32; i += 4) {
+          float w[4];
+#pragma unroll
+          for (int u = 0; u < 4; u += 2) {
+            const float2 x = unpack_f32x2(
+                fma_f32x2(pack_f32x2(__uint_as_float(sr[c][i + u]), __uint_as_float(sr[c][i + u + 1])), scale2, shift2));
+            w[u] = fast_exp2(x.x), w[u + 1] = fast_exp2(x.y);
+            packed[(i + u) >> 1] = pack_bf16x2(w[u], w[u + 1]);
+          }
+          sum4[(i >> 1) & 3] += w[0] + w[1];
+          sum4[((i >> 1) & 3) + 1] += w[2] + w[3];
         }
         tmem_st16(tp + c * 16, packed);
       }
