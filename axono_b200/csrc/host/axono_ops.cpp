@@ -70,10 +70,11 @@ Status ScaledDotProductAttention(const Context &, const Tensor &q, const Tensor 
   if (hkv == 0 || hq % hkv != 0) return Status::SHAPE_MISMATCH;
   Status st = result.Resize({sq, hq, d});
   if (st != Status::OK) return st;
-  const size_t ws = axb200_sdpa_workspace_bytes((int)sq, (int)hq, (int)hkv, (int)d, (int64_t)skv, Dt(q.dtype()));
-  Tensor scratch = Scratch(ws, q.device());
-  return St(axb200_sdpa(q.data(), k.data(), v.data(), result.data(), (int)sq, (int)hq, (int)hkv, (int)d, (int64_t)skv,
-                        is_causal ? 1 : 0, Dt(q.dtype()), scratch.data(), scratch.num_bytes(), Stream()));
+  const int n = (int)sq, heads = (int)hq, kv_heads = (int)hkv, dim = (int)d, causal = is_causal ? 1 : 0, dt = Dt(q.dtype());
+  Tensor rows = Scratch(axb200_sdpa_workspace_bytes(n, heads, kv_heads, dim, (int64_t)skv, dt), q.device());
+  Tensor fast = Scratch(axb200_sdpa_scratch_bytes(n, heads, kv_heads, dim, (int64_t)skv, causal, dt), q.device());
+  return St(axb200_sdpa_scratch(q.data(), k.data(), v.data(), result.data(), n, heads, kv_heads, dim, (int64_t)skv, causal, dt,
+                                rows.data(), rows.num_bytes(), fast.data(), fast.num_bytes(), Stream()));
 }
 
 Status SiluMul(const Context &, const Tensor &gate, const Tensor &up, Tensor &result) {

@@ -38,9 +38,9 @@ bool sdpa_tiled_supported(int sq, int hq, int hkv, int d, int64_t skv);
 int sdpa_tiled(const void *q, const void *k, const void *v, void *out, int sq, int hq, int hkv, int d, int64_t skv,
                int is_causal, int dtype, cudaStream_t st);
 // FLOAT32 on the tensor cores (prefill_f32.cu); the scratch it wants is 0 where it does not apply.
-size_t sdpa_split_workspace_bytes(int sq, int hq, int hkv, int d, int64_t skv);
+size_t sdpa_split_scratch_bytes(int sq, int hq, int hkv, int d, int64_t skv, int is_causal);
 int sdpa_split(const void *q, const void *k, const void *v, void *out, int sq, int hq, int hkv, int d, int64_t skv, int is_causal,
-               void *workspace, cudaStream_t st);
+               void *scratch, cudaStream_t st);
 
 namespace {
 
@@ -750,21 +750,30 @@ bool aligned16(const void *p) { return (reinterpret_cast<uintptr_t>(p) & 15u) ==
 extern "C" {
 
 size_t axb200_sdpa_workspace_bytes(int sq, int hq, int hkv, int d, int64_t skv, int dtype) {
-  // the row-by-row evaluation on the decode kernels needs room for partials, the fp32 form for the tiles of parts, the
-  // 256-row form for what divided blocks leave (without it FMA kernel and whole blocks)
-  const bool tiled = hkv > 0 && hq % hkv == 0 && axb::sdpa_tiled_supported(sq, hq, hkv, d, skv);
-  if (tiled && dtype == AXB200_FLOAT32) return axb::sdpa_split_workspace_bytes(sq, hq, hkv, d, skv);
-  size_t most = tiled ? 0 : axb::sdpa_rows_workspace_bytes(sq, hq, hkv, d, skv);
-  if (dtype == AXB200_FLOAT16 && sq > 0 && hq > 0 && skv > 0 && axb::pair_form(sq, d))
-    for (int causal = 0; causal < 2; ++causal) {  // the caller does not name the mask here
-      const size_t n = axb::key_split_bytes(axb::pair_plan(sq, hq, skv, causal), hq, 2 * axb::kBlockM, d);
-      most = n > most ? n : most;
-    }
-  return most;
+  // the tensor-core kernels and the tiled FMA kernel can keep everything on chip; only the row-by-row evaluation on the decode
+  // kernels needs room for partials (whatever the tensor-core path does not take - unaligned pointers, say - the tiled kernel does)
+  if (hkv > 0 && hq % hkv == 0 && axb::sdpa_tiled_supported(sq, hq, hkv, d, skv)) return 0;
+  return axb::sdpa_rows_workspace_bytes(sq, hq, hkv, d, skv);
+}
+
+size_t axb200_sdpa_scratch_bytes(int sq, int hq, int hkv, int d, int64_t skv, int is_causal, int dtype) {
+  // what makes prompts faster: the fp32 form's tiles of parts, and what blocks with divided keys leave
+  if (sq <= 0 || hq <= 0 || hkv <= 0 || d <= 0 || skv <= 0 || skv > 0x7fffffff - 4096 || hq % hkv != 0) return 0;
+  if (dtype == AXB200_FLOAT32 && axb::sdpa_tiled_supported(sq, hq, hkv, d, skv))
+    return axb::sdpa_split_scratch_bytes(sq, hq, hkv, d, skv, is_causal);
+  if (dtype == AXB200_FLOAT16 && axb::pair_form(sq, d))
+    return axb::key_split_bytes(axb::pair_plan(sq, hq, skv, is_causal), hq, 2 * axb::kBlockM, d);
+  return 0;
 }
 
 int axb200_sdpa(const void *q, const void *k, const void *v, void *out, int sq, int hq, int hkv, int d,
                 int64_t skv, int is_causal, int dtype, void *workspace, size_t workspace_bytes, void *stream) {
+  return axb200_sdpa_scratch(q, k, v, out, sq, hq, hkv, d, skv, is_causal, dtype, workspace, workspace_bytes, nullptr, 0, stream);
+}
+
+int axb200_sdpa_scratch(const void *q, const void *k, const void *v, void *out, int sq, int hq, int hkv, int d, int64_t skv,
+                        int is_causal, int dtype, void *workspace, size_t workspace_bytes, void *scratch, size_t scratch_bytes,
+                        void *stream) {
   if (dtype != AXB200_FLOAT16 && dtype != AXB200_FLOAT32) return AXB200_UNSUPPORTED_TYPE;
   if (!q || !k || !v || !out) return AXB200_INVALID_PTR;
   if (sq <= 0 || hq <= 0 || hkv <= 0 || d <= 0 || skv <= 0 || skv > 0x7fffffff - 4096) return AXB200_INVALID_ARGUMENT;
@@ -775,10 +784,10 @@ int axb200_sdpa(const void *q, const void *k, const void *v, void *out, int sq, 
                            axb::aligned16(k) && axb::aligned16(v) && axb::aligned16(out) && axb::tensor_map_encoder();
   if (!tensor_path) {
     const bool tiled = axb::sdpa_tiled_supported(sq, hq, hkv, d, skv);
-    const size_t split = tiled && dtype == AXB200_FLOAT32 ? axb::sdpa_split_workspace_bytes(sq, hq, hkv, d, skv) : 0;
-    if (split && workspace && workspace_bytes >= split && axb::aligned16(workspace) && axb::aligned16(q) && axb::aligned16(k) &&
-        axb::aligned16(v) && axb::aligned16(out))
-      return axb::sdpa_split(q, k, v, out, sq, hq, hkv, d, skv, is_causal, workspace, st);
+    const bool split = tiled && dtype == AXB200_FLOAT32 && scratch && axb::aligned16(scratch) && axb::aligned16(q) &&
+                       axb::aligned16(k) && axb::aligned16(v) && axb::aligned16(out);
+    const size_t need = split ? axb::sdpa_split_scratch_bytes(sq, hq, hkv, d, skv, is_causal) : 0;
+    if (need && scratch_bytes >= need) return axb::sdpa_split(q, k, v, out, sq, hq, hkv, d, skv, is_causal, scratch, st);
     if (tiled)
       return axb::sdpa_tiled(q, k, v, out, sq, hq, hkv, d, skv, is_causal, dtype, st);
     return axb::sdpa_rows_fallback(q, k, v, out, sq, hq, hkv, d, skv, is_causal, dtype, workspace, workspace_bytes, st);
@@ -819,10 +828,13 @@ int axb200_sdpa(const void *q, const void *k, const void *v, void *out, int sq, 
   p.k = static_cast<const __half *>(k);
   p.v = static_cast<const __half *>(v);
   if (pair) {
-    axb::KeySplit split = axb::pair_plan(sq, hq, skv, is_causal);
-    if (split.units && (!workspace || !axb::aligned16(workspace) || workspace_bytes < axb::key_split_bytes(split, hq, 2 * axb::kBlockM, d)))
-      split.units = 0;
-    const axb::Partials partials = axb::partials_at(workspace, split, hq, 2 * axb::kBlockM);
+    axb::KeySplit split;
+    split.units = 0;
+    if (scratch && axb::aligned16(scratch)) {
+      split = axb::pair_plan(sq, hq, skv, is_causal);
+      if (scratch_bytes < axb::key_split_bytes(split, hq, 2 * axb::kBlockM, d)) split.units = 0;
+    }
+    const axb::Partials partials = axb::partials_at(scratch, split, hq, 2 * axb::kBlockM);
     const dim3 grid((unsigned)hq * (split.units ? split.units : (sq + 2 * axb::kBlockM - 1) / (2 * axb::kBlockM)));
     auto *kernel = narrow ? axb::prefill_attn_f16_pair_kernel<true> : axb::prefill_attn_f16_pair_kernel<false>;
     kernel<<<grid, axb::kPairThreads, axb::kPairSmemBytes, st>>>(mq, mk, mv, p, split, partials);

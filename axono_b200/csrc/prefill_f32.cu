@@ -427,24 +427,20 @@ int launch(const Params &p, void *parts_at, cudaStream_t st) {
 // Scratch that the split form wants for this problem; 0 where the FMA kernel serves it: problems that are one launch of few key
 // tiles in a row there, waves of blocks times tiles of keys.  48 rows and keys, 16 / 8 heads of 128: 23 us in one launch, 32 in
 // three.  100 rows and keys: 55 and 29; 2000 rows, 64 keys: 70 and 39; 16 rows, 128 keys, 2 heads of 64: 25 and 28.
-size_t sdpa_split_workspace_bytes(int sq, int hq, int hkv, int d, int64_t skv) {
+size_t sdpa_split_scratch_bytes(int sq, int hq, int hkv, int d, int64_t skv, int is_causal) {
   const int64_t in_a_row = (((int64_t)sq * hq + 128 * 148 - 1) / (128 * 148)) * ((skv + kKeys - 1) / kKeys);
   const int64_t rows = (int64_t)sq * (hq / hkv);
   if (d % 4 || d > 128 || sq < 16 || hkv > 65535 || in_a_row < (rows >= kRows ? 2 : 3)) return 0;
   const int64_t n_tiles = (skv + kKeys - 1) / kKeys, q_blocks = ((int64_t)sq + kRows - 1) / kRows;
-  size_t parts = 0;
-  for (int causal = 0; causal < 2; ++causal) {  // the caller does not name the mask here
-    const size_t n = key_split_bytes(split_plan(sq, hq, skv, causal), hq, kRows, d);
-    parts = n > parts ? n : parts;
-  }
+  const size_t parts = key_split_bytes(split_plan(sq, hq, skv, is_causal), hq, kRows, d);
   const size_t total = up256((size_t)hq * q_blocks * 4) + kv_flag_bytes(hkv, n_tiles) +
                        tile_bytes(hkv, n_tiles, d) + parts;
   return total <= kMostScratch ? total : 0;
 }
 
-// q, k, v, out and workspace on 16-byte boundaries; workspace of the size above.
+// q, k, v, out and scratch on 16-byte boundaries; scratch of the size above.
 int sdpa_split(const void *q, const void *k, const void *v, void *out, int sq, int hq, int hkv, int d, int64_t skv, int is_causal,
-               void *workspace, cudaStream_t st) {
+               void *scratch, cudaStream_t st) {
   Params p{};
   p.q = static_cast<const float *>(q);
   p.k = static_cast<const float *>(k);
@@ -460,7 +456,7 @@ int sdpa_split(const void *q, const void *k, const void *v, void *out, int sq, i
   p.q_blocks = (sq + kRows - 1) / kRows;
   p.scale_log2 = (1.0f / sqrtf((float)d)) * kLog2e;
   p.wait_ns = wait_limit_ns();
-  uint8_t *at = static_cast<uint8_t *>(workspace);
+  uint8_t *at = static_cast<uint8_t *>(scratch);
   p.q_flags = reinterpret_cast<uint32_t *>(at);
   at += up256((size_t)hq * p.q_blocks * 4);
   p.kv_flags = reinterpret_cast<uint32_t *>(at);

@@ -199,13 +199,22 @@ int axb200_gqa_decode_paged_window(const void *q, void *out, const void *k_pages
  * of 8 below it, and FLOAT32 with d a multiple of 4 up to 128 run on the tcgen05 tensor cores (FLOAT32 as
  * products of three bf16 parts per value, the error of fp32 arithmetic); other head sizes (d a multiple
  * of 4 up to 192, sq >= 16) on a tiled FMA kernel with fp32 arithmetic; the remaining cases row by row on
- * the decode kernels.  Scratch: axb200_sdpa_workspace_bytes, a multiple of 16 bytes in address, of this call
- * alone while it runs.  The row-by-row form cannot do without it; with less or none FLOAT32 takes the FMA
- * kernel and fp16 does not divide a block's keys among CTAs.  There is no shared-memory limit on skv. */
+ * the decode kernels, which need axb200_sdpa_workspace_bytes of workspace (0 for the others, which leave it
+ * alone).  There is no shared-memory limit on skv.
+ *
+ * axb200_sdpa_scratch is the same with memory that makes prompts faster: axb200_sdpa_scratch_bytes (0: of no
+ * use here), at a multiple of 16 bytes, written and read by this call alone until its kernels are done, so one
+ * buffer per stream.  With less or none - and in axb200_sdpa - FLOAT32 takes the FMA kernel and fp16 does not
+ * divide a block's keys among CTAs.  A KV head (of K, V or its queries) with FLOAT32 values that are not finite,
+ * above 3.39e38 or, unless zero, below 2^-100 is computed a second time by the FMA kernel, at its speed. */
 size_t axb200_sdpa_workspace_bytes(int sq, int hq, int hkv, int d, int64_t skv, int dtype);
 int axb200_sdpa(const void *q, const void *k, const void *v, void *out,
                 int sq, int hq, int hkv, int d, int64_t skv, int is_causal, int dtype,
                 void *workspace, size_t workspace_bytes, void *stream);
+size_t axb200_sdpa_scratch_bytes(int sq, int hq, int hkv, int d, int64_t skv, int is_causal, int dtype);
+int axb200_sdpa_scratch(const void *q, const void *k, const void *v, void *out,
+                        int sq, int hq, int hkv, int d, int64_t skv, int is_causal, int dtype,
+                        void *workspace, size_t workspace_bytes, void *scratch, size_t scratch_bytes, void *stream);
 
 /* ---- decode attention fused with the all-gather of per-head outputs ------------------------------
  * For KV heads sharded over `world` GPUs of one node (one process per GPU): rank `rank` holds hkv KV

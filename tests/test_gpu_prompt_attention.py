@@ -136,3 +136,19 @@ def test_fp16_narrow_heads_with_infinities(d, sq, skv, hq, hkv):
         want[150, hq - 1] = nan
         torch.testing.assert_close(out, want, rtol=2.0 ** -10, atol=1e-5, equal_nan=True)
     assert ops.last_error() == 0
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.float32])
+@pytest.mark.parametrize("d", [64, 128])
+def test_plain_call_leaves_the_workspace_alone(dtype, d):
+    """axb200_sdpa writes no workspace where it asks for none, so that calls on several streams may be given one buffer."""
+    from axono_b200 import _capi
+
+    lib, dt = _capi.lib(), _capi.FLOAT32 if dtype == torch.float32 else _capi.FLOAT16
+    q, k, v = tensors(1300, 1300, 2, 2, d, dtype)
+    buf, out = torch.full((64 << 20,), 77, dtype=torch.uint8, device="cuda"), torch.empty_like(q)
+    assert lib.axb200_sdpa_workspace_bytes(1300, 2, 2, d, 1300, dt) == 0
+    for causal in (0, 1):
+        assert lib.axb200_sdpa(q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), 1300, 2, 2, d, 1300, causal, dt, buf.data_ptr(),
+                               buf.numel(), torch.cuda.current_stream().cuda_stream) == 0
+        assert (buf == 77).all()
