@@ -552,14 +552,13 @@ def scaled_dot_product_attention(q, k, v, is_causal: bool = False):
     q, k, v = _c(q), _c(k), _c(v)
     out = torch.empty_like(q)
     lib = _capi.lib()
-    def new(nbytes):  # memory of this call alone: streams may overlap
-        return torch.empty(nbytes, dtype=torch.uint8, device=q.device) if nbytes else None
-
     causal = int(bool(is_causal))
-    rows, fast = lib.axb200_sdpa_workspace_bytes(sq, hq, hkv, d, skv, dt), lib.axb200_sdpa_scratch_bytes(sq, hq, hkv, d, skv, causal, dt)
-    ws, scratch = new(rows), new(fast)
-    _call(lib.axb200_sdpa_scratch(q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), sq, hq, hkv, d, skv, causal, dt, _ptr(ws), rows,
-                                  _ptr(scratch), fast, _stream(q)), op)
+    need = lib.axb200_sdpa_scratch_bytes(sq, hq, hkv, d, skv, causal, dt)
+    scratch = torch.empty(need, dtype=torch.uint8, device=q.device) if need else None  # of this call alone: streams may overlap
+    # of the row-by-row form, the buffer kept for the decode operators: an address keeps counters of its own for good
+    ws = workspace(q.device, lib.axb200_sdpa_workspace_bytes(sq, hq, hkv, d, skv, dt))
+    _call(lib.axb200_sdpa_scratch(q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), sq, hq, hkv, d, skv, causal, dt, ws.data_ptr(),
+                                  ws.numel(), _ptr(scratch), need, _stream(q)), op)
     return out
 
 

@@ -152,3 +152,35 @@ def test_plain_call_leaves_the_workspace_alone(dtype, d):
         assert lib.axb200_sdpa(q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), 1300, 2, 2, d, 1300, causal, dt, buf.data_ptr(),
                                buf.numel(), torch.cuda.current_stream().cuda_stream) == 0
         assert (buf == 77).all()
+
+
+ROWS_THEN_DECODE = """
+import torch
+from axono_b200 import ops
+from torch.profiler import ProfilerActivity, profile
+
+rnd = lambda *s: torch.randn(s, device="cuda")
+held = []
+for i in range(80):  # ever other addresses are free
+    q, k, v = rnd(4, 8, 64), rnd(4096, 8, 64), rnd(4096, 8, 64)
+    held += [ops.scaled_dot_product_attention(q, k, v), torch.empty(4 << 20, dtype=torch.uint8, device="cuda")]
+ops.workspace("cuda", 256 << 20)  # a buffer at an address not seen before
+with profile(activities=[ProfilerActivity.CUDA]) as prof:
+    ops.gqa_decode_attention(rnd(1, 8, 64), k, v)
+    torch.cuda.synchronize()
+names = [e.key for e in prof.key_averages()]
+assert any("gqa_split" in n for n in names), names
+assert not any("gqa_combine" in n for n in names), names
+assert ops.last_error() == 0
+"""
+
+
+def test_row_by_row_calls_leave_counters_to_others():
+    """A workspace's address takes one of 64 regions of counters for good: calls of a few rows, however many, take one in all,
+    and a buffer first seen after them still gets its own (without one the merge is a launch of its own)."""
+    import subprocess
+    import sys
+
+    from conftest import ROOT
+
+    subprocess.run([sys.executable, "-c", ROWS_THEN_DECODE], cwd=ROOT, check=True, timeout=300)
