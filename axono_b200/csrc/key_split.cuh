@@ -13,10 +13,12 @@
 namespace axb {
 
 constexpr int kMostUnits = 448, kSms = 148;
+constexpr size_t kMostScratch = (size_t)2 << 30;
 
-// What CTAs work on, per head: unit u is part `part` of `parts` of row block `block`.  units == 0: blocks as they are.
+// What CTAs work on, per head: unit u is part `part` of `parts` of row block `block`.  units == 0: blocks as they are.  Units of
+// divided blocks follow one another: `divided` of them from `first` on; only they have scratch.
 struct KeySplit {
-  int units;
+  int units, first, divided;
   uint16_t block[kMostUnits];
   uint8_t part[kMostUnits], parts[kMostUnits];
 };
@@ -29,7 +31,7 @@ __host__ __device__ inline int split_begin(int tiles, int part, int parts) { ret
 template <typename Tiles>
 KeySplit plan_key_split(int64_t blocks, int heads, bool causal, float part_cost, float least_gain, Tiles tiles) {
   KeySplit plan;
-  plan.units = 0;
+  plan.units = plan.first = plan.divided = 0;
   if (blocks > kMostUnits || heads > 2 * kSms) return plan;
   const int most = tiles((int)blocks - 1);
   int unsplit = 0, parts = 1, limit = 0;
@@ -74,11 +76,16 @@ KeySplit plan_key_split(int64_t blocks, int heads, bool causal, float part_cost,
     }
     if (parts == 1) return plan;
   }
-  int units = 0;
+  int units = 0, divided = 0;
   for (int i = 0; i < blocks; ++i) {
     const int b = (int)blocks - 1 - i;  // under a causal mask the longest first
+    // causal: the longest first, so the divided ones first; else the divided ones last
     const int n = causal ? (tiles(b) + limit - 1) / limit : i < unsplit ? 1 : parts;
     if (units + n > kMostUnits || n > 255) return plan;
+    if (n > 1) {
+      if (divided == 0) plan.first = units;
+      divided += n;
+    }
     for (int part = 0; part < n; ++part, ++units) {
       plan.block[units] = (uint16_t)b;
       plan.part[units] = (uint8_t)part;
@@ -86,37 +93,38 @@ KeySplit plan_key_split(int64_t blocks, int heads, bool causal, float part_cost,
     }
   }
   plan.units = units;
+  plan.divided = divided;
   return plan;
 }
 
-// Scratch of a plan: per unit and head `rows` rows of d floats, and (maximum, denominator) of each row.
+// Scratch of a plan: per divided unit and head `rows` rows of d floats, and (maximum, denominator) of each row.
 inline size_t key_split_bytes(const KeySplit &plan, int heads, int rows, int d) {
-  return (size_t)plan.units * heads * rows * (d + 2) * sizeof(float);
+  return (size_t)plan.divided * heads * rows * (d + 2) * sizeof(float);
 }
 
 struct Partials {
-  float *sums;  // (unit, head, row, d)
-  float2 *ml;   // (unit, head, row): maximum in powers of two (-inf: no key), denominator
+  float *sums;  // (divided unit, head, row, d)
+  float2 *ml;   // (divided unit, head, row): maximum in powers of two (-inf: no key), denominator
 };
 inline Partials partials_at(void *scratch, const KeySplit &plan, int heads, int rows) {
   Partials p{nullptr, nullptr};
   if (plan.units == 0) return p;
   p.ml = static_cast<float2 *>(scratch);
-  p.sums = reinterpret_cast<float *>(p.ml + (size_t)plan.units * heads * rows);
+  p.sums = reinterpret_cast<float *>(p.ml + (size_t)plan.divided * heads * rows);
   return p;
 }
 
-// A warp per row of a divided block: out = sum_i 2^(m_i - m) sums_i / sum_i 2^(m_i - m) l_i.  blockIdx.y: unit (those that are no
-// first part of several leave at once); blockIdx.x: head and 8 rows.  d: a multiple of 4 up to 128.
+// A warp per row of a divided block: out = sum_i 2^(m_i - m) sums_i / sum_i 2^(m_i - m) l_i.  blockIdx.y: divided unit (those that are
+// no first part leave at once); blockIdx.x: head and 8 rows.  d: a multiple of 4 up to 128.
 template <typename O, int kRowsPerBlock>
 __global__ void __launch_bounds__(256) join_parts_kernel(const __grid_constant__ KeySplit plan, const Partials p, O *out, int sq, int hq, int d) {
-  const int u = blockIdx.y, n = plan.parts[u];
-  if (n == 1 || plan.part[u] != 0) return;
+  const int u = plan.first + blockIdx.y, n = plan.parts[u];
+  if (plan.part[u] != 0) return;
   grid_dependency_wait();
   const int h = blockIdx.x / (kRowsPerBlock / 8), row = blockIdx.x % (kRowsPerBlock / 8) * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   const int64_t t = (int64_t)plan.block[u] * kRowsPerBlock + row;
   if (t >= sq) return;
-  const size_t step = (size_t)hq * kRowsPerBlock, first = ((size_t)u * hq + h) * kRowsPerBlock + row;
+  const size_t step = (size_t)hq * kRowsPerBlock, first = ((size_t)blockIdx.y * hq + h) * kRowsPerBlock + row;
   float m = -INFINITY;
   for (int i = 0; i < n; ++i) m = fmaxf(m, p.ml[first + i * step].x);
   float l = 0.f;

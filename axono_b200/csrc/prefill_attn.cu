@@ -654,7 +654,7 @@ prefill_attn_f16_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __gr
     // ---- epilogue: O / l -> out ----
     if (ok && my_nkv > 0) ok = __all_sync(0xffffffffu, mbar_wait_bounded(&bar_fin[g], 0, abort_flag));
     tc_fence_after();
-    const size_t at = ((size_t)unit * p.hq + h) * (2 * kBlockM) + g * kBlockM + row;  // of divided blocks
+    const size_t at = ((size_t)(unit - split.first) * p.hq + h) * (2 * kBlockM) + g * kBlockM + row;  // of divided blocks
     float bad = 0.f;  // NaN once a stored sum is not finite
     if (parts > 1) {
       const bool any = ok && my_nkv > 0;
@@ -728,12 +728,14 @@ bool rows_map(CUtensorMap *map, const void *base, int64_t rows, int heads, int d
 
 // The 256-row form's plan; a tile of 128 keys takes about 2 us of a block.  2000 rows of 8 heads of 128 under a causal mask, 4
 // tiles saved: 37 us whole, 35 in parts; 4096 rows of 2 heads, 22 saved: 68 and 25.
-KeySplit pair_plan(int sq, int hq, int64_t skv, int is_causal) {
+KeySplit pair_plan(int sq, int hq, int64_t skv, int d, int is_causal) {
   const auto tiles = [&](int b) {
     const int64_t last = ((int64_t)b + 1) * 2 * kBlockM, end = last < sq ? last : sq;
     return (int)(((is_causal && end < skv ? end : skv) + kPairN - 1) / kPairN);
   };
-  return plan_key_split(((int64_t)sq + 2 * kBlockM - 1) / (2 * kBlockM), hq, is_causal != 0, 1.5f, 6.f, tiles);
+  KeySplit plan = plan_key_split(((int64_t)sq + 2 * kBlockM - 1) / (2 * kBlockM), hq, is_causal != 0, 1.5f, 6.f, tiles);
+  if (key_split_bytes(plan, hq, 2 * kBlockM, d) > kMostScratch) plan.units = plan.divided = 0;
+  return plan;
 }
 
 // Heads below 128 in prompts: a TMA row is a multiple of 16 bytes, and below 16 rows (of 128 that a tile holds) the
@@ -762,7 +764,7 @@ size_t axb200_sdpa_scratch_bytes(int sq, int hq, int hkv, int d, int64_t skv, in
   if (dtype == AXB200_FLOAT32 && axb::sdpa_tiled_supported(sq, hq, hkv, d, skv))
     return axb::sdpa_split_scratch_bytes(sq, hq, hkv, d, skv, is_causal);
   if (dtype == AXB200_FLOAT16 && axb::pair_form(sq, d))
-    return axb::key_split_bytes(axb::pair_plan(sq, hq, skv, is_causal), hq, 2 * axb::kBlockM, d);
+    return axb::key_split_bytes(axb::pair_plan(sq, hq, skv, d, is_causal), hq, 2 * axb::kBlockM, d);
   return 0;
 }
 
@@ -831,7 +833,7 @@ int axb200_sdpa_scratch(const void *q, const void *k, const void *v, void *out, 
     axb::KeySplit split;
     split.units = 0;
     if (scratch && axb::aligned16(scratch)) {
-      split = axb::pair_plan(sq, hq, skv, is_causal);
+      split = axb::pair_plan(sq, hq, skv, d, is_causal);
       if (scratch_bytes < axb::key_split_bytes(split, hq, 2 * axb::kBlockM, d)) split.units = 0;
     }
     const axb::Partials partials = axb::partials_at(scratch, split, hq, 2 * axb::kBlockM);
@@ -840,7 +842,7 @@ int axb200_sdpa_scratch(const void *q, const void *k, const void *v, void *out, 
     kernel<<<grid, axb::kPairThreads, axb::kPairSmemBytes, st>>>(mq, mk, mv, p, split, partials);
     if (split.units && cudaPeekAtLastError() == cudaSuccess)
       return axb::launch_dependent(axb::join_parts_kernel<__half, 2 * axb::kBlockM>,
-                                   dim3((unsigned)hq * (2 * axb::kBlockM / 8), split.units), dim3(256), 0, st, split, partials,
+                                   dim3((unsigned)hq * (2 * axb::kBlockM / 8), split.divided), dim3(256), 0, st, split, partials,
                                    static_cast<__half *>(out), sq, hq, d);
   } else {
     const dim3 grid((sq + axb::kBlockM - 1) / axb::kBlockM, hq);

@@ -41,7 +41,6 @@ namespace {
 constexpr int kRows = 128, kKeys = 64, kBox = kKeys * 64 * 2;
 constexpr int kThreads = 320, kMmaWarp = 8, kLoadWarp = 9, kSplitThreads = 256;
 constexpr float kLog2e = 1.4426950408889634f;
-constexpr size_t kMostScratch = (size_t)2 << 30;  // 170 K tokens of 8 heads of 128
 
 // kB: 64-wide blocks of the head size
 template <int kB>
@@ -361,7 +360,7 @@ split_attn_kernel(const Params p, const __grid_constant__ KeySplit split, const 
       float inv = l > 0.f ? 1.0f / l : 0.f;
       float *dst = p.out + ((size_t)t_row * p.hq + h) * p.d;
       if (parts > 1) {  // un-normalised
-        const size_t at = ((size_t)unit * p.hq + h) * kRows + row;
+        const size_t at = ((size_t)(unit - split.first) * p.hq + h) * kRows + row;
         partials.ml[at] = make_float2(l_s[kRows + row], l);
         dst = partials.sums + at * p.d;
         inv = 1.f;
@@ -418,7 +417,7 @@ int launch(const Params &p, void *parts_at, cudaStream_t st) {
   const int rc = launch_dependent(split_attn_kernel<kB>, dim3((unsigned)p.hq * (split.units ? split.units : p.q_blocks)), dim3(kThreads),
                                   Layout<kB>::kSmem, st, p, split, partials);
   if (rc != AXB200_OK || split.units == 0) return rc;
-  return launch_dependent(join_parts_kernel<float, kRows>, dim3((unsigned)p.hq * (kRows / 8), split.units), dim3(256), 0, st, split,
+  return launch_dependent(join_parts_kernel<float, kRows>, dim3((unsigned)p.hq * (kRows / 8), split.divided), dim3(256), 0, st, split,
                           partials, p.out, p.sq, p.hq, p.d);
 }
 
@@ -435,7 +434,7 @@ size_t sdpa_split_scratch_bytes(int sq, int hq, int hkv, int d, int64_t skv, int
   const size_t parts = key_split_bytes(split_plan(sq, hq, skv, is_causal), hq, kRows, d);
   const size_t total = up256((size_t)hq * q_blocks * 4) + kv_flag_bytes(hkv, n_tiles) +
                        tile_bytes(hkv, n_tiles, d) + parts;
-  return total <= kMostScratch ? total : 0;
+  return total <= kMostScratch ? total : 0;  // 170 K tokens of 8 heads of 128
 }
 
 // q, k, v, out and scratch on 16-byte boundaries; scratch of the size above.
