@@ -39,6 +39,16 @@ Tensor Scratch(size_t bytes, const std::string &device) {
   return Tensor::Uninitialized(DataType::INT8, {std::max<size_t>(bytes, 16)}, device);
 }
 
+// Scratch that a call can do without: none where memory is short.
+Tensor SpareScratch(size_t bytes, const std::string &device) {
+  if (bytes == 0) return Tensor();
+  try {
+    return Scratch(bytes, device);
+  } catch (const std::exception &) {
+    return Tensor();
+  }
+}
+
 }  // namespace
 
 Status GqaDecodeAttention(const Context &, const Tensor &q, const Tensor &k, const Tensor &v, Tensor &result) {
@@ -72,7 +82,7 @@ Status ScaledDotProductAttention(const Context &, const Tensor &q, const Tensor 
   if (st != Status::OK) return st;
   const int n = (int)sq, heads = (int)hq, kv_heads = (int)hkv, dim = (int)d, causal = is_causal ? 1 : 0, dt = Dt(q.dtype());
   Tensor rows = Scratch(axb200_sdpa_workspace_bytes(n, heads, kv_heads, dim, (int64_t)skv, dt), q.device());
-  Tensor fast = Scratch(axb200_sdpa_scratch_bytes(n, heads, kv_heads, dim, (int64_t)skv, causal, dt), q.device());
+  Tensor fast = SpareScratch(axb200_sdpa_scratch_bytes(n, heads, kv_heads, dim, (int64_t)skv, causal, dt), q.device());
   return St(axb200_sdpa_scratch(q.data(), k.data(), v.data(), result.data(), n, heads, kv_heads, dim, (int64_t)skv, causal, dt,
                                 rows.data(), rows.num_bytes(), fast.data(), fast.num_bytes(), Stream()));
 }

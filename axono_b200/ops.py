@@ -554,7 +554,12 @@ def scaled_dot_product_attention(q, k, v, is_causal: bool = False):
     lib = _capi.lib()
     causal = int(bool(is_causal))
     need = lib.axb200_sdpa_scratch_bytes(sq, hq, hkv, d, skv, causal, dt)
-    scratch = torch.empty(need, dtype=torch.uint8, device=q.device) if need else None  # of this call alone: streams may overlap
+    scratch = None
+    if need:
+        try:
+            scratch = torch.empty(need, dtype=torch.uint8, device=q.device)  # of this call alone: streams may overlap
+        except torch.OutOfMemoryError:  # the kernels that need none
+            need = 0
     # of the row-by-row form, the buffer kept for the decode operators: an address keeps counters of its own for good
     ws = workspace(q.device, lib.axb200_sdpa_workspace_bytes(sq, hq, hkv, d, skv, dt))
     _call(lib.axb200_sdpa_scratch(q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), sq, hq, hkv, d, skv, causal, dt, ws.data_ptr(),

@@ -184,3 +184,23 @@ def test_row_by_row_calls_leave_counters_to_others():
     from conftest import ROOT
 
     subprocess.run([sys.executable, "-c", ROWS_THEN_DECODE], cwd=ROOT, check=True, timeout=300)
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.float32])
+def test_prompts_where_memory_is_short(dtype, monkeypatch):
+    """An allocation of scratch that fails: the call goes on without."""
+    from axono_b200 import ops
+
+    q, k, v = tensors(1300, 1300, 2, 2, 64, dtype)
+    refused, empty = [], torch.empty
+
+    def short(*size, **kw):
+        if kw.get("dtype") is torch.uint8:
+            refused.append(size)
+            raise torch.OutOfMemoryError("no memory")
+        return empty(*size, **kw)
+
+    ops.workspace(q.device, 256)
+    monkeypatch.setattr(torch, "empty", short)
+    out = ops.scaled_dot_product_attention(q, k, v, True)
+    assert refused and torch.equal(out, without_scratch(q, k, v, True)) and ops.last_error() == 0
