@@ -386,6 +386,18 @@ def test_silu_mul_rows():
         assert oracle.rel_err(host(ops.silu_mul_rows(t16, n)), ref16) <= F16_TOL
 
 
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("rows,n", [(5000, 8), (300000, 16), (1000, 264), (66000, 1024), (3, 2048), (2, 2056), (70, 4104)])
+def test_silu_mul_rows_shapes(dtype, rows, n):
+    """Rows of less than a block, of a block and more; more row blocks than a grid has in one dimension."""
+    from axono_b200 import ops
+
+    x = torch.randn((rows, 2 * n), generator=torch.Generator(device="cuda").manual_seed(n), device="cuda").to(dtype)
+    ref = torch.nn.functional.silu(x[:, :n].float()) * x[:, n:].float()
+    tol = {torch.float32: 1e-5, torch.float16: 2.0 ** -11, torch.bfloat16: 2.0 ** -8}[dtype]  # the result's rounding; fp32: expf
+    assert ((ops.silu_mul_rows(x, n).float() - ref).abs() <= tol * ref.abs() + 1e-6).all()
+
+
 def test_context_parallel_single_rank_matches_plain():
     """World of one: exchange + merge kernels on local records give the plain result."""
     from axono_b200 import ops
