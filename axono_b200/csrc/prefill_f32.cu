@@ -2,7 +2,7 @@
 // ScaledDotProductAttention takes (src/ops/cuda/sequence.cu:451-472), head sizes up to 128.
 //
 // A float is the exact sum of three bf16 parts (8 bits each, round to nearest), so a product of two floats is nine products
-// of parts, of which the three smallest (2^-24 of the whole) are left out: six tcgen05.mma products per Q.K^T and per P.V,
+// of parts, of which the three smallest (2^-26 of the whole) are left out: six tcgen05.mma products per Q.K^T and per P.V,
 // smallest first, stand in for fp32 multiply-adds.  What remains is the tensor core's own accumulation, which truncates: a
 // running sum over all keys would lose a bit per product step, so every tile of 64 keys starts O anew in tensor memory and
 // the tiles are added up in fp32 registers, rescaled as the row's maximum moves.
@@ -396,6 +396,9 @@ KeySplit split_plan(int sq, int hq, int64_t skv, int is_causal) {
   return plan_key_split(((int64_t)sq + kRows - 1) / kRows, hq, is_causal != 0, 3.f, 5.f, tiles);
 }
 
+// Keys that some row sees: the others are not split into parts (16 rows over 8192 keys, 16 / 8 heads of 128, causal: 41 us with all).
+int64_t visible_keys(int sq, int64_t skv, int is_causal) { return is_causal && skv > sq ? sq : skv; }
+
 template <int kB>
 int launch(const Params &p, void *parts_at, cudaStream_t st) {
   static std::mutex mu;
@@ -427,6 +430,7 @@ int launch(const Params &p, void *parts_at, cudaStream_t st) {
 // tiles in a row there, waves of blocks times tiles of keys.  48 rows and keys, 16 / 8 heads of 128: 23 us in one launch, 32 in
 // three.  100 rows and keys: 55 and 29; 2000 rows, 64 keys: 70 and 39; 16 rows, 128 keys, 2 heads of 64: 25 and 28.
 size_t sdpa_split_scratch_bytes(int sq, int hq, int hkv, int d, int64_t skv, int is_causal) {
+  skv = visible_keys(sq, skv, is_causal);
   const int64_t in_a_row = (((int64_t)sq * hq + 128 * 148 - 1) / (128 * 148)) * ((skv + kKeys - 1) / kKeys);
   const int64_t rows = (int64_t)sq * (hq / hkv);
   if (d % 4 || d > 128 || sq < 16 || hkv > 65535 || in_a_row < (rows >= kRows ? 2 : 3)) return 0;
@@ -440,6 +444,7 @@ size_t sdpa_split_scratch_bytes(int sq, int hq, int hkv, int d, int64_t skv, int
 // q, k, v, out and scratch on 16-byte boundaries; scratch of the size above.
 int sdpa_split(const void *q, const void *k, const void *v, void *out, int sq, int hq, int hkv, int d, int64_t skv, int is_causal,
                void *scratch, cudaStream_t st) {
+  skv = visible_keys(sq, skv, is_causal);
   Params p{};
   p.q = static_cast<const float *>(q);
   p.k = static_cast<const float *>(k);

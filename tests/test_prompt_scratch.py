@@ -31,6 +31,12 @@ def test_scratch_is_bounded(dtype):
     assert scratch(4096, 2, 2, 128, 4096, 1, dtype) > 0
 
 
+def test_keys_that_no_row_sees_take_none():
+    """Under a causal mask row t sees key t at most: a few rows over a long cache are the small problem they are alone."""
+    assert scratch(16, 16, 8, 128, 8192, 1, _capi.FLOAT32) == 0 < scratch(16, 16, 8, 128, 8192, 0, _capi.FLOAT32)
+    assert scratch(300, 16, 8, 128, 50000, 1, _capi.FLOAT32) == scratch(300, 16, 8, 128, 300, 1, _capi.FLOAT32)
+
+
 @pytest.mark.parametrize("bad", [(0, 2, 2, 64, 64), (64, 0, 2, 64, 64), (64, 2, 0, 64, 64), (64, 3, 2, 64, 64), (64, 2, 2, 0, 64),
                                  (64, 2, 2, 64, 0), (64, 2, 2, 64, 2 ** 31)])
 def test_calls_that_are_refused_want_none(bad):
