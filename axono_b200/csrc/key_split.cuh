@@ -30,8 +30,7 @@ __host__ __device__ inline int split_begin(int tiles, int part, int parts) { ret
 // its tiles, in tiles; least_gain: tiles in a row that a division has to save, as many as joining takes (4 to 6 us with its launch).
 template <typename Tiles>
 KeySplit plan_key_split(int64_t blocks, int heads, bool causal, float part_cost, float least_gain, Tiles tiles) {
-  KeySplit plan;
-  plan.units = plan.first = plan.divided = 0;
+  KeySplit plan{};
   if (blocks > kMostUnits || heads > 2 * kSms) return plan;
   const int most = tiles((int)blocks - 1);
   int unsplit = 0, parts = 1, limit = 0;
