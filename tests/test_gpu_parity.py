@@ -540,6 +540,8 @@ def test_sdpa_fp16_tensor_core_path(ops, orc, causal, sq, skv):
 
 @pytest.mark.parametrize("dtype,hq,hkv,d", [(torch.float32, 16, 8, 128), (torch.float32, 4, 2, 64), (torch.float16, 4, 4, 64)])
 def test_sdpa_row_fallback(ops, orc, dtype, hq, hkv, d):
+    """70 rows over 300 keys: fp32 through the form in three bf16 parts, fp16 with heads of 64 through the tensor-core form for
+    narrow heads (the row-by-row form: test_sdpa_row_by_row)."""
     rng = np.random.default_rng(d + hq)
     sq, skv = 70, 300
     q = rng.standard_normal((sq, hq, d)).astype(np.float32)
@@ -552,12 +554,27 @@ def test_sdpa_row_fallback(ops, orc, dtype, hq, hkv, d):
         assert_close(out, orc.sdpa(q, k, v, causal), F32_TOL if dtype == torch.float32 else F16_TOL)
 
 
+@pytest.mark.parametrize("dtype,hq,hkv,d,sq", [(torch.float32, 16, 8, 128, 5), (torch.float32, 4, 2, 6, 70), (torch.float32, 4, 2, 256, 40),
+                                               (torch.float16, 4, 4, 64, 15), (torch.float16, 4, 2, 250, 40)])
+def test_sdpa_row_by_row(ops, orc, dtype, hq, hkv, d, sq):
+    """Fewer than 16 rows, head sizes that are no multiple of 4 or above 192: each row a sequence of the decode kernels."""
+    rng = np.random.default_rng(d + sq)
+    q, k, v = (rng.standard_normal(s).astype(np.float32) for s in ((sq, hq, d), (300, hkv, d), (300, hkv, d)))
+    if dtype == torch.float16:
+        q, k, v = widen(q), widen(k), widen(v)
+    for causal in (False, True):
+        out = host(ops.scaled_dot_product_attention(dev(q, dtype), dev(k, dtype), dev(v, dtype), causal))
+        assert_close(out, orc.sdpa(q, k, v, causal), F32_TOL if dtype == torch.float32 else F16_TOL)
+    assert ops.last_error() == 0
+
+
 @pytest.mark.parametrize("dtype", [torch.float32, torch.float16])
 @pytest.mark.parametrize("hq,hkv,d", [(16, 8, 128), (4, 4, 64), (6, 2, 80), (16, 2, 96), (3, 1, 8), (8, 8, 192)])
 @pytest.mark.parametrize("sq,skv", [(16, 16), (70, 300), (300, 70), (257, 257), (1000, 1000), (33, 2049)])
 def test_sdpa_tiled_fma_path(ops, orc, dtype, hq, hkv, d, sq, skv):
-    """The tiled FMA prefill kernel (FLOAT32, and head sizes other than 128): both mask modes, query
-    blocks that do not divide sq, groups 1 / 2 / 3 / 8, more queries than keys and the reverse."""
+    """Prompts in FLOAT32 and with head sizes other than 128: both mask modes, query blocks that do not divide sq, groups
+    1 / 2 / 3 / 8, more queries than keys and the reverse.  Heads of 192 and the smallest FLOAT32 prompts run on the tiled FMA
+    kernel, the others on the tensor cores (the FMA kernel at their sizes: tests/test_gpu_prompt_attention.py)."""
     rng = np.random.default_rng(sq * 31 + skv * 7 + d + hq)
     q = rng.standard_normal((sq, hq, d)).astype(np.float32)
     k = rng.standard_normal((skv, hkv, d)).astype(np.float32)
@@ -626,8 +643,7 @@ def test_sdpa_long_prefill_rows_match_decode(ops):
 
 @pytest.mark.parametrize("d", [128, 64])
 def test_sdpa_tiled_long_rows_match_decode(ops, d):
-    """The tiled FMA prefill kernel at 3000 tokens in FLOAT32 (both CTA shapes: 128 virtual rows at
-    head_dim 128, and the same at 64): sampled causal rows against decode attention over their prefixes."""
+    """A FLOAT32 prompt of 3000 tokens: sampled causal rows against decode attention over their prefixes."""
     g = torch.Generator(device="cuda").manual_seed(78 + d)
     s = 3000
     q = torch.randn((s, 16, d), generator=g, device="cuda")

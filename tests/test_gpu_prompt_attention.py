@@ -83,6 +83,69 @@ def test_fp32_values_without_three_parts(d):
     assert ops.last_error() == 0
 
 
+@pytest.mark.parametrize("source", ["k", "v", "q"])
+@pytest.mark.parametrize("sq,skv,hq,hkv", [(200, 260, 8, 4), (1536, 1536, 16, 8)])  # the second divides keys where nothing is masked
+def test_fp32_only_the_flagged_head_is_done_over(source, sq, skv, hq, hkv):
+    """One value without three parts, in one head's keys or values or in one query row of the last block: that KV head comes out
+    as from the FMA kernel, the others bit for bit as from clean inputs."""
+    from axono_b200 import ops
+
+    for causal in (True, False):
+        q, k, v = tensors(sq, skv, hq, hkv, 64, torch.float32)
+        clean = ops.scaled_dot_product_attention(q, k, v, causal)
+        {"k": k, "v": v, "q": q}[source][sq - 1 if source == "q" else 100, 2 if source == "q" else 1, 5] = 1e-33
+        out, fma = ops.scaled_dot_product_attention(q, k, v, causal), without_scratch(q, k, v, causal)
+        flagged = torch.arange(hq, device="cuda") // (hq // hkv) == 1
+        assert torch.equal(out[:, flagged], fma[:, flagged]) and not torch.equal(fma[:, flagged], clean[:, flagged])
+        assert torch.equal(out[:, ~flagged], clean[:, ~flagged])
+    assert ops.last_error() == 0
+
+
+@pytest.mark.parametrize("d", [64, 128])
+@pytest.mark.parametrize("qo,ko,vo", [(0, 2, 0), (2, 2, 0), (0, 0, 4), (2, 2, 4)])
+def test_fp32_with_common_offsets(d, qo, ko, vo):
+    """Where the sums' terms have one sign, truncation has too: the error stays below that of the FMA kernel, which rounds."""
+    from axono_b200 import ops
+
+    for sq, skv, causal in ((300, 300, True), (300, 2700, False), (1536, 1536, False)):
+        q, k, v = tensors(sq, skv, 4, 2, d, torch.float32)
+        q, k, v = q + qo, k + ko, v + vo
+        ref = attention(q, k, v, causal)
+        err = [(out.double() - ref).norm().item() for out in (ops.scaled_dot_product_attention(q, k, v, causal), without_scratch(q, k, v, causal))]
+        assert err[0] <= err[1], (sq, skv, err)
+    assert ops.last_error() == 0
+
+
+def plain(q, k, v, causal, dtype, tol):
+    out, ref = without_scratch(q, k, v, causal).double(), attention(q, k, v, causal)
+    group = q.shape[1] // k.shape[1]
+    top = (torch.einsum("qhd,khd->hqk", q.float(), k.float().repeat_interleave(group, 1)).abs().max() * q.shape[2] ** -0.5).item()
+    bound = v.float().abs().max().item() * (2 * top * 2.0 ** -21 + 2.0 ** -20) + (ref.abs() * tol if tol else 0.0)
+    assert ((out - ref).abs() <= bound).all()
+
+
+@pytest.mark.parametrize("hq,hkv,d", [(16, 8, 128), (4, 4, 64), (6, 2, 80), (16, 2, 96), (3, 1, 8)])
+@pytest.mark.parametrize("sq,skv", [(16, 16), (70, 300), (300, 70), (257, 257), (33, 2049)])
+def test_fp32_without_scratch(hq, hkv, d, sq, skv):
+    """The FMA kernel in fp32, which serves calls without scratch and the heads whose values have no three parts.  A score is off
+    by 2^-21 of the largest one, sums and the result by 2^-20."""
+    for causal in (True, False):
+        plain(*tensors(sq, skv, hq, hkv, d, torch.float32), causal, torch.float32, 0.0)
+
+
+@pytest.mark.parametrize("hq,hkv,d", [(4, 2, 12), (3, 3, 20), (8, 1, 68), (4, 2, 100), (4, 2, 64), (4, 2, 128)])
+@pytest.mark.parametrize("sq,skv", [(16, 16), (70, 300), (257, 257), (33, 1025)])
+def test_fp16_on_the_fma_kernel(hq, hkv, d, sq, skv):
+    """fp16 head sizes off the multiples of 8, and (64 and 128) tensors one element off 16 bytes: the result's rounding is 2^-11 of
+    it, the rest as in fp32."""
+    for causal in (True, False):
+        q, k, v = tensors(sq, skv, hq, hkv, d, torch.float16)
+        if d % 8 == 0:
+            q, k, v = (torch.cat([t.new_zeros(1), t.flatten()])[1:].view(t.shape) for t in (q, k, v))
+            assert k.data_ptr() % 16
+        plain(q, k, v, causal, torch.float16, 2.0 ** -11)
+
+
 @pytest.mark.parametrize("d", [8, 64, 128])
 @pytest.mark.parametrize("sq,skv,hq,hkv", [(256, 4100, 2, 1), (300, 1500, 3, 3), (1300, 1300, 2, 2), (2700, 2700, 16, 8),
                                            (2305, 900, 16, 16), (3000, 3100, 4, 2)])
