@@ -355,6 +355,27 @@ __device__ __forceinline__ uint32_t split_half2(float a, float b, uint32_t &lo) 
   return *reinterpret_cast<const uint32_t *>(&hi);
 }
 
+// The tensor core adds up by truncation: a running sum over all keys loses about a quarter of a unit of its last bit, towards zero,
+// with each of a tile's 16 products (1.8e-5 of the values by 8192 keys, 6e-5 where these have a common offset).  So every
+// kFlushTiles tiles O starts anew, and what it held joins a thread's sums in local memory, kept in fp32 with the rescaling they
+// still owe.  (Out of line, so that the sums stay out of the registers of the loop that calls it.)  8192 keys, heads of 64: error
+// 2.084e-4 without, 2.075e-4 so, as on the FMA pipe; with a common offset 2.316e-4, 2.239e-4 and 2.238e-4.  2700 patches, 16 heads
+// of 64: 112 us without, 116 so, 121 with every fourth tile; sums in shared memory that heads of 64 leave free: 117.
+constexpr int kFlushTiles = 8;
+__device__ __noinline__ void flush_sums(float4 *sums, uint32_t tmem_o, int d, bool first, float owed) {
+#pragma unroll 1
+  for (int c = 0; c * 32 < d; ++c) {
+    uint32_t r[32];
+    tmem_ld32(tmem_o + c * 32, r);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const float4 old = first ? make_float4(0.f, 0.f, 0.f, 0.f) : sums[c * 8 + i];
+      sums[c * 8 + i] = make_float4(fmaf(old.x, owed, __uint_as_float(r[4 * i])), fmaf(old.y, owed, __uint_as_float(r[4 * i + 1])),
+                                    fmaf(old.z, owed, __uint_as_float(r[4 * i + 2])), fmaf(old.w, owed, __uint_as_float(r[4 * i + 3])));
+    }
+  }
+}
+
 // One row over the keys [key0, key1) with a weight of one part, as the definition has it.  A weight in two parts meets V twice, and
 // where V is infinite hi * V + lo * V is NaN (lo may be 0 or negative) though the row's value is +-inf; and every row of a block
 // multiplies the V of all its tiles, also those that its mask hides.  So a thread whose row is not finite does it over - only
@@ -568,7 +589,7 @@ prefill_attn_f16_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __gr
 #pragma unroll
             for (int ks = 0; ks < kPairN / 16; ++ks)
               umma_f16_ts(tmem_base + 256 + g * 128, tmem_base + g * 128 + part * 64 + ks * 8, dvs + (uint64_t)(ks * (2048 >> 4)),
-                          idesc_pv, j > 0 || part > 0 || ks > 0);
+                          idesc_pv, (kNarrow ? j % kFlushTiles != 0 : j > 0) || part > 0 || ks > 0);
           if (j == nkv_g[g] - 1) umma_commit(&bar_fin[g]);
           if (j + 1 < nkv_g[g]) issue_s(g, j + 1);
         }
@@ -585,6 +606,8 @@ prefill_attn_f16_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __gr
     const uint32_t lane_base = (uint32_t)((warp & 3) * 32) << 16;
     const uint32_t tmem_s = tmem_base + g * 128 + lane_base, tmem_o = tmem_base + 256 + g * 128 + lane_base;
     float m_run = -INFINITY, l_run = 0.f;
+    float4 sums[kNarrow ? kD / 4 : 1];  // what flush_sums has taken, and the factor it has to be multiplied with
+    float owed = 1.f;
     bool ok = true;
     for (int j = 0; j < my_nkv && ok; ++j) {
       ok = __all_sync(0xffffffffu, mbar_wait_bounded(&bar_s[g], j & 1, abort_flag));
@@ -635,7 +658,11 @@ prefill_attn_f16_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __gr
       const float2 sum = unpack_f32x2(add_f32x2(add_f32x2(sum2[0], sum2[1]), add_f32x2(sum2[2], sum2[3])));
       l_run = l_run * corr + (sum.x + sum.y);
       // S_g(j) was queued behind P_g(j-1).V_{j-1}, so that product is complete: O_g may be rescaled
-      if (j > 0 && moved) {
+      if (kNarrow && j > 0 && j % kFlushTiles == 0) {  // P_g(j).V_j starts O_g anew
+        flush_sums(sums, tmem_o, p.d, j == kFlushTiles, owed);
+        owed = corr;
+      } else if (j > 0 && moved) {
+        if (kNarrow) owed *= corr;
 #pragma unroll
         for (int c = 0; c < 4; ++c) {
           if (kNarrow && c * 32 >= p.d) break;
@@ -656,6 +683,14 @@ prefill_attn_f16_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __gr
     tc_fence_after();
     const size_t at = ((size_t)(unit - split.first) * p.hq + h) * (2 * kBlockM) + g * kBlockM + row;  // of divided blocks
     float bad = 0.f;  // NaN once a stored sum is not finite
+    const auto load_o = [&](int c, uint32_t (&r)[32]) {
+      tmem_ld32(tmem_o + c * 32, r);
+      if (kNarrow && my_nkv > kFlushTiles) {
+        const float *old = reinterpret_cast<const float *>(sums) + c * 32;
+#pragma unroll
+        for (int i = 0; i < 32; ++i) r[i] = __float_as_uint(fmaf(old[i], owed, __uint_as_float(r[i])));
+      }
+    };
     if (parts > 1) {
       const bool any = ok && my_nkv > 0;
       if (t_row < p.sq) partials.ml[at] = any ? make_float2(m_run, l_run) : make_float2(-INFINITY, 0.f);
@@ -665,7 +700,7 @@ prefill_attn_f16_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __gr
         for (int c = 0; c < 4; ++c) {
           if (kNarrow && c * 32 >= p.d) break;
           uint32_t r[32];
-          tmem_ld32(tmem_o + c * 32, r);
+          load_o(c, r);
           if (t_row < p.sq) {
 #pragma unroll
             for (int u = 0; u < 8; ++u) {
@@ -685,7 +720,7 @@ prefill_attn_f16_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __gr
       for (int c = 0; c < 4; ++c) {
         if (kNarrow && c * 32 >= p.d) break;
         uint32_t r[32];
-        tmem_ld32(tmem_o + c * 32, r);
+        load_o(c, r);
         if (t_row < p.sq) {
 #pragma unroll
           for (int u = 0; u < 4; ++u) {
@@ -830,8 +865,7 @@ int axb200_sdpa_scratch(const void *q, const void *k, const void *v, void *out, 
   p.k = static_cast<const __half *>(k);
   p.v = static_cast<const __half *>(v);
   if (pair) {
-    axb::KeySplit split;
-    split.units = 0;
+    axb::KeySplit split{};
     if (scratch && axb::aligned16(scratch)) {
       split = axb::pair_plan(sq, hq, skv, d, is_causal);
       if (scratch_bytes < axb::key_split_bytes(split, hq, 2 * axb::kBlockM, d)) split.units = 0;

@@ -146,6 +146,22 @@ def test_fp16_on_the_fma_kernel(hq, hkv, d, sq, skv):
         plain(q, k, v, causal, torch.float16, 2.0 ** -11)
 
 
+@pytest.mark.parametrize("d", [64, 80])
+@pytest.mark.parametrize("offset", [0, 4])
+def test_fp16_narrow_sums_do_not_drift(d, offset):
+    """Sums over thousands of values: the tensor core's truncation pulls them towards zero with each of the 16 products of a tile of
+    128 keys, by some 1e-5 over the 8 tiles after which a sum starts anew, which adds its square to that of the result's rounding
+    (2.2e-4): a thousandth above the FMA kernel's error at most."""
+    from axono_b200 import ops
+
+    q, k, v = tensors(8192, 8192, 4, 2, d, torch.float16)
+    v = v + offset
+    off = [torch.cat([t.new_zeros(1), t.flatten()])[1:].view(t.shape) for t in (q, k, v)]  # off 16 bytes: the FMA kernel
+    ref = attention(q, k, v, False)
+    err = [(ops.scaled_dot_product_attention(*args, False).double() - ref).norm().item() for args in ((q, k, v), off)]
+    assert err[0] <= 1.001 * err[1], err
+
+
 @pytest.mark.parametrize("d", [8, 64, 128])
 @pytest.mark.parametrize("sq,skv,hq,hkv", [(256, 4100, 2, 1), (300, 1500, 3, 3), (1300, 1300, 2, 2), (2700, 2700, 16, 8),
                                            (2305, 900, 16, 16), (3000, 3100, 4, 2)])
