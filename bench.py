@@ -45,6 +45,7 @@ import ctypes
 import gc
 import json
 import os
+import re
 import statistics
 import sys
 import threading
@@ -1140,9 +1141,11 @@ def run_reference_cuda(args):
 
 def run_prefill(args):
     """`prefill`: causal prefill attention (sq = skv = --prefill-len, 16 q / 8 kv heads, head_dim 128).
-    fp16 runs on the tcgen05 kernel: tensor-bound, the roofline is the measured dense GEMM peak.
-    `--dtype f32` (the reference's own type) runs on the tiled FMA kernel: the bound is the fp32 FMA
-    pipe, 148 SMs x 128 lanes x 2 flop x the maximum SM clock (nominal; no measured figure exists)."""
+    fp16 runs on the tcgen05 kernels: tensor-bound, the roofline is the measured dense GEMM peak.
+    `--dtype f32` (the reference's own type) runs there as six bf16 products of parts per product (a sixth of
+    that peak), and the smallest prompts on the tiled FMA kernel: the bound is then the fp32 FMA pipe, 148 SMs
+    x 128 lanes x 2 flop x the maximum SM clock (nominal; no measured figure exists).  Kernel and number of
+    launches are those of one more call, after the timed ones, under torch's profiler."""
     import torch
 
     from axono_b200 import ops
@@ -1177,17 +1180,24 @@ def run_prefill(args):
             peak, kind = float(json.load(f)["bf16_tflops"]), "measured"
     except Exception:
         peak, kind = 1590.0, "fallback"
-    kernel = "prefill_attn_f16_pair_kernel" if S >= 256 else "prefill_attn_f16_kernel"
+    with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA]) as prof:
+        ops.scaled_dot_product_attention(q, k, v, True)
+        torch.cuda.synchronize()
+    own = [e for e in prof.events() if "axb::" in e.name]
+    longest = max(own, key=lambda e: e.device_time).name
+    kernel = re.search(r"(\w+_kernel)", longest).group(1)
     bound = "tensor"
-    if f32:  # six bf16 products of parts for one of floats
-        peak, kind, kernel = peak / 6, f"{kind} bf16 / 6", "split_attn_kernel"
+    if kernel == "split_attn_kernel":
+        peak, kind = peak / 6, f"{kind} bf16 / 6"
+    elif kernel == "sdpa_tiled_kernel":
+        peak, kind, bound = 148 * 128 * 2 * 1.965e9 / 1e12, "nominal fp32 FMA", "fma"
     err = ops.last_error()
     print(json.dumps({
         "metric": "prefill_attention_tflops", "value": tflops, "unit": "TFLOP/s", "n_gpus": 1, "steps": args.steps,
         "warmup": args.warmup, "ms_per_step": ms, "higher_is_better": True, "scaling": "weak", "vs_baseline": None,
         "dtype": args.dtype, "data": "synthetic",
         "config": {"workload": "prefill", "sq": S, "skv": S, "hq": HQ, "hkv": HKV, "head_dim": D, "causal": True},
-        "tokens_per_s": S / (ms / 1e3), "gpu_launches": args.steps, "error_word": err, "clocks": sampler.summary(),
+        "tokens_per_s": S / (ms / 1e3), "gpu_launches": args.steps * len(own), "error_word": err, "clocks": sampler.summary(),
         "roofline": {"bound": bound, "kernel": kernel, "achieved": tflops, "peak": peak,
                      "unit": "TFLOP/s", "frac": tflops / peak, "peak_source": f"of {kind}", "traffic": None},
     }), flush=True)
