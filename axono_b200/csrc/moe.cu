@@ -120,6 +120,7 @@ __global__ void __launch_bounds__(kRouteWarps * 32) moe_route_kernel(const Route
 // Every CTA forms the offsets for itself (a scan over the experts in shared memory) and copies its tokens'
 // rows to their places; CTA 0 also stores offsets and tiles.
 constexpr int kSortThreads = 256, kSortWarps = kSortThreads / 32;
+template <bool kWarps>  // a warp per row, else a block
 __global__ void __launch_bounds__(kSortThreads)
 moe_sort_kernel(const uint8_t *x, uint8_t *sorted, const int32_t *ids, const int32_t *place, const int32_t *counts,
                 int32_t *row_of, int32_t *offsets, int4 *tiles, int32_t *n_tiles, int rows, int experts, int top,
@@ -157,17 +158,13 @@ moe_sort_kernel(const uint8_t *x, uint8_t *sorted, const int32_t *ids, const int
       }
     if (threadIdx.x == 0) *n_tiles = toffs[experts];
   }
-  // a warp per row, its pieces in flight eight at a time (2000 tokens, 6 experts each, rows of 4 KB: 18.8 us with a block per row,
-  // whose threads had one piece each to wait for; now 16.2)
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  for (int64_t item = (int64_t)blockIdx.x * kSortWarps + warp; item < (int64_t)rows * top; item += (int64_t)gridDim.x * kSortWarps) {
-    const int dst = offs[ids[item]] + place[item];
-    if (lane == 0) row_of[item] = dst;
-    const uint8_t *s = x + (size_t)(item / top) * row_bytes;
-    uint8_t *d = sorted + (size_t)dst * row_bytes;
-    if (unit == 16) {
-      const uint4 *from = reinterpret_cast<const uint4 *>(s);
-      uint4 *to = reinterpret_cast<uint4 *>(d);
+  if constexpr (kWarps) {  // 16-byte pieces, eight in flight at a time
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    for (int64_t item = (int64_t)blockIdx.x * kSortWarps + warp; item < (int64_t)rows * top; item += (int64_t)gridDim.x * kSortWarps) {
+      const int dst = offs[ids[item]] + place[item];
+      if (lane == 0) row_of[item] = dst;
+      const uint4 *from = reinterpret_cast<const uint4 *>(x + (size_t)(item / top) * row_bytes);
+      uint4 *to = reinterpret_cast<uint4 *>(sorted + (size_t)dst * row_bytes);
       const int n = row_bytes / 16;
       int i = lane;
       for (; i + 7 * 32 < n; i += 8 * 32) {
@@ -178,8 +175,19 @@ moe_sort_kernel(const uint8_t *x, uint8_t *sorted, const int32_t *ids, const int
         for (int u = 0; u < 8; ++u) to[i + u * 32] = v[u];
       }
       for (; i < n; i += 32) to[i] = from[i];
-    } else {
-      for (int i = lane; i < row_bytes / 2; i += 32) reinterpret_cast<uint16_t *>(d)[i] = reinterpret_cast<const uint16_t *>(s)[i];
+    }
+  } else {
+    for (int item = blockIdx.x; item < rows * top; item += gridDim.x) {
+      const int e = ids[item], dst = offs[e] + place[item];
+      if (threadIdx.x == 0) row_of[item] = dst;
+      const uint8_t *s = x + (size_t)(item / top) * row_bytes;
+      uint8_t *d = sorted + (size_t)dst * row_bytes;
+      if (unit == 16)
+        for (int i = threadIdx.x; i < row_bytes / 16; i += kSortThreads)
+          reinterpret_cast<uint4 *>(d)[i] = reinterpret_cast<const uint4 *>(s)[i];
+      else
+        for (int i = threadIdx.x; i < row_bytes / 2; i += kSortThreads)
+          reinterpret_cast<uint16_t *>(d)[i] = reinterpret_cast<const uint16_t *>(s)[i];
     }
   }
 }
@@ -319,9 +327,14 @@ int axb200_moe_sort(const void *x, void *sorted, const int32_t *ids, const int32
   if (rows == 0) return AXB200_OK;
   const int row_bytes = (int)(width * es);
   const bool vec = row_bytes % 16 == 0 && ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(sorted)) & 15u) == 0;
-  const int64_t blocks = (rows * top + axb::kSortWarps - 1) / axb::kSortWarps;
+  // A block per row, or a warp, which has eight loads to wait for instead of one: better where the rows are many (us, block and
+  // warp: 12000 rows of 4 KB 12.4 and 10.0, 6000 7.5 and 7.2, 3000 5.0 and 5.1; 6000 of 8 KB 10.4 and 10.2, 3000 7.0 and 8.1; 48
+  // of 4 KB 2.4 and 2.9), and never with 2-byte pieces (12000 rows of 2050: 22 and 35).
+  const bool warps = vec && rows * top >= 6000;
+  const int64_t blocks = warps ? (rows * top + axb::kSortWarps - 1) / axb::kSortWarps : rows * top;
   const int grid = (int)(blocks < 148 * 8 ? blocks : 148 * 8);
-  return axb::launch_dependent(axb::moe_sort_kernel, dim3(grid), dim3(axb::kSortThreads), (size_t)2 * (experts + 1) * sizeof(int),
+  auto *kernel = warps ? axb::moe_sort_kernel<true> : axb::moe_sort_kernel<false>;
+  return axb::launch_dependent(kernel, dim3(grid), dim3(axb::kSortThreads), (size_t)2 * (experts + 1) * sizeof(int),
                                static_cast<cudaStream_t>(stream), static_cast<const uint8_t *>(x), static_cast<uint8_t *>(sorted),
                                ids, place, counts, row_of, offsets, reinterpret_cast<int4 *>(tiles), n_tiles, (int)rows, experts,
                                top, tile_rows, row_bytes, vec ? 16 : 2);

@@ -254,6 +254,21 @@ def test_route_many_rows():
 
 
 @pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("width", [2050, 2048, 4104])  # 2-byte pieces (bf16); more than a warp's eight loads
+@pytest.mark.parametrize("n", [1, 40, 999, 1000, 2000])  # a block per row and, from 6000 rows on, a warp
+def test_sort_copies_rows(dtype, width, n):
+    from axono_b200 import ops
+
+    logits = torch.randn(n, 64, generator=torch.Generator().manual_seed(n)).cuda()
+    ids, _, place, counts = ops.moe_route(logits, None, 1, 1, 6, 1.0)
+    x = torch.randn(n, width, generator=torch.Generator().manual_seed(width)).cuda().to(dtype)
+    rows, row_of, offsets, _, _ = ops.moe_sort(x, ids, place, counts, 64)
+    assert torch.equal(rows[row_of.flatten().long()], x.repeat_interleave(6, 0))
+    assert torch.equal(row_of, offsets[ids.long()] + place)
+    assert sorted(row_of.flatten().tolist()) == list(range(6 * n))
+
+
+@pytest.mark.parametrize("dtype", DTYPES)
 @pytest.mark.parametrize("width,ff,experts,top,n", [(76, 44, 6, 3, 50), (200, 72, 12, 3, 9), (264, 104, 7, 2, 1), (384, 192, 16, 4, 300),
                                                     (512, 384, 4, 2, 1500), (256, 128, 8, 2, 60), (256, 128, 3, 3, 33), (128, 256, 32, 1, 40)])
 def test_experts(dtype, width, ff, experts, top, n):
