@@ -1174,9 +1174,9 @@ gqa_split_f16_kernel(const __grid_constant__ CUtensorMap tmK,
 // by exchanges that halve the number of values a lane still holds (4 + 2 + 1, then one value each): 9 or 8 shuffles
 // instead of 40, and every lane ends with the score of one token, so that a token's exponential is taken by the 4 or 2
 // lanes that hold it instead of all 32.
-// Bound by HBM at long lengths, by the latency of its one wave at short ones.  us per call, 16 / 8 heads: d = 128, 1000
-// tokens 10.4 before the exchanges and 9.1 with them, 32768 tokens 48.5 and 47.2 (5.7 TB/s); d = 64, 16001 tokens 66.5 on
-// the generic kernel and 17.4 here; d = 96, 26000 tokens 136 and 31; d = 8, 4096 tokens (8 / 8 heads) 21.3 and 6.6.
+// Bound by HBM at long lengths, by the latency of its one wave at short ones.  us per call in a graph, 16 / 8 heads: d = 128, 1000
+// tokens 10.7 before the exchanges and 9.5 with them (a single call takes 12.3 either way: its host side), 32768 tokens 48.5 and
+// 47.2 (5.7 TB/s); d = 64, 16001 tokens 66.5 on the generic kernel and 17.4 here; d = 96, 26000 tokens 136 and 31; d = 8, 4096 tokens (8 / 8 heads) 21.3 and 6.6.
 __host__ __device__ constexpr int f32_tile_width(int d) { return d <= 64 ? 64 : 128; }
 __host__ __device__ constexpr int f32_tile_tokens(int tile_width) { return kStageBytes / 2 / 4 / tile_width; }
 

@@ -447,8 +447,8 @@ __device__ __noinline__ void redo_narrow_row(const PrefillParams &p, int t_row, 
 // out - Q.K^T does not step into it, and the columns of O that P.V forms from whatever stands there are never stored.
 // P.V keeps N = 128 whatever the head size: products of one shape need no wait between P.V and the S that overwrites P.
 // Bound by the products of P.V and the softmax about equally.  2700 x 2700 keys, 16 heads of 64, not causal:
-// 111 us, 91 with the last blocks divided (key_split.cuh), against 1921 us on the FMA pipe; the same error against 64 bits
-// (2.1e-4, the rounding of the result).
+// 111 us, 91 with the last blocks divided (key_split.cuh) and 95 with sums that start anew, against 1921 us on the FMA pipe; the
+// same error against 64 bits (2.1e-4, the rounding of the result).
 template <bool kNarrow>
 __global__ void __launch_bounds__(kPairThreads, 1)
 prefill_attn_f16_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,

@@ -21,7 +21,7 @@
 // the flags of their tiles make the FMA kernel of prefill_tiled.cu, launched behind, redo that KV head; else it returns at once.
 //
 // Bound by the tensor core: 12 products per tile.  Those of P.V take 71 cycles of the possible 64, those of Q.K^T, only 64 wide,
-// 62 instead of 32 (their A operand comes no faster).  1536 tokens, 16 / 8 heads of 128, causal: 744 us on the FMA pipe, 97
+// 62 instead of 32 (their A operand comes no faster).  1536 tokens, 16 / 8 heads of 128, causal: 744 us on the FMA pipe, 100
 // here, the error against 64 bits 4.2e-7 there and 1.9e-7 here; 4096 tokens, 32 heads, not causal: 11.3 and 1.46 ms.
 #include <math.h>
 
@@ -387,7 +387,7 @@ size_t kv_flag_bytes(int hkv, int64_t n_tiles) { return up256((size_t)2 * hkv * 
 
 // A tile of 64 keys takes 2 to 3 us of a block, a block three tiles more (Q's parts, the first copies, the result).  1536 rows of 16
 // heads of 128, not causal: 176 us whole, 140 in parts; 4096 rows of 2 heads, causal: 208 and 91.  Where the SMs are nearly full
-// a division gains nothing (1536 rows of 16 heads, causal: 92 us both, before the joining), hence the five tiles.
+// a division gains nothing (1536 rows of 16 heads, causal: the attention kernel alone 92 us both, before the joining), hence the five tiles.
 KeySplit split_plan(int sq, int hq, int64_t skv, int is_causal) {
   const auto tiles = [&](int b) {
     const int64_t last = ((int64_t)b + 1) * kRows, end = last < sq ? last : sq;
