@@ -10,7 +10,8 @@ projections are library GEMMs (one cuBLASLt call each through `ops.linear_nobias
 timed per shape on first use; `lt_gemm=False` takes torch.matmul), which stay outside the rewritten path;
 everything between them is this package's kernels.  Two fusions the reference's layer does not have:
 the residual add that ends a layer is folded into the next layer's input norm (one add_rms_norm),
-and rope + append is one launch.  KV heads shard across ranks (`world`, `rank`): each rank projects
+and rope + append is one launch.  With few rows on one rank a layer is two launches: the attention's step and
+everything up to the next one (`ops.row_chain`).  KV heads shard across ranks (`world`, `rank`): each rank projects
 and attends its own heads and the per-head outputs are all-gathered before o_proj - the only
 collective of the step.
 """
@@ -79,6 +80,7 @@ class TextTower:
                  fused_gather: bool = True, fused_qkv: bool = True, lt_gemm: bool = True):
         self.cfg, self.batch, self.device, self.dtype = cfg, batch, torch.device(device), dtype
         self.fused_qkv = fused_qkv
+        self.lt_gemm = lt_gemm
         self._linear = ops.linear_nobias if lt_gemm else (lambda x, w: torch.matmul(x, w.t()))
         self.world, self.rank = world, rank
         self.peer_gather = None
@@ -163,6 +165,8 @@ class TextTower:
         the greedy next token back into `token_ids`, advances `pos3`, and returns the next ids."""
         cfg = self.cfg
         h = ops.embedding(self.token_ids, self.embed)
+        if self._chains():
+            return self._finish_step(self._chained_layers(h))
         mlp_out: Optional[torch.Tensor] = None
         for li, lw in enumerate(self.layers):
             if mlp_out is None:
@@ -178,7 +182,30 @@ class TextTower:
                 act = ops.silu_mul(gu[:, :cfg.intermediate].contiguous(), gu[:, cfg.intermediate:].contiguous())
             mlp_out = self._linear(act, lw["down"])
         _, xf = ops.add_rms_norm(mlp_out, h, self.final_ln, cfg.eps)
-        logits = self._linear(xf, self.embed)
+        return self._finish_step(self._linear(xf, self.embed))
+
+    def _chains(self) -> bool:
+        """Whether everything between two attention calls is one launch (`ops.row_chain`): one rank, the fused forms, and few
+        enough rows."""
+        cfg = self.cfg
+        return self.world == 1 and self.fused_qkv and self.lt_gemm and type(self.cache) is PagedKVCache and ops.row_chain_supported(
+            self.batch, cfg.n_q_heads * cfg.head_dim, cfg.hidden, cfg.intermediate, cfg.vocab, self.dtype)
+
+    def _chained_layers(self, h) -> torch.Tensor:
+        """The layers with two launches each: the step of the attention (norms, rope, append and attention) and `ops.row_chain`,
+        whose last product is the next layer's QKV projection or the logits."""
+        cfg, last = self.cfg, self.cfg.n_layers - 1
+        out = self._linear(ops.rms_norm(h, self.layers[0]["input_ln"], cfg.eps), self.layers[0]["qkv"])
+        for li, lw in enumerate(self.layers):
+            attn = self.cache.step_qkv(li, out, cfg.n_q_heads, lw["q_norm"] if cfg.qk_norm else None,
+                                       lw["k_norm"] if cfg.qk_norm else None, cfg.eps, pos=self.pos3 if cfg.use_mrope else self.pos3[0],
+                                       inv_freq=self.inv_freq if cfg.use_mrope else None, theta=cfg.rope_theta,
+                                       mrope_section=cfg.mrope_section if cfg.use_mrope else None)
+            norm, w = (self.final_ln, self.embed) if li == last else (self.layers[li + 1]["input_ln"], self.layers[li + 1]["qkv"])
+            h, out = ops.row_chain(attn.view(self.batch, -1), lw["o"], h, lw["post_ln"], lw["gate_up"], lw["down"], norm, w, cfg.eps)
+        return out
+
+    def _finish_step(self, logits) -> torch.Tensor:
         self.last_logits = logits
         nxt = ops.argmax_last_dim(logits)
         self.token_ids.copy_(nxt)

@@ -33,6 +33,17 @@ class KVCache:
             self._host_len_bound += 1
         return q
 
+    def step_qkv(self, layer_idx: int, qkv, n_q_heads, q_norm_weight=None, k_norm_weight=None, eps=1e-6, pos=None, inv_freq=None,
+                 theta=10000.0, mrope_section=None):
+        """`append_qkv` and `attend` as one operator (one launch where the library can): the attention output (batch, hq, d)."""
+        first = layer_idx == 0
+        if first:
+            self._host_len_bound += 1
+        bound = self.max_seq_len if torch.cuda.is_current_stream_capturing() else min(self.max_seq_len, self._host_len_bound)
+        return ops.qkv_decode_step_paged(qkv, n_q_heads, q_norm_weight, k_norm_weight, eps, *self.get(layer_idx), max(bound, 1), pos=pos,
+                                         inv_freq=inv_freq, theta=theta, mrope_section=mrope_section, advance=first,
+                                         slot_delta=0 if first else -1)
+
     def step_host(self, q_host, k_new_host, v_new_host, out_host, theta=10000.0, pos=None, inv_freq=None,
                   mrope_section=None, layer_idx: int = 0):
         """One decode step with host activations (pinned CPU tensors): stage in, rope + append, attend,

@@ -465,6 +465,31 @@ def linear_nobias(x, weight):
     return out
 
 
+def row_chain_supported(rows, attn, width, ff, next_, dtype) -> bool:
+    """Whether `row_chain` takes these sizes: fp16, up to 8 rows, widths in multiples of 64."""
+    return dtype == torch.float16 and bool(_capi.lib().axb200_row_chain_supported(rows, attn, width, ff, next_, _capi.FLOAT16))
+
+
+def row_chain(x, w_o, residual, norm1, w_gate_up, w_down, norm2, w_next, eps):
+    """From an attention's output x (rows, attn) to the next input product in one launch: y = x . w_o^T + residual, the gated
+    feed-forward of its norm added to it, and its norm . w_next^T.  Returns (residual, product); all operands contiguous."""
+    op = "row_chain"
+    dt = _dt(x, op)
+    rows, attn = x.shape
+    width, ff, n = w_o.shape[0], w_down.shape[1], w_next.shape[0]
+    for t, shape in ((x, (rows, attn)), (w_o, (width, attn)), (residual, (rows, width)), (norm1, (width,)), (w_gate_up, (2 * ff, width)),
+                     (w_down, (width, ff)), (norm2, (width,)), (w_next, (n, width))):
+        if t.dtype != x.dtype or tuple(t.shape) != shape or not t.is_contiguous():
+            _capi.check(4, op)
+    lib = _capi.lib()
+    end, out = torch.empty_like(residual), torch.empty((rows, n), dtype=x.dtype, device=x.device)
+    ws = torch.empty(lib.axb200_row_chain_workspace_bytes(rows, width, ff), dtype=torch.uint8, device=x.device)
+    _call(lib.axb200_row_chain(x.data_ptr(), w_o.data_ptr(), residual.data_ptr(), norm1.data_ptr(), w_gate_up.data_ptr(),
+                               w_down.data_ptr(), norm2.data_ptr(), w_next.data_ptr(), end.data_ptr(), out.data_ptr(), rows, attn, width,
+                               ff, n, float(eps), dt, ws.data_ptr(), ws.numel(), _stream(x)), op)
+    return end, out
+
+
 def cast(x, dtype):
     """Tensor.cast_to on the device (src/core/cuda/tensor/kernel.cu:175-193): float16 <-> float32."""
     op = "cast"
