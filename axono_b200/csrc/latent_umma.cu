@@ -305,7 +305,6 @@ latent_umma_kernel(const __grid_constant__ CUtensorMap tmPages, const __grid_con
     }
   } else if (warp == kMmaWarp) {
     // ================= products of the scores (the warp walks, one lane issues) =================
-    const uint32_t lead = lane == 0;
     constexpr uint32_t idesc = kIdesc<kN>;                                // A K-major
     const uint64_t da = smem_desc(smem_u32(smem), 16, 1024);             // a chunk as [keys][elements]
     const uint64_t dq = smem_desc(smem_u32(smem + S::off_q(u)), 16, 1024);
@@ -323,8 +322,10 @@ latent_umma_kernel(const __grid_constant__ CUtensorMap tmPages, const __grid_con
       bool first = true;
       auto score_chunk = [&](int offset, int c) {
         const uint64_t a = da + (uint64_t)(offset >> 4), b = dq + (uint64_t)(c * (S::kQBox >> 4));
+        if (elect_one()) {
 #pragma unroll
-        for (int ks = 0; ks < 4; ++ks) umma_f16_lead(ts, a + ks * 2, b + ks * 2, idesc, !first || ks > 0, lead);
+          for (int ks = 0; ks < 4; ++ks) umma_f16(ts, a + ks * 2, b + ks * 2, idesc, !first || ks > 0);
+        }
         first = false;
       };
       for (int i = 0; i < u.singles && ok; ++i, rs.next(u.single_slots)) {
@@ -333,7 +334,7 @@ latent_umma_kernel(const __grid_constant__ CUtensorMap tmPages, const __grid_con
         if (!ok) break;
         tc_fence_after();
         score_chunk(off_single + s * kChunk, 2 * u.pairs + i);
-        umma_commit_lead(&empty_s[s], lead);
+        if (elect_one()) umma_commit(&empty_s[s]);
       }
       for (int i = 0; i < u.pairs && ok; ++i, rp.next(u.pair_slots)) {
         const int s = rp.slot;
@@ -342,11 +343,10 @@ latent_umma_kernel(const __grid_constant__ CUtensorMap tmPages, const __grid_con
         tc_fence_after();
         for (int c = 0; c < 2 && 2 * i + c < u.chunks; ++c) score_chunk(s * 2 * kChunk + c * kChunk, 2 * i + c);
       }
-      if (ok) umma_commit_lead(&bar_s[tile & 1], lead);
+      if (ok && elect_one()) umma_commit(&bar_s[tile & 1]);
     }
   } else if (warp == kSumWarp) {
     // ================= products of the sum =================
-    const uint32_t lead = lane == 0;
     constexpr uint32_t idesc = kIdesc<kN> | (1u << 15);             // A MN-major
     const uint64_t dv = smem_desc(smem_u32(smem), kChunk, 1024);    // a pair as latent elements x keys
     const uint64_t dp = smem_desc(smem_u32(smem + S::off_p(u)), 16, 1024);
@@ -360,13 +360,15 @@ latent_umma_kernel(const __grid_constant__ CUtensorMap tmPages, const __grid_con
       for (int i = 0; i < u.pairs; ++i, pv.next(u.pair_slots)) {
         const int s = pv.slot;
         const uint64_t a = dv + (uint64_t)(s * (2 * kChunk >> 4));
+        if (elect_one()) {
 #pragma unroll
-        for (int ks = 0; ks < kKeys / 16; ++ks)  // 16 keys: 2 KB of the chunk, 32 bytes of P
-          umma_f16_lead(tmem_o + i * kN, a + (uint64_t)(ks * (2048 >> 4)),
-                        dpt + (uint64_t)(((ks >> 2) * (kN * 128) + (ks & 3) * 32) >> 4), idesc, !fresh || ks > 0, lead);
-        umma_commit_lead(&empty_p[s], lead);
+          for (int ks = 0; ks < kKeys / 16; ++ks)  // 16 keys: 2 KB of the chunk, 32 bytes of P
+            umma_f16(tmem_o + i * kN, a + (uint64_t)(ks * (2048 >> 4)),
+                     dpt + (uint64_t)(((ks >> 2) * (kN * 128) + (ks & 3) * 32) >> 4), idesc, !fresh || ks > 0);
+          umma_commit(&empty_p[s]);
+        }
       }
-      umma_commit_lead(&bar_o[tile & 1], lead);
+      if (elect_one()) umma_commit(&bar_o[tile & 1]);
     }
   } else {
     // ================= softmax warps: thread = key of the tile =================

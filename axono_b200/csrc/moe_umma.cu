@@ -105,8 +105,7 @@ moe_umma_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__
           }
     }
   } else if (warp == kMmaWarp) {
-    const uint32_t lead = lane == 0;  // the warp walks, one lane issues
-    {
+    {  // the warp walks, one lane issues
       // fp32 accumulate, bf16 operands, both K-major, M = 128, N = the tile's rows to a multiple of 16
       const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(cols >> 3) << 17) | ((kMTile >> 4) << 24);
       const uint64_t base = smem_desc(smem_u32(smem), 16, 1024);
@@ -117,13 +116,15 @@ moe_umma_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__
         if (!ok) break;
         tc_fence_after();
         const uint64_t a0 = base + (uint64_t)(s * (S::kStageBytes >> 4)), a1 = a0 + (kATile >> 4), b = a0 + (2 * kATile >> 4);
+        if (elect_one()) {
 #pragma unroll
-        for (int ks = 0; ks < kKTile / 16; ++ks) umma_f16_lead(tmem, a0 + ks * 2, b + ks * 2, idesc, k > 0 || ks > 0, lead);
+          for (int ks = 0; ks < kKTile / 16; ++ks) umma_f16(tmem, a0 + ks * 2, b + ks * 2, idesc, k > 0 || ks > 0);
 #pragma unroll
-        for (int ks = 0; ks < kKTile / 16; ++ks) umma_f16_lead(tmem + kN, a1 + ks * 2, b + ks * 2, idesc, k > 0 || ks > 0, lead);
-        umma_commit_lead(&empty[s], lead);
+          for (int ks = 0; ks < kKTile / 16; ++ks) umma_f16(tmem + kN, a1 + ks * 2, b + ks * 2, idesc, k > 0 || ks > 0);
+          umma_commit(&empty[s]);
+        }
       }
-      if (ok) umma_commit_lead(done, lead);
+      if (ok && elect_one()) umma_commit(done);
     }
   } else {
     mbar_wait_bounded(done, 0, abort_flag, p.wait_ns);

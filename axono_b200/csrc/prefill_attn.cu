@@ -98,7 +98,7 @@ prefill_attn_f16_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
   const int qb = gridDim.x - 1 - blockIdx.x, h = blockIdx.y;
   const int hk = h / (p.hq / p.hkv);
   const int q0 = qb * kBlockM;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = uniform_warp(), lane = threadIdx.x & 31;
   const int t_last = min(q0 + kBlockM, p.sq) - 1;
   const int kv_end_max = p.causal ? min(t_last + 1, p.skv) : p.skv;  // reference rule: min(t+1, skv)
   const int nkv = (kv_end_max + kBlockN - 1) / kBlockN;
@@ -158,8 +158,8 @@ prefill_attn_f16_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
       }
     }
   } else if (warp == kMmaWarp) {
-    // ================= MMA warp (one lane) =================
-    if (lane == 0) {
+    // ================= MMA warp: all lanes walk, one issues =================
+    {
       // instruction descriptors: fp32 accumulate, fp16 operands, M = 128.  Q.K^T: N = 64 keys, B
       // K-major; P.V: N = 128 dims, B MN-major (a V tile is [keys][d], d contiguous)
       const uint32_t idesc_qk = (1u << 4) | ((kBlockN >> 3) << 17) | ((kBlockM >> 4) << 24);
@@ -172,44 +172,48 @@ prefill_attn_f16_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
       // S_j = Q . K_j^T into S buffer j&1; arrives on bar_s[j&1], and frees the K stage when done
       auto issue_s = [&](int j) -> bool {
         const int s = j & 1, sk = j % kKStages;
-        if (!mbar_wait_bounded(&full_k[sk], (j / kKStages) & 1, abort_flag)) return false;
+        if (!mbar_wait_warp(&full_k[sk], (j / kKStages) & 1, abort_flag, kWaitNanos)) return false;
         tc_fence_after();
         const uint64_t dks = dk + (uint64_t)(sk * (kKvTileBytes >> 4));
+        if (elect_one()) {
 #pragma unroll
-        for (int ks = 0; ks < 8; ++ks) {  // head_dim 128 = 8 steps of 16; each 64-wide half of d is one box
-          const uint32_t q_off = (ks >> 2) * (kQTileBytes / 2) + (ks & 3) * 32;
-          const uint32_t k_off = (ks >> 2) * (kKvTileBytes / 2) + (ks & 3) * 32;
-          umma_f16(tmem_base + s * kBlockN, dq + (q_off >> 4), dks + (k_off >> 4), idesc_qk, ks > 0);
+          for (int ks = 0; ks < 8; ++ks) {  // head_dim 128 = 8 steps of 16; each 64-wide half of d is one box
+            const uint32_t q_off = (ks >> 2) * (kQTileBytes / 2) + (ks & 3) * 32;
+            const uint32_t k_off = (ks >> 2) * (kKvTileBytes / 2) + (ks & 3) * 32;
+            umma_f16(tmem_base + s * kBlockN, dq + (q_off >> 4), dks + (k_off >> 4), idesc_qk, ks > 0);
+          }
+          umma_commit(&bar_s[s]);
+          umma_commit(&empty_k[sk]);
         }
-        umma_commit(&bar_s[s]);
-        umma_commit(&empty_k[sk]);
         return true;
       };
-      bool ok = mbar_wait_bounded(bar_q, 0, abort_flag) && issue_s(0);
+      bool ok = mbar_wait_warp(bar_q, 0, abort_flag, kWaitNanos) && issue_s(0);
       if (ok && nkv > 1) ok = issue_s(1);
       for (int j = 0; j < nkv && ok; ++j) {
         // P_j stands in the first 32 columns of S buffer j&1: O += P_j . V_j
         const int sv = j % kVStages;
-        ok = mbar_wait_bounded(&bar_p[j & 1], (j >> 1) & 1, abort_flag) &&
-             mbar_wait_bounded(&full_v[sv], (j / kVStages) & 1, abort_flag);
+        ok = mbar_wait_warp(&bar_p[j & 1], (j >> 1) & 1, abort_flag, kWaitNanos) &&
+             mbar_wait_warp(&full_v[sv], (j / kVStages) & 1, abort_flag, kWaitNanos);
         if (!ok) break;
         tc_fence_after();
         const uint64_t dvs = dv + (uint64_t)(sv * (kKvTileBytes >> 4));
         const uint32_t p_tmem = tmem_base + (j & 1) * kBlockN;
+        if (elect_one()) {
 #pragma unroll
-        for (int ks = 0; ks < kBlockN / 16; ++ks) {
-          // V as the MN-major B operand: the two 64-wide d atoms are one box (8 KB) apart, 8-key
-          // groups 1 KB apart, 16 keys per instruction = 2 KB
-          umma_f16_ts(tmem_o, p_tmem + ks * 8, dvs + (uint64_t)(ks * (2048 >> 4)), idesc_pv, j > 0 || ks > 0);
+          for (int ks = 0; ks < kBlockN / 16; ++ks) {
+            // V as the MN-major B operand: the two 64-wide d atoms are one box (8 KB) apart, 8-key
+            // groups 1 KB apart, 16 keys per instruction = 2 KB
+            umma_f16_ts(tmem_o, p_tmem + ks * 8, dvs + (uint64_t)(ks * (2048 >> 4)), idesc_pv, j > 0 || ks > 0);
+          }
+          umma_commit(bar_o);
+          umma_commit(&empty_v[sv]);
+          if (j == nkv - 1) umma_commit(bar_fin);
         }
-        umma_commit(bar_o);
-        umma_commit(&empty_v[sv]);
-        if (j == nkv - 1) umma_commit(bar_fin);
         if (j + 2 < nkv) {
           // P_j.V_j complete: P_j is consumed, so S_{j+2} may overwrite S buffer j&1 (queueing it behind
           // P_j.V_j instead would lean on issue-order execution, which is documented only for MMAs of
           // one shape; measured no faster)
-          ok = mbar_wait_bounded(bar_o, j & 1, abort_flag);
+          ok = mbar_wait_warp(bar_o, j & 1, abort_flag, kWaitNanos);
           if (!ok) break;
           ok = issue_s(j + 2);
         }
@@ -340,7 +344,8 @@ prefill_attn_f16_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
 // softmax warps that P_g(j).V_j is done and O_g may be rescaled.
 // Blocks start in the order of their key tiles over all heads, so that under a causal mask the last ones to start are the
 // short ones (head by head, the last head's longest block began when three quarters of the time were gone), and the softmax
-// works on pairs of scores.  8192 tokens, 16 / 8 heads of 128, causal: 332 us before both, 283 after (828 and 972 TFLOP/s).
+// works on pairs of scores.  8192 tokens, 16 / 8 heads of 128, causal: 332 us before both, 283 after (828 and 972 TFLOP/s);
+// with the products issued behind elect_one, 267.
 constexpr int kPairN = 128, kPairTileBytes = 128 * kD * 2;  // 32 KB: two swizzled boxes of [128 rows][64 halves]
 constexpr int kPairThreads = 320, kPairMmaWarp = 8, kPairLoadWarp = 9;
 constexpr int kPairOffQ = 0, kPairOffK = 2 * kPairTileBytes, kPairOffV = kPairOffK + 2 * kPairTileBytes;
@@ -477,7 +482,7 @@ prefill_attn_f16_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __gr
   const int parts = split.units ? split.parts[unit] : 1;
   const int hk = h / (p.hq / p.hkv);
   const int q0 = qb * 2 * kBlockM;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = uniform_warp(), lane = threadIdx.x & 31;
   // key tiles per query tile: none for a tile past the last query row; under the causal rule
   // min(t+1, skv) keys for its last row
   int nkv_g[2];
@@ -545,8 +550,8 @@ prefill_attn_f16_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __gr
       }
     }
   } else if (warp == kPairMmaWarp) {
-    // ================= MMA warp (one lane) =================
-    if (lane == 0) {
+    // ================= MMA warp: all lanes walk, one issues =================
+    {
       // fp32 accumulate, fp16 operands, M = 128, N = 128; Q.K^T: B K-major; P.V: B MN-major
       const uint32_t idesc_qk = (1u << 4) | ((kPairN >> 3) << 17) | ((kBlockM >> 4) << 24);
       const uint32_t idesc_pv = idesc_qk | (1u << 16);
@@ -557,44 +562,48 @@ prefill_attn_f16_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __gr
       auto issue_s = [&](int g, int j) {  // S_g(j) = Q_g . K_j^T; K_j is known to have landed
         const uint64_t dqg = dq + (uint64_t)(g * (kPairTileBytes >> 4));
         const uint64_t dks = dk + (uint64_t)((j & 1) * (kPairTileBytes >> 4));
+        if (elect_one()) {
 #pragma unroll
-        for (int ks = 0; ks < 8; ++ks) {  // head_dim 128 = 8 steps of 16; each 64-wide half of d is one box
-          if (kNarrow && ks >= d_steps) break;
-          const uint32_t off = ((ks >> 2) * (kPairTileBytes / 2) + (ks & 3) * 32) >> 4;
-          umma_f16(tmem_base + g * 128, dqg + off, dks + off, idesc_qk, ks > 0);
+          for (int ks = 0; ks < 8; ++ks) {  // head_dim 128 = 8 steps of 16; each 64-wide half of d is one box
+            if (kNarrow && ks >= d_steps) break;
+            const uint32_t off = ((ks >> 2) * (kPairTileBytes / 2) + (ks & 3) * 32) >> 4;
+            umma_f16(tmem_base + g * 128, dqg + off, dks + off, idesc_qk, ks > 0);
+          }
+          umma_commit(&bar_s[g]);
         }
-        umma_commit(&bar_s[g]);
       };
-      bool ok = mbar_wait_bounded(bar_q, 0, abort_flag);
+      bool ok = mbar_wait_warp(bar_q, 0, abort_flag, kWaitNanos);
       if (ok) {
         tc_fence_after();
         if (nkv_g[0] > 0) issue_s(0, 0);
         if (nkv_g[1] > 0) issue_s(1, 0);
-        umma_commit(&empty_kv[1]);  // K_0 has been read: the stage may take K_2
+        if (elect_one()) umma_commit(&empty_kv[1]);  // K_0 has been read: the stage may take K_2
       }
       for (int j = 0; j < nkv && ok; ++j) {
-        ok = mbar_wait_bounded(&full_kv[j & 1], (j >> 1) & 1, abort_flag);
+        ok = mbar_wait_warp(&full_kv[j & 1], (j >> 1) & 1, abort_flag, kWaitNanos);
         if (!ok) break;
         const uint64_t dvs = dv + (uint64_t)((j & 1) * (kPairTileBytes >> 4));
 #pragma unroll
         for (int g = 0; g < 2; ++g) {
           if (j >= nkv_g[g]) continue;
-          ok = mbar_wait_bounded(&bar_p[g], j & 1, abort_flag);
+          ok = mbar_wait_warp(&bar_p[g], j & 1, abort_flag, kWaitNanos);
           if (!ok) break;
           tc_fence_after();
           // O_g += P_g(j) . V_j: P from tensor memory (16 keys = 8 columns); V as the MN-major B
           // operand: the two 64-wide d atoms are one box (16 KB) apart, 8-key groups 1 KB apart
+          if (elect_one()) {
 #pragma unroll
-          for (int part = 0; part < (kNarrow ? 2 : 1); ++part)
+            for (int part = 0; part < (kNarrow ? 2 : 1); ++part)
 #pragma unroll
-            for (int ks = 0; ks < kPairN / 16; ++ks)
-              umma_f16_ts(tmem_base + 256 + g * 128, tmem_base + g * 128 + part * 64 + ks * 8, dvs + (uint64_t)(ks * (2048 >> 4)),
-                          idesc_pv, (kNarrow ? j % kFlushTiles != 0 : j > 0) || part > 0 || ks > 0);
-          if (j == nkv_g[g] - 1) umma_commit(&bar_fin[g]);
+              for (int ks = 0; ks < kPairN / 16; ++ks)
+                umma_f16_ts(tmem_base + 256 + g * 128, tmem_base + g * 128 + part * 64 + ks * 8, dvs + (uint64_t)(ks * (2048 >> 4)),
+                            idesc_pv, (kNarrow ? j % kFlushTiles != 0 : j > 0) || part > 0 || ks > 0);
+            if (j == nkv_g[g] - 1) umma_commit(&bar_fin[g]);
+          }
           if (j + 1 < nkv_g[g]) issue_s(g, j + 1);
         }
         if (!ok) break;
-        umma_commit(&empty_kv[j & 1]);
+        if (elect_one()) umma_commit(&empty_kv[j & 1]);
       }
     }
   } else {

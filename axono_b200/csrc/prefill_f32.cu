@@ -20,9 +20,9 @@
 // Non-finite inputs (inf - inf among the parts) and magnitudes that have no three normal parts are noticed while splitting:
 // the flags of their tiles make the FMA kernel of prefill_tiled.cu, launched behind, redo that KV head; else it returns at once.
 //
-// Bound by the tensor core: 12 products per tile.  Those of P.V take 71 cycles of the possible 64, those of Q.K^T, only 64 wide,
-// 62 instead of 32 (their A operand comes no faster).  1536 tokens, 16 / 8 heads of 128, causal: 744 us on the FMA pipe, 100
-// here, the error against 64 bits 4.2e-7 there and 1.9e-7 here; 4096 tokens, 32 heads, not causal: 11.3 and 1.46 ms.
+// Bound by the tensor core: 12 products per tile.  Those of P.V take 66 cycles of the possible 64, those of Q.K^T, only 64 wide,
+// 50 instead of 32.  1536 tokens, 16 / 8 heads of 128, causal: 744 us on the FMA pipe, 72 here (100 while a product's issue took
+// 62 to 71 cycles, see elect_one), the error against 64 bits 4.2e-7 there and 1.9e-7 here.
 #include <math.h>
 
 #include <mutex>
@@ -219,7 +219,6 @@ split_attn_kernel(const Params p, const __grid_constant__ KeySplit split, const 
       }
     }
   } else if (warp == kMmaWarp) {
-    const uint32_t lead = lane == 0;
     // fp32 accumulate, bf16 operands, M = 128, A from tensor memory.  Q.K^T: N = 64 keys, B K-major; P.V: N = the head size
     // to a multiple of 16, B MN-major
     const uint32_t bf16 = (1u << 4) | (1u << 7) | (1u << 10) | ((kRows >> 4) << 24);
@@ -232,16 +231,18 @@ split_attn_kernel(const Params p, const __grid_constant__ KeySplit split, const 
       if (!mbar_wait_warp(&full_k[s], (j >> 1) & 1, abort_flag, p.wait_ns)) return false;
       tc_fence_after();
       const uint64_t dks = dk + (uint64_t)(s * (L::kTile >> 4));
+      if (elect_one()) {
 #pragma unroll
-      for (int i = 0; i < 6; ++i)
+        for (int i = 0; i < 6; ++i)
 #pragma unroll
-        for (int ks = 0; ks < 4 * kB; ++ks) {
-          if (ks >= d_steps) break;
-          umma_f16_ts_lead(tmem_sp + s * L::kSpCols, tmem + kA[i] * 32 * kB + ks * 8,
-                           dks + (uint64_t)((kC[i] * L::kPart + (ks >> 2) * kBox + (ks & 3) * 32) >> 4), idesc_qk, i > 0 || ks > 0, lead);
-        }
-      umma_commit_lead(&bar_s[s], lead);
-      umma_commit_lead(&empty_k[s], lead);
+          for (int ks = 0; ks < 4 * kB; ++ks) {
+            if (ks >= d_steps) break;
+            umma_f16_ts(tmem_sp + s * L::kSpCols, tmem + kA[i] * 32 * kB + ks * 8,
+                        dks + (uint64_t)((kC[i] * L::kPart + (ks >> 2) * kBox + (ks & 3) * 32) >> 4), idesc_qk, i > 0 || ks > 0);
+          }
+        umma_commit(&bar_s[s]);
+        umma_commit(&empty_k[s]);
+      }
       return true;
     };
     bool ok = mbar_wait_warp(bar_q, 0, abort_flag, p.wait_ns) && issue_s(0);
@@ -254,14 +255,16 @@ split_attn_kernel(const Params p, const __grid_constant__ KeySplit split, const 
       if (!ok) break;
       tc_fence_after();
       const uint64_t dvs = dv + (uint64_t)(s * (L::kTile >> 4));
+      if (elect_one()) {
 #pragma unroll
-      for (int i = 0; i < 6; ++i)
+        for (int i = 0; i < 6; ++i)
 #pragma unroll
-        for (int ks = 0; ks < kKeys / 16; ++ks)
-          umma_f16_ts_lead(tmem_o, tmem_sp + s * L::kSpCols + kA[i] * 32 + ks * 8,
-                           dvs + (uint64_t)((kC[i] * L::kPart + ks * 2048) >> 4), idesc_pv, i > 0 || ks > 0, lead);
-      umma_commit_lead(bar_o, lead);
-      umma_commit_lead(&empty_v[s], lead);
+          for (int ks = 0; ks < kKeys / 16; ++ks)
+            umma_f16_ts(tmem_o, tmem_sp + s * L::kSpCols + kA[i] * 32 + ks * 8,
+                        dvs + (uint64_t)((kC[i] * L::kPart + ks * 2048) >> 4), idesc_pv, i > 0 || ks > 0);
+        umma_commit(bar_o);
+        umma_commit(&empty_v[s]);
+      }
       // S_{j+2} takes the place of P_j: products of unlike shapes have no order of their own, so P_j.V_j is waited for
       if (j + 2 < nkv) ok = mbar_wait_warp(bar_o, j & 1, abort_flag, p.wait_ns) && issue_s(j + 2);
     }
