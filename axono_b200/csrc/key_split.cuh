@@ -27,9 +27,10 @@ struct KeySplit {
 __host__ __device__ inline int split_begin(int tiles, int part, int parts) { return (int)((int64_t)tiles * part / parts); }
 
 // blocks row blocks of `heads` heads; tiles(b) key tiles in block b, not decreasing in b; part_cost: what a block or part costs beside
-// its tiles, in tiles; least_gain: tiles in a row that a division has to save, as many as joining takes (4 to 6 us with its launch).
+// its tiles, in tiles; least_gain: tiles in a row that a division has to save, as many as joining takes (4 to 6 us with its launch);
+// places: blocks that run at once.
 template <typename Tiles>
-KeySplit plan_key_split(int64_t blocks, int heads, bool causal, float part_cost, float least_gain, Tiles tiles) {
+KeySplit plan_key_split(int64_t blocks, int heads, bool causal, float part_cost, float least_gain, Tiles tiles, int places = kSms) {
   KeySplit plan{};
   if (blocks > kMostUnits || heads > 2 * kSms) return plan;
   const int most = tiles((int)blocks - 1);
@@ -47,14 +48,14 @@ KeySplit plan_key_split(int64_t blocks, int heads, bool causal, float part_cost,
         shortest = t / n < shortest ? t / n : shortest;
       }
       const float alone = longest + part_cost;
-      if (count * heads <= kSms) return alone;
-      const float even = (total + part_cost * count) * heads / kSms + (shortest + part_cost) / 2;
+      if (count * heads <= places) return alone;
+      const float even = (total + part_cost * count) * heads / places + (shortest + part_cost) / 2;
       return even > alone ? even : alone;
     };
     float best = estimate(most) - least_gain;
     int64_t total = 0;
     for (int b = 0; b < blocks; ++b) total += tiles(b);
-    const int first = (int)((total * heads + kSms - 1) / kSms);
+    const int first = (int)((total * heads + places - 1) / places);
     for (int at_most = first < 2 ? 2 : first; at_most < most && at_most < first + 8; ++at_most) {
       const float time = estimate(at_most);
       if (time < best) best = time, limit = at_most;
@@ -62,12 +63,12 @@ KeySplit plan_key_split(int64_t blocks, int heads, bool causal, float part_cost,
     if (limit == 0) return plan;
   } else {
     // blocks of one length: whole waves of them as they are, the rest in parts that fill one, two or three rounds of the SMs
-    const int64_t all = blocks * heads, waves = all / kSms;
-    unsplit = (int)(waves * kSms / heads);
+    const int64_t all = blocks * heads, waves = all / places;
+    unsplit = (int)(waves * places / heads);
     const int64_t rest = all - (int64_t)unsplit * heads;
-    float best = ((all + kSms - 1) / kSms - waves) * (most + part_cost) - least_gain;
+    float best = ((all + places - 1) / places - waves) * (most + part_cost) - least_gain;
     for (int rounds = 1; rounds <= 3; ++rounds) {
-      int64_t n = rest ? rounds * kSms / rest : 0;
+      int64_t n = rest ? rounds * places / rest : 0;
       n = n > 16 ? 16 : n;
       n = n > most / 2 ? most / 2 : n;
       const float time = n > 1 ? rounds * ((float)most / n + part_cost) : INFINITY;

@@ -283,3 +283,21 @@ def test_prompts_where_memory_is_short(dtype, monkeypatch):
     monkeypatch.setattr(torch, "empty", short)
     out = ops.scaled_dot_product_attention(q, k, v, True)
     assert refused and torch.equal(out, without_scratch(q, k, v, True)) and ops.last_error() == 0
+
+
+@pytest.mark.parametrize("d", [16, 64, 80, 128])
+@pytest.mark.parametrize("sq,skv", [(17, 63), (128, 64), (129, 65), (255, 1024), (256, 1025), (384, 1088), (40, 2113)])
+def test_fp16_at_the_edges_of_key_tiles(d, sq, skv):
+    """Tiles of 64 keys, of which the scores of two are ahead, and sums of narrow heads that start anew every sixteen: one tile, a
+    tile and a key, one group of tiles and the next.  The bound of `test_fp16_keys_divided_among_blocks`."""
+    from axono_b200 import ops
+
+    for causal in (True, False):
+        q, k, v = tensors(sq, skv, 2, 1, d, torch.float16, 2.0)
+        ref, mass = attention(q, k, v, causal), attention(q, k, v.abs(), causal)
+        top = (torch.einsum("qhd,khd->hqk", q.float(), k.float().repeat_interleave(2, 1)).abs().max() * d ** -0.5).item()
+        weight = 2 * top * 2.0 ** -21 + 2.0 ** -20 + (2.0 ** -11 if d == 128 else 0.0)
+        small = 2.0 ** -25 * v.double().abs().sum(0).repeat_interleave(2, 0)
+        for out in (ops.scaled_dot_product_attention(q, k, v, causal), without_scratch(q, k, v, causal)):
+            assert ((out.double() - ref).abs() <= ref.abs() * 2.0 ** -11 + weight * mass + small + 2.0 ** -24).all()
+    assert ops.last_error() == 0
