@@ -10,11 +10,14 @@
 // A row may see only the last `window` keys (a CTA starts at the tile that holds its first row's first key), and a
 // per-head sink may join the denominator.
 //
-// Structure as the 256-row form of prefill_attn.cu: one CTA per (256 query rows, head) works on two query tiles
-// against key tiles of 128; S_g and O_g in tensor memory; warps 0-7 own one query row per thread and do the
-// online softmax; warp 8 issues the MMAs, warp 9 the TMA loads.  What differs: K is 128 x up to 192 elements
-// per tile, so K is double-buffered while V has one buffer whose two halves of 64 keys are freed and refilled
-// separately; rows stand at positions start .. start + n - 1 of a longer key sequence.  Every wait is bounded.
+// Structure as prefill_attn.cu: one CTA per (128 query rows, head), two per SM, against key tiles of 64; two buffers of S and O in
+// tensor memory, P over S; warps 0-3 own one query row per thread and do the online softmax, warp 4 issues the MMAs - the
+// scores two tiles ahead -, warp 5 the TMA loads.  What differs: K is 64 x up to 192 elements per tile, so that with a rotated
+// part K and V have a buffer less; rows stand at positions start .. start + n - 1 of a longer key sequence.  Every wait is bounded.
+// Bound by the tensor core as there.  2048 rows over 8192 keys, 16 heads of 128: 133 us, now 115; with a window of 4096: 76 and 70;
+// 2000 rows, 16 heads of 128 + 64 rotated: 43 and 37; 8192 of these: 293 and 290 (before: one CTA per SM with two blocks of rows and
+// tiles of 128 keys, whose scores had to wait for the tile before, and products issued one by one; these issued as here, the
+// last is 275: three blocks of K make 64-wide scores dear, but one form serves all, and the blocks of short prompts are finer).
 #include <math.h>
 
 #include <mutex>
@@ -25,8 +28,9 @@
 namespace axb {
 namespace {
 
-constexpr int kRows = 128, kKeys = 128, kBox = kRows * 64 * 2;  // one [128 rows][64 elements] block: 16 KB
-constexpr int kThreads = 320, kMmaWarp = 8, kLoadWarp = 9;
+constexpr int kRows = 128, kKeys = 64, kBox = kRows * 64 * 2;  // one [128 rows][64 elements] block: 16 KB
+constexpr int kKeyBox = kKeys * 64 * 2;                        // of [64 keys][64 elements]
+constexpr int kThreads = 192, kMmaWarp = 4, kLoadWarp = 5;
 constexpr float kLog2e = 1.4426950408889634f, kLazy = 8.0f;
 
 struct Params {
@@ -42,50 +46,48 @@ struct Params {
 template <int kQB, int kVB, int kRot>
 struct Layout {
   static constexpr int kBlocks = kQB + kRot;
-  static constexpr int kTile = kBlocks * kBox;        // a query tile or a key tile
-  static constexpr int kVHalf = 64 * kVB * 64 * 2;    // 64 keys: kVB boxes of [64 keys][64]
-  static constexpr int kOffK = 2 * kTile, kOffV = kOffK + 2 * kTile, kOffBar = kOffV + 2 * kVHalf;
+  static constexpr int kQ = kBlocks * kBox, kK = kBlocks * kKeyBox, kV = kVB * kKeyBox;  // a query tile, tiles of keys and values
+  static constexpr bool kDeep = kQ + 3 * kK + 2 * kV <= 112 * 1024;  // two CTAs share an SM
+  static constexpr int kKStages = kDeep ? 3 : 2, kVStages = kDeep ? 2 : 1;
+  static constexpr int kOffK = kQ, kOffV = kOffK + kKStages * kK, kOffBar = kOffV + kVStages * kV;
   static constexpr int kSmem = kOffBar + 256;
+  static_assert(kOffBar <= 112 * 1024, "two CTAs per SM");
 };
 
 template <int kQB, int kVB, int kRot>
-__global__ void __launch_bounds__(kThreads, 1)
+__global__ void __launch_bounds__(kThreads, 2)
 latent_prefill_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmQr,
                       const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmKr,
                       const __grid_constant__ CUtensorMap tmV, const Params p) {
   using L = Layout<kQB, kVB, kRot>;
   extern __shared__ __align__(1024) uint8_t smem[];
   uint64_t *bars = reinterpret_cast<uint64_t *>(smem + L::kOffBar);
-  uint64_t *bar_q = bars, *full_k = bars + 1, *empty_k = bars + 3, *full_v = bars + 5, *empty_v = bars + 7;
-  uint64_t *bar_s = bars + 9, *bar_fin = bars + 11, *bar_p = bars + 13;
-  uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(bars + 15);
-  volatile int *abort_flag = reinterpret_cast<volatile int *>(bars + 16);
+  uint64_t *bar_q = bars, *full_k = bars + 1, *empty_k = bars + 4, *full_v = bars + 7, *empty_v = bars + 9;
+  uint64_t *bar_s = bars + 11, *bar_o = bars + 13;  // S_j ready (per buffer); P_j.V_j done
+  uint64_t *bar_fin = bars + 14;  // the last P.V: the softmax warps skip phases of bar_o, a parity wait there would alias
+  uint64_t *bar_p = bars + 15;    // P_j written (per S buffer), one arrival per softmax warp
+  uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(bars + 17);
+  volatile int *abort_flag = reinterpret_cast<volatile int *>(bars + 18);
   if ((smem_u32(smem) & 1023u) != 0) {
     if (threadIdx.x == 0) atomicOr(&g_error_word, AXB200_ERR_WAIT_TIMEOUT);
     return;
   }
   // heaviest blocks of all heads first: the last query block has the most key tiles
-  const int h = blockIdx.x % p.heads, q0 = (int)((gridDim.x - 1 - blockIdx.x) / p.heads) * 2 * kRows;
+  const int h = blockIdx.x % p.heads, q0 = (int)((gridDim.x - 1 - blockIdx.x) / p.heads) * kRows;
   const int warp = uniform_warp(), lane = threadIdx.x & 31;
   const int hk = h / p.group;
   const int tile0 = p.window > 0 ? max(0, p.start + q0 + 1 - p.window) / kKeys : 0;  // the first key tile
-  int nkv_g[2];
-#pragma unroll
-  for (int g = 0; g < 2; ++g) {
-    const int first = q0 + g * kRows, last = min(first + kRows, p.n) - 1;
-    nkv_g[g] = first < p.n ? (min(p.start + last + 1, p.skv) + kKeys - 1) / kKeys - tile0 : 0;
-  }
-  const int nkv = max(nkv_g[0], nkv_g[1]);
+  const int nkv = (min(p.start + min(q0 + kRows, p.n), p.skv) + kKeys - 1) / kKeys - tile0;
 
   if (threadIdx.x == 0) {
-    for (int i = 0; i < 13; ++i) mbar_init(&bars[i], 1);
+    for (int i = 0; i < 15; ++i) mbar_init(&bars[i], 1);
     mbar_init(&bar_p[0], 4);
     mbar_init(&bar_p[1], 4);
     *abort_flag = 0;
     mbar_fence_init();
   }
   if (warp == kMmaWarp) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(smem_u32(tmem_slot)) : "memory");
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 256;" ::"r"(smem_u32(tmem_slot)) : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
   tc_fence_before();
@@ -93,48 +95,38 @@ latent_prefill_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
   tc_fence_after();
   grid_dependency_wait();
   grid_dependency_launch();
-  // S_g at g * 128.  With 128 value columns O_g is at 256 + g * 128 and P_g overwrites the front of S_g; with 64,
-  // O_g is at 256 + g * 64 and P_g has columns of its own (the products then differ in shape, and the reuse of
-  // S_g would lean on the issue order of unlike products).
-  const uint32_t tmem = *tmem_slot;
-  auto tmem_o = [&](int g) { return tmem + 256 + g * (kVB * 64); };
-  auto tmem_p = [&](int g) { return kVB == 2 ? tmem + g * 128 : tmem + 384 + g * 64; };
+  const uint32_t tmem = *tmem_slot, tmem_o = tmem + 128;  // S buffers at columns 0 and 64; P_j over the front of its S
 
   if (warp == kLoadWarp) {
     if (lane == 0) {
       tma_prefetch_descriptor(&tmK);
       if (kRot) tma_prefetch_descriptor(&tmKr);
       tma_prefetch_descriptor(&tmV);
-      mbar_arrive_expect_tx(bar_q, 2 * L::kTile);
-#pragma unroll
-      for (int g = 0; g < 2; ++g) {  // rows past n are zero-filled
-        uint8_t *dst = smem + g * L::kTile;
-        for (int b = 0; b < kQB; ++b) tma_load_3d(dst + b * kBox, &tmQ, bar_q, b * 64, h, q0 + g * kRows);
-        if (kRot) tma_load_3d(dst + kQB * kBox, &tmQr, bar_q, 0, h, q0 + g * kRows);
-      }
+      mbar_arrive_expect_tx(bar_q, L::kQ);
+      for (int b = 0; b < kQB; ++b) tma_load_3d(smem + b * kBox, &tmQ, bar_q, b * 64, h, q0);  // rows past n are zero-filled
+      if (kRot) tma_load_3d(smem + kQB * kBox, &tmQr, bar_q, 0, h, q0);
       bool ok = true;
-      auto load_k = [&](int t) {
-        const int s = t & 1;
-        if (t >= 2) ok = mbar_wait_bounded(&empty_k[s], ((t >> 1) - 1) & 1, abort_flag, p.wait_ns);
+      int nk = 0, nv = 0;  // tiles asked for
+      auto load_k = [&] {
+        const int s = nk % L::kKStages;
+        if (nk >= L::kKStages) ok = ok && mbar_wait_bounded(&empty_k[s], (nk / L::kKStages - 1) & 1, abort_flag, p.wait_ns);
         if (!ok) return;
-        uint8_t *dst = smem + L::kOffK + s * L::kTile;
-        mbar_arrive_expect_tx(&full_k[s], L::kTile);
-        for (int b = 0; b < kQB; ++b) tma_load_3d(dst + b * kBox, &tmK, &full_k[s], b * 64, hk, (tile0 + t) * kKeys);
-        if (kRot) tma_load_3d(dst + kQB * kBox, &tmKr, &full_k[s], 0, 0, (tile0 + t) * kKeys);
+        uint8_t *dst = smem + L::kOffK + s * L::kK;
+        mbar_arrive_expect_tx(&full_k[s], L::kK);
+        for (int b = 0; b < kQB; ++b) tma_load_3d(dst + b * kKeyBox, &tmK, &full_k[s], b * 64, hk, (tile0 + nk) * kKeys);
+        if (kRot) tma_load_3d(dst + kQB * kKeyBox, &tmKr, &full_k[s], 0, 0, (tile0 + nk) * kKeys);
+        ++nk;
       };
-      load_k(0);
-      int j = 0;
-      for (; j < nkv; ++j) {
-        if (j + 1 < nkv) load_k(j + 1);
-#pragma unroll
-        for (int half = 0; half < 2 && ok; ++half) {
-          if (j >= 1) ok = mbar_wait_bounded(&empty_v[half], (j - 1) & 1, abort_flag, p.wait_ns);
-          if (!ok) break;
-          uint8_t *dst = smem + L::kOffV + half * L::kVHalf;
-          mbar_arrive_expect_tx(&full_v[half], L::kVHalf);
-          for (int b = 0; b < kVB; ++b) tma_load_3d(dst + b * (64 * 64 * 2), &tmV, &full_v[half], b * 64, hk, (tile0 + j) * kKeys + half * 64);
-        }
+      // consumption order is S_0 S_1 (PV_0 S_2) (PV_1 S_3) ...: K_0 K_1 V_0 K_2 V_1 K_3 ..., K ahead where it has the buffer
+      while (nk < min(nkv, L::kKStages)) load_k();
+      for (; nv < nkv; ++nv) {
+        const int s = nv % L::kVStages;
+        if (nv >= L::kVStages) ok = ok && mbar_wait_bounded(&empty_v[s], (nv / L::kVStages - 1) & 1, abort_flag, p.wait_ns);
         if (!ok) break;
+        uint8_t *dst = smem + L::kOffV + s * L::kV;
+        mbar_arrive_expect_tx(&full_v[s], L::kV);
+        for (int b = 0; b < kVB; ++b) tma_load_3d(dst + b * kKeyBox, &tmV, &full_v[s], b * 64, hk, (tile0 + nv) * kKeys);
+        if (nk < nkv) load_k();
       }
       if (*abort_flag) {  // no copy may still be on its way when the CTA leaves
         const unsigned long long t0 = global_timer_ns();
@@ -143,100 +135,81 @@ latent_prefill_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
           }
         };
         drain(bar_q, 0);
-        for (int t = max(0, j - 1); t <= min(j + 1, nkv - 1); ++t) drain(&full_k[t & 1], (t >> 1) & 1);
-        for (int half = 0; half < 2; ++half) drain(&full_v[half], max(0, min(j, nkv - 1) - (j < nkv ? 1 : 0)) & 1);
+        for (int t = max(0, nk - L::kKStages); t < nk; ++t) drain(&full_k[t % L::kKStages], (t / L::kKStages) & 1);
+        for (int t = max(0, nv - L::kVStages); t < nv; ++t) drain(&full_v[t % L::kVStages], (t / L::kVStages) & 1);
       }
     }
   } else if (warp == kMmaWarp) {
-    {  // the warp walks, one lane issues
-      // fp32 accumulate, bf16 operands, M = 128.  Q.K^T: N = 128, B K-major; P.V: N = kVB * 64, B MN-major
-      constexpr uint32_t kBf16 = (1u << 4) | (1u << 7) | (1u << 10) | ((kRows >> 4) << 24);
-      constexpr uint32_t idesc_qk = kBf16 | ((kKeys >> 3) << 17), idesc_pv = kBf16 | (1u << 16) | ((kVB * 64 >> 3) << 17);
-      const uint64_t dq = smem_desc(smem_u32(smem), 16, 1024);
-      const uint64_t dk = smem_desc(smem_u32(smem + L::kOffK), 16, 1024);
-      const uint64_t dv = smem_desc(smem_u32(smem + L::kOffV), 64 * 64 * 2, 1024);
-      auto issue_s = [&](int g, int t) {
-        const uint64_t dqg = dq + (uint64_t)(g * (L::kTile >> 4)), dks = dk + (uint64_t)((t & 1) * (L::kTile >> 4));
-        if (elect_one()) {
+    // the warp walks, one lane issues.  fp32 accumulate, bf16 operands, M = 128.  Q.K^T: N = 64, B K-major; P.V: N = kVB * 64, B
+    // MN-major
+    constexpr uint32_t kBf16 = (1u << 4) | (1u << 7) | (1u << 10) | ((kRows >> 4) << 24);
+    constexpr uint32_t idesc_qk = kBf16 | ((kKeys >> 3) << 17), idesc_pv = kBf16 | (1u << 16) | ((kVB * 64 >> 3) << 17);
+    const uint64_t dq = smem_desc(smem_u32(smem), 16, 1024);
+    const uint64_t dk = smem_desc(smem_u32(smem + L::kOffK), 16, 1024);
+    const uint64_t dv = smem_desc(smem_u32(smem + L::kOffV), kKeyBox, 1024);
+    RingPos k, v;
+    auto issue_s = [&](int j) -> bool {
+      if (!mbar_wait_warp(&full_k[k.slot], k.parity, abort_flag, p.wait_ns)) return false;
+      tc_fence_after();
+      const uint64_t dks = dk + (uint64_t)(k.slot * (L::kK >> 4));
+      if (elect_one()) {
 #pragma unroll
-          for (int ks = 0; ks < L::kBlocks * 4; ++ks) {
-            const uint32_t off = ((ks >> 2) * kBox + (ks & 3) * 32) >> 4;
-            umma_f16(tmem + g * 128, dqg + off, dks + off, idesc_qk, ks > 0);
-          }
-          umma_commit(&bar_s[g]);
-        }
-      };
-      bool ok = mbar_wait_warp(bar_q, 0, abort_flag, p.wait_ns) && mbar_wait_warp(&full_k[0], 0, abort_flag, p.wait_ns);
-      if (ok) {
-        tc_fence_after();
-        if (nkv_g[0] > 0) issue_s(0, 0);
-        if (nkv_g[1] > 0) issue_s(1, 0);
-        if (elect_one()) umma_commit(&empty_k[0]);
+        for (int ks = 0; ks < L::kBlocks * 4; ++ks)
+          umma_f16(tmem + (j & 1) * kKeys, dq + (uint64_t)(((ks >> 2) * kBox + (ks & 3) * 32) >> 4),
+                   dks + (uint64_t)(((ks >> 2) * kKeyBox + (ks & 3) * 32) >> 4), idesc_qk, ks > 0);
+        umma_commit(&bar_s[j & 1]);
+        umma_commit(&empty_k[k.slot]);
       }
-      for (int j = 0; j < nkv && ok; ++j) {
-        const int last_g = nkv_g[1] > j ? 1 : 0;
-        bool have_k = false;
-#pragma unroll
-        for (int g = 0; g < 2; ++g) {
-          if (j >= nkv_g[g]) continue;
-          ok = mbar_wait_warp(&bar_p[g], j & 1, abort_flag, p.wait_ns);
-          if (!ok) break;
-#pragma unroll
-          for (int half = 0; half < 2; ++half) {
-            ok = ok && mbar_wait_warp(&full_v[half], j & 1, abort_flag, p.wait_ns);
-            if (!ok) break;
-            tc_fence_after();
-            const uint64_t dvh = dv + (uint64_t)(half * (L::kVHalf >> 4));
-            if (elect_one()) {
-#pragma unroll
-              for (int ks = 0; ks < 4; ++ks)  // 16 keys: 8 columns of P, 2 KB of V
-                umma_f16_ts(tmem_o(g), tmem_p(g) + half * 32 + ks * 8, dvh + (uint64_t)(ks * (2048 >> 4)), idesc_pv,
-                            j > 0 || half > 0 || ks > 0);
-              if (g == last_g) umma_commit(&empty_v[half]);
-            }
-          }
-          if (!ok) break;
-          if (j == nkv_g[g] - 1 && elect_one()) umma_commit(&bar_fin[g]);
-          if (j + 1 < nkv_g[g]) {
-            if (!have_k) ok = mbar_wait_warp(&full_k[(j + 1) & 1], ((j + 1) >> 1) & 1, abort_flag, p.wait_ns);
-            if (!ok) break;
-            have_k = true;
-            tc_fence_after();
-            issue_s(g, j + 1);
-          }
-        }
-        if (ok && j + 1 < nkv && elect_one()) umma_commit(&empty_k[(j + 1) & 1]);
-      }
-    }
-  } else {
-    // ---- softmax warps: query tile g, thread = row ----
-    const int g = warp >> 2, row = threadIdx.x & (kRows - 1);
-    const int my_nkv = g ? nkv_g[1] : nkv_g[0];
-    const int t_row = q0 + g * kRows + row;
-    const int kv_end = min(p.start + t_row + 1, p.skv), kv_begin = p.window > 0 ? max(0, p.start + t_row + 1 - p.window) : 0;
-    const uint32_t lane_base = (uint32_t)((warp & 3) * 32) << 16;
-    const uint32_t ts = tmem + g * 128 + lane_base, to = tmem_o(g) + lane_base, tp = tmem_p(g) + lane_base;
-    float m_run = -INFINITY, l_run = 0.f;
-    bool ok = true;
-    for (int j = 0; j < my_nkv && ok; ++j) {
-      ok = __all_sync(0xffffffffu, mbar_wait_bounded(&bar_s[g], j & 1, abort_flag, p.wait_ns));
+      k.next(L::kKStages);
+      return true;
+    };
+    bool ok = mbar_wait_warp(bar_q, 0, abort_flag, p.wait_ns) && issue_s(0);
+    if (ok && nkv > 1) ok = issue_s(1);
+    for (int j = 0; j < nkv && ok; ++j) {
+      ok = mbar_wait_warp(&bar_p[j & 1], (j >> 1) & 1, abort_flag, p.wait_ns) &&
+           mbar_wait_warp(&full_v[v.slot], v.parity, abort_flag, p.wait_ns);
       if (!ok) break;
       tc_fence_after();
-      uint32_t sr[4][32];
+      const uint64_t dvs = dv + (uint64_t)(v.slot * (L::kV >> 4));
+      if (elect_one()) {
 #pragma unroll
-      for (int c = 0; c < 4; ++c) tmem_ld32_async(ts + c * 32, sr[c]);
+        for (int ks = 0; ks < kKeys / 16; ++ks)  // 16 keys: 8 columns of P, 2 KB of V
+          umma_f16_ts(tmem_o, tmem + (j & 1) * kKeys + ks * 8, dvs + (uint64_t)(ks * (2048 >> 4)), idesc_pv, j > 0 || ks > 0);
+        umma_commit(bar_o);
+        umma_commit(&empty_v[v.slot]);
+        if (j == nkv - 1) umma_commit(bar_fin);
+      }
+      v.next(L::kVStages);
+      // S_{j+2} takes the place of P_j: products of unlike shapes have no order of their own, so P_j.V_j is waited for
+      if (j + 2 < nkv) ok = mbar_wait_warp(bar_o, j & 1, abort_flag, p.wait_ns) && issue_s(j + 2);
+    }
+  } else {
+    // ---- softmax warps: thread = row ----
+    const int row = threadIdx.x, t_row = q0 + row;
+    const int kv_end = min(p.start + t_row + 1, p.skv), kv_begin = p.window > 0 ? max(0, p.start + t_row + 1 - p.window) : 0;
+    const uint32_t lane_base = (uint32_t)(warp * 32) << 16, to = tmem_o + lane_base;
+    float m_run = -INFINITY, l_run = 0.f, sum4[4] = {0.f, 0.f, 0.f, 0.f};
+    bool ok = true;
+    for (int j = 0; j < nkv && ok; ++j) {
+      ok = mbar_wait_warp(&bar_s[j & 1], (j >> 1) & 1, abort_flag, p.wait_ns);
+      if (!ok) break;
+      tc_fence_after();
+      const uint32_t ts = tmem + (j & 1) * kKeys + lane_base;
+      uint32_t sr[2][32];
+#pragma unroll
+      for (int c = 0; c < 2; ++c) tmem_ld32_async(ts + c * 32, sr[c]);
       tmem_wait_ld();
       const int n0 = (tile0 + j) * kKeys;
       if (n0 < kv_begin) {
 #pragma unroll
-        for (int c = 0; c < 4; ++c)
+        for (int c = 0; c < 2; ++c)
 #pragma unroll
           for (int i = 0; i < 32; ++i)
             if (n0 + c * 32 + i < kv_begin) sr[c][i] = 0xff800000u;  // -inf
       }
       if (n0 + kKeys > kv_end) {
 #pragma unroll
-        for (int c = 0; c < 4; ++c)
+        for (int c = 0; c < 2; ++c)
 #pragma unroll
           for (int i = 0; i < 32; ++i)
             if (n0 + c * 32 + i >= kv_end) sr[c][i] = 0xff800000u;  // -inf
@@ -253,11 +226,11 @@ latent_prefill_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
       }
       const float m_safe = (m_run == -INFINITY) ? 0.f : m_run;
       const uint64_t scale2 = pack_f32x2(p.scale_log2, p.scale_log2), shift2 = pack_f32x2(-m_safe, -m_safe);
-      // neighbours first: the order of these additions shows in the last bit of the results (even and odd scores apart, two
-      // additions per instruction: 152 us instead of 157 at 2048 rows over 8192 keys, 16 heads of 128)
-      float sum4[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
-      for (int c = 0; c < 4; ++c) {
+      for (int i = 0; i < 4; ++i) sum4[i] *= corr;
+      // neighbours first, and 128 keys together: the order of these additions shows in the last bit of the results
+#pragma unroll
+      for (int c = 0; c < 2; ++c) {
         uint32_t packed[16];
 #pragma unroll
         for (int i = 0; i < 32; i += 4) {
@@ -272,11 +245,20 @@ latent_prefill_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
           sum4[(i >> 1) & 3] += w[0] + w[1];
           sum4[((i >> 1) & 3) + 1] += w[2] + w[3];
         }
-        tmem_st16(tp + c * 16, packed);
+        tmem_st16(ts + c * 16, packed);
       }
-      l_run = l_run * corr + ((sum4[0] + sum4[1]) + (sum4[2] + sum4[3]));
-      // bar_s of tile j was committed after P(j-1).V_{j-1}: that product is complete and O_g may be rescaled
+      l_run *= corr;
+      if (((tile0 + j) & 1) || j == nkv - 1) {
+        l_run += (sum4[0] + sum4[1]) + (sum4[2] + sum4[3]);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) sum4[i] = 0.f;
+      }
+      // O is in use by P_{j-1}.V_{j-1} until that completes (P_j.V_j is not issued before this warp arrives below, so the barrier
+      // cannot be more than one phase ahead of the parity asked for)
       if (j > 0 && moved) {
+        ok = mbar_wait_warp(bar_o, (j - 1) & 1, abort_flag, p.wait_ns);
+        if (!ok) break;
+        tc_fence_after();
 #pragma unroll
         for (int c = 0; c < kVB * 2; ++c) {
           uint32_t r[32];
@@ -289,11 +271,11 @@ latent_prefill_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
       asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
       tc_fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive(&bar_p[g]);
+      if (lane == 0) mbar_arrive(&bar_p[j & 1]);
     }
-    if (ok && my_nkv > 0) ok = __all_sync(0xffffffffu, mbar_wait_bounded(&bar_fin[g], 0, abort_flag, p.wait_ns));
+    if (ok && nkv > 0) ok = mbar_wait_warp(bar_fin, 0, abort_flag, p.wait_ns);
     tc_fence_after();
-    if (ok && my_nkv > 0) {
+    if (ok && nkv > 0) {
       float inv = l_run > 0.f ? 1.0f / l_run : 0.f;
       if (p.sink) {
         const float s = p.sink[h] * kLog2e, top = fmaxf(m_run, s), w = fast_exp2(m_run - top);
@@ -322,7 +304,7 @@ latent_prefill_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
   tc_fence_before();
   __syncthreads();
   if (warp == kMmaWarp)
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;" ::"r"(tmem) : "memory");
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 256;" ::"r"(tmem) : "memory");
 }
 
 // (rows, heads, elems) with row and head strides in elements -> boxes of [box_rows rows][64 elements]
@@ -353,7 +335,7 @@ int launch(const CUtensorMap (&m)[5], const Params &p, cudaStream_t st) {
       opted[dev] = true;
     }
   }
-  const dim3 grid((unsigned)p.heads * ((p.n + 2 * kRows - 1) / (2 * kRows)));
+  const dim3 grid((unsigned)p.heads * ((p.n + kRows - 1) / kRows));
   return launch_dependent(kernel, grid, dim3(kThreads), L::kSmem, st, m[0], m[1], m[2], m[3], m[4], p);
 }
 
