@@ -165,6 +165,13 @@ rms_norm_warp_kernel(const T *x, const T *w, float eps, T *out, int64_t rows, in
 
 // ---- silu_mul -----------------------------------------------------------------------------------
 __device__ __forceinline__ float silu_mul1(float g, float u) { return g / (1.0f + expf(-g)) * u; }
+// The same for results of 16 bits, with the fast exponential and division (a few units in the last of 24 bits; e^-|g|, so that the
+// divisor stays in [1, 2] and neither leaves its range).  With the exact ones the instructions, not the bytes, set the pace:
+// 2048 rows of 2 x 6144 just written, 15.5 us; so 10.6; the same error against 64 bits.
+__device__ __forceinline__ float silu_mul1_fast(float g, float u) {
+  const float t = __expf(-fabsf(g));
+  return __fdividef(g >= 0.f ? g : g * t, 1.0f + t) * u;
+}
 
 template <typename T>
 __global__ void __launch_bounds__(256)
@@ -199,7 +206,7 @@ silu_mul_rows_kernel(const T *in, long long ld, int n, long long rows, T *out, b
   using V = Vec<T>;
   if (vec) {
     // Rows and columns from the block's two dimensions (see silu_mul_rows_block): a division of 64-bit indexes per 16 bytes set
-    // the pace before (2048 rows of 2 x 6144: 17.7 us, now 15.4).
+    // the pace before (2048 rows of 2 x 6144: 17.7 us, then 15.4).
     const int nv = n / V::kN;
     for (long long r = (long long)blockIdx.y * blockDim.y + threadIdx.y; r < rows; r += (long long)gridDim.y * blockDim.y) {
       const V *row = reinterpret_cast<const V *>(in + r * ld);
@@ -207,7 +214,7 @@ silu_mul_rows_kernel(const T *in, long long ld, int n, long long rows, T *out, b
         const V g = row[c], u = row[c + nv];
         V o;
 #pragma unroll
-        for (int e = 0; e < V::kN; ++e) o.set(e, silu_mul1(g.get(e), u.get(e)));
+        for (int e = 0; e < V::kN; ++e) o.set(e, sizeof(T) == 2 ? silu_mul1_fast(g.get(e), u.get(e)) : silu_mul1(g.get(e), u.get(e)));
         reinterpret_cast<V *>(out + r * n)[c] = o;
       }
     }

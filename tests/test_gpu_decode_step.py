@@ -398,6 +398,24 @@ def test_silu_mul_rows_shapes(dtype, rows, n):
     assert ((ops.silu_mul_rows(x, n).float() - ref).abs() <= tol * ref.abs() + 1e-6).all()
 
 
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+def test_silu_mul_rows_at_the_ends_of_the_gate(dtype):
+    """Gates where an exponential overflows, vanishes or is not a number: half a unit of the result's type beside the fp64 value,
+    and what 32 bits flush to zero."""
+    from axono_b200 import ops
+
+    gate = torch.tensor([-float("inf"), -3e4, -200, -104, -89, -88.5, -88, -87.5, -87, -30, -1e-3, -0.0, 0.0, 1e-3, 30, 88, 89, 3e4, float("inf"),
+                         float("nan"), 1, -1, 5, -5]).to(dtype)
+    up = torch.tensor([1.0, -2.0, 3.0, 0.5, 1.5, -1.0, 0.25, 2.0]).to(dtype).repeat(3)
+    got = ops.silu_mul_rows(torch.cat([gate, up])[None].cuda(), 24)[0].cpu().double()
+    g, u = gate.double(), up.double()
+    want = torch.where(g == -float("inf"), torch.nan, g * torch.sigmoid(g)) * u
+    want = want.to(dtype).double()  # infinite where it is beyond the type
+    assert torch.equal(got.isnan(), want.isnan()) and torch.equal(got.isinf(), want.isinf())
+    fin = want.isfinite()
+    assert ((got - want).abs()[fin] <= torch.finfo(dtype).eps * want.abs()[fin] + 1e-35).all()
+
+
 def test_context_parallel_single_rank_matches_plain():
     """World of one: exchange + merge kernels on local records give the plain result."""
     from axono_b200 import ops
