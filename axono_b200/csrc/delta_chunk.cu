@@ -83,17 +83,23 @@ __device__ __forceinline__ void portion_input(const DeltaParams<__nv_bfloat16> &
 }
 
 // Convolution and silu of four channels from c on over kCount tokens from t0 on of a portion, of which `valid` are real;
-// put(i, values).
+// put(i, values of tokens i to i + 3).
 template <int kCount, typename Put>
 __device__ __forceinline__ void conv_walk(const DeltaParams<__nv_bfloat16> &p, const int4 &portion, int t0, int valid, int c, Put put) {
+  static_assert(kCount % 4 == 0, "groups of four tokens");
   const int channels = p.channels();
+  valid = min(valid, kCount);
   if (p.taps <= 4) {
-    uint2 raw[kCount];  // all on their way at once
+    const __nv_bfloat16 *x = p.proj + (int64_t)(portion.y + t0) * p.ld + c;
+    auto fetch = [&](uint2(&raw)[4], int i0) {
 #pragma unroll
-    for (int i = 0; i < kCount; ++i) {
-      raw[i] = make_uint2(0, 0);
-      if (i < valid) raw[i] = *reinterpret_cast<const uint2 *>(p.proj + (int64_t)(portion.y + t0 + i) * p.ld + c);
-    }
+      for (int i = 0; i < 4; ++i) {
+        raw[i] = make_uint2(0, 0);
+        if (i0 + i < valid) raw[i] = *reinterpret_cast<const uint2 *>(x + (i0 + i) * p.ld);
+      }
+    };
+    uint2 next[4];
+    fetch(next, 0);
     float w[4][4], past[3][4];
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
@@ -107,44 +113,55 @@ __device__ __forceinline__ void conv_walk(const DeltaParams<__nv_bfloat16> &p, c
       for (int e = 0; e < 4; ++e) past[j][e] = 0.f;
       if (j + 1 < p.taps && valid > 0) portion_input(p, portion, t0 - j - 1, c, past[j]);
     }
+#pragma unroll 1
+    for (int i0 = 0; i0 < kCount; i0 += 4) {
+      const uint2 raw[4] = {next[0], next[1], next[2], next[3]};
+      fetch(next, i0 + 4);  // on their way meanwhile
+      float y[4][4];
 #pragma unroll
-    for (int i = 0; i < kCount; ++i) {
-      const float now[4] = {bf_lo(raw[i].x), bf_hi(raw[i].x), bf_lo(raw[i].y), bf_hi(raw[i].y)};
-      float y[4];
+      for (int i = 0; i < 4; ++i) {
+        const float now[4] = {bf_lo(raw[i].x), bf_hi(raw[i].x), bf_lo(raw[i].y), bf_hi(raw[i].y)};
 #pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        y[e] = fmaf(past[2][e], w[3][e], fmaf(past[1][e], w[2][e], fmaf(past[0][e], w[1][e], now[e] * w[0][e])));
-        y[e] = i < valid ? fast_silu(y[e]) : 0.f;
-        past[2][e] = past[1][e];
-        past[1][e] = past[0][e];
-        past[0][e] = now[e];
+        for (int e = 0; e < 4; ++e) {
+          const float sum = fmaf(past[2][e], w[3][e], fmaf(past[1][e], w[2][e], fmaf(past[0][e], w[1][e], now[e] * w[0][e])));
+          y[i][e] = i0 + i < valid ? fast_silu(sum) : 0.f;
+          past[2][e] = past[1][e];
+          past[1][e] = past[0][e];
+          past[0][e] = now[e];
+        }
       }
-      put(i, y);
+      put(i0, y);
     }
     return;
   }
+#pragma unroll 1
+  for (int i0 = 0; i0 < kCount; i0 += 4) {
+    float y[4][4] = {};
 #pragma unroll
-  for (int i = 0; i < kCount; ++i) {
-    float y[4] = {};
-    if (i < valid) {
+    for (int i = 0; i < 4; ++i) {
+      if (i0 + i >= valid) continue;
       for (int j = 0; j < p.taps; ++j) {
         float in[4], w[4];
-        portion_input(p, portion, t0 + i - j, c, in);
+        portion_input(p, portion, t0 + i0 + i - j, c, in);
         load_vec<4>(p.conv + (size_t)(p.taps - 1 - j) * channels + c, w);
 #pragma unroll
-        for (int e = 0; e < 4; ++e) y[e] = fmaf(in[e], w[e], y[e]);
+        for (int e = 0; e < 4; ++e) y[i][e] = fmaf(in[e], w[e], y[i][e]);
       }
 #pragma unroll
-      for (int e = 0; e < 4; ++e) y[e] = fast_silu(y[e]);
+      for (int e = 0; e < 4; ++e) y[i][e] = fast_silu(y[i][e]);
     }
-    put(i, y);
+    put(i0, y);
   }
 }
 
 // A warp takes 16 tokens of a query or key head (all its channels: the unit norm stays inside the warp) or of 128 value
 // channels; the four warps of a block the four runs of a chunk.
+// Bound by instructions, of which a warp runs each once or four times: with all sixteen tokens unrolled the warps waited for the
+// instruction cache (42 % of their time, one instruction per scheduler in 3.2 cycles).  Groups of four tokens in a loop, the next
+// group's inputs on their way, and 72 registers, so that a portion of 2048 (16 / 8 heads of 128: 1024 blocks) is one wave: 22.9 us,
+// now 12.3, the same bits.  64 registers spill (12.7).
 template <int kDK>
-__global__ void __launch_bounds__(128)
+__global__ void __launch_bounds__(128, 7)
 delta_chunk_conv_kernel(const DeltaParams<__nv_bfloat16> p, const int4 *portions, int first, uint8_t *keys, uint8_t *values) {
   using K = KeyTiles<kDK>;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, unit = blockIdx.z;
@@ -163,8 +180,10 @@ delta_chunk_conv_kernel(const DeltaParams<__nv_bfloat16> p, const int4 *portions
     const int c = (unit - 2 * p.kv_heads) * 128 + lane * 4;
     if (c >= p.heads * p.vdim) return;
     uint8_t *dst = values + (chunk * (p.heads * p.vdim / 8) + c / 8) * (size_t)kValueTile + (c & 7) * 2;
-    conv_walk<16>(p, portion, t0, valid, 2 * p.kv_heads * p.dim + c, [&](int i, const float (&y)[4]) {
-      *reinterpret_cast<uint2 *>(dst + (run + i) * 16) = make_uint2(pack_bf16x2(y[0], y[1]), pack_bf16x2(y[2], y[3]));
+    conv_walk<16>(p, portion, t0, valid, 2 * p.kv_heads * p.dim + c, [&](int i0, const float (&y)[4][4]) {
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+        *reinterpret_cast<uint2 *>(dst + (run + i0 + i) * 16) = make_uint2(pack_bf16x2(y[i][0], y[i][1]), pack_bf16x2(y[i][2], y[i][3]));
     });
     return;
   }
@@ -172,27 +191,31 @@ delta_chunk_conv_kernel(const DeltaParams<__nv_bfloat16> p, const int4 *portions
   const int hk = is_k ? unit - p.kv_heads : unit, c = lane * 4;
   uint8_t *tiles = keys + (chunk * p.kv_heads + hk) * (size_t)K::kBytes, *tile = tiles + (is_k ? 0 : K::kTile);
   const bool real = c < p.dim;
-  float sq[16];  // of the rounded rows: their unit vectors are exact
-  conv_walk<16>(p, portion, t0, real ? valid : 0, real ? unit * p.dim + c : 0, [&](int i, const float (&y)[4]) {
-    const uint2 packed = make_uint2(pack_bf16x2(y[0], y[1]), pack_bf16x2(y[2], y[3]));
-    const float a = bf_lo(packed.x), b = bf_hi(packed.x), d = bf_lo(packed.y), e = bf_hi(packed.y);
-    sq[i] = a * a + b * b + d * d + e * e;
-    if (c < kDK) *reinterpret_cast<uint2 *>(tile + tile_at(run + i, c >> 3, kDK / 8) + (c & 4) * 2) = packed;
-  });
-  // all sixteen sums over the warp by halving exchanges: lanes 2 i and 2 i + 1 end with row i's
-#pragma unroll
-  for (int n = 8, off = 16; n > 0; n >>= 1, off >>= 1) {
-    const bool upper = lane & off;
-#pragma unroll
-    for (int i = 0; i < n; ++i) {
-      const float send = upper ? sq[i] : sq[i + n], keep = upper ? sq[i + n] : sq[i];
-      sq[i] = keep + __shfl_xor_sync(0xffffffffu, send, off);
-    }
-  }
-  sq[0] += __shfl_xor_sync(0xffffffffu, sq[0], 1);
   const float gain = is_k ? 1.f : 1.0f / sqrtf((float)p.dim);
-  if ((lane & 1) == 0)
-    reinterpret_cast<float *>(tiles + K::kOffInv)[(is_k ? 0 : kC) + run + (lane >> 1)] = gain / sqrtf(sq[0] + kUnitEps);
+  float *inv = reinterpret_cast<float *>(tiles + K::kOffInv) + (is_k ? 0 : kC) + run;
+  conv_walk<16>(p, portion, t0, real ? valid : 0, real ? unit * p.dim + c : 0, [&](int i0, const float (&y)[4][4]) {
+    float sq[4];  // of the rounded rows: their unit vectors are exact
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const uint2 packed = make_uint2(pack_bf16x2(y[i][0], y[i][1]), pack_bf16x2(y[i][2], y[i][3]));
+      const float a = bf_lo(packed.x), b = bf_hi(packed.x), d = bf_lo(packed.y), e = bf_hi(packed.y);
+      sq[i] = a * a + b * b + d * d + e * e;
+      if (c < kDK) *reinterpret_cast<uint2 *>(tile + tile_at(run + i0 + i, c >> 3, kDK / 8) + (c & 4) * 2) = packed;
+    }
+    // the four sums over the warp, two of them by halving exchanges: lanes 8 i to 8 i + 7 end with row i's
+#pragma unroll
+    for (int n = 2, off = 16; n > 0; n >>= 1, off >>= 1) {
+      const bool upper = lane & off;
+#pragma unroll
+      for (int i = 0; i < n; ++i) {
+        const float send = upper ? sq[i] : sq[i + n], keep = upper ? sq[i + n] : sq[i];
+        sq[i] = keep + __shfl_xor_sync(0xffffffffu, send, off);
+      }
+    }
+#pragma unroll
+    for (int off = 4; off > 0; off >>= 1) sq[0] += __shfl_xor_sync(0xffffffffu, sq[0], off);
+    if ((lane & 7) == 0) inv[i0 + (lane >> 3)] = gain / sqrtf(sq[0] + kUnitEps);
+  });
 }
 
 // One warp: out (16 x 8) = sign * a (16 x 16 n) . b (16 n x 8), fp32 matrices of stride kLd in shared memory, in bf16

@@ -333,6 +333,20 @@ def test_delta_in_portions_and_tokens(sizes, dtype):
             assert torch.equal(ring[0, p % mixer.taps].cpu(), proj[p, :mixer.channels])
 
 
+@pytest.mark.parametrize("taps", [1, 3, 4, 6])
+@pytest.mark.parametrize("dim", [100, 128])
+def test_delta_convolution_at_the_ends_of_its_groups(dim, taps):
+    """Portions that end, begin and hand over at every place of a group of four tokens and of a run of sixteen (two bf16 roundings of
+    an activation, 2^-8 each, within the tolerance of the tests above)."""
+    mixer = Mixer(4, 2, dim, 40, taps, torch.bfloat16, seed=8)
+    proj = mixer.inputs(24 + 25 + 26 + 27 + 1 + 33 + 64, 11)
+    want, states = mixer.plain(proj)
+    state, ring = mixer.slots(1)
+    got, = run_delta(mixer, mixer.weights(), [proj], [[c] for c in (24, 25, 26, 27, 1, 33, 64)], state, ring)
+    close(got, want, 2e-2)
+    close(state[0], states, 2e-2)
+
+
 @pytest.mark.parametrize("dtype", DTYPES)
 def test_delta_unequal_batch_and_slots_used_again(dtype):
     mixer = Mixer(8, 4, 128, 128, 4, dtype, seed=3)
