@@ -77,9 +77,10 @@ class ModelRunner:
         order = sorted(range(len(entries)), key=lambda i: len(entries[i][1]))
         total, wanted = sum(len(e[1]) for e in entries), sum(len(e[2]) for e in entries)
         # One copy for the step's integers, from page-locked memory: portions (32 bits, read 16 bytes at a time), token ids and wanted
-        # rows (64 bits), then sequences, positions and rows before (32 bits).  A copy from pageable memory waits for everything launched before it: three of them per step left the
-        # GPU idle while the host prepared and launched the first kernels (a prompt of 8192 in four portions: 5.2 ms, 4.5 of kernels).
-        # The allocator of page-locked blocks gives one out again only after the copies from it are done.
+        # rows (64 bits), then sequences, positions and rows before (32 bits).  A copy from pageable memory waits for everything
+        # launched before it: three of them per step left the GPU idle while the host prepared and launched the first kernels (a
+        # prompt of 8192 in four portions: 5.2 ms, 4.5 of kernels).  The allocator of page-locked blocks gives one out again only
+        # after the copies from it are done.
         n_portions = sum(len(e[1]) > 1 for e in entries)
         ids_at, small_at = 2 * n_portions, 2 * n_portions + total + wanted  # in units of 64 bits
         staged = torch.empty(small_at + (3 * total + 1) // 2, dtype=torch.int64, pin_memory=self.model.device.type == "cuda")
