@@ -39,10 +39,10 @@ constexpr int kBlock = 64;              // K per tile
 constexpr int kUnit = 32;               // weight rows per tile
 constexpr int kTile = kUnit * kBlock * 2;
 constexpr int kStages = 4;
-// Buffers of the exchange in a pair.  A CTA sends its sums of unit u + 3 after it has those of unit u + 2 from the other, which
-// sent them behind a barrier that its threads reached after they had read what they got for unit u: three can be written
-// without asking.
-constexpr int kRecvs = 3;
+// Buffers of the exchange in a pair.  A CTA's senders send its sums of unit n behind a barrier that its owners reached after they had
+// read the other CTA's sums of unit n - 2 (they read those of n - 1 beside this send).  The other CTA sent n - 2 behind a barrier that
+// its owners reached after they had read what they got for unit n - 4: four can be written without asking, three cannot.
+constexpr int kRecvs = 4;
 
 constexpr int kHeld = 4;    // blocks whose inputs a warp holds
 constexpr int kSlots = 3;   // tiles in flight per warp
