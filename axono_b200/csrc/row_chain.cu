@@ -25,7 +25,8 @@
 //
 // Between stages all CTAs meet at a counter, so the launch is cooperative with one CTA per SM: two launches of this
 // kernel cannot be resident together (each takes most of every SM's shared memory), which is also why the counter can be the
-// device's.  Every wait is bounded; after one that ran out the CTA goes through the remaining stages without waiting.
+// device's.  Every wait is bounded; after one that ran out the CTA goes through the remaining stages without waiting, sends all that
+// its pair may wait for, arms no more barriers, and leaves when what the other CTA sends has landed.
 #include <mutex>
 
 #include "tcgen05.cuh"
@@ -124,6 +125,34 @@ __device__ __forceinline__ void send2(uint32_t to, float a, float b, uint32_t ba
                : "memory");
 }
 
+// More bytes that the barrier's phase has to wait for, without an arrival.
+__device__ __forceinline__ void mbar_expect_tx(uint64_t *bar, uint32_t bytes) {
+  asm volatile("mbarrier.expect_tx.relaxed.cta.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes) : "memory");
+}
+
+// After a wait that ran out: nothing that the other CTA sends may still be on its way when this one leaves its shared memory.  The
+// other sends `sent` units of kRecv bytes into the barriers in turn, whatever happened to it, and this CTA armed phases for the first
+// `armed`.  What is left is added to whichever phase a barrier is in - the armed one where sums of later units landed in it, else the
+// next - and one more arrival ends that; so the last phase of each completes when all bytes are there.  (A phase counts less than
+// 1 MB: for more columns than any vocabulary has, the time alone has to do.)
+__device__ __noinline__ void drain(uint64_t *got, int sent, int armed, unsigned long long limit_ns) {
+  const unsigned long long t0 = global_timer_ns();
+  for (int i = 0; i < kRecvs; ++i) {
+    const int phases = (armed - i + kRecvs - 1) / kRecvs, rest = (sent - i + kRecvs - 1) / kRecvs - phases;
+    auto wait = [&](int phase) {
+      while (!mbar_try_wait(&got[i], phase & 1) && global_timer_ns() - t0 < limit_ns) {
+      }
+    };
+    const bool counts = rest <= ((1 << 20) - 1) / kRecv;
+    if (rest > 0 && counts) mbar_expect_tx(&got[i], (uint32_t)(rest * kRecv));
+    if (phases > 0) wait(phases - 1);
+    if (rest > 0) {
+      if (counts) mbar_arrive(&got[i]);
+      wait(phases);
+    }
+  }
+}
+
 // KC: blocks of the norms' width that a warp has.
 template <int KC>
 __global__ void __launch_bounds__(kThreads, 1) row_chain_kernel(const __grid_constant__ ChainParams p) {
@@ -216,7 +245,7 @@ __global__ void __launch_bounds__(kThreads, 1) row_chain_kernel(const __grid_con
   const float2 *const recv = reinterpret_cast<const float2 *>(smem + kOffRecv);
   const uint32_t peer_recv = in_cta(recv, half ^ 1), peer_got = in_cta(got_all, half ^ 1);
   RingPos sent, got;
-  int units_done = 0;
+  int units_done = 0, armed = 0;
 
   asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
   grid_dependency_wait();
@@ -301,7 +330,7 @@ __global__ void __launch_bounds__(kThreads, 1) row_chain_kernel(const __grid_con
     // sums of the unit, complete after the exchange
     auto finish = [&](int u) {
       if (owner) {
-        mbar_wait_warp(&got_all[got.slot], got.parity, abort_flag, p.wait_ns);
+        if (!__any_sync(0xffffffffu, *abort_flag)) mbar_wait_warp(&got_all[got.slot], got.parity, abort_flag, p.wait_ns);
         const float2 other = recv[got.slot * (kRecv / 8) + v_i];
         mine[0] += other.x, mine[1] += other.y;
       }
@@ -358,7 +387,10 @@ __global__ void __launch_bounds__(kThreads, 1) row_chain_kernel(const __grid_con
         for (int i = 0; i < 4; ++i) red[((warp * 2 + m) * 4 + i) * 32 + lane] = acc[m][i];
       __syncthreads();
       if (last >= 0) finish(last);
-      if (threadIdx.x == 0) mbar_arrive_expect_tx(&got_all[sent.slot], kRecv);
+      if (threadIdx.x == 0 && !*abort_flag) {  // this warp has waited for every phase armed so far, so none is armed twice
+        mbar_arrive_expect_tx(&got_all[sent.slot], kRecv);
+        ++armed;
+      }
       if (owner || sender) {  // accumulators 0 and 1 are the rows of the first CTA, 2 and 3 of the second
         const int e = (owner ? half : half ^ 1) * 2 + v_e;
 #pragma unroll
@@ -384,14 +416,8 @@ __global__ void __launch_bounds__(kThreads, 1) row_chain_kernel(const __grid_con
       if (g == 0 && v_n < p.rows) p.squares[(size_t)v_n * gridDim.x + blockIdx.x] = sq;
     }
   }
-  // after a wait that ran out: nothing of the other CTA's may still be on its way when this one leaves
-  if (*abort_flag) {
-    for (int i = 0; i < units_done && i < kRecvs; ++i) {  // its last sums, in the three barriers
-      const int back = units_done - 1 - i;
-      for (int spin = 0; spin < (1 << 20) && !mbar_try_wait(&got_all[back % kRecvs], (back / kRecvs) & 1); ++spin) {
-      }
-    }
-  }
+  // the other CTA may still be in its own waits, each as long as the limit at most: three meetings and one exchange
+  if (threadIdx.x == 0 && *abort_flag) drain(got_all, units_done, armed, kWaitNanos + 4 * min(p.wait_ns, 1ull << 60));
 }
 
 bool al16(const void *p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }

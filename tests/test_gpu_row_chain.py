@@ -93,6 +93,27 @@ def test_row_chain_in_a_graph_and_on_two_streams():
     assert ops.last_error() == 0
 
 
+def test_row_chain_whose_waits_run_out_returns():
+    """Two pairs of CTAs have 64 MB of the first product each, the others meet without them after 100 us: they go on, the call returns with
+    the flag set, and the next one is as the one before."""
+    from axono_b200 import _capi
+
+    lib = _capi.lib()
+    x, w = _inputs(8, 1 << 20, 64, 2048, 4864)
+    _, want = ops.row_chain(x, eps=1e-6, **w)
+    assert ops.last_error() == 0
+    try:
+        assert lib.axb200_set_wait_limit_ns(1) == 0
+        ops.row_chain(x, eps=1e-6, **w)
+        torch.cuda.synchronize()
+        assert ops.last_error() == 1  # AXB200_ERR_WAIT_TIMEOUT
+    finally:
+        lib.axb200_set_wait_limit_ns(2_000_000_000)
+    for _ in range(2):
+        assert torch.equal(ops.row_chain(x, eps=1e-6, **w)[1], want)
+    assert ops.last_error() == 0
+
+
 @pytest.mark.parametrize("batch", [1, 8, 9])
 def test_tower_step_with_and_without_the_chain(batch):
     """The step with two launches per layer against the step of single operators, from the same state."""

@@ -1,6 +1,7 @@
 """The exchange between the two CTAs of a pair in row_chain.cu as a model, every order of its steps (no GPU): the warps of a CTA meet at
-barriers and nowhere else, and sums that were sent arrive at any later time.  The number of buffers is read from the source."""
+barriers and nowhere else, and sums that were sent arrive at any later time.  The number of buffers is read from the source.  And what becomes of the exchange when a wait runs out, with barriers that count arrivals and bytes."""
 import pathlib
+import random
 import re
 
 import pytest
@@ -76,3 +77,105 @@ def test_the_model_tells_enough_buffers_from_too_few(slots, bad):
 
 def test_sums_are_read_before_others_take_their_place():
     assert not overwritten(buffers())
+
+
+class Barrier:
+    """One arrival and the bytes it announces per phase."""
+
+    def __init__(self):
+        self.phase, self.pending, self.bytes = 0, 1, 0
+
+    def change(self, arrivals=0, expected=0, landed=0):
+        assert self.pending >= arrivals, "an arrival too many"
+        self.pending -= arrivals
+        self.bytes += expected - landed
+        if self.pending == 0 and self.bytes == 0:
+            self.phase, self.pending = self.phase + 1, 1
+
+    def ended(self, phase):  # what a wait on the phase's parity says
+        return (self.phase & 1) != (phase & 1)
+
+
+def run_pair(rng, arm_after_giving_up: bool) -> bool:
+    """A pair in a random order of steps in which waits run out at random; whether every send of a CTA had landed when the other left."""
+    slots = buffers()
+    bars = [[Barrier() for _ in range(slots)] for _ in (0, 1)]
+    under_way, left, gave_up = [[], []], [False, False], [False, False]
+    met = [[0, 0], [0, 0]]
+    lost = False
+
+    def meet(cta, who, n):
+        met[cta][who] = n
+        while met[cta][1 - who] < n:
+            yield
+
+    def owners(cta):
+        armed = 0
+
+        def read(n):
+            while not gave_up[cta] and not bars[cta][n % slots].ended(n // slots):
+                if rng.random() < 0.02:
+                    gave_up[cta] = True
+                yield
+
+        for n in range(UNITS):
+            yield from meet(cta, 0, n + 1)
+            if n:
+                yield from read(n - 1)
+            if arm_after_giving_up or not gave_up[cta]:
+                bars[cta][n % slots].change(arrivals=1, expected=1)
+                armed += 1
+            yield
+        yield from read(UNITS - 1)
+        yield from meet(cta, 0, UNITS + 1)
+        if gave_up[cta]:
+            for i, bar in enumerate(bars[cta]):
+                phases = (armed - i + slots - 1) // slots
+                rest = (UNITS - i + slots - 1) // slots - phases
+                if rest:
+                    bar.change(expected=rest)
+                yield
+                while phases and not bar.ended(phases - 1):
+                    yield
+                if rest:
+                    bar.change(arrivals=1)
+                    while not bar.ended(phases):
+                        yield
+        left[cta] = True
+
+    def senders(cta):
+        for n in range(UNITS):
+            yield from meet(cta, 1, n + 1)
+            under_way[1 - cta].append(n)
+            yield
+        yield from meet(cta, 1, UNITS + 1)
+
+    threads = [owners(0), senders(0), owners(1), senders(1)]
+    for _ in range(200000):
+        if rng.random() < 0.5:
+            cta = rng.randrange(2)
+            if under_way[cta]:
+                n = under_way[cta].pop(rng.randrange(len(under_way[cta])))
+                lost |= left[cta]
+                if not left[cta]:
+                    bars[cta][n % slots].change(landed=1)
+        elif threads:
+            t = rng.choice(threads)
+            try:
+                next(t)
+            except StopIteration:
+                threads.remove(t)
+        elif not any(under_way):
+            return not lost
+    raise TimeoutError("a wait without an end")
+
+
+def test_all_sums_have_landed_when_a_cta_leaves():
+    for seed in range(3000):
+        assert run_pair(random.Random(seed), arm_after_giving_up=False)
+
+
+def test_barriers_armed_after_a_wait_ran_out_would_miscount():
+    with pytest.raises(AssertionError, match="an arrival too many"):
+        for seed in range(3000):
+            run_pair(random.Random(seed), arm_after_giving_up=True)
