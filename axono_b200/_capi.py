@@ -103,6 +103,7 @@ SIGNATURES = {
     "axb200_row_chain_supported": (_i, [_i64, _i, _i, _i, _i, _i]),
     "axb200_row_chain_workspace_bytes": (_sz, [_i64, _i, _i]),
     "axb200_row_chain": (_i, [*[_vp] * 10, _i64, _i, _i, _i, _i, _f, _i, _vp, _sz, _vp]),
+    "axb200_row_chain_constant": (_i, [*[_vp] * 10, _i64, _i, _i, _i, _i, _f, _i, _i, _vp, _sz, _vp]),
     "axb200_residual_post_norm": (_i, [_vp, _vp, _vp, _f, _f, _vp, _vp, _i64, _i, _i, _vp]),
     "axb200_latent_prepare": (_i, [_vp, _i64, _i, _i, _vp, _i64, _i, _vp, _vp, _vp, _i64, _i, _vp, _f] + [_vp] * 5 +
                               [_i, _i, _i64] + [_i] * 5 + [_vp]),

@@ -68,6 +68,7 @@ struct ChainParams {
   float *squares;       // (rows, grid): sums of squares of the CTAs' columns, for the norm of the stage that follows
   float eps;
   int rows;
+  int weights_ready;  // weights may be read before the launch in front of this one is over
   unsigned long long wait_ns;
 };
 
@@ -225,6 +226,7 @@ __global__ void __launch_bounds__(kThreads, 1) row_chain_kernel(const __grid_con
     asm volatile("cp.async.commit_group;" ::: "memory");  // an empty one at the end: every tile stays a group of its own
     put = put + 1 == kSlots ? 0 : put + 1;
   };
+  if (!p.weights_ready) grid_dependency_wait();
 #pragma unroll 1
   for (int i = 0; i < kSlots; ++i) ask();
   // the warp's oldest tile, and its slot given back
@@ -503,6 +505,14 @@ size_t axb200_row_chain_workspace_bytes(int64_t rows, int width, int ff) {
 int axb200_row_chain(const void *x, const void *w_o, const void *residual, const void *norm1, const void *w_gate_up, const void *w_down,
                      const void *norm2, const void *w_next, void *residual_out, void *out, int64_t rows, int attn, int width, int ff,
                      int next, float eps, int dtype, void *workspace, size_t workspace_bytes, void *stream) {
+  return axb200_row_chain_constant(x, w_o, residual, norm1, w_gate_up, w_down, norm2, w_next, residual_out, out, rows, attn, width, ff, next,
+                                   eps, dtype, 0, workspace, workspace_bytes, stream);
+}
+
+int axb200_row_chain_constant(const void *x, const void *w_o, const void *residual, const void *norm1, const void *w_gate_up,
+                              const void *w_down, const void *norm2, const void *w_next, void *residual_out, void *out, int64_t rows,
+                              int attn, int width, int ff, int next, float eps, int dtype, int weights_ready, void *workspace,
+                              size_t workspace_bytes, void *stream) {
   for (const void *q : {x, w_o, residual, norm1, w_gate_up, w_down, norm2, w_next, static_cast<const void *>(residual_out),
                         static_cast<const void *>(out), static_cast<const void *>(workspace)}) {
     if (!q) return AXB200_INVALID_PTR;
@@ -523,7 +533,7 @@ int axb200_row_chain(const void *x, const void *w_o, const void *residual, const
   p.st[3] = {w_next, residual_out, out, width, next, blocks(width), units(next, axb::kUnit), 0};
   p.res_in = residual, p.res_mid = mid;
   p.norm[0] = norm1, p.norm[1] = norm2;
-  p.eps = eps, p.rows = (int)rows, p.wait_ns = axb::wait_limit_ns();
+  p.eps = eps, p.rows = (int)rows, p.weights_ready = weights_ready != 0, p.wait_ns = axb::wait_limit_ns();
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   return axb::blocks_held(width) <= 1 ? axb::launch<1>(p, st) : axb::launch<2>(p, st);
 }

@@ -193,7 +193,8 @@ class TextTower:
 
     def _chained_layers(self, h) -> torch.Tensor:
         """The layers with two launches each: the step of the attention (norms, rope, append and attention) and `ops.row_chain`,
-        whose last product is the next layer's QKV projection or the logits."""
+        whose last product is the next layer's QKV projection or the logits.  The weights are ready for every chain: the embedding
+        that a step begins with is launched behind all that came before it."""
         cfg, last = self.cfg, self.cfg.n_layers - 1
         out = self._linear(ops.rms_norm(h, self.layers[0]["input_ln"], cfg.eps), self.layers[0]["qkv"])
         for li, lw in enumerate(self.layers):
@@ -202,7 +203,8 @@ class TextTower:
                                        inv_freq=self.inv_freq if cfg.use_mrope else None, theta=cfg.rope_theta,
                                        mrope_section=cfg.mrope_section if cfg.use_mrope else None)
             norm, w = (self.final_ln, self.embed) if li == last else (self.layers[li + 1]["input_ln"], self.layers[li + 1]["qkv"])
-            h, out = ops.row_chain(attn.view(self.batch, -1), lw["o"], h, lw["post_ln"], lw["gate_up"], lw["down"], norm, w, cfg.eps)
+            h, out = ops.row_chain(attn.view(self.batch, -1), lw["o"], h, lw["post_ln"], lw["gate_up"], lw["down"], norm, w, cfg.eps,
+                                   weights_ready=True)
         return out
 
     def _finish_step(self, logits) -> torch.Tensor:

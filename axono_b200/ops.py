@@ -470,9 +470,10 @@ def row_chain_supported(rows, attn, width, ff, next_, dtype) -> bool:
     return dtype == torch.float16 and bool(_capi.lib().axb200_row_chain_supported(rows, attn, width, ff, next_, _capi.FLOAT16))
 
 
-def row_chain(x, w_o, residual, norm1, w_gate_up, w_down, norm2, w_next, eps):
+def row_chain(x, w_o, residual, norm1, w_gate_up, w_down, norm2, w_next, eps, weights_ready: bool = False):
     """From an attention's output x (rows, attn) to the next input product in one launch: y = x . w_o^T + residual, the gated
-    feed-forward of its norm added to it, and its norm . w_next^T.  Returns (residual, product); all operands contiguous."""
+    feed-forward of its norm added to it, and its norm . w_next^T.  Returns (residual, product); all operands contiguous.
+    weights_ready: the matrices were complete before the launch in front of this one began, so that they may be read early."""
     op = "row_chain"
     dt = _dt(x, op)
     rows, attn = x.shape
@@ -484,9 +485,9 @@ def row_chain(x, w_o, residual, norm1, w_gate_up, w_down, norm2, w_next, eps):
     lib = _capi.lib()
     end, out = torch.empty_like(residual), torch.empty((rows, n), dtype=x.dtype, device=x.device)
     ws = torch.empty(lib.axb200_row_chain_workspace_bytes(rows, width, ff), dtype=torch.uint8, device=x.device)
-    _call(lib.axb200_row_chain(x.data_ptr(), w_o.data_ptr(), residual.data_ptr(), norm1.data_ptr(), w_gate_up.data_ptr(),
-                               w_down.data_ptr(), norm2.data_ptr(), w_next.data_ptr(), end.data_ptr(), out.data_ptr(), rows, attn, width,
-                               ff, n, float(eps), dt, ws.data_ptr(), ws.numel(), _stream(x)), op)
+    _call(lib.axb200_row_chain_constant(x.data_ptr(), w_o.data_ptr(), residual.data_ptr(), norm1.data_ptr(), w_gate_up.data_ptr(),
+                                        w_down.data_ptr(), norm2.data_ptr(), w_next.data_ptr(), end.data_ptr(), out.data_ptr(), rows,
+                                        attn, width, ff, n, float(eps), dt, int(weights_ready), ws.data_ptr(), ws.numel(), _stream(x)), op)
     return end, out
 
 

@@ -505,13 +505,19 @@ int axb200_residual_layer_norm(float *x, const void *a, const void *b, const voi
  * fp32 sums; y, z, the activations, residual_out and the last norm are rounded to `dtype`.
  * x (rows, attn); residual, residual_out (rows, width); w_o (width, attn); w_gate_up (2 ff, width), gates first; w_down (width, ff);
  * w_next (next, width); FLOAT16, all pointers 16-byte aligned; outputs overlap no input.  Sizes: row_chain_supported (attn, width
- * and ff multiples of 64, width <= 4096).  The launch needs every SM of the device at once. */
+ * and ff multiples of 64, width <= 4096).  The launch needs every SM of the device at once.
+ * row_chain_constant with weights_ready: the four matrices were complete before the launch in front of this one began (constant
+ * weights), so that reading them need not wait for the end of that launch. */
 int axb200_row_chain_supported(int64_t rows, int attn, int width, int ff, int next, int dtype);
 size_t axb200_row_chain_workspace_bytes(int64_t rows, int width, int ff);
 int axb200_row_chain(const void *x, const void *w_o, const void *residual, const void *norm1, const void *w_gate_up,
                      const void *w_down, const void *norm2, const void *w_next, void *residual_out, void *out, int64_t rows,
                      int attn, int width, int ff, int next, float eps, int dtype, void *workspace, size_t workspace_bytes,
                      void *stream);
+int axb200_row_chain_constant(const void *x, const void *w_o, const void *residual, const void *norm1, const void *w_gate_up,
+                              const void *w_down, const void *norm2, const void *w_next, void *residual_out, void *out, int64_t rows,
+                              int attn, int width, int ff, int next, float eps, int dtype, int weights_ready, void *workspace,
+                              size_t workspace_bytes, void *stream);
 
 /* The stream of layers that norm what a sublayer puts out:
  *   embed_residual: x = table[ids] in fp32 and h (optional) the same in `dtype`; bad ids as above.

@@ -93,6 +93,33 @@ def test_row_chain_in_a_graph_and_on_two_streams():
     assert ops.last_error() == 0
 
 
+@pytest.mark.parametrize("made", ["w_o", "w_gate_up"])
+def test_row_chain_waits_for_weights_that_the_launch_before_it_writes(made):
+    """The launch in front of the chain makes one of its matrices (the rotated q of 4096 sequences), and lets dependents begin long
+    before it is done."""
+    from axono_b200.kv_cache import PagedKVCache
+
+    batch, heads, d = 4096, 16, 128
+    width, ff = (4096, 256) if made == "w_o" else (2048, 2048)
+    x, w = _inputs(8, 2048, width, ff, 128)
+    g = torch.Generator(device="cuda").manual_seed(5)
+    qkv = [(torch.randn((batch, (heads + 2) * d), generator=g, device="cuda") * 2048 ** -0.5).half() for _ in range(4)]
+    cache = PagedKVCache(1, batch, 1, d, 64)
+
+    def step(t):
+        cache.seq_lens.zero_()
+        w[made] = cache.append_qkv(0, t, heads).view(batch, heads * d)
+        return ops.row_chain(x, eps=1e-6, **w)
+
+    outs = [step(t) for t in qkv * 3]
+    for i, (_, out) in enumerate(outs):
+        cache.seq_lens.zero_()
+        w[made] = cache.append_qkv(0, qkv[i % 4], heads).view(batch, heads * d)
+        torch.cuda.synchronize()
+        assert torch.equal(out, ops.row_chain(x, eps=1e-6, weights_ready=True, **w)[1])
+    assert ops.last_error() == 0
+
+
 def test_row_chain_whose_waits_run_out_returns():
     """Two pairs of CTAs have 64 MB of the first product each, the others meet without them after 100 us: they go on, the call returns with
     the flag set, and the next one is as the one before."""
