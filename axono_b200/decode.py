@@ -77,10 +77,10 @@ class TextTower:
 
     def __init__(self, cfg: TextTowerConfig, batch: int, max_seq_len: int, device="cuda",
                  dtype=torch.float16, world: int = 1, rank: int = 0, seed: int = 0, page_tokens: int = 64,
-                 fused_gather: bool = True, fused_qkv: bool = True, lt_gemm: bool = True):
+                 fused_gather: bool = True, fused_qkv: bool = True, lt_gemm: bool = True, row_chain: bool = True):
         self.cfg, self.batch, self.device, self.dtype = cfg, batch, torch.device(device), dtype
         self.fused_qkv = fused_qkv
-        self.lt_gemm = lt_gemm
+        self.lt_gemm, self.row_chain = lt_gemm, row_chain
         self._linear = ops.linear_nobias if lt_gemm else (lambda x, w: torch.matmul(x, w.t()))
         self.world, self.rank = world, rank
         self.peer_gather = None
@@ -185,11 +185,19 @@ class TextTower:
         return self._finish_step(self._linear(xf, self.embed))
 
     def _chains(self) -> bool:
-        """Whether everything between two attention calls is one launch (`ops.row_chain`): one rank, the fused forms, and few
-        enough rows."""
+        """Whether everything between two attention calls is one launch (`ops.row_chain`): one rank, the fused forms, few
+        enough rows, and weights as that takes them (`layers` is open to a program's own, whose views the single products copy)."""
         cfg = self.cfg
-        return self.world == 1 and self.fused_qkv and self.lt_gemm and type(self.cache) is PagedKVCache and ops.row_chain_supported(
-            self.batch, cfg.n_q_heads * cfg.head_dim, cfg.hidden, cfg.intermediate, cfg.vocab, self.dtype)
+        return self.row_chain and self.world == 1 and self.fused_qkv and self.lt_gemm and type(self.cache) is PagedKVCache and \
+            ops.row_chain_supported(self.batch, cfg.n_q_heads * cfg.head_dim, cfg.hidden, cfg.intermediate, cfg.vocab, self.dtype) and \
+            all(t.is_contiguous() and t.data_ptr() % 16 == 0 for t in self._chain_weights())
+
+    def _chain_weights(self):
+        yield from (self.embed, self.final_ln)
+        for li, lw in enumerate(self.layers):
+            yield from (lw["o"], lw["post_ln"], lw["gate_up"], lw["down"])
+            if li > 0:  # the first layer's input is not a chain's
+                yield from (lw["input_ln"], lw["qkv"])
 
     def _chained_layers(self, h) -> torch.Tensor:
         """The layers with two launches each: the step of the attention (norms, rope, append and attention) and `ops.row_chain`,

@@ -141,6 +141,25 @@ def test_row_chain_whose_waits_run_out_returns():
     assert ops.last_error() == 0
 
 
+def test_row_chain_on_streams_of_unequal_priority():
+    """Each launch needs all SMs at once, with ordinary launches between them and other streams' in front."""
+    x, w = _inputs(8, 2048, 2048, 6144, 4096)
+    _, want = ops.row_chain(x, eps=1e-6, **w)
+    square = torch.randn((2048, 2048), device="cuda").half()
+    streams = [torch.cuda.Stream(priority=p) for p in (0, -1, -2)]
+    outs = []
+    for s in streams:
+        s.wait_stream(torch.cuda.current_stream())
+    for i in range(30):
+        for j, s in enumerate(streams):
+            with torch.cuda.stream(s):
+                if (i + j) % 3 == 0:
+                    ops.silu_mul_rows(square @ square, 1024)
+                outs.append(ops.row_chain(x, eps=1e-6, weights_ready=bool(i & 1), **w)[1])
+    torch.cuda.synchronize()
+    assert all(torch.equal(o, want) for o in outs) and ops.last_error() == 0
+
+
 @pytest.mark.parametrize("batch", [1, 8, 9])
 def test_tower_step_with_and_without_the_chain(batch):
     """The step with two launches per layer against the step of single operators, from the same state."""
@@ -162,3 +181,30 @@ def test_tower_step_with_and_without_the_chain(batch):
         assert (a - b).norm() <= 8 * torch.finfo(torch.float16).eps * b.norm()
         towers[1].token_ids.copy_(towers[0].token_ids)
     assert torch.equal(towers[0].cache.seq_lens, towers[1].cache.seq_lens) and ops.last_error() == 0
+
+
+def _strided(t):
+    return torch.stack([t, t], dim=-1)[..., 0]
+
+
+def _shifted(t):
+    flat = torch.empty(t.numel() + 1, dtype=t.dtype, device=t.device)
+    return flat[1:].view(t.shape).copy_(t)
+
+
+@pytest.mark.parametrize("name", ["input_ln", "qkv", "o", "post_ln", "gate_up", "down", "embed", "final_ln"])
+@pytest.mark.parametrize("view", [_strided, _shifted])
+def test_tower_with_weights_that_the_chain_does_not_take(name, view):
+    """A program's own weights as views: the step runs as single operators, with the same results as with contiguous ones."""
+    cfg = TextTowerConfig(hidden=256, intermediate=512, n_q_heads=4, n_kv_heads=2, head_dim=64, vocab=300, n_layers=2, mrope_section=(12, 10, 10))
+    towers = [TextTower(cfg, 2, 64, seed=3, row_chain=chain) for chain in (True, False)]
+    holder, key = (towers[0].layers[1], name) if name in towers[0].layers[1] else (vars(towers[0]), name)
+    assert towers[0]._chains() and not towers[1]._chains()
+    holder[key] = view(holder[key])
+    assert not towers[0]._chains()
+    for tower in towers:
+        tower.set_state([1, 2], [0, 0])
+        tower.decode_step()
+    a, b = (t.last_logits.double() for t in towers)
+    assert (a - b).norm() <= 4 * torch.finfo(torch.float16).eps * b.norm()  # a product's algorithm depends on its operands' alignment
+    assert ops.last_error() == 0
