@@ -101,6 +101,7 @@ SIGNATURES = {
     "axb200_residual_layer_norm": (_i, [_vp] * 6 + [_i] + [_vp] * 4 + [_f, _i64, _i, _i, _vp]),
     "axb200_embed_residual": (_i, [_vp] * 4 + [_i64, _i64, _i, _i, _vp]),
     "axb200_row_chain_supported": (_i, [_i64, _i, _i, _i, _i, _i]),
+    "axb200_row_chain_gains": (_i, [_i64, _i, _i, _i, _i, _i]),
     "axb200_row_chain_workspace_bytes": (_sz, [_i64, _i, _i]),
     "axb200_row_chain": (_i, [*[_vp] * 10, _i64, _i, _i, _i, _i, _f, _i, _vp, _sz, _vp]),
     "axb200_row_chain_constant": (_i, [*[_vp] * 10, _i64, _i, _i, _i, _i, _f, _i, _i, _vp, _sz, _vp]),

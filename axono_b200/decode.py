@@ -173,24 +173,34 @@ class TextTower:
                 xn = ops.rms_norm(h, lw["input_ln"], cfg.eps)
             else:  # previous layer's h + mlp folded into this layer's input norm
                 h, xn = ops.add_rms_norm(mlp_out, h, lw["input_ln"], cfg.eps)
-            attn_out = self._attention(li, xn)
-            h, xn2 = ops.add_rms_norm(attn_out, h, lw["post_ln"], cfg.eps)
-            gu = self._linear(xn2, lw["gate_up"])
-            if self.fused_qkv:
-                act = ops.silu_mul_rows(gu, cfg.intermediate)
-            else:
-                act = ops.silu_mul(gu[:, :cfg.intermediate].contiguous(), gu[:, cfg.intermediate:].contiguous())
-            mlp_out = self._linear(act, lw["down"])
-        _, xf = ops.add_rms_norm(mlp_out, h, self.final_ln, cfg.eps)
-        return self._finish_step(self._linear(xf, self.embed))
+            h, mlp_out = self._feed_forward(lw, self._attention(li, xn), h)
+        return self._finish_step(self._logits(mlp_out, h))
+
+    def _feed_forward(self, lw, attn_out, h):
+        """The second half of a layer as single operators: (h, what is still to be added to it)."""
+        cfg = self.cfg
+        h, xn2 = ops.add_rms_norm(attn_out, h, lw["post_ln"], cfg.eps)
+        gu = self._linear(xn2, lw["gate_up"])
+        if self.fused_qkv:
+            act = ops.silu_mul_rows(gu, cfg.intermediate)
+        else:
+            act = ops.silu_mul(gu[:, :cfg.intermediate].contiguous(), gu[:, cfg.intermediate:].contiguous())
+        return h, self._linear(act, lw["down"])
+
+    def _logits(self, mlp_out, h):
+        _, xf = ops.add_rms_norm(mlp_out, h, self.final_ln, self.cfg.eps)
+        return self._linear(xf, self.embed)
 
     def _chains(self) -> bool:
         """Whether everything between two attention calls is one launch (`ops.row_chain`): one rank, the fused forms, few
         enough rows, and weights as that takes them (`layers` is open to a program's own, whose views the single products copy)."""
         cfg = self.cfg
         return self.row_chain and self.world == 1 and self.fused_qkv and self.lt_gemm and type(self.cache) is PagedKVCache and \
-            ops.row_chain_supported(self.batch, cfg.n_q_heads * cfg.head_dim, cfg.hidden, cfg.intermediate, cfg.vocab, self.dtype) and \
-            all(t.is_contiguous() and t.data_ptr() % 16 == 0 for t in self._chain_weights())
+            self._chain_gains((cfg.n_q_heads + 2 * cfg.n_kv_heads) * cfg.head_dim) and all(t.is_contiguous() and t.data_ptr() % 16 == 0 for t in self._chain_weights())
+
+    def _chain_gains(self, columns: int) -> bool:
+        cfg = self.cfg
+        return ops.row_chain_gains(self.batch, cfg.n_q_heads * cfg.head_dim, cfg.hidden, cfg.intermediate, columns, self.dtype)
 
     def _chain_weights(self):
         yield from (self.embed, self.final_ln)
@@ -201,8 +211,9 @@ class TextTower:
 
     def _chained_layers(self, h) -> torch.Tensor:
         """The layers with two launches each: the step of the attention (norms, rope, append and attention) and `ops.row_chain`,
-        whose last product is the next layer's QKV projection or the logits.  The weights are ready for every chain: the embedding
-        that a step begins with is launched behind all that came before it."""
+        whose last product is the next layer's QKV projection or the logits (a narrow tower's many logits are quicker on their
+        own).  The weights are ready for every chain: the embedding that a step begins with is launched behind all that came
+        before it."""
         cfg, last = self.cfg, self.cfg.n_layers - 1
         out = self._linear(ops.rms_norm(h, self.layers[0]["input_ln"], cfg.eps), self.layers[0]["qkv"])
         for li, lw in enumerate(self.layers):
@@ -210,6 +221,9 @@ class TextTower:
                                        lw["k_norm"] if cfg.qk_norm else None, cfg.eps, pos=self.pos3 if cfg.use_mrope else self.pos3[0],
                                        inv_freq=self.inv_freq if cfg.use_mrope else None, theta=cfg.rope_theta,
                                        mrope_section=cfg.mrope_section if cfg.use_mrope else None)
+            if li == last and not self._chain_gains(cfg.vocab):
+                h, mlp_out = self._feed_forward(lw, self._linear(attn.view(self.batch, -1), lw["o"]), h)
+                return self._logits(mlp_out, h)
             norm, w = (self.final_ln, self.embed) if li == last else (self.layers[li + 1]["input_ln"], self.layers[li + 1]["qkv"])
             h, out = ops.row_chain(attn.view(self.batch, -1), lw["o"], h, lw["post_ln"], lw["gate_up"], lw["down"], norm, w, cfg.eps,
                                    weights_ready=True)

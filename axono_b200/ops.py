@@ -470,6 +470,11 @@ def row_chain_supported(rows, attn, width, ff, next_, dtype) -> bool:
     return dtype == torch.float16 and bool(_capi.lib().axb200_row_chain_supported(rows, attn, width, ff, next_, _capi.FLOAT16))
 
 
+def row_chain_gains(rows, attn, width, ff, next_, dtype) -> bool:
+    """Whether `row_chain` takes these sizes and is faster than the same as single operators."""
+    return dtype == torch.float16 and bool(_capi.lib().axb200_row_chain_gains(rows, attn, width, ff, next_, _capi.FLOAT16))
+
+
 def row_chain(x, w_o, residual, norm1, w_gate_up, w_down, norm2, w_next, eps, weights_ready: bool = False):
     """From an attention's output x (rows, attn) to the next input product in one launch: y = x . w_o^T + residual, the gated
     feed-forward of its norm added to it, and its norm . w_next^T.  Returns (residual, product); all operands contiguous.

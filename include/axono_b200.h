@@ -509,6 +509,8 @@ int axb200_residual_layer_norm(float *x, const void *a, const void *b, const voi
  * row_chain_constant with weights_ready: the four matrices were complete before the launch in front of this one began (constant
  * weights), so that reading them need not wait for the end of that launch. */
 int axb200_row_chain_supported(int64_t rows, int attn, int width, int ff, int next, int dtype);
+/* ... and whether the chain is faster than the same as launches of their own (narrow layers with many columns are not). */
+int axb200_row_chain_gains(int64_t rows, int attn, int width, int ff, int next, int dtype);
 size_t axb200_row_chain_workspace_bytes(int64_t rows, int width, int ff);
 int axb200_row_chain(const void *x, const void *w_o, const void *residual, const void *norm1, const void *w_gate_up,
                      const void *w_down, const void *norm2, const void *w_next, void *residual_out, void *out, int64_t rows,

@@ -160,12 +160,14 @@ def test_row_chain_on_streams_of_unequal_priority():
     assert all(torch.equal(o, want) for o in outs) and ops.last_error() == 0
 
 
-@pytest.mark.parametrize("batch", [1, 8, 9])
-def test_tower_step_with_and_without_the_chain(batch):
-    """The step with two launches per layer against the step of single operators, from the same state."""
-    cfg = TextTowerConfig(hidden=512, intermediate=1024, n_q_heads=8, n_kv_heads=4, head_dim=64, vocab=1000, n_layers=3, mrope_section=(12, 10, 10))
+@pytest.mark.parametrize("batch,vocab", [(1, 1000), (8, 1000), (9, 1000), (8, 40000)])
+def test_tower_step_with_and_without_the_chain(batch, vocab):
+    """The step with two launches per layer (and single operators for a narrow tower's many logits) against the step of single
+    operators, from the same state."""
+    cfg = TextTowerConfig(hidden=512, intermediate=1024, n_q_heads=8, n_kv_heads=4, head_dim=64, vocab=vocab, n_layers=3, mrope_section=(12, 10, 10))
     towers = [TextTower(cfg, batch, 192, seed=3, lt_gemm=lt) for lt in (True, False)]
     assert towers[0]._chains() == (batch <= 8) and not towers[1]._chains()
+    assert towers[0]._chain_gains(vocab) == (batch <= 8 and vocab == 1000)
     lens = [64 + 5 * b % 64 for b in range(batch)]
     g = torch.Generator(device="cuda").manual_seed(4)
     kv = [[torch.randn((batch, 128, 4, 64), generator=g, device="cuda").half() for _ in range(2)] for _ in range(cfg.n_layers)]

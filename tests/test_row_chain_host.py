@@ -1,4 +1,4 @@
-"""The exchange between the two CTAs of a pair in row_chain.cu as a model, every order of its steps (no GPU): the warps of a CTA meet at
+"""What of row_chain.cu needs no GPU.  The exchange between the two CTAs of a pair as a model, every order of its steps: the warps of a CTA meet at
 barriers and nowhere else, and sums that were sent arrive at any later time.  The number of buffers is read from the source.  And what becomes of the exchange when a wait runs out, with barriers that count arrivals and bytes."""
 import pathlib
 import random
@@ -179,3 +179,15 @@ def test_barriers_armed_after_a_wait_ran_out_would_miscount():
     with pytest.raises(AssertionError, match="an arrival too many"):
         for seed in range(3000):
             run_pair(random.Random(seed), arm_after_giving_up=True)
+
+
+@pytest.mark.parametrize("width,ff,next_,gains", [
+    (2048, 6144, 4096, 1), (2048, 6144, 151936, 1), (4096, 12288, 6144, 1), (1024, 3072, 4096, 1), (512, 1536, 1024, 1), (128, 384, 256, 1),
+    (1024, 3072, 151936, 0), (512, 1536, 32000, 0), (128, 512, 32000, 0)])
+def test_the_chain_is_taken_where_it_was_measured_faster(width, ff, next_, gains):
+    from axono_b200 import _capi
+
+    lib = _capi.lib()
+    assert lib.axb200_row_chain_supported(8, 2048, width, ff, next_, _capi.FLOAT16)
+    assert lib.axb200_row_chain_gains(8, 2048, width, ff, next_, _capi.FLOAT16) == gains
+    assert not lib.axb200_row_chain_gains(9, 2048, width, ff, next_, _capi.FLOAT16)
