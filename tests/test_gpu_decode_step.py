@@ -487,3 +487,30 @@ def test_prefill_then_decode_flow(dtype):
     vv = np.concatenate([v, vn[1:2]])
     assert oracle.rel_err(out[1:2], orc.gqa_decode(host(qn_d)[1:2], kk, vv)) <= tol
     assert cache.seq_lens.cpu().tolist() == [1, n + 1] and ops.last_error() == 0
+
+
+@pytest.mark.parametrize("window", [1, 100, 4000])
+def test_step_qkv_of_a_cache_with_a_window(window):
+    """Two layers' steps as one operator and as append and attention, over a cache that sees the last tokens alone."""
+    from axono_b200 import ops
+    from axono_b200.kv_cache import PagedKVCache, SlidingWindowKVCache
+
+    g = torch.Generator(device="cuda").manual_seed(6)
+    lens, hq, hkv, d = [300, 64, 1500], 4, 2, 64
+    qkv = torch.randn((3, (hq + 2 * hkv) * d), generator=g, device="cuda").half()
+    k, v = (torch.randn((3, 1500, hkv, d), generator=g, device="cuda").half() for _ in range(2))
+    outs = []
+    for one in (True, False):
+        cache = SlidingWindowKVCache(window, 2, 3, hkv, d, 1600)
+        for layer in (0, 1):
+            cache.fill(layer, k, v, lens)
+        if one:
+            outs.append([cache.step_qkv(layer, qkv, hq) for layer in (0, 1)])
+        else:
+            outs.append([cache.attend(layer, cache.append_qkv(layer, qkv, hq)) for layer in (0, 1)])
+        assert cache.seq_lens.tolist() == [n + 1 for n in lens] and cache._host_len_bound == 1501
+    assert all(torch.equal(a, b) for a, b in zip(*outs))
+    whole = PagedKVCache(2, 3, hkv, d, 1600)
+    whole.fill(0, k, v, lens)
+    assert torch.equal(whole.step_qkv(0, qkv, hq), outs[0][0]) == (window > 1500)
+    assert ops.last_error() == 0
