@@ -64,6 +64,9 @@ class ModelRunner:
     def step(self, entries, trace=None):
         """entries: (sequence, tokens, want) - the sequence's next tokens and the places among them whose logits
         are asked for.  Returns fp32 logits (wanted, vocab), entry by entry, or None when nothing is wanted."""
+        if self.model.device.type == "cuda" and torch.cuda.is_current_stream_capturing():
+            # a replay would copy the step's integers from a page-locked block that has long been given out again
+            raise RuntimeError("ModelRunner.step copies from the host and cannot be captured (DecodeGraph captures decoding)")
         if len({e[0] for e in entries}) != len(entries):
             raise ValueError("a sequence may appear once in a step")
         for seq, tokens, want in entries:

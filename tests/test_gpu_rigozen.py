@@ -158,6 +158,22 @@ def test_cache_overflow_is_an_error(built):
         r.step([(s, (tokens * 2)[:200], [])])
 
 
+def test_a_step_cannot_be_captured(built):
+    """Its integers come from the host: refused, with nothing changed, so that the steps after it are those of a runner that was not asked."""
+    cfg, w, tokens, _ = built("odd", 150)
+    outs = []
+    for ask in (False, True):
+        r = runner_of(cfg, w, torch.float32, 64)
+        s = r.open()
+        r.step([(s, tokens[:5], [])])
+        if ask:
+            torch.cuda.synchronize()
+            with pytest.raises(RuntimeError, match="cannot be captured"), torch.cuda.graph(torch.cuda.CUDAGraph()):
+                r.step([(s, tokens[5:9], [3])])
+        outs.append(r.step([(s, tokens[5:12], [6])]))
+    assert torch.equal(*outs)
+
+
 @pytest.mark.parametrize("name", ["odd", "recurrent"])
 def test_greedy_generation(built, name):
     """The scheduler's tokens (portions of prompts beside decoding, then graph replays) are the plain ones."""
