@@ -165,12 +165,19 @@ rms_norm_warp_kernel(const T *x, const T *w, float eps, T *out, int64_t rows, in
 
 // ---- silu_mul -----------------------------------------------------------------------------------
 __device__ __forceinline__ float silu_mul1(float g, float u) { return g / (1.0f + expf(-g)) * u; }
-// The same for results of 16 bits, with the fast exponential and division (a few units in the last of 24 bits; e^-|g|, so that the
-// divisor stays in [1, 2] and neither leaves its range).  With the exact ones the instructions, not the bytes, set the pace:
-// 2048 rows of 2 x 6144 just written, 15.5 us; so 10.6; the same error against 64 bits.
+// The same for results of 16 bits, with the fast exponential and division.  Of e^-|g|, so that the divisor stays in [1, 2] and neither
+// leaves its range; the exponential's error grows with |g| (2 + 1.16 |g| units in the last of 24 bits: 6e-6 at g = -87, a
+// three-hundredth of half a unit of bfloat16, an eightieth of float16's), and below -87.3 it is zero where the value is
+// less than 1e-36.  With the exact ones the instructions, not the bytes, set the pace: 2048 rows of 2 x 6144 just written, 15.5 us; so 10.6;
+// the same error against 64 bits.
 __device__ __forceinline__ float silu_mul1_fast(float g, float u) {
   const float t = __expf(-fabsf(g));
   return __fdividef(g >= 0.f ? g : g * t, 1.0f + t) * u;
+}
+// One element of rows, whichever pieces they are read in.
+template <typename T>
+__device__ __forceinline__ float silu_mul1_row(float g, float u) {
+  return sizeof(T) == 2 ? silu_mul1_fast(g, u) : silu_mul1(g, u);
 }
 
 template <typename T>
@@ -214,7 +221,7 @@ silu_mul_rows_kernel(const T *in, long long ld, int n, long long rows, T *out, b
         const V g = row[c], u = row[c + nv];
         V o;
 #pragma unroll
-        for (int e = 0; e < V::kN; ++e) o.set(e, sizeof(T) == 2 ? silu_mul1_fast(g.get(e), u.get(e)) : silu_mul1(g.get(e), u.get(e)));
+        for (int e = 0; e < V::kN; ++e) o.set(e, silu_mul1_row<T>(g.get(e), u.get(e)));
         reinterpret_cast<V *>(out + r * n)[c] = o;
       }
     }
@@ -224,7 +231,7 @@ silu_mul_rows_kernel(const T *in, long long ld, int n, long long rows, T *out, b
          i += (long long)gridDim.x * blockDim.x) {
       const long long r = i / n;
       const int c = (int)(i % n);
-      stf(out + i, silu_mul1(ldf(in + r * ld + c), ldf(in + r * ld + n + c)));
+      stf(out + i, silu_mul1_row<T>(ldf(in + r * ld + c), ldf(in + r * ld + n + c)));
     }
   }
 }

@@ -400,8 +400,8 @@ def test_silu_mul_rows_shapes(dtype, rows, n):
 
 @pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
 def test_silu_mul_rows_at_the_ends_of_the_gate(dtype):
-    """Gates where an exponential overflows, vanishes or is not a number: half a unit of the result's type beside the fp64 value,
-    and what 32 bits flush to zero."""
+    """Gates where an exponential overflows, vanishes or is not a number: half a unit of the result's type beside the fp64 value
+    (and a fiftieth of one for the fast exponential), of float16's smallest ones too, and less than 1e-35 where 32 bits flush to zero."""
     from axono_b200 import ops
 
     gate = torch.tensor([-float("inf"), -3e4, -200, -104, -89, -88.5, -88, -87.5, -87, -30, -1e-3, -0.0, 0.0, 1e-3, 30, 88, 89, 3e4, float("inf"),
@@ -410,10 +410,22 @@ def test_silu_mul_rows_at_the_ends_of_the_gate(dtype):
     got = ops.silu_mul_rows(torch.cat([gate, up])[None].cuda(), 24)[0].cpu().double()
     g, u = gate.double(), up.double()
     want = torch.where(g == -float("inf"), torch.nan, g * torch.sigmoid(g)) * u
-    want = want.to(dtype).double()  # infinite where it is beyond the type
-    assert torch.equal(got.isnan(), want.isnan()) and torch.equal(got.isinf(), want.isinf())
-    fin = want.isfinite()
-    assert ((got - want).abs()[fin] <= torch.finfo(dtype).eps * want.abs()[fin] + 1e-35).all()
+    stored = want.to(dtype)  # infinite where it is beyond the type
+    assert torch.equal(got.isnan(), stored.isnan()) and torch.equal(got.isinf(), stored.isinf())
+    fin = stored.isfinite()
+    assert ((got - want).abs()[fin] <= 0.51 * torch.finfo(dtype).eps * want.abs()[fin] + (2 ** -25 if dtype == torch.float16 else 1e-35)).all()
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16, torch.float32])
+def test_silu_mul_rows_bits_are_the_same_in_pieces_and_one_by_one(dtype):
+    """Rows that start on 16 bytes and the same rows one element further."""
+    from axono_b200 import ops
+
+    n, rows = 1024, 37
+    x = (6 * torch.randn((rows, 2 * n), generator=torch.Generator().manual_seed(9))).to(dtype).cuda()
+    shifted = torch.empty(rows * 2 * n + 1, dtype=dtype, device="cuda")[1:].view(rows, 2 * n)
+    shifted.copy_(x)
+    assert torch.equal(ops.silu_mul_rows(x, n), ops.silu_mul_rows(shifted, n))
 
 
 def test_context_parallel_single_rank_matches_plain():
