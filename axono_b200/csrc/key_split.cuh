@@ -1,8 +1,8 @@
 // Blocks of query rows whose keys are divided among several CTAs, and the kernel that joins their partial results.
 //
-// The blocks of a prompt are few (a block is 128 or 256 rows of a head) and, under a causal mask, of very different length, so that
-// the last of them leave most SMs without work: 2700 rows of 16 heads are 176 blocks, one full wave and 28 more that
-// take as long again.  A plan divides the blocks that would run alone; the parts leave un-normalised sums, their maxima and
+// The blocks of a prompt are few (a block is 128 rows of a head) and, under a causal mask, of very different length, so that
+// the last of them leave most SMs without work: 2700 rows of 16 heads are 352 blocks, which two CTAs per SM take as one full wave and
+// 56 more that take as long again.  A plan divides the blocks that would run alone; the parts leave un-normalised sums, their maxima and
 // denominators in scratch memory.
 #pragma once
 
@@ -12,27 +12,31 @@
 
 namespace axb {
 
-constexpr int kMostUnits = 448, kSms = 148;
+constexpr int kSms = 148;
 constexpr size_t kMostScratch = (size_t)2 << 30;
 
 // What CTAs work on, per head: unit u is part `part` of `parts` of row block `block`.  units == 0: blocks as they are.  Units of
-// divided blocks follow one another: `divided` of them from `first` on; only they have scratch.
+// divided blocks follow one another: `divided` of them from `first` on; only they have scratch.  kMost: units that a plan can have (it
+// travels as a kernel's argument, so a kernel for whole blocks does without).
+template <int kMost>
 struct KeySplit {
+  static constexpr int kMostUnits = kMost;
   int units, first, divided;
-  uint16_t block[kMostUnits];
-  uint8_t part[kMostUnits], parts[kMostUnits];
+  uint16_t block[kMost];
+  uint8_t part[kMost], parts[kMost];
 };
 
 // The first tile of part i of n.
 __host__ __device__ inline int split_begin(int tiles, int part, int parts) { return (int)((int64_t)tiles * part / parts); }
 
 // blocks row blocks of `heads` heads; tiles(b) key tiles in block b, not decreasing in b; part_cost: what a block or part costs beside
-// its tiles, in tiles; least_gain: tiles in a row that a division has to save, as many as joining takes (4 to 6 us with its launch);
-// places: blocks that run at once.
-template <typename Tiles>
-KeySplit plan_key_split(int64_t blocks, int heads, bool causal, float part_cost, float least_gain, Tiles tiles, int places = kSms) {
-  KeySplit plan{};
-  if (blocks > kMostUnits || heads > 2 * kSms) return plan;
+// its tiles, in tiles; least_gain: tiles in a row that a division has to save, as many as joining takes with its launch (the callers say what they measured);
+// join_cost: what joining costs for each further part of a block, in tiles; places: blocks that run at once.
+template <typename Plan, typename Tiles>
+Plan plan_key_split(int64_t blocks, int heads, bool causal, float part_cost, float least_gain, Tiles tiles, int places = kSms,
+                    float join_cost = 0.f) {
+  Plan plan{};
+  if (blocks > Plan::kMostUnits || heads > 2 * kSms) return plan;
   const int most = tiles((int)blocks - 1);
   int unsplit = 0, parts = 1, limit = 0;
   if (causal) {
@@ -47,7 +51,7 @@ KeySplit plan_key_split(int64_t blocks, int heads, bool causal, float part_cost,
         longest = (t + n - 1) / n > longest ? (t + n - 1) / n : longest;
         shortest = t / n < shortest ? t / n : shortest;
       }
-      const float alone = longest + part_cost;
+      const float alone = longest + part_cost + join_cost * ((most - 1) / at_most);
       if (count * heads <= places) return alone;
       const float even = (total + part_cost * count) * heads / places + (shortest + part_cost) / 2;
       return even > alone ? even : alone;
@@ -71,7 +75,7 @@ KeySplit plan_key_split(int64_t blocks, int heads, bool causal, float part_cost,
       int64_t n = rest ? rounds * places / rest : 0;
       n = n > 16 ? 16 : n;
       n = n > most / 2 ? most / 2 : n;
-      const float time = n > 1 ? rounds * ((float)most / n + part_cost) : INFINITY;
+      const float time = n > 1 ? rounds * ((float)most / n + part_cost) + join_cost * (n - 1) : INFINITY;
       if (time < best) best = time, parts = (int)n;
     }
     if (parts == 1) return plan;
@@ -81,7 +85,7 @@ KeySplit plan_key_split(int64_t blocks, int heads, bool causal, float part_cost,
     const int b = (int)blocks - 1 - i;  // under a causal mask the longest first
     // causal: the longest first, so the divided ones first; else the divided ones last
     const int n = causal ? (tiles(b) + limit - 1) / limit : i < unsplit ? 1 : parts;
-    if (units + n > kMostUnits || n > 255) return plan;
+    if (units + n > Plan::kMostUnits || n > 255) return plan;
     if (n > 1) {
       if (divided == 0) plan.first = units;
       divided += n;
@@ -98,7 +102,8 @@ KeySplit plan_key_split(int64_t blocks, int heads, bool causal, float part_cost,
 }
 
 // Scratch of a plan: per divided unit and head `rows` rows of d floats, and (maximum, denominator) of each row.
-inline size_t key_split_bytes(const KeySplit &plan, int heads, int rows, int d) {
+template <typename Plan>
+size_t key_split_bytes(const Plan &plan, int heads, int rows, int d) {
   return (size_t)plan.divided * heads * rows * (d + 2) * sizeof(float);
 }
 
@@ -106,7 +111,8 @@ struct Partials {
   float *sums;  // (divided unit, head, row, d)
   float2 *ml;   // (divided unit, head, row): maximum in powers of two (-inf: no key), denominator
 };
-inline Partials partials_at(void *scratch, const KeySplit &plan, int heads, int rows) {
+template <typename Plan>
+Partials partials_at(void *scratch, const Plan &plan, int heads, int rows) {
   Partials p{nullptr, nullptr};
   if (plan.units == 0) return p;
   p.ml = static_cast<float2 *>(scratch);
@@ -116,8 +122,8 @@ inline Partials partials_at(void *scratch, const KeySplit &plan, int heads, int 
 
 // A warp per row of a divided block: out = sum_i 2^(m_i - m) sums_i / sum_i 2^(m_i - m) l_i.  blockIdx.y: divided unit (those that are
 // no first part leave at once); blockIdx.x: head and 8 rows.  d: a multiple of 4 up to 128.
-template <typename O, int kRowsPerBlock>
-__global__ void __launch_bounds__(256) join_parts_kernel(const __grid_constant__ KeySplit plan, const Partials p, O *out, int sq, int hq, int d) {
+template <typename O, int kRowsPerBlock, typename Plan>
+__global__ void __launch_bounds__(256) join_parts_kernel(const __grid_constant__ Plan plan, const Partials p, O *out, int sq, int hq, int d) {
   const int u = plan.first + blockIdx.y, n = plan.parts[u];
   if (plan.part[u] != 0) return;
   grid_dependency_wait();

@@ -22,6 +22,7 @@
 #include <math.h>
 
 #include <mutex>
+#include <type_traits>
 
 #include "key_split.cuh"
 #include "tcgen05.cuh"
@@ -64,6 +65,11 @@ struct PrefillParams {
 };
 
 constexpr float kLazyLog2 = 8.0f;
+
+// The plan of a prompt whose keys are divided, and what a kernel of whole blocks takes in its place: 5 KB of arguments cost a launch
+// of 16 to 64 rows 0.3 of 4.8 us.
+using PromptSplit = KeySplit<1216>;
+struct WholeBlocks {};
 
 // Two fp16 parts of a pair of weights: hi + lo holds 22 bits of each (2^-24 absolute where a part is subnormal).
 __device__ __forceinline__ uint32_t split_half2(float a, float b, uint32_t &lo) {
@@ -180,11 +186,12 @@ __device__ __noinline__ void redo_narrow_row(const PrefillParams &p, int t_row, 
 // wide as the head.  Elements past the head size are zeros that TMA fills in; head sizes up to 64 leave the second 64-wide block
 // of every tile out.  2700 x 2700 keys, 16 heads of 64, not causal: 1921 us on the FMA pipe, 91 with two blocks per CTA (whose P.V
 // had to be 128 wide), 71 here; the same error against 64 bits (2.1e-4, the rounding of the result).
-template <bool kNarrow>
+template <bool kNarrow, typename Split>
 __global__ void __launch_bounds__(kThreads, 2)
 prefill_attn_f16_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                         const __grid_constant__ CUtensorMap tmV, const __grid_constant__ PrefillParams p,
-                        const __grid_constant__ KeySplit split, const Partials partials) {
+                        const __grid_constant__ Split split, const Partials partials) {
+  constexpr bool kDivided = std::is_same<Split, PromptSplit>::value;
   extern __shared__ __align__(1024) uint8_t smem[];
   uint64_t *bars = reinterpret_cast<uint64_t *>(smem + kOffBar);
   uint64_t *bar_q = bars;                                    // Q landed
@@ -204,17 +211,24 @@ prefill_attn_f16_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
   // heaviest blocks of all heads first: under a causal mask the last query block has the most key tiles
   // (or in the plan's order, where keys are divided)
   const int h = blockIdx.x % p.hq, unit = blockIdx.x / p.hq;
-  const int qb = split.units ? split.block[unit] : (int)((gridDim.x - 1 - blockIdx.x) / p.hq);
-  const int parts = split.units ? split.parts[unit] : 1;
+  int qb, parts = 1;
+  if constexpr (kDivided)
+    qb = split.block[unit], parts = split.parts[unit];
+  else
+    qb = (int)((gridDim.x - 1 - blockIdx.x) / p.hq);
   const int hk = h / (p.hq / p.hkv);
   const int q0 = qb * kBlockM;
   const int warp = uniform_warp(), lane = threadIdx.x & 31;
   const int t_last = min(q0 + kBlockM, p.sq) - 1;
   const int kv_end_max = p.causal ? min(t_last + 1, p.skv) : p.skv;  // reference rule: min(t+1, skv)
   int nkv = (kv_end_max + kBlockN - 1) / kBlockN, tile0 = 0;
-  if (parts > 1) {
-    tile0 = split_begin(nkv, split.part[unit], parts);
-    nkv = split_begin(nkv, split.part[unit] + 1, parts) - tile0;
+  size_t at = 0;  // of the rows of a divided block, their places among the partial results
+  if constexpr (kDivided) {
+    if (parts > 1) {
+      tile0 = split_begin(nkv, split.part[unit], parts);
+      nkv = split_begin(nkv, split.part[unit] + 1, parts) - tile0;
+    }
+    at = ((size_t)(unit - split.first) * p.hq + h) * kBlockM;
   }
   const bool two_blocks = !kNarrow || p.d > 64;
   const uint32_t kv_bytes = two_blocks ? kKvTileBytes : kKvTileBytes / 2;
@@ -422,7 +436,7 @@ prefill_attn_f16_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
     // ---- epilogue: O / l -> out ----
     if (ok && nkv > 0) ok = __all_sync(0xffffffffu, mbar_wait_bounded(bar_fin, 0, abort_flag));
     tc_fence_after();
-    const size_t at = ((size_t)(unit - split.first) * p.hq + h) * kBlockM + row;  // of divided blocks
+    at += row;
     float bad = 0.f;  // NaN once a stored sum is not finite
     const auto load_o = [&](int c, uint32_t (&r)[32]) {
       tmem_ld32(tmem_o + lane_base + c * 32, r);
@@ -501,15 +515,21 @@ bool rows_map(CUtensorMap *map, const void *base, int64_t rows, int heads, int d
             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-// A tile takes about 0.7 us of a block; a block costs six tiles more, joining with its launch 18 (7 to 9 us, and what the parts of
-// full SMs take from each other).  Whole and divided, the joining included: 4096 rows of 2 heads, causal: 46 and 24 us; 2700 of 16
-// heads of 64, not causal: 76 and 68; 2000 of 8 heads, causal: 25 both; 2048 of 16 heads, causal: 28 and 38, left whole.
-KeySplit prompt_plan(int sq, int hq, int64_t skv, int d, int is_causal) {
+// A tile takes about 0.7 us of a block; a block costs six tiles more.  Joining with its launch costs 18 (7 to 9 us, and what the parts of
+// full SMs take from each other), fewer where heads are few and narrow: 14, or 10 for one head and a fifth for each part that a row is
+// joined of.  Whole and divided, the joining included: 4096 rows of 2 heads of 128, causal: 46 and 24 us; 2700 of 16 heads of 64, not
+// causal: 76 and 68; 2000 of 8 heads of 128, causal: 25 both; 2048 of 16, causal: 28 and 38, left whole.  1100 rows, causal, at 18 tiles (whole) and
+// here: 2 heads of 64 16.5 and 11.6, 8 heads 16.9 and 15.4, 2 heads of 128 16.0 and 12.6; not causal, 4 heads of 64 17.4 and 16.1, but 4 of 128 at
+// 14 tiles 18.8 instead of 16.9.  2700 rows of one head of 128, causal: 20.5 in 22 parts, 18.9 in fewer.  One head, not causal, whole (a plan of 448
+// units did not hold the parts) and divided: 40000 rows of 128, 959 and 608; 77000, 3126 and 2564.
+PromptSplit prompt_plan(int sq, int hq, int64_t skv, int d, int is_causal) {
   const auto tiles = [&](int b) {
     const int64_t last = ((int64_t)b + 1) * kBlockM, end = last < sq ? last : sq;
     return (int)(((is_causal && end < skv ? end : skv) + kBlockN - 1) / kBlockN);
   };
-  KeySplit plan = plan_key_split(((int64_t)sq + kBlockM - 1) / kBlockM, hq, is_causal != 0, 6.f, 18.f, tiles, 2 * kSms);
+  const float least_gain = hq == 1 ? 10.f : hq * d <= (is_causal ? 640 : 256) ? 14.f : 18.f;
+  PromptSplit plan = plan_key_split<PromptSplit>(((int64_t)sq + kBlockM - 1) / kBlockM, hq, is_causal != 0, 6.f, least_gain, tiles,
+                                                 2 * kSms, hq == 1 ? 0.2f : 0.f);
   if (key_split_bytes(plan, hq, kBlockM, d) > kMostScratch) plan.units = plan.divided = 0;
   return plan;
 }
@@ -579,10 +599,11 @@ int axb200_sdpa_scratch(const void *q, const void *k, const void *v, void *out, 
   {
     std::lock_guard<std::mutex> lock(mu);
     if (!opted[dev]) {
-      if (cudaFuncSetAttribute(axb::prefill_attn_f16_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               axb::kSmemBytes) != cudaSuccess ||
-          cudaFuncSetAttribute(axb::prefill_attn_f16_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               axb::kSmemBytes) != cudaSuccess)
+      const auto opt = [](auto kernel) {
+        return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, axb::kSmemBytes) == cudaSuccess;
+      };
+      if (!opt(&axb::prefill_attn_f16_kernel<false, axb::WholeBlocks>) || !opt(&axb::prefill_attn_f16_kernel<true, axb::WholeBlocks>) ||
+          !opt(&axb::prefill_attn_f16_kernel<false, axb::PromptSplit>) || !opt(&axb::prefill_attn_f16_kernel<true, axb::PromptSplit>))
         return AXB200_DEVICE_ERROR;
       opted[dev] = true;
     }
@@ -599,17 +620,22 @@ int axb200_sdpa_scratch(const void *q, const void *k, const void *v, void *out, 
   p.q = static_cast<const __half *>(q);
   p.k = static_cast<const __half *>(k);
   p.v = static_cast<const __half *>(v);
-  axb::KeySplit split{};
+  axb::PromptSplit split{};
   if (scratch && axb::aligned16(scratch)) {
     split = axb::prompt_plan(sq, hq, skv, d, is_causal);
     if (scratch_bytes < axb::key_split_bytes(split, hq, axb::kBlockM, d)) split.units = 0;
   }
+  if (split.units == 0) {
+    const dim3 grid((unsigned)hq * ((sq + axb::kBlockM - 1) / axb::kBlockM));
+    auto *kernel = narrow ? axb::prefill_attn_f16_kernel<true, axb::WholeBlocks> : axb::prefill_attn_f16_kernel<false, axb::WholeBlocks>;
+    kernel<<<grid, axb::kThreads, axb::kSmemBytes, st>>>(mq, mk, mv, p, axb::WholeBlocks{}, axb::Partials{nullptr, nullptr});
+    return axb::launch_status();
+  }
   const axb::Partials partials = axb::partials_at(scratch, split, hq, axb::kBlockM);
-  const dim3 grid((unsigned)hq * (split.units ? split.units : (sq + axb::kBlockM - 1) / axb::kBlockM));
-  auto *kernel = narrow ? axb::prefill_attn_f16_kernel<true> : axb::prefill_attn_f16_kernel<false>;
-  kernel<<<grid, axb::kThreads, axb::kSmemBytes, st>>>(mq, mk, mv, p, split, partials);
-  if (split.units && cudaPeekAtLastError() == cudaSuccess)
-    return axb::launch_dependent(axb::join_parts_kernel<__half, axb::kBlockM>, dim3((unsigned)hq * (axb::kBlockM / 8), split.divided),
+  auto *kernel = narrow ? axb::prefill_attn_f16_kernel<true, axb::PromptSplit> : axb::prefill_attn_f16_kernel<false, axb::PromptSplit>;
+  kernel<<<dim3((unsigned)hq * split.units), axb::kThreads, axb::kSmemBytes, st>>>(mq, mk, mv, p, split, partials);
+  if (cudaPeekAtLastError() == cudaSuccess)
+    return axb::launch_dependent(axb::join_parts_kernel<__half, axb::kBlockM, axb::PromptSplit>, dim3((unsigned)hq * (axb::kBlockM / 8), split.divided),
                                  dim3(256), 0, st, split, partials, static_cast<__half *>(out), sq, hq, d);
   return axb::launch_status();
 }

@@ -184,6 +184,22 @@ def test_fp16_keys_divided_among_blocks(d, sq, skv, hq, hkv):
     assert ops.last_error() == 0
 
 
+@pytest.mark.parametrize("sq,d", [(40000, 64), (60000, 128)])
+def test_fp16_long_prompts_of_one_head(sq, d):
+    """Plans of more than 448 blocks and parts: the last blocks, which are divided, and some others, within the bound above."""
+    from axono_b200 import ops
+
+    q, k, v = tensors(sq, sq, 1, 1, d, torch.float16)
+    out = ops.scaled_dot_product_attention(q, k, v, False)
+    weight = 2 * (q.float().norm(dim=-1).max() * k.float().norm(dim=-1).max() * d ** -0.5).item() * 2.0 ** -21 + 2.0 ** -20 + 2.0 ** -11
+    small = 2.0 ** -25 * v.double().abs().sum(0)
+    for at in (0, sq // 2, sq - 2000, sq - 1000):
+        rows = slice(at, at + 1000)
+        ref, mass = attention(q[rows], k, v, False), attention(q[rows], k, v.abs(), False)
+        assert ((out[rows].double() - ref).abs() <= ref.abs() * 2.0 ** -11 + weight * mass + small + 2.0 ** -24).all()
+    assert ops.last_error() == 0
+
+
 @pytest.mark.parametrize("d", [8, 64, 72])
 @pytest.mark.parametrize("sq,skv,hq,hkv", [(200, 260, 4, 2), (300, 4100, 2, 1), (1300, 1300, 2, 2)])  # the later two divide keys
 def test_fp16_narrow_heads_with_infinities(d, sq, skv, hq, hkv):

@@ -15,6 +15,14 @@ def test_only_divided_blocks_take_scratch(tokens, heads, causal, most):
     assert scratch(tokens, heads, heads // 2, 128, tokens, causal, _capi.FLOAT16) <= most
 
 
+@pytest.mark.parametrize("tokens,heads,d,causal,divided", [
+    (1100, 1, 64, 1, True), (1100, 2, 64, 1, True), (1100, 4, 64, 0, True), (1100, 8, 64, 1, True), (1100, 2, 128, 1, True),
+    (1100, 4, 128, 0, False), (1100, 8, 128, 1, False), (1100, 16, 64, 0, False), (2048, 16, 128, 1, False),
+    (40000, 1, 128, 0, True), (57600, 1, 64, 0, True), (77000, 1, 128, 0, True)])  # more than 448 blocks or units
+def test_prompts_are_divided_where_that_was_measured_faster(tokens, heads, d, causal, divided):
+    assert (scratch(tokens, heads, heads, d, tokens, causal, _capi.FLOAT16) > 0) == divided
+
+
 @pytest.mark.parametrize("dtype", [_capi.FLOAT16, _capi.FLOAT32])
 def test_scratch_is_bounded(dtype):
     """2 GB at most; fp32 that would want more (its tiles of K and V) asks for none."""
