@@ -15,9 +15,9 @@
 // scores two tiles ahead -, warp 5 the TMA loads.  What differs: K is 64 x up to 192 elements per tile, so that with a rotated
 // part K and V have a buffer less; rows stand at positions start .. start + n - 1 of a longer key sequence.  Every wait is bounded.
 // Bound by the tensor core as there.  2048 rows over 8192 keys, 16 heads of 128: 133 us, now 115; with a window of 4096: 76 and 70;
-// 2000 rows, 16 heads of 128 + 64 rotated: 43 and 37; 8192 of these: 293 and 290 (before: one CTA per SM with two blocks of rows and
-// tiles of 128 keys, whose scores had to wait for the tile before, and products issued one by one; these issued as here, the
-// last is 275: three blocks of K make 64-wide scores dear, but one form serves all, and the blocks of short prompts are finer).
+// 2000 rows, 16 heads of 128 + 64 rotated: 43 and 36 (before: one CTA per SM with two blocks of rows and tiles of 128 keys, whose
+// scores had to wait for the tile before, and products issued one by one).  That form, issued as here, is still the faster one for
+// much work with a rotated part: the second kernel (8192 rows of these: 272, 288 in the first).
 #include <math.h>
 
 #include <mutex>
@@ -41,6 +41,101 @@ struct Params {
   float scale_log2;
   unsigned long long wait_ns;
 };
+
+// A thread's row of scores of a tile from key n0 on: those outside [begin, end) are masked, the running maximum m_run (of the scaled
+// scores: scale may be negative or zero in principle) moves where some row of the warp found a score more than kLazy above it, and the
+// weights go to tensor memory in bf16.  The sums of weights so far and the row's accumulator then owe the factor corr; true where it may not be one.
+template <int kChunks>
+__device__ __forceinline__ bool softmax_tile(uint32_t (&sr)[kChunks][32], int n0, int begin, int end, float scale_log2, uint32_t weights,
+                                             float &m_run, float &corr, float (&sum4)[4]) {
+  if (n0 < begin) {
+#pragma unroll
+    for (int c = 0; c < kChunks; ++c)
+#pragma unroll
+      for (int i = 0; i < 32; ++i)
+        if (n0 + c * 32 + i < begin) sr[c][i] = 0xff800000u;  // -inf
+  }
+  if (n0 + kChunks * 32 > end) {
+#pragma unroll
+    for (int c = 0; c < kChunks; ++c)
+#pragma unroll
+      for (int i = 0; i < 32; ++i)
+        if (n0 + c * 32 + i >= end) sr[c][i] = 0xff800000u;  // -inf
+  }
+  const float m_tile = row_max(sr) * scale_log2;
+  corr = 1.f;
+  const bool moved = __any_sync(0xffffffffu, m_tile > m_run + kLazy);
+  if (moved) {
+    const float m_new = fmaxf(m_run, m_tile);
+    corr = fast_exp2(m_run - ((m_new == -INFINITY) ? 0.f : m_new));
+    m_run = m_new;
+  }
+  const float m_safe = (m_run == -INFINITY) ? 0.f : m_run;
+  const uint64_t scale2 = pack_f32x2(scale_log2, scale_log2), shift2 = pack_f32x2(-m_safe, -m_safe);
+#pragma unroll
+  for (int i = 0; i < 4; ++i) sum4[i] *= corr;
+  // neighbours first, and 128 keys together: the order of these additions shows in the last bit of the results
+#pragma unroll
+  for (int c = 0; c < kChunks; ++c) {
+    uint32_t packed[16];
+#pragma unroll
+    for (int i = 0; i < 32; i += 4) {
+      float w[4];
+#pragma unroll
+      for (int u = 0; u < 4; u += 2) {
+        const float2 x =
+            unpack_f32x2(fma_f32x2(pack_f32x2(__uint_as_float(sr[c][i + u]), __uint_as_float(sr[c][i + u + 1])), scale2, shift2));
+        w[u] = fast_exp2(x.x), w[u + 1] = fast_exp2(x.y);
+        packed[(i + u) >> 1] = pack_bf16x2(w[u], w[u + 1]);
+      }
+      sum4[(i >> 1) & 3] += w[0] + w[1];
+      sum4[((i >> 1) & 3) + 1] += w[2] + w[3];
+    }
+    tmem_st16(weights + c * 16, packed);
+  }
+  return moved;
+}
+
+// A row of the accumulator times corr.
+template <int kVB>
+__device__ __forceinline__ void rescale_row(uint32_t acc, float corr) {
+#pragma unroll
+  for (int c = 0; c < kVB * 2; ++c) {
+    uint32_t r[32];
+    tmem_ld32(acc + c * 32, r);
+#pragma unroll
+    for (int i = 0; i < 32; ++i) r[i] = __float_as_uint(__uint_as_float(r[i]) * corr);
+    tmem_st32(acc + c * 32, r);
+  }
+}
+
+// A row's result from its accumulator, maximum and denominator.
+template <int kVB>
+__device__ __forceinline__ void store_row(const Params &p, int t_row, int h, uint32_t acc, float m_run, float l_run) {
+  float inv = l_run > 0.f ? 1.0f / l_run : 0.f;
+  if (p.sink) {
+    const float s = p.sink[h] * kLog2e, top = fmaxf(m_run, s), w = fast_exp2(m_run - top);
+    inv = w / fmaf(l_run, w, fast_exp2(s - top));
+  }
+  __nv_bfloat16 *dst = p.out + ((size_t)t_row * p.heads + h) * p.vdim;
+#pragma unroll
+  for (int c = 0; c < kVB * 2; ++c) {
+    uint32_t r[32];
+    tmem_ld32(acc + c * 32, r);
+    if (t_row < p.n) {
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        if (c * 32 + u * 8 >= p.vdim) break;
+        uint4 w;
+        w.x = pack_bf16x2(__uint_as_float(r[u * 8 + 0]) * inv, __uint_as_float(r[u * 8 + 1]) * inv);
+        w.y = pack_bf16x2(__uint_as_float(r[u * 8 + 2]) * inv, __uint_as_float(r[u * 8 + 3]) * inv);
+        w.z = pack_bf16x2(__uint_as_float(r[u * 8 + 4]) * inv, __uint_as_float(r[u * 8 + 5]) * inv);
+        w.w = pack_bf16x2(__uint_as_float(r[u * 8 + 6]) * inv, __uint_as_float(r[u * 8 + 7]) * inv);
+        *reinterpret_cast<uint4 *>(dst + c * 32 + u * 8) = w;
+      }
+    }
+  }
+}
 
 // kQB / kVB: 64-wide blocks of the heads' own key part and of the values; kRot: one more block for the rotated part
 template <int kQB, int kVB, int kRot>
@@ -199,54 +294,9 @@ latent_prefill_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
 #pragma unroll
       for (int c = 0; c < 2; ++c) tmem_ld32_async(ts + c * 32, sr[c]);
       tmem_wait_ld();
-      const int n0 = (tile0 + j) * kKeys;
-      if (n0 < kv_begin) {
-#pragma unroll
-        for (int c = 0; c < 2; ++c)
-#pragma unroll
-          for (int i = 0; i < 32; ++i)
-            if (n0 + c * 32 + i < kv_begin) sr[c][i] = 0xff800000u;  // -inf
-      }
-      if (n0 + kKeys > kv_end) {
-#pragma unroll
-        for (int c = 0; c < 2; ++c)
-#pragma unroll
-          for (int i = 0; i < 32; ++i)
-            if (n0 + c * 32 + i >= kv_end) sr[c][i] = 0xff800000u;  // -inf
-      }
-      const float mx = row_max(sr);
-      // scale may be negative or zero in principle: the running maximum is kept of the scaled scores
-      const float m_tile = mx * p.scale_log2;
-      float corr = 1.f;
-      const bool moved = __any_sync(0xffffffffu, m_tile > m_run + kLazy);
-      if (moved) {
-        const float m_new = fmaxf(m_run, m_tile);
-        corr = fast_exp2(m_run - ((m_new == -INFINITY) ? 0.f : m_new));
-        m_run = m_new;
-      }
-      const float m_safe = (m_run == -INFINITY) ? 0.f : m_run;
-      const uint64_t scale2 = pack_f32x2(p.scale_log2, p.scale_log2), shift2 = pack_f32x2(-m_safe, -m_safe);
-#pragma unroll
-      for (int i = 0; i < 4; ++i) sum4[i] *= corr;
-      // neighbours first, and 128 keys together: the order of these additions shows in the last bit of the results
-#pragma unroll
-      for (int c = 0; c < 2; ++c) {
-        uint32_t packed[16];
-#pragma unroll
-        for (int i = 0; i < 32; i += 4) {
-          float w[4];
-#pragma unroll
-          for (int u = 0; u < 4; u += 2) {
-            const float2 x = unpack_f32x2(
-                fma_f32x2(pack_f32x2(__uint_as_float(sr[c][i + u]), __uint_as_float(sr[c][i + u + 1])), scale2, shift2));
-            w[u] = fast_exp2(x.x), w[u + 1] = fast_exp2(x.y);
-            packed[(i + u) >> 1] = pack_bf16x2(w[u], w[u + 1]);
-          }
-          sum4[(i >> 1) & 3] += w[0] + w[1];
-          sum4[((i >> 1) & 3) + 1] += w[2] + w[3];
-        }
-        tmem_st16(ts + c * 16, packed);
-      }
+      float corr;
+      const bool moved =
+          softmax_tile(sr, (tile0 + j) * kKeys, kv_begin, kv_end, p.scale_log2, ts, m_run, corr, sum4);
       l_run *= corr;
       if (((tile0 + j) & 1) || j == nkv - 1) {
         l_run += (sum4[0] + sum4[1]) + (sum4[2] + sum4[3]);
@@ -259,14 +309,7 @@ latent_prefill_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
         ok = mbar_wait_warp(bar_o, (j - 1) & 1, abort_flag, p.wait_ns);
         if (!ok) break;
         tc_fence_after();
-#pragma unroll
-        for (int c = 0; c < kVB * 2; ++c) {
-          uint32_t r[32];
-          tmem_ld32(to + c * 32, r);
-#pragma unroll
-          for (int i = 0; i < 32; ++i) r[i] = __float_as_uint(__uint_as_float(r[i]) * corr);
-          tmem_st32(to + c * 32, r);
-        }
+        rescale_row<kVB>(to, corr);
       }
       asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
       tc_fence_before();
@@ -275,36 +318,209 @@ latent_prefill_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
     }
     if (ok && nkv > 0) ok = mbar_wait_warp(bar_fin, 0, abort_flag, p.wait_ns);
     tc_fence_after();
-    if (ok && nkv > 0) {
-      float inv = l_run > 0.f ? 1.0f / l_run : 0.f;
-      if (p.sink) {
-        const float s = p.sink[h] * kLog2e, top = fmaxf(m_run, s), w = fast_exp2(m_run - top);
-        inv = w / fmaf(l_run, w, fast_exp2(s - top));
-      }
-      __nv_bfloat16 *dst = p.out + ((size_t)t_row * p.heads + h) * p.vdim;
-#pragma unroll
-      for (int c = 0; c < kVB * 2; ++c) {
-        uint32_t r[32];
-        tmem_ld32(to + c * 32, r);
-        if (t_row < p.n) {
-#pragma unroll
-          for (int u = 0; u < 4; ++u) {
-            if (c * 32 + u * 8 >= p.vdim) break;
-            uint4 w;
-            w.x = pack_bf16x2(__uint_as_float(r[u * 8 + 0]) * inv, __uint_as_float(r[u * 8 + 1]) * inv);
-            w.y = pack_bf16x2(__uint_as_float(r[u * 8 + 2]) * inv, __uint_as_float(r[u * 8 + 3]) * inv);
-            w.z = pack_bf16x2(__uint_as_float(r[u * 8 + 4]) * inv, __uint_as_float(r[u * 8 + 5]) * inv);
-            w.w = pack_bf16x2(__uint_as_float(r[u * 8 + 6]) * inv, __uint_as_float(r[u * 8 + 7]) * inv);
-            *reinterpret_cast<uint4 *>(dst + c * 32 + u * 8) = w;
-          }
-        }
-      }
-    }
+    if (ok && nkv > 0) store_row<kVB>(p, t_row, h, to, m_run, l_run);
   }
   tc_fence_before();
   __syncthreads();
   if (warp == kMmaWarp)
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 256;" ::"r"(tmem) : "memory");
+}
+
+// The form for much work with a rotated part, 65 to 128 own elements and as many value columns: one CTA per SM has two blocks of
+// rows against tiles of 128 keys.  A key's 192 elements make 64-wide scores dear (12 products of 50 cycles, 12 of 66 for twice the keys), and
+// four boxes of 16 KB more are under way per CTA; but scores wait for the tile before, and the blocks are coarser.  S_g at g * 128,
+// P_g over its front, O_g at 256 + g * 128; K is double-buffered, V has one buffer whose halves of 64 keys are freed and
+// refilled separately.  Scores take P's place in the order of issue, which products of one shape keep.
+struct Wide {
+  static constexpr int kKeys = 128, kThreads = 320, kMmaWarp = 8, kLoadWarp = 9;
+  static constexpr int kTile = 3 * kBox, kVHalf = 2 * kKeyBox;  // a query tile or a key tile; 64 keys' values
+  static constexpr int kOffK = 2 * kTile, kOffV = kOffK + 2 * kTile, kOffBar = kOffV + 2 * kVHalf, kSmem = kOffBar + 256;
+};
+
+__global__ void __launch_bounds__(Wide::kThreads, 1)
+latent_prefill_wide_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmQr,
+                           const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmKr,
+                           const __grid_constant__ CUtensorMap tmV, const Params p) {
+  using L = Wide;
+  extern __shared__ __align__(1024) uint8_t smem[];
+  uint64_t *bars = reinterpret_cast<uint64_t *>(smem + L::kOffBar);
+  uint64_t *bar_q = bars, *full_k = bars + 1, *empty_k = bars + 3, *full_v = bars + 5, *empty_v = bars + 7;
+  uint64_t *bar_s = bars + 9, *bar_fin = bars + 11, *bar_p = bars + 13;  // per block of rows
+  uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(bars + 15);
+  volatile int *abort_flag = reinterpret_cast<volatile int *>(bars + 16);
+  if ((smem_u32(smem) & 1023u) != 0) {
+    if (threadIdx.x == 0) atomicOr(&g_error_word, AXB200_ERR_WAIT_TIMEOUT);
+    return;
+  }
+  const int h = blockIdx.x % p.heads, q0 = (int)((gridDim.x - 1 - blockIdx.x) / p.heads) * 2 * kRows;
+  const int warp = uniform_warp(), lane = threadIdx.x & 31;
+  const int hk = h / p.group;
+  const int tile0 = p.window > 0 ? max(0, p.start + q0 + 1 - p.window) / L::kKeys : 0;
+  int nkv_g[2];  // key tiles; none for a block past the last row
+#pragma unroll
+  for (int g = 0; g < 2; ++g) {
+    const int first = q0 + g * kRows;
+    nkv_g[g] = first < p.n ? (min(p.start + min(first + kRows, p.n), p.skv) + L::kKeys - 1) / L::kKeys - tile0 : 0;
+  }
+  const int nkv = max(nkv_g[0], nkv_g[1]);
+
+  if (threadIdx.x == 0) {
+    for (int i = 0; i < 13; ++i) mbar_init(&bars[i], 1);
+    mbar_init(&bar_p[0], 4);
+    mbar_init(&bar_p[1], 4);
+    *abort_flag = 0;
+    mbar_fence_init();
+  }
+  if (warp == L::kMmaWarp) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(smem_u32(tmem_slot)) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  grid_dependency_wait();
+  grid_dependency_launch();
+  const uint32_t tmem = *tmem_slot;
+
+  if (warp == L::kLoadWarp) {
+    if (lane == 0) {
+      tma_prefetch_descriptor(&tmK);
+      tma_prefetch_descriptor(&tmKr);
+      tma_prefetch_descriptor(&tmV);
+      mbar_arrive_expect_tx(bar_q, 2 * L::kTile);
+      for (int g = 0; g < 2; ++g) {  // rows past n are zero-filled
+        uint8_t *dst = smem + g * L::kTile;
+        for (int b = 0; b < 2; ++b) tma_load_3d(dst + b * kBox, &tmQ, bar_q, b * 64, h, q0 + g * kRows);
+        tma_load_3d(dst + 2 * kBox, &tmQr, bar_q, 0, h, q0 + g * kRows);
+      }
+      bool ok = true;
+      int nk = 0, nv[2] = {0, 0};  // tiles, and halves of them, asked for
+      auto load_k = [&] {
+        const int s = nk & 1;
+        if (nk >= 2) ok = ok && mbar_wait_bounded(&empty_k[s], ((nk >> 1) - 1) & 1, abort_flag, p.wait_ns);
+        if (!ok) return;
+        uint8_t *dst = smem + L::kOffK + s * L::kTile;
+        mbar_arrive_expect_tx(&full_k[s], L::kTile);
+        for (int b = 0; b < 2; ++b) tma_load_3d(dst + b * kBox, &tmK, &full_k[s], b * 64, hk, (tile0 + nk) * L::kKeys);
+        tma_load_3d(dst + 2 * kBox, &tmKr, &full_k[s], 0, 0, (tile0 + nk) * L::kKeys);
+        ++nk;
+      };
+      load_k();
+      for (int j = 0; j < nkv && ok; ++j) {
+        if (nk < nkv) load_k();
+        for (int half = 0; half < 2 && ok; ++half) {
+          if (j >= 1) ok = mbar_wait_bounded(&empty_v[half], (j - 1) & 1, abort_flag, p.wait_ns);
+          if (!ok) break;
+          uint8_t *dst = smem + L::kOffV + half * L::kVHalf;
+          mbar_arrive_expect_tx(&full_v[half], L::kVHalf);
+          for (int b = 0; b < 2; ++b) tma_load_3d(dst + b * kKeyBox, &tmV, &full_v[half], b * 64, hk, (tile0 + j) * L::kKeys + half * 64);
+          ++nv[half];
+        }
+      }
+      if (*abort_flag) {  // no copy may still be on its way when the CTA leaves
+        const unsigned long long t0 = global_timer_ns();
+        auto drain = [&](uint64_t *bar, uint32_t parity) {
+          while (!mbar_try_wait(bar, parity) && global_timer_ns() - t0 < 100000000ull) {
+          }
+        };
+        drain(bar_q, 0);
+        for (int t = max(0, nk - 2); t < nk; ++t) drain(&full_k[t & 1], (t >> 1) & 1);
+        for (int half = 0; half < 2; ++half)
+          if (nv[half] > 0) drain(&full_v[half], (nv[half] - 1) & 1);
+      }
+    }
+  } else if (warp == L::kMmaWarp) {
+    constexpr uint32_t idesc_qk = (1u << 4) | (1u << 7) | (1u << 10) | ((L::kKeys >> 3) << 17) | ((kRows >> 4) << 24);
+    constexpr uint32_t idesc_pv = idesc_qk | (1u << 16);  // as wide; B MN-major
+    const uint64_t dq = smem_desc(smem_u32(smem), 16, 1024);
+    const uint64_t dk = smem_desc(smem_u32(smem + L::kOffK), 16, 1024);
+    const uint64_t dv = smem_desc(smem_u32(smem + L::kOffV), kKeyBox, 1024);
+    auto issue_s = [&](int g, int t) {
+      const uint64_t dqg = dq + (uint64_t)(g * (L::kTile >> 4)), dks = dk + (uint64_t)((t & 1) * (L::kTile >> 4));
+      if (elect_one()) {
+#pragma unroll
+        for (int ks = 0; ks < 12; ++ks) {
+          const uint32_t off = ((ks >> 2) * kBox + (ks & 3) * 32) >> 4;
+          umma_f16(tmem + g * 128, dqg + off, dks + off, idesc_qk, ks > 0);
+        }
+        umma_commit(&bar_s[g]);
+      }
+    };
+    bool ok = mbar_wait_warp(bar_q, 0, abort_flag, p.wait_ns) && mbar_wait_warp(&full_k[0], 0, abort_flag, p.wait_ns);
+    if (ok) {
+      tc_fence_after();
+      if (nkv_g[0] > 0) issue_s(0, 0);
+      if (nkv_g[1] > 0) issue_s(1, 0);
+      if (elect_one()) umma_commit(&empty_k[0]);
+    }
+    for (int j = 0; j < nkv && ok; ++j) {
+      const int last_g = nkv_g[1] > j ? 1 : 0;
+      bool have_k = false;
+#pragma unroll
+      for (int g = 0; g < 2; ++g) {
+        if (j >= nkv_g[g]) continue;
+        ok = mbar_wait_warp(&bar_p[g], j & 1, abort_flag, p.wait_ns);
+        if (!ok) break;
+#pragma unroll
+        for (int half = 0; half < 2; ++half) {
+          ok = ok && mbar_wait_warp(&full_v[half], j & 1, abort_flag, p.wait_ns);
+          if (!ok) break;
+          tc_fence_after();
+          const uint64_t dvh = dv + (uint64_t)(half * (L::kVHalf >> 4));
+          if (elect_one()) {
+#pragma unroll
+            for (int ks = 0; ks < 4; ++ks)  // 16 keys: 8 columns of P, 2 KB of V
+              umma_f16_ts(tmem + 256 + g * 128, tmem + g * 128 + half * 32 + ks * 8, dvh + (uint64_t)(ks * (2048 >> 4)), idesc_pv,
+                          j > 0 || half > 0 || ks > 0);
+            if (g == last_g) umma_commit(&empty_v[half]);
+          }
+        }
+        if (!ok) break;
+        if (j == nkv_g[g] - 1 && elect_one()) umma_commit(&bar_fin[g]);
+        if (j + 1 < nkv_g[g]) {
+          if (!have_k) ok = mbar_wait_warp(&full_k[(j + 1) & 1], ((j + 1) >> 1) & 1, abort_flag, p.wait_ns);
+          if (!ok) break;
+          have_k = true;
+          tc_fence_after();
+          issue_s(g, j + 1);
+        }
+      }
+      if (ok && j + 1 < nkv && elect_one()) umma_commit(&empty_k[(j + 1) & 1]);
+    }
+  } else {
+    // ---- softmax warps: block of rows g, thread = row ----
+    const int g = warp >> 2, my_nkv = g ? nkv_g[1] : nkv_g[0];
+    const int t_row = q0 + g * kRows + (threadIdx.x & (kRows - 1));
+    const int kv_end = min(p.start + t_row + 1, p.skv), kv_begin = p.window > 0 ? max(0, p.start + t_row + 1 - p.window) : 0;
+    const uint32_t lane_base = (uint32_t)((warp & 3) * 32) << 16, ts = tmem + g * 128 + lane_base, to = ts + 256;
+    float m_run = -INFINITY, l_run = 0.f;
+    bool ok = true;
+    for (int j = 0; j < my_nkv && ok; ++j) {
+      ok = mbar_wait_warp(&bar_s[g], j & 1, abort_flag, p.wait_ns);
+      if (!ok) break;
+      tc_fence_after();
+      uint32_t sr[4][32];
+#pragma unroll
+      for (int c = 0; c < 4; ++c) tmem_ld32_async(ts + c * 32, sr[c]);
+      tmem_wait_ld();
+      float corr, sum4[4] = {0.f, 0.f, 0.f, 0.f};
+      const bool moved = softmax_tile(sr, (tile0 + j) * L::kKeys, kv_begin, kv_end, p.scale_log2, ts, m_run, corr, sum4);
+      l_run = l_run * corr + ((sum4[0] + sum4[1]) + (sum4[2] + sum4[3]));
+      // S_g(j) stands where P_g(j-1) was read, so P_g(j-1).V_{j-1} is complete and O_g may be rescaled
+      if (j > 0 && moved) rescale_row<2>(to, corr);
+      asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&bar_p[g]);
+    }
+    if (ok && my_nkv > 0) ok = mbar_wait_warp(&bar_fin[g], 0, abort_flag, p.wait_ns);
+    tc_fence_after();
+    if (ok && my_nkv > 0) store_row<2>(p, t_row, h, to, m_run, l_run);
+  }
+  tc_fence_before();
+  __syncthreads();
+  if (warp == L::kMmaWarp)
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;" ::"r"(tmem) : "memory");
 }
 
 // (rows, heads, elems) with row and head strides in elements -> boxes of [box_rows rows][64 elements]
@@ -319,10 +535,8 @@ bool map_of(CUtensorMap *map, const void *base, int elems, int heads, int64_t ro
                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-template <int kQB, int kVB, int kRot>
-int launch(const CUtensorMap (&m)[5], const Params &p, cudaStream_t st) {
-  using L = Layout<kQB, kVB, kRot>;
-  auto *kernel = latent_prefill_kernel<kQB, kVB, kRot>;
+template <auto kKernel>
+int launch_form(int rows, int threads, int smem, const CUtensorMap (&m)[5], const Params &p, cudaStream_t st) {
   static std::mutex mu;
   static bool opted[64] = {false};
   int dev = 0;
@@ -330,13 +544,34 @@ int launch(const CUtensorMap (&m)[5], const Params &p, cudaStream_t st) {
   {
     std::lock_guard<std::mutex> lock(mu);
     if (!opted[dev]) {
-      if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, L::kSmem) != cudaSuccess)
-        return AXB200_DEVICE_ERROR;
+      if (cudaFuncSetAttribute(kKernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) return AXB200_DEVICE_ERROR;
       opted[dev] = true;
     }
   }
-  const dim3 grid((unsigned)p.heads * ((p.n + kRows - 1) / kRows));
-  return launch_dependent(kernel, grid, dim3(kThreads), L::kSmem, st, m[0], m[1], m[2], m[3], m[4], p);
+  const dim3 grid((unsigned)p.heads * ((p.n + rows - 1) / rows));
+  return launch_dependent(kKernel, grid, dim3(threads), smem, st, m[0], m[1], m[2], m[3], m[4], p);
+}
+
+template <int kQB, int kVB, int kRot>
+int launch(const CUtensorMap (&m)[5], const Params &p, cudaStream_t st) {
+  return launch_form<&latent_prefill_kernel<kQB, kVB, kRot>>(kRows, kThreads, Layout<kQB, kVB, kRot>::kSmem, m, p, st);
+}
+
+// Whether the wide form is the faster one.  The tensor core sets the pace from about 64 tiles of 64 keys for each of the 296 CTAs that run at
+// once (wide and narrow tiles, with 16 heads: 4096 rows, 57 tiles, 76 us and 76; 8192, 223, 272 and 288; 32 heads: 3000 rows, 63, 95 and
+// 94; 2048 rows over 8192 keys, 194, 251 and 269); and where a CTA per SM reads keys and values that do not fit into L2, copies under
+// way do (100 rows over 8100 keys: 16 heads, 66 MB, 125 and 117; 32 heads, 133 MB, 125 and 142; 128 heads 138 and 171).
+bool wide_gains(const Params &p, int kv_heads, int dim, int rot_dim) {
+  if (rot_dim == 0 || dim <= 64 || p.vdim <= 64) return false;
+  const int64_t blocks = ((int64_t)p.n + kRows - 1) / kRows;
+  int64_t tiles = 0;
+  for (int64_t b = 0; b < blocks; ++b) {
+    const int64_t first = p.start + b * kRows, last = first + kRows < p.skv ? first + kRows : p.skv;
+    tiles += (last + kKeys - 1) / kKeys - (p.window > 0 && first + 1 > p.window ? (first + 1 - p.window) / kKeys : 0);
+  }
+  const int64_t first_key = p.window > 0 && p.start + 1 > p.window ? p.start + 1 - p.window : 0;
+  const int64_t bytes = (p.skv - first_key) * kv_heads * (dim + p.vdim) * 2;
+  return tiles * p.heads >= 64 * 296 || (blocks * p.heads <= 148 && bytes > (int64_t)100 << 20);
 }
 
 bool al16(const void *p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
@@ -364,18 +599,21 @@ int axb200_latent_prefill(const void *q, int64_t q_ld, const void *k, const void
   if (n == 0) return AXB200_OK;
   const int per = dim + rot_dim;
   const int64_t skv = start + n;
+  axb::Params p{static_cast<__nv_bfloat16 *>(out), n, (int)start, (int)skv, heads, heads / kv_heads, vdim, window, sink,
+                scale * axb::kLog2e, axb::wait_limit_ns()};
+  const bool wide = axb::wide_gains(p, kv_heads, dim, rot_dim);
+  const int key_rows = wide ? axb::Wide::kKeys : axb::kKeys;
   CUtensorMap m[5] = {};
   const __nv_bfloat16 *qb = static_cast<const __nv_bfloat16 *>(q);
   if (!axb::map_of(&m[0], qb, dim, heads, n, per, q_ld, axb::kRows) ||
-      !axb::map_of(&m[2], k, dim, kv_heads, skv, dim, (int64_t)kv_heads * dim, axb::kKeys) ||
+      !axb::map_of(&m[2], k, dim, kv_heads, skv, dim, (int64_t)kv_heads * dim, key_rows) ||
       !axb::map_of(&m[4], v, vdim, kv_heads, skv, vdim, (int64_t)kv_heads * vdim, 64))
     return AXB200_INTERNAL_ERROR;
   if (rot_dim > 0 && (!axb::map_of(&m[1], qb + dim, rot_dim, heads, n, per, q_ld, axb::kRows) ||
-                      !axb::map_of(&m[3], rot, rot_dim, 1, skv, rot_ld, rot_ld, axb::kKeys)))
+                      !axb::map_of(&m[3], rot, rot_dim, 1, skv, rot_ld, rot_ld, key_rows)))
     return AXB200_INTERNAL_ERROR;
-  axb::Params p{static_cast<__nv_bfloat16 *>(out), n, (int)start, (int)skv, heads, heads / kv_heads, vdim, window, sink,
-                scale * axb::kLog2e, axb::wait_limit_ns()};
   cudaStream_t st = static_cast<cudaStream_t>(stream);
+  if (wide) return axb::launch_form<&axb::latent_prefill_wide_kernel>(2 * axb::kRows, axb::Wide::kThreads, axb::Wide::kSmem, m, p, st);
   auto go = [&](auto rot_tag) {
     constexpr int kRot = decltype(rot_tag)::value;
     if (dim > 64) return vdim > 64 ? axb::launch<2, 2, kRot>(m, p, st) : axb::launch<2, 1, kRot>(m, p, st);

@@ -303,3 +303,37 @@ def test_experts(dtype, width, ff, experts, top, n):
             got[hit] = rows[hit]
     close(got, want, tol(dtype))
     assert sorted(slot.cpu().flatten().tolist()) == list(range(n * top))
+
+
+@pytest.mark.parametrize("heads,kv_heads,dim,rot,vdim,n,start,window", [
+    (64, 4, 128, 64, 128, 300, 20000, 0), (64, 4, 72, 8, 80, 257, 20011, 0), (64, 2, 128, 40, 128, 513, 20000, 9000),
+    (32, 2, 128, 64, 128, 2700, 1000, 0), (40, 40, 128, 64, 128, 3100, 0, 0),                             # much work
+    (128, 128, 128, 64, 128, 100, 1900, 0), (128, 128, 96, 64, 128, 7, 2100, 0), (128, 128, 128, 64, 128, 100, 3900, 2000)])  # few blocks, many keys
+def test_latent_prefill_in_the_form_of_two_blocks(heads, kv_heads, dim, rot, vdim, n, start, window):
+    """The sizes that take the kernel with two blocks of rows per CTA: edges of its blocks and tiles, sizes that fill their 64-wide blocks
+    in part, windows, sinks.  Weights and results are rounded to bf16: half of its spacing, 2^-7 between 1 and 2, is at most 2^-8 of a value each
+    time; a score is off by its sum of products in fp32."""
+    from axono_b200 import ops
+
+    g = torch.Generator(device="cuda").manual_seed(n)
+    rnd = lambda *shape: torch.randn(shape, generator=g, device="cuda").bfloat16()  # noqa: E731
+    q, k, v, r = rnd(n, heads * (dim + rot)), rnd(start + n, kv_heads * dim), rnd(start + n, kv_heads * vdim), rnd(start + n, rot)
+    scale = (dim + rot) ** -0.5
+    at = torch.arange(start, start + n, device="cuda")[:, None]
+    keys = torch.arange(start + n, device="cuda")[None, :]
+    hidden = (keys > at) | ((keys <= at - window) if window else False)
+    for sink in (None, torch.linspace(-4, 10, heads, device="cuda")):
+        out = ops.latent_prefill(q, start, k, v, r, heads, dim, rot, vdim, scale, window=window, sink=sink, kv_heads=kv_heads)
+        assert ops.last_error() == 0
+        for h in (0, heads // 2 + 1, heads - 1):
+            hk = h // (heads // kv_heads)
+            mine = q.view(n, heads, dim + rot)[:, h].double()
+            s = scale * (mine[:, :dim] @ k.view(-1, kv_heads, dim)[:, hk].double().T + mine[:, dim:] @ r.double().T)
+            s.masked_fill_(hidden, -float("inf"))
+            top = s.amax(-1, keepdim=True) if sink is None else torch.maximum(s.amax(-1, keepdim=True), sink[h].double())
+            w = torch.exp(s - top)
+            total = w.sum(-1, keepdim=True) + (0 if sink is None else torch.exp(sink[h].double() - top))
+            values = v.view(-1, kv_heads, vdim)[:, hk].double()
+            want, mass = w @ values / total, w @ values.abs() / total
+            err = (out.view(n, heads, vdim)[:, h].double() - want).abs()
+            assert (err <= want.abs() * 2.0 ** -8 + mass * (2.0 ** -8 + 2.0 ** -14) + 1e-30).all(), (h, err.max())
