@@ -66,9 +66,7 @@ struct PrefillParams {
 
 constexpr float kLazyLog2 = 8.0f;
 
-// The plan of a prompt whose keys are divided, and what a kernel of whole blocks takes in its place: 5 KB of arguments cost a launch
-// of 16 to 64 rows 0.3 of 4.8 us.
-using PromptSplit = KeySplit<1216>;
+// What a kernel of whole blocks takes in the place of a plan: 2 KB of arguments cost a launch of 16 to 64 rows 0.3 of 4.8 us.
 struct WholeBlocks {};
 
 // Two fp16 parts of a pair of weights: hi + lo holds 22 bits of each (2^-24 absolute where a part is subnormal).
@@ -80,11 +78,11 @@ __device__ __forceinline__ uint32_t split_half2(float a, float b, uint32_t &lo) 
 }
 
 // The tensor core adds up by truncation: a running sum over all keys loses about a quarter of a unit of its last bit, towards zero,
-// with each of a tile's 16 products (1.8e-5 of the values by 8192 keys, 6e-5 where these have a common offset).  So every
-// kFlushTiles tiles O starts anew, and what it held joins a thread's sums in local memory, kept in fp32 with the rescaling they
-// still owe.  (Out of line, so that the sums stay out of the registers of the loop that calls it.)  8192 keys, heads of 64: error
-// 2.084e-4 without, 2.075e-4 so, as on the FMA pipe; with a common offset 2.316e-4, 2.239e-4 and 2.238e-4.  It costs 4 % of the
-// time, twice as often 8 %.
+// with each of the 8 products of a tile of 64 keys, two parts of the weights times 64 / 16 (1.8e-5 of the values by 8192 keys, 6e-5
+// where these have a common offset).  So every kFlushTiles tiles, 1024 keys, O starts anew, and what it held joins a thread's sums
+// in local memory, kept in fp32 with the rescaling they still owe.  (Out of line, so that the sums stay out of the registers of the
+// loop that calls it.)  8192 keys, heads of 64: error 2.084e-4 without, 2.075e-4 so, as on the FMA pipe; with a common offset
+// 2.316e-4, 2.239e-4 and 2.238e-4.  It costs 4 % of the time, twice as often 8 %.
 constexpr int kFlushTiles = 16;
 __device__ __noinline__ void flush_sums(float4 *sums, uint32_t tmem_o, int d, bool first, float owed) {
 #pragma unroll 1
@@ -179,8 +177,9 @@ __device__ __noinline__ void redo_narrow_row(const PrefillParams &p, int t_row, 
 // Bound by the tensor core: a tile's 8 products of Q.K^T take 50 cycles each (Q is read from shared memory for 64 columns at a time) and
 // its 4 of P.V 66, 1330 cycles for the tiles of the two CTAs of an SM; a tile takes 1410.  One CTA per SM with two blocks of 128
 // rows and tiles of 128 keys needed a fifth less of the tensor core, but had no room for scores ahead of the softmax: a tile's
-// chain of 3600 cycles was its time.  16 / 8 heads of 128: 8192 tokens, causal, 283 us in that form, 266 here (2048: 42 and 30); 4096,
-// not causal: 131 and 119 (1150 TFLOP/s).
+// chain of 3600 cycles was its time.  16 / 8 heads of 128, many calls in a row (under the power cap; ten calls after a pause take 235
+// us at 8192): 8192 tokens, causal, 283 us in that form, 266 here - that form issued behind elect_one, as here, took 263 to 267, so 8192
+// tokens owe their gain to the issue; 2048: 42 and 30; 4096, not causal: 131 and 119 (1150 TFLOP/s).
 // kNarrow: head sizes below 128 (multiples of 8).  They ran on the FMA pipe at first, whose weights were fp32, so P enters
 // P.V as two fp16 parts here: P's two parts take the two halves of an S buffer, and a tile costs 8 products for P.V instead of 4, as
 // wide as the head.  Elements past the head size are zeros that TMA fills in; head sizes up to 64 leave the second 64-wide block
@@ -191,7 +190,7 @@ __global__ void __launch_bounds__(kThreads, 2)
 prefill_attn_f16_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                         const __grid_constant__ CUtensorMap tmV, const __grid_constant__ PrefillParams p,
                         const __grid_constant__ Split split, const Partials partials) {
-  constexpr bool kDivided = std::is_same<Split, PromptSplit>::value;
+  constexpr bool kDivided = std::is_same<Split, KeySplit>::value;
   extern __shared__ __align__(1024) uint8_t smem[];
   uint64_t *bars = reinterpret_cast<uint64_t *>(smem + kOffBar);
   uint64_t *bar_q = bars;                                    // Q landed
@@ -211,11 +210,13 @@ prefill_attn_f16_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
   // heaviest blocks of all heads first: under a causal mask the last query block has the most key tiles
   // (or in the plan's order, where keys are divided)
   const int h = blockIdx.x % p.hq, unit = blockIdx.x / p.hq;
-  int qb, parts = 1;
-  if constexpr (kDivided)
-    qb = split.block[unit], parts = split.parts[unit];
-  else
+  int qb, part = 0, parts = 1;
+  if constexpr (kDivided) {
+    const KeyUnit u = key_unit(split, unit);
+    qb = u.block, part = u.part, parts = u.parts;
+  } else {
     qb = (int)((gridDim.x - 1 - blockIdx.x) / p.hq);
+  }
   const int hk = h / (p.hq / p.hkv);
   const int q0 = qb * kBlockM;
   const int warp = uniform_warp(), lane = threadIdx.x & 31;
@@ -225,8 +226,8 @@ prefill_attn_f16_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
   size_t at = 0;  // of the rows of a divided block, their places among the partial results
   if constexpr (kDivided) {
     if (parts > 1) {
-      tile0 = split_begin(nkv, split.part[unit], parts);
-      nkv = split_begin(nkv, split.part[unit] + 1, parts) - tile0;
+      tile0 = split_begin(nkv, part, parts);
+      nkv = split_begin(nkv, part + 1, parts) - tile0;
     }
     at = ((size_t)(unit - split.first) * p.hq + h) * kBlockM;
   }
@@ -515,21 +516,22 @@ bool rows_map(CUtensorMap *map, const void *base, int64_t rows, int heads, int d
             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-// A tile takes about 0.7 us of a block; a block costs six tiles more.  Joining with its launch costs 18 (7 to 9 us, and what the parts of
-// full SMs take from each other), fewer where heads are few and narrow: 14, or 10 for one head and a fifth for each part that a row is
-// joined of.  Whole and divided, the joining included: 4096 rows of 2 heads of 128, causal: 46 and 24 us; 2700 of 16 heads of 64, not
-// causal: 76 and 68; 2000 of 8 heads of 128, causal: 25 both; 2048 of 16, causal: 28 and 38, left whole.  1100 rows, causal, at 18 tiles (whole) and
-// here: 2 heads of 64 16.5 and 11.6, 8 heads 16.9 and 15.4, 2 heads of 128 16.0 and 12.6; not causal, 4 heads of 64 17.4 and 16.1, but 4 of 128 at
-// 14 tiles 18.8 instead of 16.9.  2700 rows of one head of 128, causal: 20.5 in 22 parts, 18.9 in fewer.  One head, not causal, whole (a plan of 448
-// units did not hold the parts) and divided: 40000 rows of 128, 959 and 608; 77000, 3126 and 2564.
-PromptSplit prompt_plan(int sq, int hq, int64_t skv, int d, int is_causal) {
+// A tile takes about 0.7 us of a block; a block costs six tiles more.  Joining with its launch counts as 18 (it took 7 to 9 us, with
+// what the parts of full SMs take from each other, and somewhat less since), as 14 where heads are few and narrow, and as 10 for one
+// head and a fifth for each further part of a row.  Whole and divided, the joining included: 4096 rows of 2 heads of 128, causal: 46
+// and 23 us; 2700 of 16 heads of 64, not causal: 76 and 66; 2000 of 8 heads of 128, causal: 25 both; 2048 of 16, causal: 28 and 38,
+// left whole.  1100 rows, causal, at 18 tiles (whole) and here: 2 heads of 64 17.1 and 10.3, 8 heads 17.4 and 14.7, 2 heads of 128
+// 16.4 and 11.3; not causal, 4 heads of 64 17.4 and 13.0.  2700 rows of one head of 128, causal: 20.8 in 22 parts, 15.7 in fewer.  One
+// head of 128, not causal, whole (a plan of 448 entries did not hold the parts) and divided: 40000 rows 959 and 608; 77000, 3126 and
+// 2570.
+KeySplit prompt_plan(int sq, int hq, int64_t skv, int d, int is_causal) {
   const auto tiles = [&](int b) {
     const int64_t last = ((int64_t)b + 1) * kBlockM, end = last < sq ? last : sq;
     return (int)(((is_causal && end < skv ? end : skv) + kBlockN - 1) / kBlockN);
   };
   const float least_gain = hq == 1 ? 10.f : hq * d <= (is_causal ? 640 : 256) ? 14.f : 18.f;
-  PromptSplit plan = plan_key_split<PromptSplit>(((int64_t)sq + kBlockM - 1) / kBlockM, hq, is_causal != 0, 6.f, least_gain, tiles,
-                                                 2 * kSms, hq == 1 ? 0.2f : 0.f);
+  KeySplit plan = plan_key_split(((int64_t)sq + kBlockM - 1) / kBlockM, hq, is_causal != 0, 6.f, least_gain, tiles, 2 * kSms, 1216,
+                                 hq == 1 ? 0.2f : 0.f);
   if (key_split_bytes(plan, hq, kBlockM, d) > kMostScratch) plan.units = plan.divided = 0;
   return plan;
 }
@@ -603,7 +605,7 @@ int axb200_sdpa_scratch(const void *q, const void *k, const void *v, void *out, 
         return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, axb::kSmemBytes) == cudaSuccess;
       };
       if (!opt(&axb::prefill_attn_f16_kernel<false, axb::WholeBlocks>) || !opt(&axb::prefill_attn_f16_kernel<true, axb::WholeBlocks>) ||
-          !opt(&axb::prefill_attn_f16_kernel<false, axb::PromptSplit>) || !opt(&axb::prefill_attn_f16_kernel<true, axb::PromptSplit>))
+          !opt(&axb::prefill_attn_f16_kernel<false, axb::KeySplit>) || !opt(&axb::prefill_attn_f16_kernel<true, axb::KeySplit>))
         return AXB200_DEVICE_ERROR;
       opted[dev] = true;
     }
@@ -620,7 +622,7 @@ int axb200_sdpa_scratch(const void *q, const void *k, const void *v, void *out, 
   p.q = static_cast<const __half *>(q);
   p.k = static_cast<const __half *>(k);
   p.v = static_cast<const __half *>(v);
-  axb::PromptSplit split{};
+  axb::KeySplit split{};
   if (scratch && axb::aligned16(scratch)) {
     split = axb::prompt_plan(sq, hq, skv, d, is_causal);
     if (scratch_bytes < axb::key_split_bytes(split, hq, axb::kBlockM, d)) split.units = 0;
@@ -632,10 +634,10 @@ int axb200_sdpa_scratch(const void *q, const void *k, const void *v, void *out, 
     return axb::launch_status();
   }
   const axb::Partials partials = axb::partials_at(scratch, split, hq, axb::kBlockM);
-  auto *kernel = narrow ? axb::prefill_attn_f16_kernel<true, axb::PromptSplit> : axb::prefill_attn_f16_kernel<false, axb::PromptSplit>;
+  auto *kernel = narrow ? axb::prefill_attn_f16_kernel<true, axb::KeySplit> : axb::prefill_attn_f16_kernel<false, axb::KeySplit>;
   kernel<<<dim3((unsigned)hq * split.units), axb::kThreads, axb::kSmemBytes, st>>>(mq, mk, mv, p, split, partials);
   if (cudaPeekAtLastError() == cudaSuccess)
-    return axb::launch_dependent(axb::join_parts_kernel<__half, axb::kBlockM, axb::PromptSplit>, dim3((unsigned)hq * (axb::kBlockM / 8), split.divided),
+    return axb::launch_dependent(axb::join_parts_kernel<__half, axb::kBlockM>, dim3((unsigned)hq * (axb::kBlockM / 8), split.divided_blocks),
                                  dim3(256), 0, st, split, partials, static_cast<__half *>(out), sq, hq, d);
   return axb::launch_status();
 }

@@ -61,8 +61,6 @@ struct Params {
   unsigned long long wait_ns;
 };
 
-using Split = KeySplit<448>;
-
 // Three bf16 parts of each of two floats; their sum is exact.
 __device__ __forceinline__ void split3(float a, float b, uint32_t &h, uint32_t &m, uint32_t &l) {
   h = pack_bf16x2(a, b);
@@ -112,7 +110,7 @@ split_kernel(const Params p) {
 
 template <int kB>
 __global__ void __launch_bounds__(kThreads, 1)
-split_attn_kernel(const Params p, const __grid_constant__ Split split, const Partials partials) {
+split_attn_kernel(const Params p, const __grid_constant__ KeySplit split, const Partials partials) {
   using L = Layout<kB>;
   extern __shared__ __align__(1024) uint8_t smem[];
   uint64_t *bars = reinterpret_cast<uint64_t *>(smem + L::kOffBar);
@@ -393,12 +391,13 @@ size_t kv_flag_bytes(int hkv, int64_t n_tiles) { return up256((size_t)2 * hkv * 
 // A tile of 64 keys takes 2 to 3 us of a block, a block three tiles more (Q's parts, the first copies, the result).  1536 rows of 16
 // heads of 128, not causal: 176 us whole, 140 in parts; 4096 rows of 2 heads, causal: 208 and 91.  Where the SMs are nearly full
 // a division gains nothing (1536 rows of 16 heads, causal: the attention kernel alone 92 us both, before the joining), hence the five tiles.
-Split split_plan(int sq, int hq, int64_t skv, int is_causal) {
+KeySplit split_plan(int sq, int hq, int64_t skv, int is_causal) {
   const auto tiles = [&](int b) {
     const int64_t last = ((int64_t)b + 1) * kRows, end = last < sq ? last : sq;
     return (int)(((is_causal && end < skv ? end : skv) + kKeys - 1) / kKeys);
   };
-  return plan_key_split<Split>(((int64_t)sq + kRows - 1) / kRows, hq, is_causal != 0, 3.f, 5.f, tiles);
+  return plan_key_split(((int64_t)sq + kRows - 1) / kRows, hq, is_causal != 0, 3.f, 5.f, tiles, kSms,
+                        KeySplit::kMostEntries);
 }
 
 // Keys that some row sees: the others are not split into parts (16 rows over 8192 keys, 16 / 8 heads of 128, causal: 41 us with all).
@@ -420,13 +419,13 @@ int launch(const Params &p, void *parts_at, cudaStream_t st) {
   }
   split_kernel<kB><<<dim3(p.n_tiles, p.hkv, 2), kSplitThreads, 0, st>>>(p);
   if (cudaGetLastError() != cudaSuccess) return AXB200_DEVICE_ERROR;
-  const Split split = split_plan(p.sq, p.hq, p.skv, p.causal);
+  const KeySplit split = split_plan(p.sq, p.hq, p.skv, p.causal);
   const Partials partials = partials_at(parts_at, split, p.hq, kRows);
   const int rc = launch_dependent(split_attn_kernel<kB>, dim3((unsigned)p.hq * (split.units ? split.units : p.q_blocks)), dim3(kThreads),
                                   Layout<kB>::kSmem, st, p, split, partials);
   if (rc != AXB200_OK || split.units == 0) return rc;
-  return launch_dependent(join_parts_kernel<float, kRows, Split>, dim3((unsigned)p.hq * (kRows / 8), split.divided), dim3(256), 0, st, split,
-                          partials, p.out, p.sq, p.hq, p.d);
+  return launch_dependent(join_parts_kernel<float, kRows>, dim3((unsigned)p.hq * (kRows / 8), split.divided_blocks), dim3(256), 0, st,
+                          split, partials, p.out, p.sq, p.hq, p.d);
 }
 
 }  // namespace
