@@ -247,7 +247,7 @@ __global__ void __launch_bounds__(kThreads, 1) row_chain_kernel(const __grid_con
   const float2 *const recv = reinterpret_cast<const float2 *>(smem + kOffRecv);
   const uint32_t peer_recv = in_cta(recv, half ^ 1), peer_got = in_cta(got_all, half ^ 1);
   RingPos sent, got;
-  int units_done = 0, armed = 0;
+  int units_done = 0, armed = 0;  // units whose phase thread 0 armed; ~ of it in a warp whose wait for the other CTA ran out
 
   asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
   grid_dependency_wait();
@@ -332,7 +332,7 @@ __global__ void __launch_bounds__(kThreads, 1) row_chain_kernel(const __grid_con
     // sums of the unit, complete after the exchange
     auto finish = [&](int u) {
       if (owner) {
-        if (!__any_sync(0xffffffffu, *abort_flag)) mbar_wait_warp(&got_all[got.slot], got.parity, abort_flag, p.wait_ns);
+        if (armed >= 0 && !mbar_wait_warp(&got_all[got.slot], got.parity, abort_flag, p.wait_ns)) armed = ~armed;
         const float2 other = recv[got.slot * (kRecv / 8) + v_i];
         mine[0] += other.x, mine[1] += other.y;
       }
@@ -389,7 +389,7 @@ __global__ void __launch_bounds__(kThreads, 1) row_chain_kernel(const __grid_con
         for (int i = 0; i < 4; ++i) red[((warp * 2 + m) * 4 + i) * 32 + lane] = acc[m][i];
       __syncthreads();
       if (last >= 0) finish(last);
-      if (threadIdx.x == 0 && !*abort_flag) {  // this warp has waited for every phase armed so far, so none is armed twice
+      if (threadIdx.x == 0 && armed >= 0) {  // this warp has waited for every phase armed so far, so none is armed twice
         mbar_arrive_expect_tx(&got_all[sent.slot], kRecv);
         ++armed;
       }
@@ -419,7 +419,7 @@ __global__ void __launch_bounds__(kThreads, 1) row_chain_kernel(const __grid_con
     }
   }
   // the other CTA may still be in its own waits, each as long as the limit at most: three meetings and one exchange
-  if (threadIdx.x == 0 && *abort_flag) drain(got_all, units_done, armed, kWaitNanos + 4 * min(p.wait_ns, 1ull << 60));
+  if (threadIdx.x == 0 && *abort_flag) drain(got_all, units_done, armed < 0 ? ~armed : armed, kWaitNanos + 4 * min(p.wait_ns, 1ull << 60));
 }
 
 bool al16(const void *p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
@@ -519,8 +519,8 @@ size_t axb200_row_chain_workspace_bytes(int64_t rows, int width, int ff) {
 int axb200_row_chain(const void *x, const void *w_o, const void *residual, const void *norm1, const void *w_gate_up, const void *w_down,
                      const void *norm2, const void *w_next, void *residual_out, void *out, int64_t rows, int attn, int width, int ff,
                      int next, float eps, int dtype, void *workspace, size_t workspace_bytes, void *stream) {
-  return axb200_row_chain_constant(x, w_o, residual, norm1, w_gate_up, w_down, norm2, w_next, residual_out, out, rows, attn, width, ff, next,
-                                   eps, dtype, 0, workspace, workspace_bytes, stream);
+  return axb200_row_chain_constant(x, w_o, residual, norm1, w_gate_up, w_down, norm2, w_next, residual_out, out, rows, attn, width, ff,
+                                   next, eps, dtype, 0, workspace, workspace_bytes, stream);
 }
 
 int axb200_row_chain_constant(const void *x, const void *w_o, const void *residual, const void *norm1, const void *w_gate_up,
