@@ -165,10 +165,10 @@ rms_norm_warp_kernel(const T *x, const T *w, float eps, T *out, int64_t rows, in
 
 // ---- silu_mul -----------------------------------------------------------------------------------
 __device__ __forceinline__ float silu_mul1(float g, float u) { return g / (1.0f + expf(-g)) * u; }
-// The same for results of 16 bits, with the fast exponential and division.  Of e^-|g|, so that the divisor stays in [1, 2] and neither
-// leaves its range; the exponential's error grows with |g| (2 + 1.16 |g| units in the last of 24 bits: 6e-6 at g = -87, a
-// three-hundredth of half a unit of bfloat16, an eightieth of float16's), and below -87.3 it is zero where the value is
-// less than 1e-36.  With the exact ones the instructions, not the bytes, set the pace: 2048 rows of 2 x 6144 just written, 15.5 us; so 10.6;
+// The same for results of 16 bits, with the fast exponential and division.  Of e^-|g|, so that the divisor stays in [1, 2] and
+// neither leaves its range; the exponential's error grows with |g| (2 + 1.16 |g| units in the last of 24 bits: 6e-6 at g = -87, a
+// three-hundredth of half a unit of bfloat16, an eightieth of float16's), and below -87.3 it is zero where the value is less than
+// 1e-36.  With the exact ones the instructions, not the bytes, set the pace: 2048 rows of 2 x 6144 just written, 15.5 us; so 10.6;
 // the same error against 64 bits.
 __device__ __forceinline__ float silu_mul1_fast(float g, float u) {
   const float t = __expf(-fabsf(g));

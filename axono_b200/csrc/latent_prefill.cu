@@ -42,9 +42,10 @@ struct Params {
   unsigned long long wait_ns;
 };
 
-// A thread's row of scores of a tile from key n0 on: those outside [begin, end) are masked, the running maximum m_run (of the scaled
-// scores: scale may be negative or zero in principle) moves where some row of the warp found a score more than kLazy above it, and the
-// weights go to tensor memory in bf16.  The sums of weights so far and the row's accumulator then owe the factor corr; true where it may not be one.
+// A thread's row of scores of a tile from key n0 on: those outside [begin, end) are masked, the running maximum m_run (of the
+// scaled scores: scale may be negative or zero in principle) moves where some row of the warp found a score more than kLazy above
+// it, and the weights go to tensor memory in bf16.  The sums of weights so far and the row's accumulator then owe the factor corr;
+// true where it may not be one.
 template <int kChunks>
 __device__ __forceinline__ bool softmax_tile(uint32_t (&sr)[kChunks][32], int n0, int begin, int end, float scale_log2, uint32_t weights,
                                              float &m_run, float &corr, float (&sum4)[4]) {
@@ -327,10 +328,10 @@ latent_prefill_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
 }
 
 // The form for much work with a rotated part, 65 to 128 own elements and as many value columns: one CTA per SM has two blocks of
-// rows against tiles of 128 keys.  A key's 192 elements make 64-wide scores dear (12 products of 50 cycles, 12 of 66 for twice the keys), and
-// four boxes of 16 KB more are under way per CTA; but scores wait for the tile before, and the blocks are coarser.  S_g at g * 128,
-// P_g over its front, O_g at 256 + g * 128; K is double-buffered, V has one buffer whose halves of 64 keys are freed and
-// refilled separately.  Scores take P's place in the order of issue, which products of one shape keep.
+// rows against tiles of 128 keys.  A key's 192 elements make 64-wide scores dear (12 products of 50 cycles, 12 of 66 for twice the
+// keys), and four boxes of 16 KB more are under way per CTA; but scores wait for the tile before, and the blocks are coarser.  S_g
+// at g * 128, P_g over its front, O_g at 256 + g * 128; K is double-buffered, V has one buffer whose halves of 64 keys are freed
+// and refilled separately.  Scores take P's place in the order of issue, which products of one shape keep.
 struct Wide {
   static constexpr int kKeys = 128, kThreads = 320, kMmaWarp = 8, kLoadWarp = 9;
   static constexpr int kTile = 3 * kBox, kVHalf = 2 * kKeyBox;  // a query tile or a key tile; 64 keys' values
@@ -557,10 +558,11 @@ int launch(const CUtensorMap (&m)[5], const Params &p, cudaStream_t st) {
   return launch_form<&latent_prefill_kernel<kQB, kVB, kRot>>(kRows, kThreads, Layout<kQB, kVB, kRot>::kSmem, m, p, st);
 }
 
-// Whether the wide form is the faster one.  The tensor core sets the pace from about 64 tiles of 64 keys for each of the 296 CTAs that run at
-// once (wide and narrow tiles, with 16 heads: 4096 rows, 57 tiles, 76 us and 76; 8192, 223, 272 and 288; 32 heads: 3000 rows, 63, 95 and
-// 94; 2048 rows over 8192 keys, 194, 251 and 269); and where a CTA per SM reads keys and values that do not fit into L2, copies under
-// way do (100 rows over 8100 keys: 16 heads, 66 MB, 125 and 117; 32 heads, 133 MB, 125 and 142; 128 heads 138 and 171).
+// Whether the wide form is the faster one.  The tensor core sets the pace from about 64 tiles of 64 keys for each of the 296 CTAs
+// that run at once (wide and narrow tiles, with 16 heads: 4096 rows, 57 tiles, 76 us and 76; 8192, 223, 272 and 288; 32 heads: 3000
+// rows, 63, 95 and 94; 2048 rows over 8192 keys, 194, 251 and 269); and where a CTA per SM reads keys and values that do not fit
+// into L2, copies under way do (100 rows over 8100 keys: 16 heads, 66 MB, 125 and 117; 32 heads, 133 MB, 125 and 142; 128 heads 138
+// and 171).
 bool wide_gains(const Params &p, int kv_heads, int dim, int rot_dim) {
   if (rot_dim == 0 || dim <= 64 || p.vdim <= 64) return false;
   const int64_t blocks = ((int64_t)p.n + kRows - 1) / kRows;

@@ -183,8 +183,8 @@ __device__ __noinline__ void redo_narrow_row(const PrefillParams &p, int t_row, 
 // kNarrow: head sizes below 128 (multiples of 8).  They ran on the FMA pipe at first, whose weights were fp32, so P enters
 // P.V as two fp16 parts here: P's two parts take the two halves of an S buffer, and a tile costs 8 products for P.V instead of 4, as
 // wide as the head.  Elements past the head size are zeros that TMA fills in; head sizes up to 64 leave the second 64-wide block
-// of every tile out.  2700 x 2700 keys, 16 heads of 64, not causal: 1921 us on the FMA pipe, 91 with two blocks per CTA (whose P.V
-// had to be 128 wide), 71 here; the same error against 64 bits (2.1e-4, the rounding of the result).
+// of every tile out.  2700 x 2700 keys, 16 heads of 64, not causal: 1921 us on the FMA pipe, 88 with two blocks per CTA (whose P.V
+// had to be 128 wide), 66 here, the joining included; the same error against 64 bits (2.1e-4, the rounding of the result).
 template <bool kNarrow, typename Split>
 __global__ void __launch_bounds__(kThreads, 2)
 prefill_attn_f16_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,

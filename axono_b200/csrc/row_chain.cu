@@ -8,8 +8,8 @@
 // What bounds it: reading the weights.  As launches of their own (product, norm, product, activation, product, norm, product)
 // the seven start and drain one after the other, each product being 1 to 8 us of reading.  Here one CTA per SM stays
 // through all stages and asks for the next stages' first weights (192 KB per SM) before it waits for the other CTAs.  8 rows,
-// width 2048, ff 6144, 4096 columns next (100 MB of weights, 15.6 us at 6.46 TB/s), in a graph: 41.3 us before, 29.6 now.  What is
-// left: three meetings of all CTAs and the reading of the inputs after each (about 3 us together each time), and 1.1 us per unit
+// width 2048, ff 6144, 4096 columns next (100 MB of weights, 15.6 us at 6.46 TB/s), in a graph: 41.3 us before, 29.6 to 32.1 now (five
+// boxes).  What is left: three meetings of all CTAs and the reading of the inputs after each (about 3 us together each time), and 1.1 us per unit
 // of a CTA, of which its copies into shared memory take 0.45 and its reads and products 0.4; the reading of a unit from HBM takes 1.5.
 //
 // Split: a unit is 32 rows of a weight matrix (16 gate and 16 up rows in stage 1, so that the activation joins values of one
@@ -25,8 +25,9 @@
 //
 // Between stages all CTAs meet at a counter, so the launch is cooperative with one CTA per SM: two launches of this
 // kernel cannot be resident together (each takes most of every SM's shared memory), which is also why the counter can be the
-// device's.  Every wait is bounded; after one that ran out the CTA goes through the remaining stages without waiting, sends all that
-// its pair may wait for, arms no more barriers, and leaves when what the other CTA sends has landed.
+// device's.  Every wait is bounded; after one that ran out the CTA goes through the remaining stages without meeting the others,
+// sends all that its pair may wait for, arms no more barriers where it was the pair that it waited for, and leaves when what the
+// other CTA sends has landed.
 #include <mutex>
 
 #include "tcgen05.cuh"

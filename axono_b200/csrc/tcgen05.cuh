@@ -60,7 +60,8 @@ __device__ __forceinline__ void umma_commit(uint64_t *bar) {
 // issues and commits behind this: the compiler knows the branch for what it is and keeps descriptors and counters in uniform
 // registers.  Behind `lane == 0` it may rebuild every operand per instruction; products that are predicated one by one were the
 // form before, and cost more too (alone, 64 in a row: 128 x 128 x 16 in 72 cycles each, 66 so; 128 x 64 x 16 in 63, 50 so).
-// 1536 tokens in fp32: 98 us, now 72; 8192 in fp16: 245 (behind `lane == 0`), 234 (predicated), 232.
+// 1536 tokens in fp32: 98 us, now 72; 8192 in fp16, the same kernel, ten calls after a pause: 245 (behind `lane == 0`), 234
+// (predicated), 232.
 __device__ __forceinline__ bool elect_one() {
   uint32_t is;
   asm volatile("{\n.reg .pred q;\nelect.sync _|q, 0xffffffff;\nselp.b32 %0, 1, 0, q;\n}\n" : "=r"(is));

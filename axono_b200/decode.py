@@ -196,7 +196,8 @@ class TextTower:
         enough rows, and weights as that takes them (`layers` is open to a program's own, whose views the single products copy)."""
         cfg = self.cfg
         return self.row_chain and self.world == 1 and self.fused_qkv and self.lt_gemm and type(self.cache) is PagedKVCache and \
-            self._chain_gains((cfg.n_q_heads + 2 * cfg.n_kv_heads) * cfg.head_dim) and all(t.is_contiguous() and t.data_ptr() % 16 == 0 for t in self._chain_weights())
+            self._chain_gains((cfg.n_q_heads + 2 * cfg.n_kv_heads) * cfg.head_dim) and \
+            all(t.is_contiguous() and t.data_ptr() % 16 == 0 for t in self._chain_weights())
 
     def _chain_gains(self, columns: int) -> bool:
         cfg = self.cfg

@@ -38,8 +38,8 @@ class KVCache:
         """`append_qkv` and `attend` as one operator (one launch where the library can; the two of a cache with a window, which the
         operator does not know): the attention output (batch, hq, d)."""
         if getattr(self, "window", 0):
-            return self.attend(layer_idx, self.append_qkv(layer_idx, qkv, n_q_heads, q_norm_weight, k_norm_weight, eps, pos, inv_freq, theta,
-                                                          mrope_section))
+            q = self.append_qkv(layer_idx, qkv, n_q_heads, q_norm_weight, k_norm_weight, eps, pos, inv_freq, theta, mrope_section)
+            return self.attend(layer_idx, q)
         first = layer_idx == 0
         if first:
             self._host_len_bound += 1

@@ -311,8 +311,8 @@ def test_experts(dtype, width, ff, experts, top, n):
     (128, 128, 128, 64, 128, 100, 1900, 0), (128, 128, 96, 64, 128, 7, 2100, 0), (128, 128, 128, 64, 128, 100, 3900, 2000)])  # few blocks, many keys
 def test_latent_prefill_in_the_form_of_two_blocks(heads, kv_heads, dim, rot, vdim, n, start, window):
     """The sizes that take the kernel with two blocks of rows per CTA: edges of its blocks and tiles, sizes that fill their 64-wide blocks
-    in part, windows, sinks.  Weights and results are rounded to bf16: half of its spacing, 2^-7 between 1 and 2, is at most 2^-8 of a value each
-    time; a score is off by its sum of products in fp32."""
+    in part, windows, sinks.  Weights and results are rounded to bf16: half of its spacing, 2^-7 between 1 and 2, is at most 2^-8 of a
+    value each time; a score is off by its sum of products in fp32."""
     from axono_b200 import ops
 
     g = torch.Generator(device="cuda").manual_seed(n)

@@ -149,8 +149,8 @@ def test_fp16_on_the_fma_kernel(hq, hkv, d, sq, skv):
 @pytest.mark.parametrize("d", [64, 80])
 @pytest.mark.parametrize("offset", [0, 4])
 def test_fp16_narrow_sums_do_not_drift(d, offset):
-    """Sums over thousands of values: the tensor core's truncation pulls them towards zero with each of the 16 products of a tile of
-    128 keys, by some 1e-5 over the 8 tiles after which a sum starts anew, which adds its square to that of the result's rounding
+    """Sums over thousands of values: the tensor core's truncation pulls them towards zero with each of the 8 products of a tile of 64
+    keys, by some 1e-5 over the 16 tiles after which a sum starts anew, which adds its square to that of the result's rounding
     (2.2e-4): a thousandth above the FMA kernel's error at most."""
     from axono_b200 import ops
 

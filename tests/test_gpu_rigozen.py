@@ -159,7 +159,8 @@ def test_cache_overflow_is_an_error(built):
 
 
 def test_a_step_cannot_be_captured(built):
-    """Its integers come from the host: refused, with nothing changed, so that the steps after it are those of a runner that was not asked."""
+    """Its integers come from the host: refused, with nothing changed, so that the steps after it are those of a runner that was not
+    asked."""
     cfg, w, tokens, _ = built("odd", 150)
     outs = []
     for ask in (False, True):

@@ -1,5 +1,6 @@
-"""What of row_chain.cu needs no GPU.  The exchange between the two CTAs of a pair as a model, every order of its steps: the warps of a CTA meet at
-barriers and nowhere else, and sums that were sent arrive at any later time.  The number of buffers is read from the source.  And what becomes of the exchange when a wait runs out, with barriers that count arrivals and bytes."""
+"""What of row_chain.cu needs no GPU.  The exchange between the two CTAs of a pair as a model, every order of its steps: the warps of
+a CTA meet at barriers and nowhere else, and sums that were sent arrive at any later time; the number of buffers is read from the
+source.  What becomes of the exchange when a wait runs out, with barriers that count arrivals and bytes.  And where the chain is taken."""
 import pathlib
 import random
 import re
