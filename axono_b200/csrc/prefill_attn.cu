@@ -262,20 +262,32 @@ prefill_attn_f16_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
       tma_load_3d(smem + kOffQ, &tmQ, bar_q, 0, h, q0);  // rows past sq are zero-filled
       if (two_blocks) tma_load_3d(smem + kOffQ + kQTileBytes / 2, &tmQ, bar_q, 64, h, q0);
       bool ok = true;
-      auto load = [&](int j, int stages, int off, const CUtensorMap &map, uint64_t *full, uint64_t *empty) {
-        const int s = j % stages;
+      int nk = 0, nv = 0;  // tiles asked for
+      auto load = [&](int &n, int stages, int off, const CUtensorMap &map, uint64_t *full, uint64_t *empty) {
+        const int j = n, s = j % stages;
         if (j >= stages) ok = ok && mbar_wait_bounded(&empty[s], (j / stages - 1) & 1, abort_flag);
         if (!ok) return;
         uint8_t *dst = smem + off + s * kKvTileBytes;
         mbar_arrive_expect_tx(&full[s], kv_bytes);
         tma_load_3d(dst, &map, &full[s], 0, hk, (tile0 + j) * kBlockN);
         if (two_blocks) tma_load_3d(dst + kKvTileBytes / 2, &map, &full[s], 64, hk, (tile0 + j) * kBlockN);
+        ++n;
       };
       // consumption order is S_0 S_1 (PV_0 S_2) (PV_1 S_3) ...: K_0 K_1 K_2 V_0 K_3 V_1 ...
-      for (int j = 0; j < 2 && j < nkv; ++j) load(j, kKStages, kOffK, tmK, full_k, empty_k);
-      for (int j = 0; j < nkv && ok; ++j) {
-        if (j + 2 < nkv) load(j + 2, kKStages, kOffK, tmK, full_k, empty_k);
-        load(j, kVStages, kOffV, tmV, full_v, empty_v);
+      while (nk < 2 && nk < nkv) load(nk, kKStages, kOffK, tmK, full_k, empty_k);
+      while (nv < nkv && ok) {
+        if (nk < nkv) load(nk, kKStages, kOffK, tmK, full_k, empty_k);
+        load(nv, kVStages, kOffV, tmV, full_v, empty_v);
+      }
+      if (*abort_flag) {  // no copy may still be on its way when the CTA leaves
+        const unsigned long long t0 = global_timer_ns();
+        auto drain = [&](uint64_t *bar, uint32_t parity) {
+          while (!mbar_try_wait(bar, parity) && global_timer_ns() - t0 < 100000000ull) {
+          }
+        };
+        drain(bar_q, 0);
+        for (int t = max(0, nk - kKStages); t < nk; ++t) drain(&full_k[t % kKStages], (t / kKStages) & 1);
+        for (int t = max(0, nv - kVStages); t < nv; ++t) drain(&full_v[t % kVStages], (t / kVStages) & 1);
       }
     }
   } else if (warp == kMmaWarp) {
